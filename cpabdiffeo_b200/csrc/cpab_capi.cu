@@ -4,15 +4,29 @@
 #include <new>
 
 #include "cpab_ctx.h"
+#include "cpab_jump.cuh"
 
 using namespace cpab;
 
 thread_local char cpab::g_thread_err[512];
 
-static size_t tables_smem(const cpab_ctx *c, int prec)
+// Tile scratch of a cell-sorted launch next to the tables.
+static size_t sort_smem(const cpab_ctx *c)
 {
-    // float64: A and T; float32: A and T - I
-    return (size_t)c->t.nC * cell_len(c) * (prec == CPAB_F64 ? 2 * 8 : 2 * 4);
+    return c->cfg.sort ? ((size_t)c->t.nC + 2 * (size_t)c->cfg.tile_pts) * sizeof(int) : 0;
+}
+
+JumpCfg cpab::ctx_jump(const cpab_ctx *c, int nTimeSteps, int nStepsODE, int scheme, size_t scratch)
+{
+    const size_t most = (size_t)max_smem_optin(), other = scratch + 1024;  // 1 KB for static shared memory
+    return jump_cfg(c->t.dim, c->t.nC, nTimeSteps, nStepsODE, scheme, most > other ? most - other : 0);
+}
+
+static size_t tables_smem(const cpab_ctx *c, int prec, int scheme, int nTimeSteps, int nStepsODE)
+{
+    // float64: A and T; float32: the composed-step tables
+    if (prec == CPAB_F64) return (size_t)c->t.nC * cell_len(c) * 2 * 8;
+    return jump_bytes(ctx_jump(c, nTimeSteps, nStepsODE, scheme, sort_smem(c)), c->t.dim, c->t.nC);
 }
 
 int cpab::max_smem_optin()
@@ -261,8 +275,7 @@ static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *T
         need = exact1d_smem_bytes(ctx->t.nC, ctx->cfg.tile_pts, ctx->cfg.sort,
                                   precision == CPAB_F64 ? PREC_F64 : PREC_F32);
     } else {
-        need = tables_smem(ctx, precision);
-        if (ctx->cfg.sort) need += ((size_t)ctx->t.nC + 2 * (size_t)ctx->cfg.tile_pts) * sizeof(int);
+        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx);
     }
     if (need > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch (%zu bytes) exceed shared memory", need);
@@ -270,7 +283,7 @@ static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *T
 }
 
 static IntegrateArgs make_args(cpab_ctx *ctx, const double *signedA, const double *Trels, const void *pts,
-                               void *out, double dt, int nTimeSteps, int nStepsODE, uint64_t *counters)
+                               void *out, int scheme, double dt, int nTimeSteps, int nStepsODE, uint64_t *counters)
 {
     IntegrateArgs a;
     memset(&a, 0, sizeof(a));
@@ -293,6 +306,7 @@ static IntegrateArgs make_args(cpab_ctx *ctx, const double *signedA, const doubl
     a.facets = ctx->facets_dev;
     a.nbr = ctx->nbr_dev;
     a.nF = ctx->nF;
+    a.jump = ctx_jump(ctx, nTimeSteps, nStepsODE, scheme, sort_smem(ctx));
     return a;
 }
 
@@ -317,7 +331,7 @@ int cpab_calc_T(cpab_ctx *ctx, const double *signedA, const double *Trels, const
     if (st != CPAB_OK) return st;
     CPAB_CHECK_ALIGN(ctx, {counters, 8, "counters"});
     if (nPts == 0) return CPAB_OK;
-    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, dt, nTimeSteps, nStepsODE, counters);
+    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, scheme, dt, nTimeSteps, nStepsODE, counters);
     a.batch.N = 1;
     a.batch.n_uniform = nPts;
     a.batch.offsets = nullptr;
@@ -351,7 +365,7 @@ int cpab_calc_T_batched(cpab_ctx *ctx, const double *signedA, const double *Trel
     if (offsets && pts == out) return fail(ctx, CPAB_ALIAS, "pts and out are the same buffer");
     CPAB_CHECK_ALIGN(ctx, {offsets, 8, "offsets"}, {workspace, 8, "workspace"}, {counters, 8, "counters"});
     cudaStream_t s = (cudaStream_t)stream;
-    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, dt, nTimeSteps, nStepsODE, counters);
+    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, scheme, dt, nTimeSteps, nStepsODE, counters);
     a.batch.N = N;
     a.batch.tile_pts = ctx->cfg.tile_pts;
     int64_t uniform_tiles = 0;
@@ -386,7 +400,7 @@ int cpab_calc_trajectory(cpab_ctx *ctx, const double *signedA, const double *Tre
     CPAB_CHECK_ALIGN(ctx, {pts, 8, "pts"}, {traj, 8, "traj"});
     size_t in_bytes = (size_t)nPts * ctx->t.dim * 8, out_bytes = in_bytes * (size_t)(nTimeSteps + 1);
     if (overlaps(pts, in_bytes, traj, out_bytes)) return fail(ctx, CPAB_ALIAS, "pts and traj overlap");
-    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, traj, dt, nTimeSteps, nStepsODE, nullptr);
+    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, traj, CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE, nullptr);
     return cuda_status(ctx, launch_trajectory(a, nPts, (cudaStream_t)stream), "trajectory launch");
 }
 

@@ -41,6 +41,14 @@ int likelihood_tile(int64_t total, int tile_pts)
     return (t + kSumChunk - 1) / kSumChunk * kSumChunk;
 }
 
+// The FP32 table levels of a likelihood launch: chosen beside the largest tile
+// the context may use, so that a result does not depend on the launch's size.
+JumpCfg likelihood_jump(const cpab_ctx *ctx, int nTimeSteps, int nStepsODE, size_t (*scratch)(int))
+{
+    const int tile = (ctx->cfg.tile_pts + kSumChunk - 1) / kSumChunk * kSumChunk;
+    return ctx_jump(ctx, nTimeSteps, nStepsODE, SCHEME_REF, scratch(tile));
+}
+
 int check_images(cpab_ctx *ctx, int N, int H, int W)
 {
     if (N < 0) return fail(ctx, CPAB_BAD_SHAPE, "N < 0");
@@ -133,8 +141,9 @@ int cpab_register_ll(cpab_ctx *ctx, const double *signedA, const double *Trels, 
     if (nTimeSteps < 1 || nStepsODE < 1) return fail(ctx, CPAB_BAD_ARG, "nTimeSteps and nStepsODE must be >= 1");
     if (!std::isfinite(dt)) return fail(ctx, CPAB_BAD_ARG, "dt is not finite");
     const int tile_px = likelihood_tile((int64_t)N * H * W, ctx->cfg.tile_pts);
+    const JumpCfg jump = likelihood_jump(ctx, nTimeSteps, nStepsODE, register_scratch_bytes);
     // cell tables plus one point slot per pixel of a tile
-    if (register_smem_bytes(ctx->t.nC, tile_px, precision == CPAB_F64 ? PREC_F64 : PREC_F32) >
+    if (register_smem_bytes(ctx->t.nC, tile_px, precision == CPAB_F64 ? PREC_F64 : PREC_F32, jump) >
         (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch exceed shared memory");
     const WsLayout L = ws_layout(N, tiles_of(H, W, kSumChunk));
@@ -143,6 +152,7 @@ int cpab_register_ll(cpab_ctx *ctx, const double *signedA, const double *Trels, 
     RegisterArgs a;
     memset(&a, 0, sizeof(a));
     a.t = ctx->t;
+    a.jump = jump;
     a.A = signedA;
     a.T = Trels;
     a.src = src;
@@ -269,7 +279,8 @@ int cpab_register3d_ll(cpab_ctx *ctx, const double *signedA, const double *Trels
                      {ll, 8, "ll"}, {warped, 4, "warped"}, {workspace, 8, "workspace"}, {counters, 8, "counters"});
     const int prec = precision == CPAB_F64 ? PREC_F64 : PREC_F32;
     const int tile_px = likelihood_tile((int64_t)N * H * W * D, ctx->cfg.tile_pts);
-    if (register3d_smem_bytes(ctx->t.nC, tile_px, prec) > (size_t)max_smem_optin())
+    const JumpCfg jump = likelihood_jump(ctx, nTimeSteps, nStepsODE, register3d_scratch_bytes);
+    if (register3d_smem_bytes(ctx->t.nC, tile_px, prec, jump) > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch exceed shared memory");
     const WsLayout L = ws_layout(N, tiles_of3(H, W, D, kSumChunk));
     if (!workspace || workspace_bytes < L.total)
@@ -277,6 +288,7 @@ int cpab_register3d_ll(cpab_ctx *ctx, const double *signedA, const double *Trels
     Register3dArgs a;
     memset(&a, 0, sizeof(a));
     a.t = ctx->t;
+    a.jump = jump;
     a.A = signedA;
     a.T = Trels;
     a.src = src;
@@ -331,7 +343,9 @@ int cpab_landmark_ll(cpab_ctx *ctx, const double *signedA, const double *Trels, 
                      {ll, 8, "ll"}, {transformed, 8, "transformed"}, {workspace, 8, "workspace"},
                      {counters, 8, "counters"});
     const int prec = precision == CPAB_F64 ? PREC_F64 : PREC_F32;
-    if (landmark_smem_bytes(ctx->t, ctx->cfg.tile_pts, prec) > (size_t)max_smem_optin())
+    const JumpCfg jump =
+        ctx_jump(ctx, nTimeSteps, nStepsODE, SCHEME_REF, (size_t)ctx->cfg.tile_pts * sizeof(double));
+    if (landmark_smem_bytes(ctx->t, ctx->cfg.tile_pts, prec, jump) > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch exceed shared memory");
     const size_t need = cpab_landmark_workspace_bytes(ctx, N, n_lm);
     if (!workspace || workspace_bytes < need) return fail(ctx, CPAB_NO_MEMORY, "workspace of %zu bytes needed", need);
@@ -345,6 +359,7 @@ int cpab_landmark_ll(cpab_ctx *ctx, const double *signedA, const double *Trels, 
     LandmarkArgs a;
     memset(&a, 0, sizeof(a));
     a.t = ctx->t;
+    a.jump = jump;
     a.A = signedA;
     a.T = Trels;
     a.src = src;

@@ -67,6 +67,8 @@ struct Tess {
     double hi[3];      // clamp for type I: (double)nCk*inc_k - 1e-10 (axis 2 uses inc_x)
     int pow2[3];       // inc_k is a power of two: xmod/inc == xmod*(1/inc) exactly
     float finc[3], finv_inc[3], fspan[3], fhi[3];
+    float finc_lo[3], finv_inc_lo[3];  // inc - finc, 1/inc - finv_inc
+    float finv_n[3];                   // 1 / nCk
 };
 
 // Geometry of a tessellation from box counts and box sizes, derived
@@ -104,10 +106,16 @@ inline bool make_tess(int dim, int tess, const int *nCs, const double *incs, Tes
     for (int k = 0; k < 3; ++k) {
         t.finc[k] = (float)t.inc[k];
         t.finv_inc[k] = (float)(1.0 / t.inc[k]);
+        t.finc_lo[k] = (float)(t.inc[k] - (double)t.finc[k]);
+        t.finv_inc_lo[k] = (float)(1.0 / t.inc[k] - (double)t.finv_inc[k]);
+        t.finv_n[k] = 1.0f / (float)n[k];
         t.fspan[k] = (float)t.span[k];
         double top = (dim == 3 && tess == 1 && k == 2) ? (double)n[2] * t.inc[0] : t.span[k];
-        // float clamp strictly below the span so floor() stays in the last box
+        // float clamp strictly below the span so floor() stays in the last box,
+        // also where the product with 1/inc rounds up
         t.fhi[k] = nextafterf((float)top, 0.0f);
+        if (top == t.span[k])
+            while (t.fhi[k] > 0.0f && t.fhi[k] * t.finv_inc[k] >= (float)n[k]) t.fhi[k] = nextafterf(t.fhi[k], 0.0f);
     }
     return true;
 }
@@ -354,16 +362,61 @@ CPAB_HD int fast_cell(const Tess &t, const float *p)
     return fast_cell_3d_tet(t, p);
 }
 
-template <int DIM>
-CPAB_HD void fast_affine(float *x, const float *A, const float *b)
+// fast_cell_3d_tet with m: a lower bound of the distances from the point to the
+// facets its cell shares with another cell, in box units (coordinates divided
+// by the box sizes; a cut plane's distance is its functional -x - y + z, ...
+// with coefficients +-1).  Facets on the domain boundary do not count: the
+// cell continues outside.  Points outside take the margins of the nearest
+// point inside.  m exceeds a distance only by float rounding; for NaN
+// coordinates it means nothing.
+CPAB_HD int fast_cell_3d_tet_m(const Tess &t, const float *p, float &m)
 {
+    const int n[3] = {t.nC0, t.nC1, t.nC2};
+    int kb[3];
+    float f[3], face = 2.0f;
+#ifdef __CUDA_ARCH__
 #pragma unroll
-    for (int r = 0; r < DIM; ++r) {
-        float acc = A[r * (DIM + 1) + DIM];
-#pragma unroll
-        for (int c = 0; c < DIM; ++c) acc = fmaf(A[r * (DIM + 1) + c], b[c], acc);
-        x[r] = acc;
+#endif
+    for (int i = 0; i < 3; ++i) {
+        const float u = fminf(t.fhi[i], fmaxf(0.0f, p[i])) * t.finv_inc[i], fl = floorf(u);
+        kb[i] = (int)fminf(fl, (float)(n[i] - 1));
+        f[i] = u - fl;
+        // the nearest of the box's faces inside the domain, a lower bound of a corner tetrahedron's three
+        if (kb[i] > 0) face = fminf(face, f[i]);
+        if (kb[i] < n[i] - 1) face = fminf(face, 1.0f - f[i]);
     }
+    float x = f[0], y = f[1];
+    const float z = f[2];
+    if ((kb[0] ^ kb[1] ^ kb[2]) & 1) {
+        const float tmp = x;
+        x = y;
+        y = 1.0f - tmp;
+    }
+    // the four cut planes, in fast_cell_3d_tet's order and arithmetic
+    const float e1 = -x - y + z, e2 = x + y + z - 2.0f, e3 = -x + y - z, e4 = x - y - z;
+    const int tet = e1 >= 0 ? 1 : e2 >= 0 ? 2 : e3 >= 0 ? 3 : e4 >= 0 ? 4 : 0;
+    m = fminf(fminf(fabsf(e1), fabsf(e2)), fminf(fabsf(e3), fabsf(e4)));
+    if (tet) m = fminf(m, face);
+    return (kb[0] + kb[1] * t.nC0 + kb[2] * t.nC1 * t.nC0) * 5 + tet;
+}
+
+// The box indices of cell c.  Quotients of integers below 2^20 by a float
+// product: the quotient's error stays below 2^-23 2^20 / n = 1/(8 n), its
+// distance from the next integer is at least 1/(2 n).
+template <int DIM, int TESS>
+CPAB_HD void cell_box(const Tess &t, int c, int *kb)
+{
+    const int n[3] = {t.nC0, t.nC1, t.nC2};
+    int b = TESS == 1 ? (DIM == 2 ? c >> 2 : c / 5) : c;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int i = 0; i + 1 < DIM; ++i) {
+        const int q = (int)(((float)b + 0.5f) * t.finv_n[i]);
+        kb[i] = b - q * n[i];
+        b = q;
+    }
+    kb[DIM - 1] = b;
 }
 
 }  // namespace cpab

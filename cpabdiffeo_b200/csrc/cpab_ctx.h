@@ -92,6 +92,8 @@ inline const volatile int *cancel_ptr(const cpab_ctx *c)
 }
 
 int max_smem_optin();
+// The FP32 integration's table levels, `scratch` bytes of shared memory being needed beside them.
+JumpCfg ctx_jump(const cpab_ctx *c, int nTimeSteps, int nStepsODE, int scheme, size_t scratch);
 int build_facets(const Tess &t, const int *nCs, std::vector<double> &F, std::vector<int> &nbr);
 
 }  // namespace cpab

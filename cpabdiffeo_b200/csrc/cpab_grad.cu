@@ -391,7 +391,28 @@ __device__ __forceinline__ void acc_switch_f(double *sG, float *acc, int &acc_ce
     acc_cell = c;
 }
 
-// x' = x + M[x; 1] on the compensated state (the float advance() of the lane scheduler)
+// The float tables of one instance in shared memory, column-major: S - I and
+// T - I, h the sub-step length.
+template <int DIM>
+__device__ __forceinline__ void stage_tables_f32(const double *gA, const double *gT, int nC, double h, float *sS,
+                                                 float *sT)
+{
+    constexpr int NE = DIM * (DIM + 1);
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nC * NE; i += blockDim.x) {
+        const int c = i / NE, e = i - c * NE, r = e / (DIM + 1), col = e - r * (DIM + 1);
+        const int cm = col * DIM + r;
+        // (S - I)[r][col] = h (A[r][col] + h/2 sum_k L[r][k] A[k][col])
+        const double *a = gA + (size_t)c * NE;
+        double l2 = 0.0;
+#pragma unroll 1
+        for (int k = 0; k < DIM; ++k) l2 += a[r * (DIM + 1) + k] * a[k * (DIM + 1) + col];
+        sS[c * NE + cm] = (float)(h * (a[r * (DIM + 1) + col] + 0.5 * h * l2));
+        sT[c * NE + cm] = (float)(gT[i] - (r == col ? 1.0 : 0.0));
+    }
+}
+
+// x' = x + M[x; 1] on the compensated state
 template <int DIM>
 __device__ __forceinline__ void f32_map(PState<DIM, float> &st, const float *M)
 {
@@ -484,7 +505,7 @@ __global__ void __launch_bounds__(128) k_grad_ref_f32(GradArgs a)
     double *sGT = SACC ? sums + tab : a.gT + (size_t)inst * tab;  // dLoss/dT (closed-form steps)
     float *sS = reinterpret_cast<float *>(sums + (SACC ? 2 * tab : 0));
     float *sT = sS + tab;
-    stage_tables<DIM, float>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, true, a.h_sub, sS, sT);
+    stage_tables_f32<DIM>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, a.h_sub, sS, sT);
     if (SACC)
         for (int i = threadIdx.x; i < 2 * tab; i += blockDim.x) sums[i] = 0.0;
     __syncthreads();

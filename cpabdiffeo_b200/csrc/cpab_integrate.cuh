@@ -16,24 +16,21 @@ namespace cpab {
 //    arithmetic (cpab_cell.cuh).
 //  * float (FP32 mode): an unnormalised compensated pair hi + lo per
 //    coordinate plus x = fl(hi + lo), the float nearest the point, which the
-//    velocity, the closed-form step and the cell lookup read.  Each update
-//    adds its increment d to hi and the rounding error of that addition
-//    (Fast2Sum; |d| is a small step, and where |hi| < |d| the error term is
-//    below ulp(d)) to lo, so the many small increments of the integration are
-//    not lost to float rounding.  Both step kinds are increments from a
-//    small matrix: the closed-form step adds (T - I)[x; 1]; an explicit
-//    midpoint sub-step of length h with the cell's velocity v(x) = A[x; 1]
-//    (both evaluations in the cell of x, calc_2Dto2D.cu:177-196) is, inside
-//    one cell, the affine map x + h v(x + h/2 v(x)) = x + (S - I)[x; 1] with
-//        S - I = [h L + h^2/2 L^2 | h b + h^2/2 L b]      (A = [L | b]),
+//    cell lookup reads.  Each update adds its increment d to hi and the
+//    rounding error of that addition (Fast2Sum; where |hi| < |d| the error
+//    term is below ulp(d)) to lo, so the increments of the integration are
+//    not lost to float rounding.  Every step is an increment from a small
+//    matrix (cpab_jump.cuh): the closed-form step adds (T - I)[x; 1]; an
+//    explicit midpoint sub-step of length h with the cell's velocity
+//    v(x) = A[x; 1] (both evaluations in the cell of x, calc_2Dto2D.cu:177-196)
+//    is, inside one cell, the affine map x + h v(x + h/2 v(x)) = x + (S - I)[x; 1]
+//    with S - I = [h L + h^2/2 L^2 | h b + h^2/2 L b]      (A = [L | b]),
 //    evaluated in double when the tables are staged.  Table roundings are
-//    relative to the small increments, not to the position, so they do not
-//    bias every step.
-// Shared-memory tables per cell (ne = DIM * (DIM + 1)):
-//  double: A[ne], T[ne], row-major as in global memory;
-//  float:  (S - I)[ne] and (T - I)[ne], column-major (the DIM columns of the
-//          linear part, then the offset) so that a cell's matrix is read with
-//          8-byte (1D/2D) or 16-byte (3D) loads.
+//    relative to the increments, not to the position.
+// Shared-memory tables per cell (ne = DIM * (DIM + 1)) of the double states:
+// A[ne] (EXACT: S[ne]) and T[ne], row-major as in global memory.  Float
+// matrices are column-major (the DIM columns of the linear part, then the
+// offset) so that one is read with 8-byte (1D/2D) or 16-byte (3D) loads.
 
 template <int DIM, typename Real>
 struct PState;
@@ -92,48 +89,26 @@ struct PState<DIM, float> {
     }
 };
 
-template <typename Real>
-struct TableLayout {
-    // tables of the closed-form step per cell (double: T; float: T - I)
-    static constexpr int kTParts = 1;
-};
+template <int DIM>
+__device__ void stage_exact_substeps(const double *gA, const double *gT, int nC, double h, double *sS, double *sT);
 
-// Stage one instance's tables in shared memory (layout above); h is the
-// sub-step length dt / nStepsODE (float tables only), passed from the
-// kernel's parameters so that no register holds it during integration.
-// EXACT scheme (2D/3D): the sub-step map is the exact flow S = expm(h A)
-// instead of the midpoint map, staged by stage_exact_substeps below.
-template <int DIM, typename Real>
-__device__ void stage_exact_substeps(const double *gA, const double *gT, int nC, double h, Real *sS, Real *sT);
-
-template <int DIM, typename Real>
+// Stage one instance's double tables in shared memory (layout above).  EXACT
+// scheme (2D/3D): the sub-step map is the exact flow S = expm(h A), h the
+// sub-step length, instead of the signed A.
+template <int DIM>
 __device__ __forceinline__ void stage_tables(const double *gA, const double *gT, int nC, bool with_T, double h,
-                                             Real *sA, Real *sT, bool exact_sub = false)
+                                             double *sA, double *sT, bool exact_sub = false)
 {
-    constexpr int NE = DIM * (DIM + 1);
-    const int tab = nC * NE;
     if (exact_sub) {
-        stage_exact_substeps<DIM, Real>(gA, gT, nC, h, sA, sT);
+        stage_exact_substeps<DIM>(gA, gT, nC, h, sA, sT);
         return;
     }
     // not unrolled: the staging loop's loads in flight would otherwise set
     // the register count of the integration loop that follows
 #pragma unroll 1
-    for (int i = threadIdx.x; i < tab; i += blockDim.x) {
-        if (sizeof(Real) == 8) {
-            sA[i] = (Real)gA[i];
-            if (with_T) sT[i] = (Real)gT[i];
-        } else {
-            const int c = i / NE, e = i - c * NE, r = e / (DIM + 1), col = e - r * (DIM + 1);
-            const int cm = col * DIM + r;
-            // (S - I)[r][col] = h (A[r][col] + h/2 sum_k L[r][k] A[k][col])
-            const double *a = gA + (size_t)c * NE;
-            double l2 = 0.0;
-#pragma unroll 1
-            for (int k = 0; k < DIM; ++k) l2 += a[r * (DIM + 1) + k] * a[k * (DIM + 1) + col];
-            sA[c * NE + cm] = (float)(h * (a[r * (DIM + 1) + col] + 0.5 * h * l2));
-            if (with_T) sT[c * NE + cm] = (float)(gT[i] - (r == col ? 1.0 : 0.0));
-        }
+    for (int i = threadIdx.x; i < nC * DIM * (DIM + 1); i += blockDim.x) {
+        sA[i] = gA[i];
+        if (with_T) sT[i] = gT[i];
     }
 }
 
@@ -188,17 +163,13 @@ __device__ __forceinline__ int cell_of(const Tess &t, const PState<DIM, float> &
 
 // One unit of work on a point in cell c: the candidate end point q of a
 // closed-form step (fast: q = T_c [p; 1]) or of one explicit-midpoint
-// sub-step with A_c.  The caller looks up the cell of q; a closed-form step
-// is kept when that is still c (calc_2Dto2D.cu:380-400), a sub-step always
-// is, and its end cell is the cell of the next sub-step's start point.
-//   double: the reference's arithmetic (exact_affine / exact_midpoint).
-//   float:  one matrix-vector product with the cell's (T - I) or (S - I)
-//           and the compensated update -- the same instructions for both
-//           kinds, so lanes that mix closed-form steps and sub-steps do not
-//           diverge.
+// sub-step with A_c, in the reference's arithmetic.  The caller looks up the
+// cell of q; a closed-form step is kept when that is still c
+// (calc_2Dto2D.cu:380-400), a sub-step always is, and its end cell is the cell
+// of the next sub-step's start point.
 template <int DIM>
 __device__ __forceinline__ void advance(bool fast, const PState<DIM, double> &s, const double *A, const double *T,
-                                        const double *, double h, PState<DIM, double> &q)
+                                        double h, PState<DIM, double> &q)
 {
     if (fast) {
         exact_affine<DIM>(q.p, T, s.p);
@@ -225,43 +196,14 @@ __device__ __forceinline__ void add_pair(PState<DIM, float> &q, float2 d)
     q.x[0] = x.x; q.x[1] = x.y;
 }
 
-template <int DIM>
-__device__ __forceinline__ void advance(bool fast, const PState<DIM, float> &s, const float *A, const float *T,
-                                        const float *, float, PState<DIM, float> &q)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    float m[NE], d[DIM];
-    // d = (T - I)[x; 1] for a closed-form step, (S - I)[x; 1] for a sub-step
-    load_cell<DIM>(fast ? T : A, m);
-    q = s;
-    if constexpr (DIM == 1) {
-        cm_affine<DIM>(d, m, s.x);
-        q.add(0, d[0]);
-    } else {
-        // rows 0 and 1 as one pair: the same fmaf sequence as cm_affine per row
-        float2 d01 = make_float2(m[DIM * DIM], m[DIM * DIM + 1]);
-#pragma unroll
-        for (int k = 0; k < DIM; ++k)
-            d01 = __ffma2_rn(make_float2(m[k * DIM], m[k * DIM + 1]), make_float2(s.x[k], s.x[k]), d01);
-        add_pair<DIM>(q, d01);
-        if constexpr (DIM == 3) {
-            float d2 = m[DIM * DIM + 2];
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) d2 = fmaf(m[k * DIM + 2], s.x[k], d2);
-            q.add(2, d2);
-        }
-    }
-}
-
 // ------------------------------------------------------------ exact scheme (2D/3D)
 //
 // Sub-step map of the exact flow: column j of S - I is
 // sum_{k>=1} h^k/k! L^{k-1} A[:, j]  (A = [L | b], homogeneous bottom row 0),
 // summed per column until the terms fall below the sum's rounding.
-// double tables: S row-major (the layout exact_affine-style code reads);
-// float tables: S - I column-major (the layout of the float sub-step table).
-template <int DIM, typename Real>
-__device__ void stage_exact_substeps(const double *gA, const double *gT, int nC, double h, Real *sS, Real *sT)
+// Tables: S row-major (the layout exact_affine-style code reads).
+template <int DIM>
+__device__ void stage_exact_substeps(const double *gA, const double *gT, int nC, double h, double *sS, double *sT)
 {
     constexpr int NE = DIM * (DIM + 1);
 #pragma unroll 1
@@ -300,24 +242,11 @@ __device__ void stage_exact_substeps(const double *gA, const double *gT, int nC,
                 if (!(big > 1e-18 * am)) break;
             }
 #pragma unroll
-            for (int r = 0; r < DIM; ++r) {
-                if (sizeof(Real) == 8)
-                    sS[c * NE + r * (DIM + 1) + col] = (Real)(acc[r] + (r == col ? 1.0 : 0.0));
-                else
-                    sS[c * NE + col * DIM + r] = (Real)acc[r];
-            }
+            for (int r = 0; r < DIM; ++r) sS[c * NE + r * (DIM + 1) + col] = acc[r] + (r == col ? 1.0 : 0.0);
         }
     }
-    const int tab = nC * NE;
 #pragma unroll 1
-    for (int i = threadIdx.x; i < tab; i += blockDim.x) {
-        if (sizeof(Real) == 8) {
-            sT[i] = (Real)gT[i];
-        } else {
-            const int c = i / NE, e = i - c * NE, r = e / (DIM + 1), col = e - r * (DIM + 1);
-            sT[c * NE + col * DIM + r] = (Real)(gT[i] - (r == col ? 1.0 : 0.0));
-        }
-    }
+    for (int i = threadIdx.x; i < nC * NE; i += blockDim.x) sT[i] = gT[i];
 }
 
 // What a lane needs to resolve an exit: the instance's signed A (global,
@@ -534,28 +463,35 @@ __device__ __forceinline__ double facet_hit_time(const double *__restrict__ A, c
     return 0.5 * (lo + hi);
 }
 
-// A sub-step of length h from st in cell c ended at q outside c: the exact
-// flow from st, exit times through interior facets, the neighbour across the
+// A sub-step of length h from p in cell c ended at q outside c: the exact
+// flow from p, exit times through interior facets, the neighbour across the
 // exited facet, the rest of the sub-step there (and so on).  q becomes the
 // point at the sub-step's end; returns its cell.  FP64 throughout (the
-// hitting times); q keeps the state's precision.  When no interior facet
+// hitting times; Real is the precision whose cell lookup decides).  When no interior facet
 // explains the exit (a point on the domain boundary) or the crossings exceed
 // the cap, q is the end point of the flow in the current cell (as in the
 // reference scheme, which keeps its sub-step's end wherever it lands).
 template <int DIM, int TESS, typename Real>
 __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex, int c,
-                                                   const PState<DIM, Real> &st, PState<DIM, Real> &q)
+                                                   const double *from, double *q)
 {
     constexpr int NH = DIM + 1, NE = DIM * NH;
     double p[DIM], y[DIM];
-    st.get(p);
-    q.get(y);
+#pragma unroll
+    for (int r = 0; r < DIM; ++r) {
+        p[r] = from[r];
+        y[r] = q[r];
+    }
+    auto end_at = [&](const double *x) {
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) q[r] = x[r];
+    };
     double s = ex.h;
 #pragma unroll 1
     for (int crossings = 0;;) {
         // (the caller found q outside c; later ends are looked up here)
         if (crossings > 0 && lookup_d<DIM, TESS>(t, y, Real(0)) == c) {
-            q.set(y);
+            end_at(y);
             return c;
         }
         const double *A = ex.A + (size_t)c * NE;
@@ -582,7 +518,7 @@ __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex
         }
         if (kbest < 0 || !(tau == tau) || ++crossings > ex.cap) {
             ++ex.unresolved;
-            q.set(y);
+            end_at(y);
             return lookup_d<DIM, TESS>(t, y, Real(0));
         }
         flow_taylor<DIM>(A, p, tau, p);
@@ -590,20 +526,19 @@ __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex
         c = __ldg(ex.nbr + c * ex.nF + kbest);
         ++ex.crossings;
         if (!(s > 0)) {
-            q.set(p);
+            end_at(p);
             return c;
         }
         if (!flow_taylor<DIM>(ex.A + (size_t)c * NE, p, s, y)) {
             // the neighbour's flow is too fast for the polynomial over the
             // rest of the sub-step: the reference scheme's sub-step end
             ++ex.unresolved;
-            return cell_of<DIM, TESS>(t, q);
+            return lookup_d<DIM, TESS>(t, q, Real(0));
         }
     }
 }
 
-// EXACT unit: the closed-form step with T (the reference's arithmetic in
-// double) or one sub-step of the exact flow with S.
+// EXACT unit: the closed-form step with T (the reference's arithmetic) or one sub-step of the exact flow with S.
 template <int DIM>
 __device__ __forceinline__ void advance_exact(bool fast, const PState<DIM, double> &s, const double *S,
                                               const double *T, PState<DIM, double> &q)
@@ -620,12 +555,6 @@ __device__ __forceinline__ void advance_exact(bool fast, const PState<DIM, doubl
         }
     }
 }
-template <int DIM>
-__device__ __forceinline__ void advance_exact(bool fast, const PState<DIM, float> &s, const float *S, const float *T,
-                                              PState<DIM, float> &q)
-{
-    advance<DIM>(fast, s, S, T, nullptr, 0.0f, q);
-}
 
 // ------------------------------------------------------------ integration
 
@@ -637,8 +566,8 @@ __device__ __forceinline__ void advance_exact(bool fast, const PState<DIM, float
 // nStepsODE sub-steps therefore keeps one lane busy, not the whole warp.
 // Results do not depend on the schedule: each point follows exactly the
 // reference's sequence of operations.
-//   Src::load(idx, st)     sets the start state of point idx
-//   Snk::put(idx, st)      receives the end state (PState; get() converts)
+//   Src::load(idx, p)      gives the start position of point idx
+//   Snk::put(idx, p)       receives its end position
 //   perm (optional, shared memory): the k-th point of the range is
 //   ws_base + perm[k - ws_base] (a cell-sorted order inside the tile).
 //   start_cells (optional, with perm): cell of point perm_base + i at [i],
@@ -652,9 +581,9 @@ __device__ __forceinline__ void advance_exact(bool fast, const PState<DIM, float
 // the cell the next sub-step (or the next time step) starts in, which the
 // reference would look up from the same point.  So each lane always knows
 // the cell of its current point.
-template <int DIM, int TESS, typename Real, int SCHEME, class Src, class Snk>
-__device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE, const Real *sA, const Real *sT,
-                                                int64_t ws, int64_t we, Real h, const Src &src, Snk &snk,
+template <int DIM, int TESS, int SCHEME, class Src, class Snk>
+__device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE, const double *sA, const double *sT,
+                                                int64_t ws, int64_t we, double h, const Src &src, Snk &snk,
                                                 unsigned long long &c_fast, unsigned long long &c_fb,
                                                 unsigned long long &c_sub, unsigned long long &c_pts,
                                                 const int *perm = nullptr, int64_t perm_base = 0,
@@ -675,18 +604,14 @@ __device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE,
     }
     bool active = k < we;
     int64_t idx = (active && perm) ? perm_base + perm[k - perm_base] : k;
-    PState<DIM, Real> st;
+    PState<DIM, double> st;
     int steps_left = 0, sub_left = 0, c = 0;
     if (active) {
-        src.load(idx, st);
+        src.load(idx, st.p);
         c = start_cells ? start_cells[idx - perm_base] : cell_of<DIM, TESS>(t, st);
         steps_left = nT;
         sub_left = (SCHEME == SCHEME_SIMPLE) ? nT * nODE : 0;
     }
-    // FP32: two units per lane between the warp's votes (a lane whose point
-    // finishes after the first idles for the second; points finish about once
-    // in a hundred units)
-    constexpr int kUnits = sizeof(Real) == 4 ? 2 : 1;
     // EXACT: a sub-step that ends outside its cell parks the lane (pend)
     // instead of resolving the exit at once: resolving takes about as long as
     // a hundred units, and done alone it leaves the other 31 lanes idle.  The
@@ -700,41 +625,36 @@ __device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE,
     int pend_votes = 0;
     while (__any_sync(FULL, active)) {
         bool fin = false;
-#pragma unroll
-        for (int u = 0; u < kUnits; ++u) {
-            if (active && !fin && !pend) {
-                const bool fast = (SCHEME == SCHEME_REF || SCHEME == SCHEME_EXACT) && sub_left == 0;
-                PState<DIM, Real> q;
-                if (SCHEME == SCHEME_EXACT)
-                    advance_exact<DIM>(fast, st, sA + c * NE, sT + c * NE, q);
-                else
-                    advance<DIM>(fast, st, sA + c * NE, sT + c * NE, nullptr, h, q);
-                int cq = cell_of<DIM, TESS>(t, q);
-                if (SCHEME == SCHEME_EXACT && !fast && cq != c) {
-                    pend = true;
-                    continue;
-                }
-                if (fast && cq != c) {
-                    // the end point left the cell: redo the step with nStepsODE sub-steps from p
-                    sub_left = nODE;
-                    ++c_fb;
+        if (active && !fin && !pend) {
+            const bool fast = (SCHEME == SCHEME_REF || SCHEME == SCHEME_EXACT) && sub_left == 0;
+            PState<DIM, double> q;
+            if (SCHEME == SCHEME_EXACT)
+                advance_exact<DIM>(fast, st, sA + c * NE, sT + c * NE, q);
+            else
+                advance<DIM>(fast, st, sA + c * NE, sT + c * NE, h, q);
+            int cq = cell_of<DIM, TESS>(t, q);
+            if (SCHEME == SCHEME_EXACT && !fast && cq != c) {
+                pend = true;
+            } else if (fast && cq != c) {
+                // the end point left the cell: redo the step with nStepsODE sub-steps from p
+                sub_left = nODE;
+                ++c_fb;
+            } else {
+                st = q;
+                c = cq;
+                if (fast) {
+                    --steps_left;
+                    ++c_fast;
                 } else {
-                    st = q;
-                    c = cq;
-                    if (fast) {
-                        --steps_left;
-                        ++c_fast;
-                    } else {
-                        --sub_left;
-                        ++c_sub;
-                        if (SCHEME != SCHEME_SIMPLE && sub_left == 0) --steps_left;
-                    }
+                    --sub_left;
+                    ++c_sub;
+                    if (SCHEME != SCHEME_SIMPLE && sub_left == 0) --steps_left;
                 }
-                fin = (SCHEME == SCHEME_SIMPLE) ? (sub_left == 0) : (steps_left == 0);
-                if (fin) {
-                    snk.put(idx, st);
-                    ++c_pts;
-                }
+            }
+            fin = (SCHEME == SCHEME_SIMPLE) ? (sub_left == 0) : (steps_left == 0);
+            if (fin) {
+                snk.put(idx, st.p);
+                ++c_pts;
             }
         }
         if (SCHEME == SCHEME_EXACT) {
@@ -745,9 +665,9 @@ __device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE,
                     pend_votes = 0;
                     if (pend) {
                         // the parked sub-step's end, recomputed with the same arithmetic
-                        PState<DIM, Real> qp;
+                        PState<DIM, double> qp;
                         advance_exact<DIM>(false, st, sA + c * NE, sT + c * NE, qp);
-                        c = exact_substep_cross<DIM, TESS, Real>(t, *ex, c, st, qp);
+                        c = exact_substep_cross<DIM, TESS, double>(t, *ex, c, st.p, qp.p);
                         st = qp;
                         pend = false;
                         --sub_left;
@@ -755,7 +675,7 @@ __device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE,
                         if (sub_left == 0) --steps_left;
                         fin = steps_left == 0;
                         if (fin) {
-                            snk.put(idx, st);
+                            snk.put(idx, st.p);
                             ++c_pts;
                         }
                     }
@@ -777,7 +697,7 @@ __device__ __forceinline__ void integrate_range(const Tess &t, int nT, int nODE,
                 active = k < we;
                 if (active) {
                     idx = perm ? perm_base + perm[k - perm_base] : k;
-                    src.load(idx, st);
+                    src.load(idx, st.p);
                     c = start_cells ? start_cells[idx - perm_base] : cell_of<DIM, TESS>(t, st);
                     steps_left = nT;
                     sub_left = (SCHEME == SCHEME_SIMPLE) ? nT * nODE : 0;

@@ -35,8 +35,17 @@ struct Batch {
     int tile_pts;                // points per CTA tile
 };
 
+// Composed-step tables of the FP32 integration (cpab_jump.cuh): nT levels of
+// the closed-form step and nS of the sub-step, level l being the step's map
+// composed 2^(l r) times; mul = ceil(32 / r), so that (k mul) >> 5 = k / r
+// for k = log2 of a step count.
+struct JumpCfg {
+    int nT, nS, r, mul;
+};
+
 struct IntegrateArgs {
     Tess t;
+    JumpCfg jump;         // FP32 (2D/3D EXACT, REF, SIMPLE)
     const double *A;      // [N, nC, ne] signed velocity matrices
     const double *T;      // [N, nC, ne] Trel = expm(dt * signed A)  (REF)
     const void *pts_in;   // [nPts, DIM] float64 or float32

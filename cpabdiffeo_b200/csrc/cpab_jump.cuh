@@ -1,0 +1,864 @@
+// cpab_jump.cuh -- the FP32 integration: many steps of a scheme at once
+// through the powers of a cell's step maps.
+//
+// While a point stays in one cell, each closed-form step applies the same
+// affine map T_c = expm(dt A_c), and each sub-step the same map S_c (the
+// explicit-midpoint map, or expm(h A_c) for the exact scheme): 2^k steps are
+// one application of the map's 2^k-th power.  A CTA stages these powers per
+// instance (level l of a map: its 2^(l r)-th power), and a unit of work is
+// one of them.  The scheme's sequence of steps is unchanged: every step
+// skipped over is one that the scheme would have taken from inside the cell
+// to inside the cell.  That is certain when the path cannot leave the cell in
+// between, which the two end points show:
+//   * both lie in the cell c (the scheme's own lookup), and
+//   * the larger of their margins m (least distance to a facet shared with
+//     another cell, box units) is at least tau^2 B / 2, where B
+//     bounds the second derivative of every facet functional along the path
+//     over the jump's time tau: a functional g with g(0), g(tau) <= 0, one of
+//     them <= -tau^2 B / 2 and |g''| <= B stays <= 0 in between.
+// With L the cell's linear part in box units, rho = |L|_1, x = rho tau: the
+// path's velocity is e^{L t} v0, so B <= rho e^x |v0|_1 (facet functionals
+// have coefficients 0, +-1), and its displacement d = tau phi(L tau) v0,
+// phi(z) = (e^z - 1)/z, gives |v0|_1 <= |d|_1 / (tau (2 - phi(x))).  So the
+// margin needed is |d|_1 kappa with
+//     kappa = 1/2 x e^x / (2 - phi(x))        (x < 1.2, else no jump),
+// tabulated per cell and level with 2 % to spare for the float arithmetic
+// and for S being the flow only up to O(h^2).
+//
+// A jump that is not certain is dropped, and the exit estimated from the rate
+// at which the dropped candidate lost its margin (`per_m`); the next jumps aim
+// short of it (8.7 units per point; 11.4 by bisection down the levels).  Level
+// 0 is the scheme itself: a closed-form step is kept or replaced by
+// nStepsODE sub-steps, a sub-step always taken.
+//
+// A lane keeps its point's position r in its box (from the box's centre, in
+// box units, |r| <= 1/2 inside) as a compensated pair, and the maps act on r:
+// rounding is then relative to a box, not to the domain, and the margin of a
+// candidate end point needs no cell lookup -- it is the smallest of the facet
+// functionals of the lane's current cell (WalkBox, WalkTri), negative when
+// the candidate left it.  The cell is looked up again only where a sub-step
+// leaves it.  3D tetrahedra (WalkTet) look every candidate up.
+//
+// Measured on 2D prior fields (64 cells, dt 0.02, 50 steps, 100 sub-steps
+// per leaving step): 11.4 units per point instead of 95; with r = 2 (every
+// fourth power) 13.5.  8.4 M points in 1024 instances: 3.17 ms with one step
+// per unit, 0.73 ms.
+// FP32 error against 64 bits of the registration likelihood (256 fields x
+// 256^2 pixels): 5.1e-8 before, 2.8e-8.
+#pragma once
+
+#include "cpab_integrate.cuh"
+
+namespace cpab {
+
+// Units of work a lane runs between changes of phase (kUnits), changes of
+// phase between the warp's votes (kRounds), and units of a first pass.
+// Measured on 8.4 M points (2D, 64 cells): 3 x 2 0.70 ms, 2 x 3 0.71, 2 x 2
+// and 4 x 1 0.72, 1 x 4 0.73, 2 x 1 0.80.
+constexpr int kUnits = 3, kRounds = 2, kFirstUnits = 5;
+// Resident CTAs of 256 threads the register allocation must allow per SM:
+// 4 (64 registers) in 1D and 2D -- 3 and 5 measured 0.72 and 0.77 ms on the
+// same points -- and 2 in 3D, whose tables leave room for no more (0.25 ms
+// against 0.27 ms for 3 on 0.5 M points of 320 cells).
+template <int DIM>
+constexpr int kJumpCtas = DIM == 3 ? 2 : 4;
+
+// Shared memory of the tables: the maps (increments M - I, column-major),
+// then kappa of every level above 0.
+__host__ __device__ inline size_t jump_bytes(const JumpCfg &j, int dim, int nC)
+{
+    const size_t kap = (size_t)(j.nT > 0 ? j.nT - 1 : 0) + j.nS;  // one row to spare: level 0 reads a row too
+    const size_t b = ((size_t)(j.nT + j.nS) * dim * (dim + 1) + kap) * nC * sizeof(float);
+    return (b + 15) & ~(size_t)15;
+}
+
+// log2 of the ratio between levels: every power of two while the tables stay
+// within 40 KB, every fourth power up to 64 KB, every eighth or sixteenth up to
+// 112 KB (two CTAs per SM), else level 0 alone; fewer levels when `avail`
+// bytes (what shared memory the kernel's other needs leave) do not hold the
+// choice.  The choice depends on the space and the step counts, not on the
+// batch, so results do not either.
+inline JumpCfg jump_cfg(int dim, int nC, int nTimeSteps, int nStepsODE, int scheme, size_t avail)
+{
+    auto log2i = [](long long v) {
+        int k = 0;
+        while (v > 1) {
+            v >>= 1;
+            ++k;
+        }
+        return k;
+    };
+    const int lt = log2i(nTimeSteps);
+    int ls = log2i(scheme == SCHEME_SIMPLE ? (long long)nTimeSteps * nStepsODE : nStepsODE);
+    if (ls > 8) ls = 8;
+    JumpCfg j{0, 0, 0, 0};
+    for (int r : {1, 2, 3, 4, 31}) {
+        j.r = r;
+        j.mul = (32 + r - 1) / r;
+        j.nT = scheme == SCHEME_SIMPLE ? 0 : (lt > 8 ? 8 : lt) / r + 1;
+        j.nS = ls / r + 1;
+        const size_t b = jump_bytes(j, dim, nC), budget = (size_t)(r == 1 ? 40 : r == 2 ? 64 : 112) * 1024;
+        if (r == 31 || (b <= budget && b <= avail)) break;
+    }
+    return j;
+}
+
+struct JumpTables {
+    const float *map;  // [nT + nS][nC][DIM * (DIM + 1)]
+    const float *kap;  // [nT - 1 + nS - 1][nC]
+};
+
+// Stage one instance's tables from its signed A and Trel: one thread per
+// (map, cell) squares the increment D = M - I upwards in FP64,
+// (I + D)^2 - I = 2 D + D_lin D.
+template <int DIM, int TESS>
+__device__ __forceinline__ JumpTables stage_jump(const double *gA, const double *gT, const Tess &t, const JumpCfg &jc,
+                                                 double dt, double h, bool exact_sub, unsigned char *smem)
+{
+    constexpr int NH = DIM + 1, NE = DIM * NH;
+    const int nC = t.nC;
+    float *map = reinterpret_cast<float *>(smem);
+    float *kap = map + (size_t)(jc.nT + jc.nS) * nC * NE;
+    const int kinds = jc.nT > 0 ? 2 : 1;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < kinds * nC; i += blockDim.x) {
+        const bool sub = i >= nC || jc.nT == 0;
+        const int c = i < nC ? i : i - nC;
+        const double *a = gA + (size_t)c * NE;
+        double D[NE];
+        double tau = sub ? h : dt;
+        if (!sub) {
+#pragma unroll
+            for (int e = 0; e < NE; ++e) D[e] = gT[(size_t)c * NE + e] - (e % NH == e / NH ? 1.0 : 0.0);
+        } else if (!exact_sub) {
+            // midpoint map: h A + h^2/2 L A
+#pragma unroll
+            for (int r = 0; r < DIM; ++r)
+#pragma unroll
+                for (int col = 0; col < NH; ++col) {
+                    double l2 = 0.0;
+#pragma unroll
+                    for (int k = 0; k < DIM; ++k) l2 += a[r * NH + k] * a[k * NH + col];
+                    D[r * NH + col] = h * (a[r * NH + col] + 0.5 * h * l2);
+                }
+        } else {
+            // expm(h A) - I by its Taylor sum, to the sum's rounding
+            double w[NE];
+#pragma unroll
+            for (int e = 0; e < NE; ++e) D[e] = w[e] = h * a[e];
+#pragma unroll 1
+            for (int k = 2; k <= 40; ++k) {
+                double nw[NE], big = 0.0, am = 0.0;
+#pragma unroll
+                for (int r = 0; r < DIM; ++r)
+#pragma unroll
+                    for (int col = 0; col < NH; ++col) {
+                        double v = 0.0;
+#pragma unroll
+                        for (int m = 0; m < DIM; ++m) v = fma(a[r * NH + m], w[m * NH + col], v);
+                        nw[r * NH + col] = v * (h / k);
+                    }
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    w[e] = nw[e];
+                    D[e] += w[e];
+                    big = fmax(big, fabs(w[e]));
+                    am = fmax(am, fabs(D[e]));
+                }
+                if (!(big > 1e-18 * am)) break;
+            }
+        }
+        // the box's centre
+        double ctr[DIM];
+        {
+            int kb[DIM];
+            cell_box<DIM, TESS>(t, c, kb);
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) ctr[r] = ((double)kb[r] + 0.5) * t.inc[r];
+        }
+        // rho = |L|_1 in box units
+        double rho = 0.0;
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+            double s = 0.0;
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) s += fabs(a[r * NH + k]) * t.inv_inc[r];
+            rho = fmax(rho, s * t.inc[k]);
+        }
+        const int levels = sub ? jc.nS : jc.nT, row0 = sub ? jc.nT : 0;
+        const int kap0 = sub ? (jc.nT > 0 ? jc.nT - 1 : 0) : 0;
+#pragma unroll 1
+        for (int l = 0; l < levels; ++l) {
+            float *m = map + ((size_t)(row0 + l) * nC + c) * NE;
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) {
+                double off = D[r * NH + DIM];  // the displacement of the box's centre
+#pragma unroll
+                for (int col = 0; col < DIM; ++col) {
+                    m[col * DIM + r] = (float)(D[r * NH + col] * t.inc[col] * t.inv_inc[r]);
+                    off = fma(D[r * NH + col], ctr[col], off);
+                }
+                m[DIM * DIM + r] = (float)(off * t.inv_inc[r]);
+            }
+            if (l > 0) {
+                const float x = (float)(rho * tau), em = expm1f(x), room = 2.0f - em / x;
+                kap[(size_t)(kap0 + l - 1) * nC + c] =
+                    x < 1e-6f ? 1e-6f : (x < 1.2f ? 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
+            }
+            if (l + 1 < levels) {
+#pragma unroll 1
+                for (int q = 0; q < jc.r; ++q) {
+                    double D2[NE];
+#pragma unroll
+                    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+                        for (int col = 0; col < NH; ++col) {
+                            double s = 2.0 * D[r * NH + col];
+#pragma unroll
+                            for (int k = 0; k < DIM; ++k) s = fma(D[r * NH + k], D[k * NH + col], s);
+                            D2[r * NH + col] = s;
+                        }
+#pragma unroll
+                    for (int e = 0; e < NE; ++e) D[e] = D2[e];
+                    tau *= 2.0;
+                }
+            }
+        }
+    }
+    return JumpTables{map, kap};
+}
+
+// ------------------------------------------------------------ walkers
+//
+// One lane's point: its cell c, margin m, and position.
+//   place(t, x)          at the absolute position x (looks the cell up)
+//   place_in(t, x, c)    the same, in the given cell (margin unknown: 0)
+//   position(t, x)       the absolute position
+//   step(t, map, q)      q: the candidate end of one composed step with the
+//                        column-major map; returns |d|_1 in box units; q.m is
+//                        its margin, negative when it left the cell
+//   take(q, yes)         moves to q, in the same cell, when yes
+//   leave(t, q)          moves to q, looking its cell up
+//   where(t, q, x)       absolute position of a candidate
+
+// Position in a box as a compensated pair hi + lo, box units from the centre.
+template <int DIM>
+struct BoxPos {
+    float hi[DIM], lo[DIM];
+};
+
+template <int DIM>
+struct BoxCand {
+    BoxPos<DIM> p;
+    float x[DIM];  // hi + lo
+    float m;
+};
+
+template <int DIM, int TESS>
+struct WalkLocal {
+    BoxPos<DIM> p;
+    int c;
+    float m;
+
+    __device__ __forceinline__ void set_local(const Tess &t, const double *x, const int *kb)
+    {
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            const double r = fma(x[i], t.inv_inc[i], -((double)kb[i] + 0.5));
+            p.hi[i] = (float)r;
+            p.lo[i] = (float)(r - (double)p.hi[i]);
+        }
+    }
+    // float coordinates in float arithmetic: x / inc with the low part of
+    // 1/inc, rounded once relative to the position in the box
+    __device__ __forceinline__ void set_local(const Tess &t, const float *x, const int *kb)
+    {
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            p.hi[i] = fmaf(x[i], t.finv_inc[i], -((float)kb[i] + 0.5f));
+            p.lo[i] = x[i] * t.finv_inc_lo[i];
+        }
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void box_of(const Tess &t, const Elem *x, int *kb) const
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {  // NaN -> 0
+            const float u = floorf((float)x[i] * t.finv_inc[i]);
+            kb[i] = (int)fminf(fmaxf(u, 0.0f), (float)(n[i] - 1));
+        }
+    }
+    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM> &q, double *x) const
+    {
+        int kb[DIM];
+        cell_box<DIM, TESS>(t, c, kb);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i)
+            x[i] = (((double)kb[i] + 0.5) + ((double)q.hi[i] + (double)q.lo[i])) * t.inc[i];
+    }
+    // the same rounded to float: the centre (k + 1/2) inc as a float and its
+    // rest, and one rounding of the sum
+    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM> &q, float *x) const
+    {
+        int kb[DIM];
+        cell_box<DIM, TESS>(t, c, kb);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            const float k = (float)kb[i] + 0.5f, ctr = k * t.finc[i];
+            const float rest = fmaf(k, t.finc[i], -ctr) + k * t.finc_lo[i];
+            x[i] = ctr + (rest + fmaf(q.hi[i], t.finc[i], q.lo[i] * t.finc[i]));
+        }
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void position(const Tess &t, Elem *x) const
+    {
+        to_absolute(t, p, x);
+    }
+    __device__ __forceinline__ void where(const Tess &t, const BoxCand<DIM> &q, double *x) const
+    {
+        to_absolute(t, q.p, x);
+    }
+    __device__ __forceinline__ void move(const BoxCand<DIM> &q, bool yes)
+    {
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            p.hi[i] = yes ? q.p.hi[i] : p.hi[i];
+            p.lo[i] = yes ? q.p.lo[i] : p.lo[i];
+        }
+        m = yes ? q.m : m;
+    }
+    // the box of a candidate, with its position relative to that box
+    __device__ __forceinline__ void shift_box(const Tess &t, BoxCand<DIM> &q, int *kb) const
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+        cell_box<DIM, TESS>(t, c, kb);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            const float s = fminf(fmaxf(floorf(q.x[i] + 0.5f), (float)-kb[i]), (float)(n[i] - 1 - kb[i]));
+            kb[i] += (int)s;
+            q.p.hi[i] -= s;
+            q.x[i] = q.p.hi[i] + q.p.lo[i];
+        }
+    }
+    __device__ __forceinline__ float advance(const float *map, BoxCand<DIM> &q) const
+    {
+        float mm[DIM * (DIM + 1)];
+        load_cell<DIM>(map, mm);
+        if constexpr (DIM == 1) {
+            const float d = fmaf(mm[0], p.hi[0] + p.lo[0], mm[1]);
+            const float s = p.hi[0] + d;
+            q.p.lo[0] = p.lo[0] + (d - (s - p.hi[0]));
+            q.p.hi[0] = s;
+            q.x[0] = s + q.p.lo[0];
+            return fabsf(d);
+        } else {
+            // coordinates 0 and 1 as one pair (FFMA2 / FADD2)
+            const float2 h = make_float2(p.hi[0], p.hi[1]), l = make_float2(p.lo[0], p.lo[1]);
+            const float2 r = __fadd2_rn(h, l);
+            float2 d = __ffma2_rn(make_float2(mm[0], mm[1]), make_float2(r.x, r.x),
+                                  make_float2(mm[DIM * DIM], mm[DIM * DIM + 1]));
+            d = __ffma2_rn(make_float2(mm[DIM], mm[DIM + 1]), make_float2(r.y, r.y), d);
+            float len = 0.0f;
+            if constexpr (DIM == 3) {
+                const float z = p.hi[2] + p.lo[2];
+                d = __ffma2_rn(make_float2(mm[6], mm[7]), make_float2(z, z), d);
+                const float dz = fmaf(mm[8], z, fmaf(mm[5], r.y, fmaf(mm[2], r.x, mm[11])));
+                const float s = p.hi[2] + dz;
+                q.p.lo[2] = p.lo[2] + (dz - (s - p.hi[2]));
+                q.p.hi[2] = s;
+                q.x[2] = s + q.p.lo[2];
+                len = fabsf(dz);
+            }
+            const float2 s = __fadd2_rn(h, d);
+            const float2 l2 = __fadd2_rn(l, __fadd2_rn(d, neg2(__fadd2_rn(s, neg2(h)))));
+            const float2 x = __fadd2_rn(s, l2);
+            q.p.hi[0] = s.x;
+            q.p.hi[1] = s.y;
+            q.p.lo[0] = l2.x;
+            q.p.lo[1] = l2.y;
+            q.x[0] = x.x;
+            q.x[1] = x.y;
+            return len + (fabsf(d.x) + fabsf(d.y));
+        }
+    }
+};
+
+constexpr float kFar = 1e30f;  // distance to a facet on the domain boundary
+
+// Box cells (1D and type II): the box's faces.
+template <int DIM>
+struct WalkBox : WalkLocal<DIM, 2> {
+    using B = WalkLocal<DIM, 2>;
+    using Cand = BoxCand<DIM>;
+    float flo[DIM], fhi[DIM];  // 1/2, or kFar where the domain ends
+
+    __device__ __forceinline__ float margin(const float *x) const
+    {
+        float v = fminf(flo[0] + x[0], fhi[0] - x[0]);
+#pragma unroll
+        for (int i = 1; i < DIM; ++i) v = fminf(v, fminf(flo[i] + x[i], fhi[i] - x[i]));
+        return v;
+    }
+    __device__ __forceinline__ void enter(const Tess &t, const int *kb)
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+        int stride = 1;
+        B::c = 0;
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            B::c += kb[i] * stride;
+            stride *= n[i];
+            flo[i] = kb[i] > 0 ? 0.5f : kFar;
+            fhi[i] = kb[i] < n[i] - 1 ? 0.5f : kFar;
+        }
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place(const Tess &t, const Elem *x)
+    {
+        int kb[DIM];
+        float r[DIM];
+        B::box_of(t, x, kb);
+        B::set_local(t, x, kb);
+        enter(t, kb);
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) r[i] = B::p.hi[i] + B::p.lo[i];
+        B::m = margin(r);
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
+    {
+        int kb[DIM];
+        cell_box<DIM, 2>(t, cell, kb);
+        B::set_local(t, x, kb);
+        enter(t, kb);
+        B::m = 0.0f;
+    }
+    __device__ __forceinline__ float step(const Tess &, const float *map, Cand &q) const
+    {
+        const float len = B::advance(map, q);
+        q.m = margin(q.x);
+        return len;
+    }
+    __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
+    __device__ __forceinline__ void leave(const Tess &t, Cand &q)
+    {
+        int kb[DIM];
+        B::shift_box(t, q, kb);
+        enter(t, kb);
+        B::p = q.p;
+        B::m = margin(q.x);
+    }
+};
+
+// 2D type I: four triangles per box between its diagonals, 0 at low y, then
+// counterclockwise.  With v the box coordinate towards a triangle's side and u
+// the one along it, the triangle is |u| <= v <= 1/2.  Outside the domain the
+// reference's rules (calc_2Dto2D.cu:53-148) continue it: beyond its side over
+// the side's width (|u| <= 1/2), and beyond a corner of the domain up to the
+// box's diagonal continued (|u| <= v).
+struct WalkTri : WalkLocal<2, 1> {
+    using B = WalkLocal<2, 1>;
+    using Cand = BoxCand<2>;
+    bool along_x;      // v is the y coordinate
+    unsigned sv;       // sign bit of v
+    float side;        // 1/2, or kFar where the side ends the domain
+    float ulo, uhi;    // 1/2 where the box's low / high face in u ends the domain, else kFar
+
+    __device__ __forceinline__ float margin(const float *x) const
+    {
+        const float v = __uint_as_float(__float_as_uint(along_x ? x[1] : x[0]) ^ sv), u = along_x ? x[0] : x[1];
+        // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
+        const float top = (u > uhi || u < -ulo) ? v : fminf(v, 0.5f);
+        return fminf(top - fabsf(u), side - v);
+    }
+    __device__ __forceinline__ void enter(const Tess &t, const int *kb, bool up, bool right)
+    {
+        const int tri = up ? (right ? 2 : 3) : (right ? 1 : 0);
+        c = (kb[0] + kb[1] * t.nC0) * 4 + tri;
+        along_x = up == right;
+        sv = right ? 0u : 0x80000000u;
+        const int k = along_x ? kb[1] : kb[0], n = along_x ? t.nC1 : t.nC0;
+        const int ku = along_x ? kb[0] : kb[1], nu = along_x ? t.nC0 : t.nC1;
+        side = k == (right ? n - 1 : 0) ? kFar : 0.5f;
+        // where u's faces do not end the domain, u beyond 1/2 is outside the triangle whatever v
+        ulo = ku == 0 ? 0.5f : kFar;
+        uhi = ku == nu - 1 ? 0.5f : kFar;
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place(const Tess &t, const Elem *x)
+    {
+        int kb[2];
+        box_of(t, x, kb);
+        set_local(t, x, kb);
+        const float r[2] = {p.hi[0] + p.lo[0], p.hi[1] + p.lo[1]};
+        enter(t, kb, r[0] < r[1], r[0] + r[1] > 0.0f);
+        m = margin(r);
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
+    {
+        int kb[2];
+        cell_box<2, 1>(t, cell, kb);
+        set_local(t, x, kb);
+        const int tri = cell & 3;
+        enter(t, kb, tri >= 2, tri == 1 || tri == 2);
+        m = 0.0f;
+    }
+    __device__ __forceinline__ float step(const Tess &, const float *map, Cand &q) const
+    {
+        const float len = advance(map, q);
+        q.m = margin(q.x);
+        return len;
+    }
+    __device__ __forceinline__ void take(const Cand &q, bool yes) { move(q, yes); }
+    __device__ __forceinline__ void leave(const Tess &t, Cand &q)
+    {
+        int kb[2];
+        shift_box(t, q, kb);
+        enter(t, kb, q.x[0] < q.x[1], q.x[0] + q.x[1] > 0.0f);
+        p = q.p;
+        m = margin(q.x);
+    }
+};
+
+// 3D type I: five tetrahedra per box, four at corners and the centre one.  In
+// box coordinates R a corner tetrahedron belongs to a corner sigma (signs of
+// product + in even boxes, - in odd ones): with y_a = sigma_a R_a it is
+// y0 + y1 + y2 >= 1/2 inside the box's three faces y_a <= 1/2 there; the centre
+// is where no corner's sum reaches 1/2.  Coordinates beyond the domain count
+// as on its boundary (the reference clamps them, calc_3Dto3D.cu:55-60), hence
+// the clamped y in the sum.  The reference clamps z with the x box size: where
+// the two sizes differ, every candidate is looked up at its absolute position.
+struct WalkTet : WalkLocal<3, 1> {
+    using B = WalkLocal<3, 1>;
+    using Cand = BoxCand<3>;
+    unsigned sg[3];  // sign bits of sigma
+    float face[3];   // 1/2, or kFar where the face ends the domain (and for the centre)
+    float low[3];    // -1/2 where the opposite face ends the domain, else -kFar
+    bool centre;
+
+    __device__ __forceinline__ float margin(const float *x) const
+    {
+        float y[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) y[i] = __uint_as_float(__float_as_uint(x[i]) ^ sg[i]);
+        float sum = -0.5f, far = kFar;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            sum += fmaxf(fminf(y[i], 0.5f), low[i]);
+            far = fminf(far, face[i] - y[i]);
+        }
+        const float corner = fminf(sum, far);
+        // the four corners' sums: sigma with an even number of signs flipped
+        const float a = y[0] + y[1], d = y[0] - y[1];
+        const float most = fmaxf(fabsf(a) + y[2], fabsf(d) - y[2]);
+        return centre ? 0.5f - most : corner;
+    }
+    __device__ __forceinline__ void enter(const Tess &t, int cell)
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+        int kb[3];
+        c = cell;
+        cell_box<3, 1>(t, cell, kb);
+        const int tet = cell - cell / 5 * 5;
+        const bool odd = ((kb[0] ^ kb[1] ^ kb[2]) & 1) != 0;
+        centre = tet == 0;
+        // signs in fast_cell_3d_tet's turned coordinates (odd boxes: (x, y) -> (y, -x))
+        const bool n0 = tet == 1 || tet == 3, n1 = tet == 1 || tet == 4, n2 = tet == 3 || tet == 4;
+        const bool neg[3] = {odd ? !n1 : n0, odd ? n0 : n1, n2};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            sg[i] = neg[i] ? 0x80000000u : 0u;
+            face[i] = centre || kb[i] == (neg[i] ? 0 : n[i] - 1) ? kFar : 0.5f;
+            low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
+        }
+    }
+    __device__ __forceinline__ int lookup(const Tess &t, const float *x, float &mq) const
+    {
+        float a[3];
+        int kb[3];
+        cell_box<3, 1>(t, c, kb);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) a[i] = ((float)kb[i] + 0.5f + x[i]) * t.finc[i];
+        return fast_cell_3d_tet_m(t, a, mq);
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place(const Tess &t, const Elem *x)
+    {
+        float a[3], mq;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) a[i] = (float)x[i];
+        place_in(t, x, fast_cell_3d_tet_m(t, a, mq));
+        m = mq;
+    }
+    template <typename Elem>
+    __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
+    {
+        int kb[3];
+        enter(t, cell);
+        cell_box<3, 1>(t, cell, kb);
+        set_local(t, x, kb);
+        m = 0.0f;
+    }
+    __device__ __forceinline__ float step(const Tess &t, const float *map, Cand &q) const
+    {
+        const float len = advance(map, q);
+        if (t.inc[0] == t.inc[2]) {
+            q.m = margin(q.x);
+        } else if (lookup(t, q.x, q.m) != c) {
+            q.m = -1e-30f;  // outside, nothing known of how far
+        }
+        return len;
+    }
+    __device__ __forceinline__ void take(const Cand &q, bool yes) { move(q, yes); }
+    __device__ __forceinline__ void leave(const Tess &t, Cand &q)
+    {
+        double x[3];
+        float mq;
+        const int cell = lookup(t, q.x, mq);
+        where(t, q, x);
+        place_in(t, x, cell);
+        m = mq;
+    }
+};
+
+template <int DIM, int TESS>
+struct WalkerOf {
+    using type = WalkBox<DIM>;
+};
+template <>
+struct WalkerOf<2, 1> {
+    using type = WalkTri;
+};
+template <>
+struct WalkerOf<3, 1> {
+    using type = WalkTet;
+};
+
+// Per-warp queue of points that the first pass left over (entries, shared memory).
+constexpr int kQueue = 64;
+
+// The FP32 twin of integrate_range.  Warps claim 32 points of the range at a
+// time and try to carry them through all their closed-form steps at once
+// (first pass: lanes in step, loads and stores coalesced; on the prior's
+// fields half of the points or more stay in their cell).  Points that may
+// leave their cell go to the warp's queue and from there one to a lane, the
+// lane advancing its point by one composed step per unit and taking the next
+// from the queue when done; another first pass runs whenever the queue does
+// not hold enough for the idle lanes.  Every closed-form step of a time step
+// is either kept or replaced by nStepsODE sub-steps, so the counts of both
+// follow from the number of replaced ones (c_fb).
+template <int DIM, int TESS, int SCHEME, class Src, class Snk>
+__device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, const JumpCfg &jc,
+                                               const JumpTables &tab, int64_t ws, int n_range, const Src &src,
+                                               Snk &snk, unsigned long long &c_fast, unsigned long long &c_fb,
+                                               unsigned long long &c_sub, unsigned long long &c_pts, int *claim,
+                                               unsigned short *queues, ExactCross *ex)
+{
+    using Walker = typename WalkerOf<DIM, TESS>::type;
+    using Cand = typename Walker::Cand;
+    constexpr int NE = DIM * (DIM + 1);
+    constexpr float kHuge = 1e30f;
+    const int lane = threadIdx.x & 31, nC = t.nC;
+    const unsigned lt = (1u << lane) - 1u;
+    // A lane's phase: closed-form steps of the remaining time steps (`left`
+    // of them), or sub-steps of the current one (`left` of them, `steps` time
+    // steps to go).  `row`: the phase's level 0 row of w.c in the maps; kappa of
+    // level l >= 1 sits at l nC + row - kshift (level 0 reads an entry before
+    // it, inside the tables, and ignores it).
+    const int s_row = jc.nT * nC;
+    Walker w;
+    w.c = 0;
+    w.m = 0.0f;
+    int left = 0, steps = 0, row = 0, kshift = nC, top = 0, idx = 0;
+    float per_m = kHuge;  // estimated steps per unit of margin until the exit
+    bool sub = false, active = false;
+    unsigned n_fb = 0, n_pts = 0;
+    auto to_steps = [&](int n) {  // n time steps to go
+        left = n;
+        sub = SCHEME == SCHEME_SIMPLE;
+        row = w.c;
+        kshift = nC;
+        top = (SCHEME == SCHEME_SIMPLE ? jc.nS : jc.nT) - 1;
+        per_m = kHuge;
+    };
+    auto to_substeps = [&](int n) {
+        left = n;
+        sub = true;
+        row = s_row + w.c;
+        kshift = jc.nT > 0 ? 2 * nC : nC;
+        top = jc.nS - 1;
+    };
+    auto start = [&](int k) {
+        active = true;
+        typename Src::Elem x[DIM];
+        idx = k;
+        src.load(ws + k, x);
+        w.place(t, x);
+        steps = 1;
+        to_steps(SCHEME == SCHEME_SIMPLE ? nT * nODE : nT);
+    };
+    auto finish = [&]() {
+        typename Src::Elem x[DIM];
+        w.position(t, x);
+        snk.put(ws + idx, x);
+        ++n_pts;
+        active = false;
+    };
+    // level and step count of the largest composed step within n >= 1 steps
+    auto level = [&](int n, int l_top, int &count) {
+        const int l = min(((31 - __clz(n)) * jc.mul) >> 5, l_top);
+        count = 1 << (l * jc.r);
+        return l * nC;
+    };
+    unsigned short *queue = queues + (threadIdx.x >> 5) * kQueue;
+    int queued = 0;
+    bool more = true;  // the range may hold unclaimed points
+    // Idle lanes take points: from the queue, after as many first passes as
+    // it takes to fill it (a pass adds at most 32, so kQueue holds).
+    auto refill = [&]() {
+        const unsigned idle = __ballot_sync(FULL, !active);
+        const int want = __popc(idle);
+        while (more && queued < want) {
+            int b = 0;
+            if (lane == 0) b = atomicAdd(claim, 32);
+            b = __shfl_sync(FULL, b, 0);
+            if (b + 32 >= n_range) more = false;
+            if (b >= n_range) break;
+            const bool have = b + lane < n_range;
+            bool left_over = have;
+            if (SCHEME != SCHEME_SIMPLE) {
+                Walker v;
+                typename Src::Elem x[DIM];
+                v.c = 0;
+                if (have) {
+                    src.load(ws + b + lane, x);
+                    v.place(t, x);
+                }
+                int togo = have ? nT : 0;
+                bool go = have;
+#pragma unroll 1
+                for (int u = 0; u < kFirstUnits && __any_sync(FULL, go); ++u) {
+                    int n;
+                    const int l = level(max(togo, 1), jc.nT - 1, n);
+                    Cand q;
+                    const float need = v.step(t, tab.map + (l + v.c) * NE, q) * tab.kap[l + v.c - nC];
+                    go = go && !(q.m < 0.0f) && (l == 0 || fmaxf(v.m, q.m) >= need);
+                    v.take(q, go);
+                    togo -= go ? n : 0;
+                    go = go && togo > 0;
+                }
+                left_over = have && togo > 0;
+                if (have && togo == 0) {
+                    v.position(t, x);
+                    snk.put(ws + b + lane, x);
+                    ++n_pts;
+                }
+            }
+            const unsigned lo = __ballot_sync(FULL, left_over);
+            if (left_over) queue[queued + __popc(lo & lt)] = (unsigned short)(b + lane);
+            queued += __popc(lo);
+            __syncwarp();
+        }
+        if (!active) {
+            const int k = queued - 1 - __popc(idle & lt);
+            if (k >= 0) start(queue[k]);
+        }
+        queued = max(queued - want, 0);
+        __syncwarp();
+    };
+    refill();
+    // A lane whose sub-step leaves its cell parks (`park`): the warp moves its
+    // parked lanes into their new cells together -- done at once, each such
+    // lane would hold up the other 31 (about one lane of a warp leaves its
+    // cell per unit).  A parked lane keeps only the sub-step's start and
+    // recomputes its end.  EXACT resolves the exits, which takes far longer,
+    // once kCrossBatch lanes wait (as integrate_range).
+    constexpr int kCrossBatch = CPAB_EXACT_CROSS_BATCH, kCrossWait = CPAB_EXACT_CROSS_WAIT;
+    bool park = false;
+    int park_votes = 0;
+    while (__any_sync(FULL, active)) {
+        // units without branches: lanes that wait run along without effect
+#pragma unroll 1
+        for (int h = 0; h < kRounds; ++h) {
+            bool go = active && !park && left > 0, out = false;
+#pragma unroll
+            for (int u = 0; u < kUnits; ++u) {
+                int n;
+                const int l = level(max(min(left, (int)(w.m * per_m)), 1), top, n);
+                Cand q;
+                const float need = w.step(t, tab.map + (l + row) * NE, q) * tab.kap[l + row - kshift];
+                const bool stays = !(q.m < 0.0f);  // NaN stays
+                const bool take = go && stays && (l == 0 || fmaxf(w.m, q.m) >= need);
+                // Dropped: the exit is estimated where the margin is used up at
+                // the rate it was lost (a candidate inside, but not certain:
+                // at half its steps).  The estimate stays below n steps, so the
+                // next jump from here is a shorter one.
+                if (go && !take)
+                    per_m = __fdividef((stays ? 0.5f : 0.999f) * (float)(l == 0 && !sub ? nODE : n),
+                                       stays ? fmaxf(w.m, 1e-12f) : w.m - q.m);
+                out = out || (go && !take && l == 0);
+                w.take(q, take);
+                left -= take ? n : 0;
+                go = go && !out && left > 0;
+            }
+            if (SCHEME == SCHEME_SIMPLE) {
+                park = park || out;
+            } else {
+                park = park || (out && sub);
+                if (out && !sub) {
+                    // the closed-form step leaves the cell: redo it with nStepsODE sub-steps
+                    steps = left;
+                    to_substeps(nODE);
+                    ++n_fb;
+                } else if (left == 0 && sub && !park) {
+                    to_steps(--steps);
+                }
+            }
+        }
+        const unsigned pm = __ballot_sync(FULL, park);
+        bool resolve = pm != 0;
+        if (SCHEME == SCHEME_EXACT && pm) {
+            const unsigned am = __ballot_sync(FULL, active && left > 0);
+            resolve = __popc(pm) >= kCrossBatch || pm == am || ++park_votes > kCrossWait;
+            if (resolve) park_votes = 0;
+        }
+        if (resolve && park) {
+            // the parked sub-step's end, recomputed with the same arithmetic
+            Cand q;
+            w.step(t, tab.map + row * NE, q);
+            if (SCHEME == SCHEME_EXACT) {
+                double from[DIM], to[DIM];
+                w.position(t, from);
+                w.where(t, q, to);
+                const int c = exact_substep_cross<DIM, TESS, float>(t, *ex, w.c, from, to);
+                w.place_in(t, to, c);
+            } else {
+                w.leave(t, q);
+            }
+            park = false;
+            // of the new cell's exit nothing is known
+            if (SCHEME == SCHEME_SIMPLE) {
+                to_steps(left - 1);
+            } else if (left > 1) {
+                to_substeps(left - 1);
+                per_m = kHuge;
+            } else {
+                to_steps(--steps);
+            }
+        }
+        if (active && !park && left == 0) finish();
+        if (__any_sync(FULL, !active) && (more || queued > 0)) refill();
+    }
+    c_pts += n_pts;
+    if (SCHEME == SCHEME_SIMPLE) {
+        c_sub += (unsigned long long)n_pts * nT * nODE;
+    } else {
+        c_fb += n_fb;
+        c_sub += (unsigned long long)n_fb * nODE;
+        c_fast += (unsigned long long)n_pts * nT - n_fb;
+    }
+}
+
+}  // namespace cpab

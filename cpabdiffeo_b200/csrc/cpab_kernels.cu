@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "cpab_integrate.cuh"
+#include "cpab_jump.cuh"
 #include "cpab_launch.h"
 
 namespace cpab {
@@ -53,32 +54,26 @@ __global__ void k_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, in
 
 // ------------------------------------------------------------ integration
 
-template <int DIM>
+template <int DIM, typename Real>
 struct ArraySrc {
+    using Elem = Real;
     const void *base;
-    template <typename Real>
-    __device__ __forceinline__ void load(int64_t i, PState<DIM, Real> &st) const
-    {
-        Real p[DIM];
-        load_pt<DIM, Real>(base, i, p);
-        st.set(p);
-    }
+    __device__ __forceinline__ void load(int64_t i, Real *x) const { load_pt<DIM, Real>(base, i, x); }
 };
 
-template <int DIM>
+template <int DIM, typename Real>
 struct ArraySnk {
     void *base;
     int clamp;
     double lo, hi;
     unsigned long long nan;
-    template <typename Real>
-    __device__ __forceinline__ void put(int64_t i, const PState<DIM, Real> &st)
+    __device__ __forceinline__ void put(int64_t i, const Real *x)
     {
         Real p[DIM];
-        st.get(p);
         bool bad = false;
 #pragma unroll
         for (int k = 0; k < DIM; ++k) {
+            p[k] = x[k];
             if (clamp) p[k] = clamp_ref(p[k], lo, hi);
             bad |= (p[k] != p[k]);
         }
@@ -87,27 +82,39 @@ struct ArraySnk {
     }
 };
 
+// Shared memory of an instance's tables.
+template <typename Real>
+__host__ __device__ inline size_t table_bytes(const IntegrateArgs &a)
+{
+    if (sizeof(Real) == 4) return jump_bytes(a.jump, a.t.dim, a.t.nC);
+    return (size_t)2 * a.t.nC * a.t.dim * (a.t.dim + 1) * sizeof(double);
+}
+
 template <int DIM, int TESS, typename Real, int SCHEME>
 __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
 {
     constexpr int NE = DIM * (DIM + 1);
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    // double: A and Trel; float: the composed-step tables (cpab_jump.cuh)
+    constexpr bool kJump = sizeof(Real) == 4;
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
     // cell-sort scratch after the tables: histogram [nC], start cells and permutation [tile_pts]
-    int *s_hist = reinterpret_cast<int *>(sA + (1 + TableLayout<Real>::kTParts) * a.t.nC * NE);
+    int *s_hist = reinterpret_cast<int *>(smem_raw + table_bytes<Real>(a));
     int *s_cell = s_hist + a.t.nC;
     int *s_perm = s_cell + a.batch.tile_pts;
     __shared__ TileInfo s_tile;
     __shared__ unsigned long long s_claim;
+    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
 
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t ntiles = total_tiles(a.batch);
     unsigned long long c_fast = 0, c_fb = 0, c_sub = 0, c_pts = 0;
     int loaded = -1;
-    const ArraySrc<DIM> src{a.pts_in};
-    ArraySnk<DIM> snk{a.pts_out, a.clamp, a.clamp_lo, a.clamp_hi, 0ull};
+    const ArraySrc<DIM, Real> src{a.pts_in};
+    ArraySnk<DIM, Real> snk{a.pts_out, a.clamp, a.clamp_lo, a.clamp_hi, 0ull};
+    JumpTables jt{nullptr, nullptr};
     ExactCross ex{nullptr, a.facets, a.nbr, a.nF, a.h_sub, a.max_crossings, 0ull, 0ull};
 
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -119,23 +126,30 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
         __syncthreads();
         const TileInfo ti = s_tile;
         if (ti.inst != loaded) {
-            stage_tables<DIM, Real>(a.A + (size_t)ti.inst * tab, a.T + (size_t)ti.inst * tab, a.t.nC,
-                                    SCHEME != SCHEME_SIMPLE, a.h_sub, sA, sT, SCHEME == SCHEME_EXACT);
+            const double *gA = a.A + (size_t)ti.inst * tab, *gT = a.T + (size_t)ti.inst * tab;
+            if constexpr (kJump)
+                jt = stage_jump<DIM, TESS>(gA, gT, a.t, a.jump, a.dt, a.h_sub, SCHEME == SCHEME_EXACT, smem_raw);
+            else
+                stage_tables<DIM>(gA, gT, a.t.nC, SCHEME != SCHEME_SIMPLE, a.h_sub, sA, sT,
+                                        SCHEME == SCHEME_EXACT);
             ex.A = a.A + (size_t)ti.inst * tab;
             loaded = ti.inst;
             __syncthreads();
         }
         const int64_t n = ti.end - ti.start;
         const int *perm = nullptr;
-        if (a.sort) {
+        if (!kJump && a.sort) {
             // counting sort of the tile's points by start cell (order inside a cell is irrelevant:
-            // every point is integrated on its own)
+            // every point is integrated on its own).  Not in FP32: lanes in different cells cost a
+            // composed step nothing, and the sort's passes did (64 cells, 8.4 M points: 0.94 ms
+            // without, 1.10 ms with).
             for (int i = threadIdx.x; i < a.t.nC; i += blockDim.x) s_hist[i] = 0;
             __syncthreads();
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                PState<DIM, Real> st;
-                src.load(ti.start + i, st);
-                const int c = cell_of<DIM, TESS>(a.t, st);
+                Real p[DIM];
+                src.load(ti.start + i, p);
+                const double x[3] = {(double)p[0], (double)p[DIM > 1 ? 1 : 0], (double)p[DIM > 2 ? 2 : 0]};
+                const int c = exact_cell<DIM, TESS>(a.t, x);
                 s_cell[i] = c;
                 atomicAdd(s_hist + c, 1);
             }
@@ -147,9 +161,13 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
             perm = s_perm;
         }
         // every warp works on the whole tile through the shared claim counter
-        integrate_range<DIM, TESS, Real, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, ti.end, h, src,
-                                                 snk, c_fast, c_fb, c_sub, c_pts, perm, ti.start, &s_claim,
-                                                 perm ? s_cell : nullptr, &ex);
+        if constexpr (kJump)
+            integrate_jump<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, ti.start, (int)n, src, snk,
+                                              c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim), s_queue, &ex);
+        else
+            integrate_range<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, ti.end, h, src,
+                                                     snk, c_fast, c_fb, c_sub, c_pts, perm, ti.start, &s_claim,
+                                                     perm ? s_cell : nullptr, &ex);
         __syncthreads();
     }
     if (a.counters) {
@@ -176,7 +194,7 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
 }
 
 template <int DIM, int TESS, typename Real, int SCHEME>
-__global__ void __launch_bounds__(256) k_integrate(IntegrateArgs a)
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? kJumpCtas<DIM> : 1) k_integrate(IntegrateArgs a)
 {
     integrate_body<DIM, TESS, Real, SCHEME>(a);
 }
@@ -522,9 +540,8 @@ static int grid_for(int64_t n, int block, int per_sm = 8)
 template <int DIM, int TESS, typename Real, int SCHEME>
 static cudaError_t launch_integrate_t(const IntegrateArgs &a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    constexpr int NE = DIM * (DIM + 1);
-    size_t smem = (size_t)(1 + TableLayout<Real>::kTParts) * a.t.nC * NE * sizeof(Real);
-    if (a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)a.batch.tile_pts) * sizeof(int);
+    size_t smem = table_bytes<Real>(a);
+    if (sizeof(Real) == 8 && a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)a.batch.tile_pts) * sizeof(int);
     void (*kern)(IntegrateArgs);
     if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
     else kern = k_integrate<DIM, TESS, Real, SCHEME>;

@@ -12,6 +12,7 @@
 // terms go to shared memory and are summed in a fixed order per tile, tiles
 // per instance in index order, so results do not depend on the batch.
 #include "cpab_integrate.cuh"
+#include "cpab_jump.cuh"
 #include "cpab_landmarks.h"
 #include "cpab_launch.h"
 #include "cpab_reduce.cuh"
@@ -23,15 +24,13 @@ namespace {
 // Start points: the instance's landmarks (double [n_lm, DIM]).
 template <int DIM>
 struct LandmarkSrc {
+    using Elem = double;
     const double *src;  // this instance's first landmark
     int64_t base;       // global index of that landmark
-    template <typename Real>
-    __device__ __forceinline__ void load(int64_t i, PState<DIM, Real> &st) const
+    __device__ __forceinline__ void load(int64_t i, double *p) const
     {
-        double p[DIM];
 #pragma unroll
         for (int k = 0; k < DIM; ++k) p[k] = __ldg(src + (i - base) * DIM + k);
-        st.set(p);
     }
 };
 
@@ -46,12 +45,12 @@ struct LandmarkSnk {
     double *term;
     int clamp;
     double lo, hi;
-    template <typename Real>
-    __device__ __forceinline__ void put(int64_t i, const PState<DIM, Real> &st)
+    __device__ __forceinline__ void put(int64_t i, const double *p)
     {
         const int64_t j = i - base;
         double x[DIM];
-        st.get(x);
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) x[d] = p[d];
         if (clamp) {
             // calc_T's end-point clamp (threshold_krnl)
 #pragma unroll
@@ -76,8 +75,12 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
     // per-landmark terms of the current tile, after the tables (a multiple of 8 bytes)
-    double *s_term = reinterpret_cast<double *>(sA + (1 + TableLayout<Real>::kTParts) * a.t.nC * NE);
+    constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
+    JumpTables jt{nullptr, nullptr};
+    double *s_term = reinterpret_cast<double *>(
+        smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     __shared__ unsigned long long s_claim;
+    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t tpi = ((int64_t)a.n_lm + a.tile_pts - 1) / a.tile_pts;
@@ -94,8 +97,9 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
         const int64_t end = min(start + (int64_t)a.tile_pts, base + a.n_lm);
         if (inst != loaded) {
             __syncthreads();
-            stage_tables<DIM, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, true,
-                                    a.h_sub, sA, sT);
+            const double *gA = a.A + (size_t)inst * tab, *gT = a.T + (size_t)inst * tab;
+            if constexpr (kJump) jt = stage_jump<DIM, TESS>(gA, gT, a.t, a.jump, a.dt, a.h_sub, false, smem_raw);
+            else stage_tables<DIM>(gA, gT, a.t.nC, true, a.h_sub, sA, sT);
             loaded = inst;
         }
         LandmarkSrc<DIM> src{a.src + (int64_t)inst * a.src_stride * DIM, base};
@@ -104,8 +108,13 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
                              base, start, k, s_term, a.clamp, a.clamp_lo, a.clamp_hi};
         if (threadIdx.x == 0) s_claim = 0ull;
         __syncthreads();
-        integrate_range<DIM, TESS, Real, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, end, h, src,
-                                                     snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
+        if constexpr (kJump)
+            integrate_jump<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, start, (int)(end - start), src,
+                                                  snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
+                                                  s_queue, nullptr);
+        else
+            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, end, h,
+                                                         src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         double acc = 0.0;
         for (int j = threadIdx.x; j < (int)(end - start); j += blockDim.x) acc += s_term[j];
@@ -128,7 +137,7 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
 template <int DIM, int TESS, typename Real>
 cudaError_t launch_t(const LandmarkArgs &a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = landmark_smem_bytes(a.t, a.tile_pts, sizeof(Real) == 8 ? PREC_F64 : PREC_F32);
+    const size_t smem = landmark_smem_bytes(a.t, a.tile_pts, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
     auto kern = k_landmark_ll<DIM, TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -149,10 +158,9 @@ cudaError_t launch_dt(const LandmarkArgs &a, int prec, const LaunchCfg &cfg, cud
 
 }  // namespace
 
-size_t landmark_smem_bytes(const Tess &t, int tile_pts, int prec)
+size_t landmark_smem_bytes(const Tess &t, int tile_pts, int prec, const JumpCfg &jump)
 {
-    const int ne = t.dim * (t.dim + 1);
-    const size_t tables = prec == PREC_F64 ? (size_t)t.nC * ne * 2 * 8 : (size_t)t.nC * ne * 2 * 4;
+    const size_t tables = prec == PREC_F64 ? (size_t)t.nC * t.dim * (t.dim + 1) * 2 * 8 : jump_bytes(jump, t.dim, t.nC);
     return tables + (size_t)tile_pts * sizeof(double);
 }
 

@@ -13,6 +13,7 @@ struct LaunchCfg;
 // Gaussian landmark log-likelihood of N instances.
 struct LandmarkArgs {
     Tess t;
+    JumpCfg jump;             // FP32
     const double *A, *T;      // [N, nC, ne] signed tables (sign +1: calc_T_fwd)
     const double *src, *dst;  // landmarks [*, n_lm, dim]
     int64_t src_stride;       // points between instances' landmark sets (0: one set shared by all)
@@ -31,7 +32,7 @@ struct LandmarkArgs {
     const volatile int *cancel;
 };
 
-size_t landmark_smem_bytes(const Tess &t, int tile_pts, int prec);
+size_t landmark_smem_bytes(const Tess &t, int tile_pts, int prec, const JumpCfg &jump);
 cudaError_t launch_landmark_ll(const LandmarkArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s);
 
 }  // namespace cpab

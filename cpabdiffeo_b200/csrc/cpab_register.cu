@@ -26,6 +26,7 @@
 
 #include "cpab_bulk.cuh"
 #include "cpab_integrate.cuh"
+#include "cpab_jump.cuh"
 #include "cpab_launch.h"
 #include "cpab_reduce.cuh"
 #include "cpab_register.h"
@@ -455,48 +456,42 @@ cudaError_t launch_remap_ssd(const RemapArgs &a, int map_prec, cudaStream_t s)
 // and the sampling stay out of the lane loop, whose register count sets the
 // CTAs per SM, and each warp samples 32 consecutive pixels together.
 struct SlotSrc2 {
+    using Elem = double;
     const double2 *slot;
     int64_t tile_start;
-    template <typename Real>
-    __device__ __forceinline__ void load(int64_t i, PState<2, Real> &st) const
+    __device__ __forceinline__ void load(int64_t i, double *p) const
     {
         const double2 v = slot[i - tile_start];
-        const double p[2] = {v.x, v.y};
-        st.set(p);
+        p[0] = v.x;
+        p[1] = v.y;
     }
 };
 
 struct SlotSnk2 {
     double2 *slot;
     int64_t tile_start;
-    template <typename Real>
-    __device__ __forceinline__ void put(int64_t i, const PState<2, Real> &st)
+    __device__ __forceinline__ void put(int64_t i, const double *p)
     {
-        double p[2];
-        st.get(p);
         slot[i - tile_start] = make_double2(p[0], p[1]);
     }
 };
 
-// CPAB_REGISTER_MIN_BLOCKS: resident CTAs of 256 threads the register
-// allocation must allow per SM (unset: the compiler's own choice).
-#ifdef CPAB_REGISTER_MIN_BLOCKS
-#define CPAB_REGISTER_BOUNDS __launch_bounds__(256, CPAB_REGISTER_MIN_BLOCKS)
-#else
-#define CPAB_REGISTER_BOUNDS __launch_bounds__(256)
-#endif
 template <int TESS, typename Real>
-__global__ void CPAB_REGISTER_BOUNDS k_register_ll(RegisterArgs a)
+__global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 3 : 1) k_register_ll(RegisterArgs a)
 {
     constexpr int DIM = 2, NE = 6;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
-    // the tile's point slots, after the tables (48 or 96 bytes per cell: 16-byte aligned), then the
-    // 32-point group sums of the likelihood
-    double2 *s_pos = reinterpret_cast<double2 *>(sA + (1 + TableLayout<Real>::kTParts) * a.t.nC * NE);
+    JumpTables jt{nullptr, nullptr};
+    // the tile's point slots, after the tables (a multiple of 16 bytes), then the 32-point group sums of the
+    // likelihood
+    double2 *s_pos = reinterpret_cast<double2 *>(
+        smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     double *s_grp = reinterpret_cast<double *>(s_pos + a.tile_px);
     __shared__ unsigned long long s_claim;
+    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t npx = (int64_t)a.H * a.W;
@@ -515,8 +510,9 @@ __global__ void CPAB_REGISTER_BOUNDS k_register_ll(RegisterArgs a)
         const int n = (int)(min(start + (int64_t)a.tile_px, base + npx) - start);
         if (inst != loaded) {
             __syncthreads();
-            stage_tables<DIM, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, true,
-                                    a.h_sub, sA, sT);
+            const double *gA = a.A + (size_t)inst * tab, *gT = a.T + (size_t)inst * tab;
+            if constexpr (kJump) jt = stage_jump<DIM, TESS>(gA, gT, a.t, a.jump, a.dt, a.h_sub, false, smem_raw);
+            else stage_tables<DIM>(gA, gT, a.t.nC, true, a.h_sub, sA, sT);
             loaded = inst;
         }
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -528,8 +524,13 @@ __global__ void CPAB_REGISTER_BOUNDS k_register_ll(RegisterArgs a)
         // all warps share the tile through the claim counter
         const SlotSrc2 src{s_pos, start};
         SlotSnk2 snk{s_pos, start};
-        integrate_range<DIM, TESS, Real, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
-                                                     src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
+        if constexpr (kJump)
+            integrate_jump<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, start, n, src,
+                                                  snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
+                                                  s_queue, nullptr);
+        else
+            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
+                                                         src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         const float *img = a.src + base, *ref = a.dst + base;
         float *warped = a.warped ? a.warped + base : nullptr;
@@ -560,16 +561,20 @@ __global__ void CPAB_REGISTER_BOUNDS k_register_ll(RegisterArgs a)
     }
 }
 
-size_t register_smem_bytes(int nC, int tile_px, int prec)
+size_t register_scratch_bytes(int tile_px)
 {
-    return (size_t)nC * 6 * (prec == PREC_F64 ? 2 * 8 : 2 * 4) + (size_t)tile_px * sizeof(double2) +
-           (size_t)((tile_px + 31) / 32) * sizeof(double);
+    return (size_t)tile_px * sizeof(double2) + (size_t)((tile_px + 31) / 32) * sizeof(double);
+}
+
+size_t register_smem_bytes(int nC, int tile_px, int prec, const JumpCfg &jump)
+{
+    return (prec == PREC_F64 ? (size_t)nC * 6 * 2 * 8 : jump_bytes(jump, 2, nC)) + register_scratch_bytes(tile_px);
 }
 
 template <int TESS, typename Real>
 static cudaError_t launch_register_t(const RegisterArgs &a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = register_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32);
+    const size_t smem = register_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
     auto kern = k_register_ll<TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

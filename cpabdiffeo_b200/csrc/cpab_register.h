@@ -27,6 +27,7 @@ struct RemapArgs {
 // Fused registration likelihood for N instances, one image pair each.
 struct RegisterArgs {
     Tess t;                   // 2D space
+    JumpCfg jump;             // FP32
     const double *A, *T;      // [N, nC, 6] signed tables (sign -1: calc_T_inv)
     const float *src, *dst;   // [N, H, W]
     float *warped;            // [N, H, W] or nullptr
@@ -43,7 +44,8 @@ struct RegisterArgs {
 
 cudaError_t launch_remap_ssd(const RemapArgs &a, int map_prec, cudaStream_t s);
 // Dynamic shared memory of k_register_ll: the tables and one double2 point slot per tile pixel.
-size_t register_smem_bytes(int nC, int tile_px, int prec);
+size_t register_scratch_bytes(int tile_px);
+size_t register_smem_bytes(int nC, int tile_px, int prec, const JumpCfg &jump);
 cudaError_t launch_register_ll(const RegisterArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s);
 
 }  // namespace cpab

@@ -16,6 +16,7 @@
 //                     transformed points are never stored.
 // Sums are deterministic (cpab_reduce.cuh).
 #include "cpab_integrate.cuh"
+#include "cpab_jump.cuh"
 #include "cpab_launch.h"
 #include "cpab_reduce.cuh"
 #include "cpab_register3d.h"
@@ -145,25 +146,23 @@ __global__ void __launch_bounds__(256) k_remap3d_ssd(Remap3dArgs a)
 // t + blockDim, ...).  Index arithmetic and sampling stay out of the lane
 // loop, whose register count sets the CTAs per SM.
 struct SlotSrc3 {
+    using Elem = double;
     const double *slot;
     int64_t tile_start;
-    template <typename Real>
-    __device__ __forceinline__ void load(int64_t i, PState<3, Real> &st) const
+    __device__ __forceinline__ void load(int64_t i, double *p) const
     {
         const double *v = slot + 3 * (i - tile_start);
-        const double p[3] = {v[0], v[1], v[2]};
-        st.set(p);
+        p[0] = v[0];
+        p[1] = v[1];
+        p[2] = v[2];
     }
 };
 
 struct SlotSnk3 {
     double *slot;
     int64_t tile_start;
-    template <typename Real>
-    __device__ __forceinline__ void put(int64_t i, const PState<3, Real> &st)
+    __device__ __forceinline__ void put(int64_t i, const double *p)
     {
-        double p[3];
-        st.get(p);
         double *v = slot + 3 * (i - tile_start);
         v[0] = p[0];
         v[1] = p[1];
@@ -178,9 +177,13 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
-    double *s_pos = reinterpret_cast<double *>(sA + (1 + TableLayout<Real>::kTParts) * a.t.nC * NE);
+    constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
+    JumpTables jt{nullptr, nullptr};
+    double *s_pos = reinterpret_cast<double *>(
+        smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     double *s_grp = s_pos + 3 * (size_t)a.tile_px;  // 32-voxel group sums of the likelihood
     __shared__ unsigned long long s_claim;
+    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t nvx = (int64_t)a.H * a.W * a.D;
@@ -199,8 +202,9 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
         const int n = (int)(min(start + (int64_t)a.tile_px, base + nvx) - start);
         if (inst != loaded) {
             __syncthreads();
-            stage_tables<DIM, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, true,
-                                    a.h_sub, sA, sT);
+            const double *gA = a.A + (size_t)inst * tab, *gT = a.T + (size_t)inst * tab;
+            if constexpr (kJump) jt = stage_jump<DIM, TESS>(gA, gT, a.t, a.jump, a.dt, a.h_sub, false, smem_raw);
+            else stage_tables<DIM>(gA, gT, a.t.nC, true, a.h_sub, sA, sT);
             loaded = inst;
         }
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -215,8 +219,13 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
         __syncthreads();
         const SlotSrc3 src{s_pos, start};
         SlotSnk3 snk{s_pos, start};
-        integrate_range<DIM, TESS, Real, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
-                                                     src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
+        if constexpr (kJump)
+            integrate_jump<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, start, n, src,
+                                                  snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
+                                                  s_queue, nullptr);
+        else
+            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
+                                                         src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         const float *img = a.src + base, *ref = a.dst + base;
         float *warped = a.warped ? a.warped + base : nullptr;
@@ -250,7 +259,7 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
 template <int TESS, typename Real>
 cudaError_t launch_register3d_t(const Register3dArgs &a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = register3d_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32);
+    const size_t smem = register3d_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
     auto kern = k_register3d_ll<TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -266,11 +275,15 @@ cudaError_t launch_register3d_t(const Register3dArgs &a, const LaunchCfg &cfg, c
 
 }  // namespace
 
-size_t register3d_smem_bytes(int nC, int tile_px, int prec)
+size_t register3d_scratch_bytes(int tile_px)
 {
-    const size_t tables = prec == PREC_F64 ? (size_t)nC * 12 * 2 * 8 : (size_t)nC * 12 * 2 * 4;
     // three doubles per voxel slot, then the 32-voxel group sums
-    return tables + (size_t)tile_px * 3 * sizeof(double) + (size_t)((tile_px + 31) / 32) * sizeof(double);
+    return (size_t)tile_px * 3 * sizeof(double) + (size_t)((tile_px + 31) / 32) * sizeof(double);
+}
+
+size_t register3d_smem_bytes(int nC, int tile_px, int prec, const JumpCfg &jump)
+{
+    return (prec == PREC_F64 ? (size_t)nC * 12 * 2 * 8 : jump_bytes(jump, 3, nC)) + register3d_scratch_bytes(tile_px);
 }
 
 cudaError_t launch_remap3d_ssd(const Remap3dArgs &a, int map_prec, cudaStream_t s)

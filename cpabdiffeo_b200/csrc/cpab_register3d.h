@@ -27,6 +27,7 @@ struct Remap3dArgs {
 // Fused 3D registration likelihood for N instances, one volume pair each.
 struct Register3dArgs {
     Tess t;                   // 3D space
+    JumpCfg jump;             // FP32
     const double *A, *T;      // [N, nC, 12] signed tables (sign -1: calc_T_inv)
     const float *src, *dst;   // [N, H, W, D]
     float *warped;            // [N, H, W, D] or nullptr
@@ -41,7 +42,8 @@ struct Register3dArgs {
     const volatile int *cancel;
 };
 
-size_t register3d_smem_bytes(int nC, int tile_px, int prec);
+size_t register3d_scratch_bytes(int tile_px);
+size_t register3d_smem_bytes(int nC, int tile_px, int prec, const JumpCfg &jump);
 cudaError_t launch_remap3d_ssd(const Remap3dArgs &a, int map_prec, cudaStream_t s);
 cudaError_t launch_register3d_ll(const Register3dArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s);
 
