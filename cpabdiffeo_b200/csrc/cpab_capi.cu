@@ -373,8 +373,11 @@ int cpab_calc_T_batched(cpab_ctx *ctx, const double *signedA, const double *Trel
         if (!workspace || workspace_bytes < cpab_batched_workspace_bytes(N))
             return fail(ctx, CPAB_NO_MEMORY, "workspace of %zu bytes needed", cpab_batched_workspace_bytes(N));
         int64_t *prefix = static_cast<int64_t *>(workspace);
-        cudaError_t e = launch_tile_prefix(offsets, prefix, N, a.batch.tile_pts, s);
-        if (e != cudaSuccess) return cuda_status(ctx, e, "tile_prefix launch");
+        // (the 1D exact kernel's intervals take ranges of points, not tiles)
+        if (!(scheme == CPAB_SCHEME_EXACT && ctx->t.dim == 1 && exact1d_uses_intervals(ctx->t.nC, precision))) {
+            cudaError_t e = launch_tile_prefix(offsets, prefix, N, a.batch.tile_pts, s);
+            if (e != cudaSuccess) return cuda_status(ctx, e, "tile_prefix launch");
+        }
         a.batch.offsets = offsets;
         a.batch.tile_prefix = prefix;
     } else {

@@ -23,6 +23,7 @@ struct LaunchCfg {
 constexpr size_t kSmemOptInAbove = 40 * 1024;
 
 int num_sms();
+int max_smem_optin();
 
 // Points per tile of a uniform integration launch over `total` points: the
 // configured tile, or a smaller one (a multiple of 32, at least 64) when the
@@ -50,6 +51,7 @@ inline int persistent_grid(K kern, const LaunchCfg &cfg, size_t smem)
 cudaError_t launch_integrate(const IntegrateArgs &a, int prec, int scheme, const LaunchCfg &cfg, cudaStream_t s);
 cudaError_t launch_integrate_exact1d(const IntegrateArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s);
 size_t exact1d_smem_bytes(int nC, int tile_pts, int sort, int prec);
+bool exact1d_uses_intervals(int nC, int prec);
 cudaError_t launch_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, cudaStream_t s);
 cudaError_t launch_trajectory(const IntegrateArgs &a, int64_t nPts, cudaStream_t s);
 cudaError_t launch_cell_idx(const Tess &t, const double *pts, int32_t *out, int64_t n, cudaStream_t s);
