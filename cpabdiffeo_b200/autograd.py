@@ -6,10 +6,10 @@ kernel (cpab_grad_theta).
 
 scheme="ref" (default): the forward is calc_T, the reference scheme
 (closed-form steps T = expm(dt A), nStepsODE midpoint sub-steps where a step
-leaves its cell); the backward (cpab_grad_theta_ref) re-runs it with
-checkpoints every `ck` time steps and propagates dLoss/dT(x) back through
-every step along the branch the forward took, mapping the per-cell
-dLoss/dT to dLoss/dA through the adjoint Frechet derivative of expm.
+leaves its cell); the backward (cpab_grad_theta_ref) re-runs it through
+composed steps and propagates dLoss/dT(x) back along the branch the forward
+took, mapping the per-cell dLoss/dT to dLoss/dA through the adjoint Frechet
+derivative of expm (`ck` only sizes its scratch).
 scheme="simple": the forward is calc_T_simple (nTimeSteps * nStepsODE
 midpoint sub-steps) and the backward (cpab_grad_theta) goes through every
 sub-step.  Either is the exact gradient of the discrete map.  theta is

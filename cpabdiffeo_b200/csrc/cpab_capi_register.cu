@@ -574,6 +574,7 @@ int cpab_mcmc_run(cpab_ctx *ctx, const double *B, int d, int C, double *theta, c
 // 448-491 computes the same derivative forward; its binding is commented out
 // in cpab/gpu/Calcs.py:196).
 #include "cpab_grad.h"
+#include "cpab_jump.cuh"
 
 extern "C" {
 
@@ -593,6 +594,16 @@ size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_i
 }
 
 }  // extern "C"
+
+// Levels of the adjoint's tables: as calc_T's, sparser where there is room for
+// fewer than `rows` sums beside level 0.
+static JumpCfg grad_jump(const cpab_ctx *ctx, int nTimeSteps, int nStepsODE, size_t most, size_t el, size_t rows)
+{
+    JumpCfg j = jump_cfg(ctx->t.dim, ctx->t.nC, nTimeSteps, nStepsODE, SCHEME_REF, most, el);
+    while (j.r < 31 && (size_t)(j.nT - 1 + j.nS - 1) > rows)
+        j = jump_cfg(ctx->t.dim, ctx->t.nC, nTimeSteps, nStepsODE, SCHEME_REF, most, el, j.r + 1);
+    return j;
+}
 
 // Shared body of cpab_grad_theta (ref == false: midpoint scheme, FP64) and
 // cpab_grad_theta_ref (reference scheme, needs Trels; FP64 or FP32 points).
@@ -638,10 +649,10 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         a.t = ctx->t;
         a.A = signedA;
         a.T = Trels;
-        a.pts = static_cast<const double *>(pts);  // float data when precision is CPAB_F32
-        a.grad_out = static_cast<const double *>(grad_out);
+        a.pts = pts;
+        a.grad_out = grad_out;
         a.out = static_cast<double *>(out);
-        a.grad_in = static_cast<double *>(grad_pts);
+        a.grad_in = grad_pts;
         a.gA = gA;
         a.ckpt = static_cast<double *>(workspace);
         a.N = N;
@@ -656,12 +667,25 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
             a.gT = reinterpret_cast<double *>(static_cast<char *>(workspace) + ck_bytes);
             a.gS = reinterpret_cast<double *>(static_cast<char *>(workspace) + ck_bytes + sum_bytes);
             e = cudaMemsetAsync(a.gT, 0, 2 * sum_bytes, s);
+            // The sums of the levels above 0 take the place of the checkpoints.  As many levels as one
+            // checkpoint has room for, so that the result does not depend on ck.
+            const size_t rows = (size_t)n_per_inst / ((size_t)ctx->t.nC * (ctx->t.dim + 1));
+            const size_t el = precision == CPAB_F64 ? 8 : 4, most = (size_t)max_smem_optin() - 1024;
+            a.jump = grad_jump(ctx, nTimeSteps, nStepsODE, most, el, rows);
+            a.gL = static_cast<double *>(workspace);
+            const size_t extra = (size_t)(a.jump.nT - 1 + a.jump.nS - 1);
+            if (e == cudaSuccess && extra) e = cudaMemsetAsync(a.gL, 0, extra * N * DA * sizeof(double), s);
             if (e != cudaSuccess) return cuda_status(ctx, e, "gradient sums reset");
-            e = precision == CPAB_F64 ? launch_grad_ref(a, s) : launch_grad_ref_f32(a, s);
+            e = launch_grad_ref(a, precision == CPAB_F64 ? PREC_F64 : PREC_F32, s);
         } else {
             e = launch_grad_simple(a, s);
         }
         if (e != cudaSuccess) return cuda_status(ctx, e, "grad launch");
+    }
+    if (ref && out && n_per_inst > 0) {
+        const int st = cpab_calc_T_batched(ctx, signedA, Trels, pts, out, N, nullptr, n_per_inst, nullptr, 0, precision,
+                                           CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE, nullptr, stream);
+        if (st != CPAB_OK) return st;
     }
     if (dtheta) {
         e = launch_bt_times(B, gA, dtheta, DA, d, N, (double)sign, s);

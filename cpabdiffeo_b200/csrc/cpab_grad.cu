@@ -20,18 +20,34 @@
 // every sub-step's start point and cell in a per-thread array.
 //
 // k_grad_ref: the same for the reference scheme (calc_T, calc_2Dto2D.cu:
-// 348-408): a time step is either the closed-form step q = T_c [p; 1] with
-// T_c = expm(dt A_c), kept when q stays in cell c, or nStepsODE sub-steps as
-// above.  Backwards through a kept step
-//     dT_c += g [p; 1]^T,   g = T_lin^T g,
-// and through a fallback step the sub-step adjoint.  The per-cell sums dT_c
-// become dLoss/dA_c once per instance and cell (k_frechet_adjoint):
+// 348-408), FP64 and FP32, through the composed steps of cpab_jump.cuh.  A
+// time step is either the closed-form step, kept when its end stays in the
+// cell, or nStepsODE sub-steps; the forward takes runs of either inside one
+// cell as one application of the map's power, r' = r + M [r; 1] on the
+// position r in the box, and records each move's table row and start.  The
+// adjoint runs down that list,
+//     dM += g [r; 1]^T,   g = g + M_lin^T g,
+// with dM summed per instance, cell and table row.  Once per instance and
+// cell, k_level_sums takes the sums down the levels -- D' = 2 D + D_lin D for
+// a map applied twice, so dD = 2 dD' + D_lin^T dD' + [dD' D^T | 0] -- to
+// dLoss/dT_c and dLoss/d(sub-step map)_c, and these become dLoss/dA_c:
+// k_frechet_adjoint:
 //     dA_c += dt L(X^T, dT_c),  X = dt [A_c; 0],
 // L the Frechet derivative of expm, read off the top-right block of
-// expm([[X^T, G], [0, X^T]]).  This is the exact gradient of the discrete
-// map along the branch the forward took (kept / fallback, cells); where a
-// step changes branch the map itself is discontinuous.
+// expm([[X^T, G], [0, X^T]]), and k_substep_map_adjoint.  This is the exact
+// gradient of the discrete map along the branch the forward took (kept /
+// fallback, cells); where a perturbation flips a branch the map itself jumps
+// by the sub-steps' discretisation error.  Nothing is checkpointed: the list
+// holds kMoves moves of a trajectory (most take 5 to 30) in local memory, and
+// a longer one is replayed in blocks from saved states.
+//
+// Measured, 3D with 320 cells, FP32, 8 theta x 64^3 points, forward and
+// backward: one step at a time 30.8 ms -- 4.8 of 32 lanes active, a fallback
+// step holding up its warp -- this 4.0 ms.
+#include <algorithm>
+
 #include "cpab_integrate.cuh"
+#include "cpab_jump.cuh"
 #include "cpab_grad.h"
 #include "cpab_launch.h"
 
@@ -176,125 +192,363 @@ __global__ void __launch_bounds__(128) k_grad_simple(GradArgs a)
     }
 }
 
-// One time step of the reference scheme from p (calc_T, the FP64 arithmetic
-// of k_integrate): the closed-form step when its end point stays in the
-// cell, else nODE sub-steps.  Returns whether the closed-form step was kept.
-template <int DIM, int TESS>
-__device__ __forceinline__ bool ref_step(const Tess &t, const double *sA, const double *sT, double *p, double h,
-                                         int nODE)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    const int c = exact_cell<DIM, TESS>(t, p);
-    double q[DIM];
-    exact_affine<DIM>(q, sT + c * NE, p);
-    if (exact_cell<DIM, TESS>(t, q) == c) {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) p[i] = q[i];
-        return true;
+// ------------------------------------------------------------ adjoint of calc_T
+
+// Moves of a trajectory kept at once, and states saved of a longer one.
+constexpr int kMoves = 48, kSaves = 24;
+// Lanes that must add to the same sums for them to be added up in the warp
+// first (the 3D case above: 8 lanes 3.98 ms, 4 4.11, 16 4.54).
+constexpr int kGroup = 8;
+
+// One point on its way through calc_T (the phases of integrate_jump, for one
+// lane on its own).
+template <int DIM, int TESS, typename Real>
+struct Path {
+    using Walker = typename WalkerOf<DIM, TESS, Real>::type;
+    Walker w;
+    Real per_m;
+    int left, steps, row, kshift, top;
+    bool sub;
+
+    __device__ __forceinline__ void to_steps(const JumpCfg &jc, int nC, int n)
+    {
+        left = n;
+        sub = false;
+        row = w.c;
+        kshift = nC;
+        top = jc.nT - 1;
+        per_m = Real(1e30);
     }
-    substeps<DIM, TESS>(t, sA, p, h, nODE);
-    return false;
+    __device__ __forceinline__ void to_substeps(const JumpCfg &jc, int nC, int n)
+    {
+        left = n;
+        sub = true;
+        row = jc.nT * nC + w.c;
+        kshift = 2 * nC;
+        top = jc.nS - 1;
+    }
+    __device__ __forceinline__ void begin(const Tess &t, const JumpCfg &jc, const Real *x, int nT)
+    {
+        w.place(t, x);
+        steps = 0;
+        to_steps(jc, t.nC, nT);
+    }
+    __device__ __forceinline__ bool done() const { return left == 0; }
+    // One unit; true when it moved, by the table row mi from r.
+    __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE,
+                                         int &mi, Real *r)
+    {
+        constexpr int NE = DIM * (DIM + 1);
+        const int nC = t.nC, lg = 31 - __clz(max(min(left, (int)(w.m * per_m)), 1));
+        const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
+        typename Walker::Cand q;
+        mi = l * nC + row;
+        const Real need = w.step(t, tab.map + (size_t)mi * NE, q) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
+        const bool stays = !(q.m < Real(0));
+        const bool take = stays && (l == 0 || most(w.m, q.m) >= need);
+        if (take || (l == 0 && sub)) {
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) r[i] = w.p.x(i);
+            left -= n;
+            if (take) {
+                w.take(q, true);
+            } else {
+                w.leave(t, q);
+                per_m = Real(1e30);
+                row = jc.nT * nC + w.c;
+            }
+            if (left == 0 && sub) to_steps(jc, nC, --steps);
+            return true;
+        }
+        // dropped: see integrate_jump
+        per_m = (stays ? Real(0.5) : Real(0.999)) * Real(l == 0 ? nODE : n) /
+                (stays ? most(w.m, Real(1e-12)) : w.m - q.m);
+        if (l == 0) {
+            steps = left;
+            const Real keep = per_m;
+            to_substeps(jc, nC, nODE);
+            per_m = keep;
+        }
+        return false;
+    }
+};
+
+// Add each lane's NE values to the sums at G (null: nothing to add; `key`
+// tells the sums apart).  Lanes with the same key -- neighbouring points make
+// the same moves -- are added up in the warp first: the sums are spread over
+// the lanes as they are halved (16 shuffles for up to 16 values), and one lane
+// per value adds its share.  Added one by one, 32 lanes to one address, the
+// additions bound the kernel (7.6 ms of 8.8 on the case above; 3.2 of 4.0 like
+// this, where the moves' list and the sums wait on L2).
+template <int NE, typename Real>
+__device__ __forceinline__ void add_grouped(double *G, int key, const Real *v)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned same = __match_any_sync(FULL, G ? key : -1 - lane);
+    const bool alone = __popc(same) < kGroup;
+    if (G && alone) {
+#pragma unroll
+        for (int e = 0; e < NE; ++e) atomicAdd(G + e, (double)v[e]);
+    }
+    unsigned todo = __ballot_sync(FULL, !alone);
+    while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const unsigned members = __shfl_sync(FULL, same, lead);
+        const bool in = (members >> lane) & 1u;
+        todo &= ~members;
+        double *base = reinterpret_cast<double *>(__shfl_sync(FULL, reinterpret_cast<unsigned long long>(G), lead));
+        constexpr int kSlots = NE <= 2 ? 2 : NE <= 8 ? 8 : 16;
+        Real s[kSlots];
+#pragma unroll
+        for (int e = 0; e < kSlots; ++e) s[e] = e < NE && in ? v[e < NE ? e : 0] : Real(0);
+        int slot = 0;
+#pragma unroll
+        for (int half = kSlots / 2, bit = 16; bit > 0; half /= 2, bit /= 2) {
+            if (half > 0) {
+                // keep one half of the values, hand the other to the partner
+                const bool up = (lane & bit) != 0;
+                if (up) slot += half;
+#pragma unroll
+                for (int e = 0; e < half; ++e) {
+                    const Real give = up ? s[e] : s[e + half], keep = up ? s[e + half] : s[e];
+                    s[e] = keep + __shfl_xor_sync(FULL, give, bit);
+                }
+            } else {
+                s[0] += __shfl_xor_sync(FULL, s[0], bit);
+            }
+        }
+        // the lanes that differ only in the bits left over hold the same sum
+        if ((lane & (32 / kSlots - 1)) == 0 && slot < NE) atomicAdd(base + slot, (double)s[0]);
+    }
 }
 
-// SACC: the gradient sums in shared memory, added to gA / gT at the end;
-// else (large tables) the per-thread accumulators go straight to gA / gT, so
-// that shared memory holds the tables only and more CTAs fit on an SM.
-template <int DIM, int TESS, bool SACC>
-__global__ void __launch_bounds__(128) k_grad_ref(GradArgs a)
+template <int DIM, int TESS, typename Real>
+__global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
 {
     constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tab = a.t.nC * NE;
-    const int inst = blockIdx.y;
-    double *sA = reinterpret_cast<double *>(smem_raw);
-    double *sT = sA + tab;
-    double *sGA = SACC ? sT + tab : a.gA + (size_t)inst * tab;   // dLoss/dA from sub-steps
-    double *sGT = SACC ? sGA + tab : a.gT + (size_t)inst * tab;  // dLoss/dT from closed-form steps
-    for (int i = threadIdx.x; i < tab; i += blockDim.x) {
-        sA[i] = a.A[(size_t)inst * tab + i];
-        sT[i] = a.T[(size_t)inst * tab + i];
-        if (SACC) {
-            sGA[i] = 0.0;
-            sGT[i] = 0.0;
-        }
-    }
+    const int nC = a.t.nC, tab = nC * NE, inst = blockIdx.y, lane = threadIdx.x & 31;
+    const JumpCfg jc = a.jump;
+    const JumpTables<Real> jt = stage_jump<DIM, TESS, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t, jc,
+                                                            a.dt, a.h_sub, false, smem_raw);
     __syncthreads();
-    const double h = XDIV(a.dt, (double)a.nStepsODE);
-    const int nT = a.nTimeSteps, nODE = a.nStepsODE, ck = a.ck;
+    // sums of level 0 (steps, sub-steps), and of the levels above in kappa's order
+    double *gT = a.gT + (size_t)inst * tab, *gS = a.gS + (size_t)inst * tab;
+    double *gL = a.gL + (size_t)inst * (jc.nT - 1 + jc.nS - 1) * tab;
+    const int s_row = jc.nT * nC;
     const int64_t n = a.n_per_inst;
-    const int64_t total = n * a.N;
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t gi = (int64_t)inst * n + j;
-        double p[DIM];
-        load_pt<DIM, double>(a.pts, gi, p);
-        for (int s = 0; s < nT; ++s) {
-            if (s % ck == 0) store_pt<DIM, double>(a.ckpt, (int64_t)(s / ck) * total + gi, p);
-            ref_step<DIM, TESS>(a.t, sA, sT, p, h, nODE);
+    const Real *pts = static_cast<const Real *>(a.pts), *gout = static_cast<const Real *>(a.grad_out);
+    Real *gin = static_cast<Real *>(a.grad_in);
+    // 32 points per warp at a time
+    for (int64_t j0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; j0 < n;
+         j0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t gi = (int64_t)inst * n + j0 + lane;
+        const bool have = j0 + lane < n;
+        Real x[DIM], g[DIM], r[kMoves][DIM];
+        int mi[kMoves];
+        Path<DIM, TESS, Real> save[kSaves], s;
+        int k = 0, block = 0;
+        if (have) {
+            load_pt<DIM, Real>(pts, gi, x);
+            s.begin(a.t, jc, x, a.nTimeSteps);
+            while (!s.done()) {
+                if (k == kMoves) {
+                    ++block;
+                    k = 0;
+                    if (block < kSaves) save[block] = s;
+                }
+                k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
+            }
+            // dLoss/d(position in the box)
+            load_pt<DIM, Real>(gout, gi, g);
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) g[i] *= (Real)a.t.inc[i];
         }
-        if (a.out) store_pt<DIM, double>(a.out, gi, p);
-        double g[DIM];
-        load_pt<DIM, double>(a.grad_out, gi, g);
-        double accA[NE], accT[NE];
+        for (;;) {
+            while (__any_sync(FULL, k > 0)) {
+                double *G = nullptr;
+                Real v[NE];
+                int key = 0;
+                if (k > 0) {
+                    --k;
+                    key = mi[k];
+                    const bool sub = key >= s_row;
+                    const int rel = key - (sub ? s_row : 0);
+                    G = rel < nC ? (sub ? gS : gT) + rel * NE
+                                 : gL + (size_t)(rel - nC + (sub ? (jc.nT - 1) * nC : 0)) * NE;
 #pragma unroll
-        for (int e = 0; e < NE; ++e) accA[e] = accT[e] = 0.0;
-        int cellA = -1, cellT = -1;
-        for (int s = nT - 1; s >= 0; --s) {
-            double q[DIM];
-            load_pt<DIM, double>(a.ckpt, (int64_t)(s / ck) * total + gi, q);
-            for (int r = 0; r < s % ck; ++r) ref_step<DIM, TESS>(a.t, sA, sT, q, h, nODE);
-            // time step s from q, along the forward's branch
-            const int c = exact_cell<DIM, TESS>(a.t, q);
-            const double *T = sT + c * NE;
-            double y[DIM];
-            exact_affine<DIM>(y, T, q);
-            if (exact_cell<DIM, TESS>(a.t, y) == c) {
-                acc_switch<NE>(sGT, accT, cellT, c);
+                    for (int i = 0; i < DIM; ++i) {
 #pragma unroll
-                for (int i = 0; i < DIM; ++i) {
+                        for (int c = 0; c < DIM; ++c) v[i * NH + c] = g[i] * r[k][c];
+                        v[i * NH + DIM] = g[i];
+                    }
+                    const Real *M = jt.map + (size_t)key * NE;
+                    Real gn[DIM];
 #pragma unroll
-                    for (int k = 0; k < DIM; ++k) accT[i * NH + k] += g[i] * q[k];
-                    accT[i * NH + DIM] += g[i];
+                    for (int c = 0; c < DIM; ++c) {
+                        Real u = g[c];
+#pragma unroll
+                        for (int i = 0; i < DIM; ++i) u += M[c * DIM + i] * g[i];
+                        gn[c] = u;
+                    }
+#pragma unroll
+                    for (int c = 0; c < DIM; ++c) g[c] = gn[c];
                 }
-                double gn[DIM];
-#pragma unroll
-                for (int k = 0; k < DIM; ++k) {
-                    double s2 = 0.0;
-#pragma unroll
-                    for (int i = 0; i < DIM; ++i) s2 += T[i * NH + k] * g[i];
-                    gn[k] = s2;
-                }
-#pragma unroll
-                for (int k = 0; k < DIM; ++k) g[k] = gn[k];
-            } else {
-                adjoint_substeps<DIM, TESS>(a.t, sA, sGA, q, g, h, nODE, accA, cellA);
+                add_grouped<NE, Real>(G, key, v);
+            }
+            if (!__any_sync(FULL, block > 0)) break;
+            if (block > 0) {
+                // the block before, replayed from the latest saved state at or before its start
+                --block;
+                const int from = min(block, kSaves - 1);
+                if (from == 0) s.begin(a.t, jc, x, a.nTimeSteps);
+                else s = save[from];
+                for (int skip = (block - from) * kMoves; skip > 0;)
+                    skip -= s.unit(a.t, jc, jt, a.nStepsODE, mi[0], r[0]) ? 1 : 0;
+                for (k = 0; k < kMoves;) k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
             }
         }
-        acc_switch<NE>(sGA, accA, cellA, -1);
-        acc_switch<NE>(sGT, accT, cellT, -1);
-        if (a.grad_in) store_pt<DIM, double>(a.grad_in, gi, g);
-    }
-    if (!SACC) return;
-    __syncthreads();
-    for (int i = threadIdx.x; i < tab; i += blockDim.x) {
-        const double va = sGA[i], vt = sGT[i];
-        if (va != 0.0) atomicAdd(a.gA + (size_t)inst * tab + i, va);
-        if (vt != 0.0) atomicAdd(a.gT + (size_t)inst * tab + i, vt);
+        if (gin && have) {
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) g[i] *= (Real)a.t.inv_inc[i];
+            store_pt<DIM, Real>(gin, gi, g);
+        }
     }
 }
 
-// E = expm(Z) for a small K x K matrix: scaling and squaring (Moler & Van
-// Loan, "Nineteen dubious ways to compute the exponential of a matrix",
-// method 3) with the degree-18 Taylor polynomial of Z / 2^s,
-// ||Z / 2^s||_1 <= 1/2 (truncation below 1e-22 relative).  Z is scaled in
-// place.
-template <int K>
-__device__ void expm_small(double (&Z)[K][K], double (&E)[K][K])
+// dLoss/dD from dLoss/d(2 D + D_lin D), in place.
+template <int DIM>
+__device__ __forceinline__ void twice_adjoint(const double *D, double *G)
 {
+    constexpr int NH = DIM + 1, NE = DIM * NH;
+    double o[NE];
+#pragma unroll
+    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+        for (int col = 0; col < NH; ++col) {
+            double v = 2.0 * G[r * NH + col];
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) v = fma(D[k * NH + r], G[k * NH + col], v);
+            if (col < DIM) {
+#pragma unroll
+                for (int q = 0; q < NH; ++q) v = fma(G[r * NH + q], D[col * NH + q], v);
+            }
+            o[r * NH + col] = v;
+        }
+#pragma unroll
+    for (int e = 0; e < NE; ++e) G[e] = o[e];
+}
+
+// The sums of all levels, in box coordinates, taken down to level 0 and to
+// the coordinates of the tables: gT becomes dLoss/dT, gS dLoss/d(sub-step map).
+template <int DIM, int TESS>
+__global__ void k_level_sums(GradArgs a)
+{
+    constexpr int NH = DIM + 1, NE = DIM * NH;
+    const int nC = a.t.nC, extra = a.jump.nT - 1 + a.jump.nS - 1;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)2 * a.N * nC;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const bool sub = (i & 1) != 0;
+        const int64_t ic = i >> 1;
+        const int inst = (int)(ic / nC), c = (int)(ic - (int64_t)inst * nC);
+        const double *A = a.A + ic * NE, *T = a.T + ic * NE;
+        double ctr[DIM], P[9][NE], G[NE];
+        {
+            int kb[DIM];
+            cell_box<DIM, TESS>(a.t, c, kb);
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) ctr[r] = ((double)kb[r] + 0.5) * a.t.inc[r];
+        }
+        double D[NE];
+        if (sub) {
+            midpoint_increment<DIM>(A, a.h_sub, D);
+        } else {
+#pragma unroll
+            for (int e = 0; e < NE; ++e) D[e] = T[e] - (e % NH == e / NH ? 1.0 : 0.0);
+        }
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            double off = D[r * NH + DIM];
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) {
+                off = fma(D[r * NH + k], ctr[k], off);
+                P[0][r * NH + k] = D[r * NH + k] * a.t.inc[k] * a.t.inv_inc[r];
+            }
+            P[0][r * NH + DIM] = off * a.t.inv_inc[r];
+        }
+        const int top = (sub ? a.jump.nS : a.jump.nT) - 1, q0 = sub ? a.jump.nT - 1 : 0, chain = top * a.jump.r;
+        for (int q = 0; q < chain; ++q) {
+#pragma unroll
+            for (int e = 0; e < NE; ++e) P[q + 1][e] = P[q][e];
+            twice<DIM>(P[q + 1]);
+        }
+        double *g0 = (sub ? a.gS : a.gT) + ic * NE;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) G[e] = 0.0;
+        for (int q = chain; q > 0; --q) {
+            if (q % a.jump.r == 0) {
+                const double *g = a.gL + (((size_t)inst * extra + q0 + q / a.jump.r - 1) * nC + c) * NE;
+#pragma unroll
+                for (int e = 0; e < NE; ++e) G[e] += g[e];
+            }
+            twice_adjoint<DIM>(P[q - 1], G);
+        }
+#pragma unroll
+        for (int e = 0; e < NE; ++e) G[e] += g0[e];
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            const double go = G[r * NH + DIM] * a.t.inv_inc[r];
+#pragma unroll
+            for (int k = 0; k < DIM; ++k)
+                g0[r * NH + k] = G[r * NH + k] * a.t.inc[k] * a.t.inv_inc[r] + go * ctr[k];
+            g0[r * NH + DIM] = go;
+        }
+    }
+}
+
+// gA[c] += dt L(X^T, G_c) for every (instance, cell) c, X = dt [A_c; 0]
+// (homogeneous) and G_c = [gT_c; 0]: the top-right block of exp(Z),
+// Z = [[X^T, G], [0, X^T]].  Scaling and squaring (Moler & Van Loan, "Nineteen
+// dubious ways to compute the exponential of a matrix", method 3) with the
+// degree-18 Taylor polynomial of Z / 2^s, |Z / 2^s|_1 <= 1/2 (truncation below
+// 1e-22 relative).  Powers of Z keep its shape [[P, Q], [0, P]], so only P and
+// Q are carried: P' = P X^T, Q' = Q X^T + P G, and (P^2, P Q + Q P) to square.
+// L is linear in G, so G is scaled to max |entry| 1 and the block scaled back,
+// which keeps the squaring count set by X.
+//
+// 16 threads per cell, one matrix entry each, matrices in shared memory: a
+// thread per cell had the 2 (DIM + 1) square matrices in local memory and
+// too few threads (2560 cells: 0.45 ms of the 3D gradient, this 0.02).
+template <int DIM>
+__global__ void __launch_bounds__(128) k_frechet_adjoint(const double *A, const double *gT, double *gA, int total,
+                                                         double dt)
+{
+    constexpr int M = DIM + 1, NE = DIM * M;
+    __shared__ double s_m[8][6][16];
+    const int grp = threadIdx.x >> 4, e = threadIdx.x & 15, i = e / M, j = e - i * M;
+    const unsigned mask = 0xffffu << ((threadIdx.x & 16) ? 16 : 0);
+    double *X = s_m[grp][0], *G = s_m[grp][1], *P = s_m[grp][2], *Q = s_m[grp][3], *P2 = s_m[grp][4], *Q2 = s_m[grp][5];
+    const bool on = e < M * M;
+    const int idx = blockIdx.x * 8 + grp;
+    if (idx >= total) return;  // whole groups; the barriers below are per group
+    const double *a = A + (size_t)idx * NE, *g = gT + (size_t)idx * NE;
+    double gs = 0.0;
+    for (int k = 0; k < NE; ++k) gs = fmax(gs, fabs(g[k]));
+    if (!(gs > 0.0)) return;  // no closed-form step in this cell
+    // X^T and G, row-major [i][j], last row of G and last column of X^T zero
+    if (on) {
+        X[e] = j < DIM ? dt * a[j * M + i] : 0.0;
+        G[e] = i < DIM ? g[i * M + j] / gs : 0.0;
+    }
+    __syncwarp(mask);
     double nrm = 0.0;
-    for (int j = 0; j < K; ++j) {
-        double cs = 0.0;
-        for (int i = 0; i < K; ++i) cs += fabs(Z[i][j]);
-        nrm = fmax(nrm, cs);
+    for (int c = 0; c < M; ++c) {
+        double cx = 0.0, cg = 0.0;
+        for (int r = 0; r < M; ++r) {
+            cx += fabs(X[r * M + c]);
+            cg += fabs(G[r * M + c]);
+        }
+        nrm = fmax(nrm, cx + cg);
     }
     int sq = 0;
     while (nrm > 0.5 && sq < 60) {
@@ -302,276 +556,56 @@ __device__ void expm_small(double (&Z)[K][K], double (&E)[K][K])
         ++sq;
     }
     const double sc = ldexp(1.0, -sq);
-    double Tm[K][K], W[K][K];
-    for (int i = 0; i < K; ++i)
-        for (int j = 0; j < K; ++j) {
-            Z[i][j] *= sc;
-            Tm[i][j] = E[i][j] = (i == j) ? 1.0 : 0.0;
-        }
+    __syncwarp(mask);
+    double p = i == j ? 1.0 : 0.0, q = 0.0;  // the term
+    double sp = p, sum = 0.0;                // the sums
+    if (on) {
+        X[e] *= sc;
+        G[e] *= sc;
+        P[e] = p;
+        Q[e] = q;
+    }
+    __syncwarp(mask);
     for (int k = 1; k <= 18; ++k) {
         const double inv = 1.0 / (double)k;
-        for (int i = 0; i < K; ++i)
-            for (int j = 0; j < K; ++j) {
-                double s2 = 0.0;
-                for (int m = 0; m < K; ++m) s2 += Tm[i][m] * Z[m][j];
-                W[i][j] = s2 * inv;
+        p = q = 0.0;
+        if (on) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) {
+                p = fma(P[i * M + m], X[m * M + j], p);
+                q = fma(Q[i * M + m], X[m * M + j], fma(P[i * M + m], G[m * M + j], q));
             }
-        for (int i = 0; i < K; ++i)
-            for (int j = 0; j < K; ++j) {
-                Tm[i][j] = W[i][j];
-                E[i][j] += W[i][j];
-            }
+            p *= inv;
+            q *= inv;
+            sp += p;
+            sum += q;
+        }
+        __syncwarp(mask);
+        if (on) {
+            P[e] = p;
+            Q[e] = q;
+        }
+        __syncwarp(mask);
     }
     for (int r = 0; r < sq; ++r) {
-        for (int i = 0; i < K; ++i)
-            for (int j = 0; j < K; ++j) {
-                double s2 = 0.0;
-                for (int m = 0; m < K; ++m) s2 += E[i][m] * E[m][j];
-                W[i][j] = s2;
-            }
-        for (int i = 0; i < K; ++i)
-            for (int j = 0; j < K; ++j) E[i][j] = W[i][j];
-    }
-}
-
-// gA[c] += dt L(X^T, G_c) for every (instance, cell) c, X = dt [A_c; 0]
-// (homogeneous, last row zero) and G_c = [gT_c; 0].  L is linear in G, so G
-// is scaled to max |entry| 1 before the exponential and the block scaled
-// back, which keeps the squaring count set by X.
-template <int DIM>
-__global__ void k_frechet_adjoint(const double *A, const double *gT, double *gA, int total, double dt)
-{
-    constexpr int M = DIM + 1, K = 2 * M, NE = DIM * M;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-        const double *a = A + (size_t)idx * NE;
-        const double *g = gT + (size_t)idx * NE;
-        double gs = 0.0;
-        for (int e = 0; e < NE; ++e) gs = fmax(gs, fabs(g[e]));
-        if (!(gs > 0.0)) continue;  // no closed-form step in this cell
-        double Z[K][K], E[K][K];
-        for (int i = 0; i < K; ++i)
-            for (int j = 0; j < K; ++j) Z[i][j] = 0.0;
-        for (int i = 0; i < DIM; ++i)
-            for (int j = 0; j < M; ++j) {
-                const double x = dt * a[i * M + j];  // X[i][j]
-                Z[j][i] = x;                         // X^T, top left
-                Z[M + j][M + i] = x;                 // X^T, bottom right
-                Z[i][M + j] = g[i * M + j] / gs;     // G, top right
-            }
-        expm_small<K>(Z, E);
-        for (int i = 0; i < DIM; ++i)
-            for (int j = 0; j < M; ++j) gA[(size_t)idx * NE + i * M + j] += dt * gs * E[i][M + j];
-    }
-}
-
-// ------------------------------------------------------------ FP32 adjoint of calc_T
-//
-// The FP32 forward (k_integrate<float>, SCHEME_REF) keeps each coordinate as
-// a compensated pair hi + lo and moves it by x + M[x; 1] with the cell's
-// float T - I (closed-form step) or S - I (one midpoint sub-step, S the
-// sub-step's affine map).  k_grad_ref_f32 replays exactly that arithmetic
-// (checkpoints hold hi and lo) and goes backwards through
-//     x' = x + M_c [x; 1]:   dM_c += g [x; 1]^T,  g = g + M_lin^T g,
-// with dM summed per cell for T (gT) and for S (gS).  Per instance and cell,
-// dLoss/dA then follows in FP64 from gT through the expm Frechet adjoint and
-// from gS through the derivative of S - I = [hL + h^2/2 L^2 | hb + h^2/2 Lb]
-// (k_substep_map_adjoint).
-
-template <int NE>
-__device__ __forceinline__ void acc_switch_f(double *sG, float *acc, int &acc_cell, int c)
-{
-    if (c == acc_cell) return;
-    if (acc_cell >= 0) {
-#pragma unroll
-        for (int e = 0; e < NE; ++e) {
-            atomicAdd(sG + acc_cell * NE + e, (double)acc[e]);
-            acc[e] = 0.0f;
+        if (on) {
+            P2[e] = sp;
+            Q2[e] = sum;
         }
-    }
-    acc_cell = c;
-}
-
-// The float tables of one instance in shared memory, column-major: S - I and
-// T - I, h the sub-step length.
-template <int DIM>
-__device__ __forceinline__ void stage_tables_f32(const double *gA, const double *gT, int nC, double h, float *sS,
-                                                 float *sT)
-{
-    constexpr int NE = DIM * (DIM + 1);
-#pragma unroll 1
-    for (int i = threadIdx.x; i < nC * NE; i += blockDim.x) {
-        const int c = i / NE, e = i - c * NE, r = e / (DIM + 1), col = e - r * (DIM + 1);
-        const int cm = col * DIM + r;
-        // (S - I)[r][col] = h (A[r][col] + h/2 sum_k L[r][k] A[k][col])
-        const double *a = gA + (size_t)c * NE;
-        double l2 = 0.0;
-#pragma unroll 1
-        for (int k = 0; k < DIM; ++k) l2 += a[r * (DIM + 1) + k] * a[k * (DIM + 1) + col];
-        sS[c * NE + cm] = (float)(h * (a[r * (DIM + 1) + col] + 0.5 * h * l2));
-        sT[c * NE + cm] = (float)(gT[i] - (r == col ? 1.0 : 0.0));
-    }
-}
-
-// x' = x + M[x; 1] on the compensated state
-template <int DIM>
-__device__ __forceinline__ void f32_map(PState<DIM, float> &st, const float *M)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    float m[NE], d[DIM];
-    load_cell<DIM>(M, m);
-    cm_affine<DIM>(d, m, st.x);
+        __syncwarp(mask);
+        p = q = 0.0;
+        if (on) {
 #pragma unroll
-    for (int r = 0; r < DIM; ++r) st.add(r, d[r]);
-}
-
-// One time step of calc_T in FP32 from st; returns whether the closed-form step was kept.
-template <int DIM, int TESS>
-__device__ __forceinline__ bool ref_step_f32(const Tess &t, const float *sS, const float *sT, PState<DIM, float> &st,
-                                             int nODE)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    const int c = fast_cell<DIM, TESS>(t, st.x);
-    PState<DIM, float> q = st;
-    f32_map<DIM>(q, sT + c * NE);
-    if (fast_cell<DIM, TESS>(t, q.x) == c) {
-        st = q;
-        return true;
-    }
-    for (int k = 0; k < nODE; ++k) f32_map<DIM>(st, sS + fast_cell<DIM, TESS>(t, st.x) * NE);
-    return false;
-}
-
-// Backwards through x' = x + M[x; 1] (M column-major float, cell c): accumulate
-// g [x; 1]^T into acc (row-major, as the FP64 tables) and set g += M_lin^T g.
-template <int DIM>
-__device__ __forceinline__ void f32_map_adjoint(const float *M, const float *x, float *g, float *acc)
-{
-    constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
-    float m[NE];
-    load_cell<DIM>(M, m);
-#pragma unroll
-    for (int r = 0; r < DIM; ++r) {
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) acc[r * NH + k] = fmaf(g[r], x[k], acc[r * NH + k]);
-        acc[r * NH + DIM] += g[r];
-    }
-    float gn[DIM];
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) {
-        float s2 = g[k];
-#pragma unroll
-        for (int r = 0; r < DIM; ++r) s2 = fmaf(m[k * DIM + r], g[r], s2);
-        gn[k] = s2;
-    }
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) g[k] = gn[k];
-}
-
-// Backwards through the nODE sub-steps of a fallback step starting at st
-// (consumed): one forward pass keeps every sub-step's point and cell in a
-// per-thread array (nODE <= 256, at most 4 KB of local memory, touched only
-// by fallback steps), then the adjoint runs down it.
-template <int DIM, int TESS>
-__device__ __forceinline__ void adjoint_substeps_f32(const Tess &t, const float *sS, double *sGS,
-                                                     PState<DIM, float> &st, float *g, int nODE, float *acc,
-                                                     int &acc_cell)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    float xs[kMaxSubsteps][DIM];
-    int cs[kMaxSubsteps];
-    for (int k = 0; k < nODE; ++k) {
-        const int c = fast_cell<DIM, TESS>(t, st.x);
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) xs[k][i] = st.x[i];
-        cs[k] = c;
-        f32_map<DIM>(st, sS + c * NE);
-    }
-    for (int k = nODE - 1; k >= 0; --k) {
-        const int c = cs[k];
-        acc_switch_f<NE>(sGS, acc, acc_cell, c);
-        f32_map_adjoint<DIM>(sS + c * NE, xs[k], g, acc);
-    }
-}
-
-template <int DIM, int TESS, bool SACC>
-__global__ void __launch_bounds__(128) k_grad_ref_f32(GradArgs a)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int tab = a.t.nC * NE;
-    const int inst = blockIdx.y;
-    double *sums = reinterpret_cast<double *>(smem_raw);
-    double *sGS = SACC ? sums : a.gS + (size_t)inst * tab;        // dLoss/dS (sub-steps)
-    double *sGT = SACC ? sums + tab : a.gT + (size_t)inst * tab;  // dLoss/dT (closed-form steps)
-    float *sS = reinterpret_cast<float *>(sums + (SACC ? 2 * tab : 0));
-    float *sT = sS + tab;
-    stage_tables_f32<DIM>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t.nC, a.h_sub, sS, sT);
-    if (SACC)
-        for (int i = threadIdx.x; i < 2 * tab; i += blockDim.x) sums[i] = 0.0;
-    __syncthreads();
-    const int nT = a.nTimeSteps, nODE = a.nStepsODE, ck = a.ck;
-    const int64_t n = a.n_per_inst;
-    const int64_t total = n * a.N;
-    float *ckpt = reinterpret_cast<float *>(a.ckpt);  // [ceil(nT/ck), N*n, 2*DIM]: hi, lo
-    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t gi = (int64_t)inst * n + j;
-        float p[DIM];
-        load_pt<DIM, float>(a.pts, gi, p);
-        PState<DIM, float> st;
-        st.set(p);
-        for (int s = 0; s < nT; ++s) {
-            if (s % ck == 0) {
-                float *c = ckpt + ((int64_t)(s / ck) * total + gi) * 2 * DIM;
-#pragma unroll
-                for (int i = 0; i < DIM; ++i) {
-                    c[i] = st.hi[i];
-                    c[DIM + i] = st.lo[i];
-                }
-            }
-            ref_step_f32<DIM, TESS>(a.t, sS, sT, st, nODE);
-        }
-        if (a.out) {
-            st.get(p);
-            store_pt<DIM, float>(a.out, gi, p);
-        }
-        float g[DIM];
-        load_pt<DIM, float>(a.grad_out, gi, g);
-        float accS[NE], accT[NE];
-#pragma unroll
-        for (int e = 0; e < NE; ++e) accS[e] = accT[e] = 0.0f;
-        int cellS = -1, cellT = -1;
-        for (int s = nT - 1; s >= 0; --s) {
-            PState<DIM, float> q;
-            const float *c = ckpt + ((int64_t)(s / ck) * total + gi) * 2 * DIM;
-#pragma unroll
-            for (int i = 0; i < DIM; ++i) {
-                q.hi[i] = c[i];
-                q.lo[i] = c[DIM + i];
-                q.x[i] = q.hi[i] + q.lo[i];
-            }
-            for (int r = 0; r < s % ck; ++r) ref_step_f32<DIM, TESS>(a.t, sS, sT, q, nODE);
-            // time step s from q, along the forward's branch
-            const int cc = fast_cell<DIM, TESS>(a.t, q.x);
-            PState<DIM, float> y = q;
-            f32_map<DIM>(y, sT + cc * NE);
-            if (fast_cell<DIM, TESS>(a.t, y.x) == cc) {
-                acc_switch_f<NE>(sGT, accT, cellT, cc);
-                f32_map_adjoint<DIM>(sT + cc * NE, q.x, g, accT);
-            } else {
-                adjoint_substeps_f32<DIM, TESS>(a.t, sS, sGS, q, g, nODE, accS, cellS);
+            for (int m = 0; m < M; ++m) {
+                p = fma(P2[i * M + m], P2[m * M + j], p);
+                q = fma(P2[i * M + m], Q2[m * M + j], fma(Q2[i * M + m], P2[m * M + j], q));
             }
         }
-        acc_switch_f<NE>(sGS, accS, cellS, -1);
-        acc_switch_f<NE>(sGT, accT, cellT, -1);
-        if (a.grad_in) store_pt<DIM, float>(a.grad_in, gi, g);
+        sp = p;
+        sum = q;
+        __syncwarp(mask);
     }
-    if (!SACC) return;
-    __syncthreads();
-    for (int i = threadIdx.x; i < tab; i += blockDim.x) {
-        const double vs = sGS[i], vt = sGT[i];
-        if (vs != 0.0) atomicAdd(a.gS + (size_t)inst * tab + i, vs);
-        if (vt != 0.0) atomicAdd(a.gT + (size_t)inst * tab + i, vt);
-    }
+    if (on && i < DIM) gA[(size_t)idx * NE + i * M + j] += dt * gs * sum;
 }
 
 // gA[c] += dLoss/dA through S - I = [hL + h^2/2 L^2 | hb + h^2/2 Lb] (A = [L | b]):
@@ -600,16 +634,27 @@ __global__ void k_substep_map_adjoint(const double *A, const double *gS, double 
     }
 }
 
-// out[n, j] = scale * sum_k B[k, j] * G[n, k]  (dLoss/dtheta = B^T dLoss/dA)
-__global__ void k_bt_times(const double *B, const double *G, double *out, int DA, int d, int N, double scale)
+// out[n, j] = scale * sum_k B[k, j] * G[n, k]  (dLoss/dtheta = B^T dLoss/dA).
+// A CTA takes 32 columns of one instance, its 16 warps a strided share of the
+// rows each, added in warp order: one thread per column ran D_A dependent
+// loads deep (D_A = 3840, 8 x 225 columns: 0.3 ms, this 0.02).
+constexpr int kBtWarps = 16;
+__global__ void __launch_bounds__(32 * kBtWarps) k_bt_times(const double *B, const double *G, double *out, int DA, int d,
+                                                             double scale)
 {
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < (int64_t)N * d;
-         g += (int64_t)gridDim.x * blockDim.x) {
-        const int n = (int)(g / d), j = (int)(g - (int64_t)n * d);
-        const double *Gn = G + (int64_t)n * DA;
-        double s = 0.0;
-        for (int k = 0; k < DA; ++k) s = fma(B[(int64_t)k * d + j], Gn[k], s);
-        out[g] = scale * s;
+    __shared__ double part[kBtWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+    const double *Gn = G + (int64_t)blockIdx.y * DA;
+    double s = 0.0;
+    if (j < d)
+        for (int k = w; k < DA; k += kBtWarps) s = fma(B[(int64_t)k * d + j], Gn[k], s);
+    part[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && j < d) {
+        s = 0.0;
+#pragma unroll
+        for (int k = 0; k < kBtWarps; ++k) s += part[k][lane];
+        out[(int64_t)blockIdx.y * d + j] = scale * s;
     }
 }
 
@@ -632,71 +677,44 @@ static cudaError_t launch_grad_t(const GradArgs &a, cudaStream_t s)
     return cudaGetLastError();
 }
 
-template <int DIM, int TESS>
+template <int DIM, int TESS, typename Real>
 static cudaError_t launch_grad_ref_t(const GradArgs &a, cudaStream_t s)
 {
-    constexpr int NE = DIM * (DIM + 1);
-    // gradient sums in shared memory only while all four arrays stay within 48 KB
-    const bool sacc = (size_t)4 * a.t.nC * NE * sizeof(double) <= 48 * 1024;
-    size_t smem = (size_t)(sacc ? 4 : 2) * a.t.nC * NE * sizeof(double);
-    auto kern = sacc ? k_grad_ref<DIM, TESS, true> : k_grad_ref<DIM, TESS, false>;
+    const size_t smem = jump_bytes(a.jump, DIM, a.t.nC, sizeof(Real));
+    auto kern = k_grad_ref<DIM, TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    int64_t bx = (a.n_per_inst + 127) / 128;
-    int64_t cap = (int64_t)num_sms() * 8 / (a.N > 0 ? a.N : 1) + 1;
+    LaunchCfg cfg;
+    cfg.block = a.n_per_inst * a.N >= (int64_t)num_sms() * 512 ? 256 : 64;
+    // one wave: a CTA over it would run alone after all others
+    int64_t bx = (a.n_per_inst + cfg.block - 1) / cfg.block;
+    const int64_t cap = std::max<int64_t>(1, persistent_grid(kern, cfg, smem) / a.N);
     if (bx > cap) bx = cap;
-    if (bx < 1) bx = 1;
     dim3 grid((unsigned)bx, (unsigned)a.N);
-    kern<<<grid, 128, smem, s>>>(a);
+    kern<<<grid, cfg.block, smem, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int total = a.N * a.t.nC;
-    k_frechet_adjoint<DIM><<<(total + 63) / 64, 64, 0, s>>>(a.A, a.gT, a.gA, total, a.dt);
-    return cudaGetLastError();
-}
-
-template <int DIM, int TESS>
-static cudaError_t launch_grad_ref_f32_t(const GradArgs &a, cudaStream_t s)
-{
-    constexpr int NE = DIM * (DIM + 1);
-    const size_t tables = (size_t)2 * a.t.nC * NE * sizeof(float), sums = (size_t)2 * a.t.nC * NE * sizeof(double);
-    const bool sacc = tables + sums <= 48 * 1024;
-    const size_t smem = tables + (sacc ? sums : 0);
-    auto kern = sacc ? k_grad_ref_f32<DIM, TESS, true> : k_grad_ref_f32<DIM, TESS, false>;
-    if (smem > kSmemOptInAbove) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    int64_t bx = (a.n_per_inst + 127) / 128;
-    int64_t cap = (int64_t)num_sms() * 8 / (a.N > 0 ? a.N : 1) + 1;
-    if (bx > cap) bx = cap;
-    if (bx < 1) bx = 1;
-    dim3 grid((unsigned)bx, (unsigned)a.N);
-    kern<<<grid, 128, smem, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const int total = a.N * a.t.nC;
-    k_frechet_adjoint<DIM><<<(total + 63) / 64, 64, 0, s>>>(a.A, a.gT, a.gA, total, a.dt);
+    k_level_sums<DIM, TESS><<<(2 * total + 63) / 64, 64, 0, s>>>(a);
+    k_frechet_adjoint<DIM><<<(total + 7) / 8, 128, 0, s>>>(a.A, a.gT, a.gA, total, a.dt);
     k_substep_map_adjoint<DIM><<<(total + 127) / 128, 128, 0, s>>>(a.A, a.gS, a.gA, total, a.h_sub);
     return cudaGetLastError();
 }
 
-cudaError_t launch_grad_ref_f32(const GradArgs &a, cudaStream_t s)
+template <typename Real>
+static cudaError_t launch_grad_ref_r(const GradArgs &a, cudaStream_t s)
 {
     const int dim = a.t.dim, tess = a.t.tess;
-    if (dim == 1) return launch_grad_ref_f32_t<1, 2>(a, s);
-    if (dim == 2) return tess == 1 ? launch_grad_ref_f32_t<2, 1>(a, s) : launch_grad_ref_f32_t<2, 2>(a, s);
-    return tess == 1 ? launch_grad_ref_f32_t<3, 1>(a, s) : launch_grad_ref_f32_t<3, 2>(a, s);
+    if (dim == 1) return launch_grad_ref_t<1, 2, Real>(a, s);
+    if (dim == 2) return tess == 1 ? launch_grad_ref_t<2, 1, Real>(a, s) : launch_grad_ref_t<2, 2, Real>(a, s);
+    return tess == 1 ? launch_grad_ref_t<3, 1, Real>(a, s) : launch_grad_ref_t<3, 2, Real>(a, s);
 }
 
-cudaError_t launch_grad_ref(const GradArgs &a, cudaStream_t s)
+cudaError_t launch_grad_ref(const GradArgs &a, int prec, cudaStream_t s)
 {
-    const int dim = a.t.dim, tess = a.t.tess;
-    if (dim == 1) return launch_grad_ref_t<1, 2>(a, s);
-    if (dim == 2) return tess == 1 ? launch_grad_ref_t<2, 1>(a, s) : launch_grad_ref_t<2, 2>(a, s);
-    return tess == 1 ? launch_grad_ref_t<3, 1>(a, s) : launch_grad_ref_t<3, 2>(a, s);
+    return prec == PREC_F64 ? launch_grad_ref_r<double>(a, s) : launch_grad_ref_r<float>(a, s);
 }
 
 cudaError_t launch_grad_simple(const GradArgs &a, cudaStream_t s)
@@ -710,11 +728,8 @@ cudaError_t launch_grad_simple(const GradArgs &a, cudaStream_t s)
 cudaError_t launch_bt_times(const double *B, const double *G, double *out, int DA, int d, int N, double scale,
                             cudaStream_t s)
 {
-    int64_t n = (int64_t)N * d;
-    int grid = (int)((n + 127) / 128);
-    if (grid < 1) grid = 1;
-    if (grid > num_sms() * 16) grid = num_sms() * 16;
-    k_bt_times<<<grid, 128, 0, s>>>(B, G, out, DA, d, N, scale);
+    // N <= 65535 (checked by the caller)
+    k_bt_times<<<dim3((unsigned)((d + 31) / 32), (unsigned)N), 32 * kBtWarps, 0, s>>>(B, G, out, DA, d, scale);
     return cudaGetLastError();
 }
 

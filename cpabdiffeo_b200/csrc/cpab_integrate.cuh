@@ -52,44 +52,6 @@ struct PState<DIM, double> {
 };
 
 template <int DIM>
-struct PState<DIM, float> {
-    float hi[DIM], lo[DIM], x[DIM];
-    __device__ __forceinline__ void set(const float *v)
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) { hi[i] = v[i]; lo[i] = 0.0f; x[i] = v[i]; }
-    }
-    __device__ __forceinline__ void set(const double *v)
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) {
-            hi[i] = (float)v[i];
-            lo[i] = (float)(v[i] - (double)hi[i]);
-            x[i] = hi[i] + lo[i];
-        }
-    }
-    __device__ __forceinline__ void get(float *v) const
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) v[i] = x[i];
-    }
-    __device__ __forceinline__ void get(double *v) const
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) v[i] = (double)hi[i] + (double)lo[i];
-    }
-    __device__ __forceinline__ const float *lookup() const { return x; }
-    // hi + lo += d
-    __device__ __forceinline__ void add(int i, float d)
-    {
-        const float s = hi[i] + d;
-        lo[i] += d - (s - hi[i]);
-        hi[i] = s;
-        x[i] = s + lo[i];
-    }
-};
-
-template <int DIM>
 __device__ void stage_exact_substeps(const double *gA, const double *gT, int nC, double h, double *sS, double *sT);
 
 // Stage one instance's double tables in shared memory (layout above).  EXACT
@@ -137,28 +99,10 @@ __device__ __forceinline__ void load_cell(const float *p, float *m)
     }
 }
 
-// y = M [x; 1] for a column-major cell matrix held in registers
-template <int DIM>
-__device__ __forceinline__ void cm_affine(float *y, const float *m, const float *x)
-{
-#pragma unroll
-    for (int r = 0; r < DIM; ++r) {
-        float acc = m[DIM * DIM + r];
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) acc = fmaf(m[k * DIM + r], x[k], acc);
-        y[r] = acc;
-    }
-}
-
 template <int DIM, int TESS>
 __device__ __forceinline__ int cell_of(const Tess &t, const PState<DIM, double> &s)
 {
     return exact_cell<DIM, TESS>(t, s.p);
-}
-template <int DIM, int TESS>
-__device__ __forceinline__ int cell_of(const Tess &t, const PState<DIM, float> &s)
-{
-    return fast_cell<DIM, TESS>(t, s.x);
 }
 
 // One unit of work on a point in cell c: the candidate end point q of a
@@ -182,19 +126,6 @@ __device__ __forceinline__ void advance(bool fast, const PState<DIM, double> &s,
 // instruction, each rounded as its scalar twin) for the (x, y) coordinates:
 // the column-major cell matrix gives column k as the pair (M[0][k], M[1][k]).
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-
-// hi + lo += d for coordinates 0 and 1 at once (PState::add, twice)
-template <int DIM>
-__device__ __forceinline__ void add_pair(PState<DIM, float> &q, float2 d)
-{
-    const float2 hi = make_float2(q.hi[0], q.hi[1]), lo = make_float2(q.lo[0], q.lo[1]);
-    const float2 sm = __fadd2_rn(hi, d);
-    const float2 l2 = __fadd2_rn(lo, __fadd2_rn(d, neg2(__fadd2_rn(sm, neg2(hi)))));
-    const float2 x = __fadd2_rn(sm, l2);
-    q.hi[0] = sm.x; q.hi[1] = sm.y;
-    q.lo[0] = l2.x; q.lo[1] = l2.y;
-    q.x[0] = x.x; q.x[1] = x.y;
-}
 
 // ------------------------------------------------------------ exact scheme (2D/3D)
 //

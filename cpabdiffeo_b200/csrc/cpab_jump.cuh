@@ -65,10 +65,10 @@ constexpr int kJumpCtas = DIM == 3 ? 2 : 4;
 
 // Shared memory of the tables: the maps (increments M - I, column-major),
 // then kappa of every level above 0.
-__host__ __device__ inline size_t jump_bytes(const JumpCfg &j, int dim, int nC)
+__host__ __device__ inline size_t jump_bytes(const JumpCfg &j, int dim, int nC, size_t el = sizeof(float))
 {
     const size_t kap = (size_t)(j.nT > 0 ? j.nT - 1 : 0) + j.nS;  // one row to spare: level 0 reads a row too
-    const size_t b = ((size_t)(j.nT + j.nS) * dim * (dim + 1) + kap) * nC * sizeof(float);
+    const size_t b = ((size_t)(j.nT + j.nS) * dim * (dim + 1) + kap) * nC * el;
     return (b + 15) & ~(size_t)15;
 }
 
@@ -78,7 +78,8 @@ __host__ __device__ inline size_t jump_bytes(const JumpCfg &j, int dim, int nC)
 // bytes (what shared memory the kernel's other needs leave) do not hold the
 // choice.  The choice depends on the space and the step counts, not on the
 // batch, so results do not either.
-inline JumpCfg jump_cfg(int dim, int nC, int nTimeSteps, int nStepsODE, int scheme, size_t avail)
+inline JumpCfg jump_cfg(int dim, int nC, int nTimeSteps, int nStepsODE, int scheme, size_t avail,
+                        size_t el = sizeof(float), int r_least = 1)
 {
     auto log2i = [](long long v) {
         int k = 0;
@@ -92,33 +93,71 @@ inline JumpCfg jump_cfg(int dim, int nC, int nTimeSteps, int nStepsODE, int sche
     int ls = log2i(scheme == SCHEME_SIMPLE ? (long long)nTimeSteps * nStepsODE : nStepsODE);
     if (ls > 8) ls = 8;
     JumpCfg j{0, 0, 0, 0};
-    for (int r : {1, 2, 3, 4, 31}) {
+    for (int r : {1, 2, 3, 4, 5, 6, 31}) {
+        if (r < r_least) continue;
         j.r = r;
         j.mul = (32 + r - 1) / r;
         j.nT = scheme == SCHEME_SIMPLE ? 0 : (lt > 8 ? 8 : lt) / r + 1;
         j.nS = ls / r + 1;
-        const size_t b = jump_bytes(j, dim, nC), budget = (size_t)(r == 1 ? 40 : r == 2 ? 64 : 112) * 1024;
+        const size_t b = jump_bytes(j, dim, nC, el), budget = (size_t)(r == 1 ? 40 : r == 2 ? 64 : 112) * 1024;
         if (r == 31 || (b <= budget && b <= avail)) break;
     }
     return j;
 }
 
+template <typename Real>
 struct JumpTables {
-    const float *map;  // [nT + nS][nC][DIM * (DIM + 1)]
-    const float *kap;  // [nT - 1 + nS - 1][nC]
+    const Real *map;  // [nT + nS][nC][DIM * (DIM + 1)]
+    const Real *kap;  // [nT - 1 + nS - 1][nC]
 };
+
+// 2 D + D_lin D: the increment of a map applied twice.
+template <int DIM>
+__device__ __forceinline__ void twice(double *D)
+{
+    constexpr int NH = DIM + 1, NE = DIM * NH;
+    double D2[NE];
+#pragma unroll
+    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+        for (int col = 0; col < NH; ++col) {
+            double s = 2.0 * D[r * NH + col];
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) s = fma(D[r * NH + k], D[k * NH + col], s);
+            D2[r * NH + col] = s;
+        }
+#pragma unroll
+    for (int e = 0; e < NE; ++e) D[e] = D2[e];
+}
+
+// The midpoint map's increment h A + h^2/2 L A  (A = [L | b]).
+template <int DIM>
+__device__ __forceinline__ void midpoint_increment(const double *a, double h, double *D)
+{
+    constexpr int NH = DIM + 1;
+#pragma unroll
+    for (int r = 0; r < DIM; ++r)
+#pragma unroll
+        for (int col = 0; col < NH; ++col) {
+            double l2 = 0.0;
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) l2 += a[r * NH + k] * a[k * NH + col];
+            D[r * NH + col] = h * (a[r * NH + col] + 0.5 * h * l2);
+        }
+}
 
 // Stage one instance's tables from its signed A and Trel: one thread per
 // (map, cell) squares the increment D = M - I upwards in FP64,
 // (I + D)^2 - I = 2 D + D_lin D.
-template <int DIM, int TESS>
-__device__ __forceinline__ JumpTables stage_jump(const double *gA, const double *gT, const Tess &t, const JumpCfg &jc,
-                                                 double dt, double h, bool exact_sub, unsigned char *smem)
+template <int DIM, int TESS, typename Real = float>
+__device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const double *gT, const Tess &t,
+                                                       const JumpCfg &jc, double dt, double h, bool exact_sub,
+                                                       unsigned char *smem)
 {
     constexpr int NH = DIM + 1, NE = DIM * NH;
     const int nC = t.nC;
-    float *map = reinterpret_cast<float *>(smem);
-    float *kap = map + (size_t)(jc.nT + jc.nS) * nC * NE;
+    Real *map = reinterpret_cast<Real *>(smem);
+    Real *kap = map + (size_t)(jc.nT + jc.nS) * nC * NE;
     const int kinds = jc.nT > 0 ? 2 : 1;
 #pragma unroll 1
     for (int i = threadIdx.x; i < kinds * nC; i += blockDim.x) {
@@ -131,16 +170,7 @@ __device__ __forceinline__ JumpTables stage_jump(const double *gA, const double 
 #pragma unroll
             for (int e = 0; e < NE; ++e) D[e] = gT[(size_t)c * NE + e] - (e % NH == e / NH ? 1.0 : 0.0);
         } else if (!exact_sub) {
-            // midpoint map: h A + h^2/2 L A
-#pragma unroll
-            for (int r = 0; r < DIM; ++r)
-#pragma unroll
-                for (int col = 0; col < NH; ++col) {
-                    double l2 = 0.0;
-#pragma unroll
-                    for (int k = 0; k < DIM; ++k) l2 += a[r * NH + k] * a[k * NH + col];
-                    D[r * NH + col] = h * (a[r * NH + col] + 0.5 * h * l2);
-                }
+            midpoint_increment<DIM>(a, h, D);
         } else {
             // expm(h A) - I by its Taylor sum, to the sum's rounding
             double w[NE];
@@ -189,16 +219,16 @@ __device__ __forceinline__ JumpTables stage_jump(const double *gA, const double 
         const int kap0 = sub ? (jc.nT > 0 ? jc.nT - 1 : 0) : 0;
 #pragma unroll 1
         for (int l = 0; l < levels; ++l) {
-            float *m = map + ((size_t)(row0 + l) * nC + c) * NE;
+            Real *m = map + ((size_t)(row0 + l) * nC + c) * NE;
 #pragma unroll
             for (int r = 0; r < DIM; ++r) {
                 double off = D[r * NH + DIM];  // the displacement of the box's centre
 #pragma unroll
                 for (int col = 0; col < DIM; ++col) {
-                    m[col * DIM + r] = (float)(D[r * NH + col] * t.inc[col] * t.inv_inc[r]);
+                    m[col * DIM + r] = (Real)(D[r * NH + col] * t.inc[col] * t.inv_inc[r]);
                     off = fma(D[r * NH + col], ctr[col], off);
                 }
-                m[DIM * DIM + r] = (float)(off * t.inv_inc[r]);
+                m[DIM * DIM + r] = (Real)(off * t.inv_inc[r]);
             }
             if (l > 0) {
                 const float x = (float)(rho * tau), em = expm1f(x), room = 2.0f - em / x;
@@ -208,24 +238,13 @@ __device__ __forceinline__ JumpTables stage_jump(const double *gA, const double 
             if (l + 1 < levels) {
 #pragma unroll 1
                 for (int q = 0; q < jc.r; ++q) {
-                    double D2[NE];
-#pragma unroll
-                    for (int r = 0; r < DIM; ++r)
-#pragma unroll
-                        for (int col = 0; col < NH; ++col) {
-                            double s = 2.0 * D[r * NH + col];
-#pragma unroll
-                            for (int k = 0; k < DIM; ++k) s = fma(D[r * NH + k], D[k * NH + col], s);
-                            D2[r * NH + col] = s;
-                        }
-#pragma unroll
-                    for (int e = 0; e < NE; ++e) D[e] = D2[e];
+                    twice<DIM>(D);
                     tau *= 2.0;
                 }
             }
         }
     }
-    return JumpTables{map, kap};
+    return JumpTables<Real>{map, kap};
 }
 
 // ------------------------------------------------------------ walkers
@@ -241,32 +260,49 @@ __device__ __forceinline__ JumpTables stage_jump(const double *gA, const double 
 //   leave(t, q)          moves to q, looking its cell up
 //   where(t, q, x)       absolute position of a candidate
 
-// Position in a box as a compensated pair hi + lo, box units from the centre.
+// Position in a box, box units from the centre: float as a compensated pair
+// hi + lo, double as it is.
+template <int DIM, typename Real>
+struct BoxPos;
 template <int DIM>
-struct BoxPos {
+struct BoxPos<DIM, float> {
     float hi[DIM], lo[DIM];
+    __device__ __forceinline__ float x(int i) const { return hi[i] + lo[i]; }
 };
-
 template <int DIM>
-struct BoxCand {
-    BoxPos<DIM> p;
-    float x[DIM];  // hi + lo
-    float m;
+struct BoxPos<DIM, double> {
+    double hi[DIM];
+    __device__ __forceinline__ double x(int i) const { return hi[i]; }
 };
 
-template <int DIM, int TESS>
+template <int DIM, typename Real>
+struct BoxCand {
+    BoxPos<DIM, Real> p;
+    Real x[DIM];
+    Real m;
+};
+
+// -v where neg (a sign bit flipped, no branch)
+__device__ __forceinline__ float flip(float v, bool neg) { return neg ? -v : v; }
+__device__ __forceinline__ double flip(double v, bool neg) { return neg ? -v : v; }
+__device__ __forceinline__ float least(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ double least(double a, double b) { return fmin(a, b); }
+__device__ __forceinline__ float most(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double most(double a, double b) { return fmax(a, b); }
+
+template <int DIM, int TESS, typename Real>
 struct WalkLocal {
-    BoxPos<DIM> p;
+    BoxPos<DIM, Real> p;
     int c;
-    float m;
+    Real m;
 
     __device__ __forceinline__ void set_local(const Tess &t, const double *x, const int *kb)
     {
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {
             const double r = fma(x[i], t.inv_inc[i], -((double)kb[i] + 0.5));
-            p.hi[i] = (float)r;
-            p.lo[i] = (float)(r - (double)p.hi[i]);
+            p.hi[i] = (Real)r;
+            if constexpr (sizeof(Real) == 4) p.lo[i] = (float)(r - (double)p.hi[i]);
         }
     }
     // float coordinates in float arithmetic: x / inc with the low part of
@@ -285,21 +321,26 @@ struct WalkLocal {
         const int n[3] = {t.nC0, t.nC1, t.nC2};
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {  // NaN -> 0
-            const float u = floorf((float)x[i] * t.finv_inc[i]);
-            kb[i] = (int)fminf(fmaxf(u, 0.0f), (float)(n[i] - 1));
+            const Real u = floor((Real)x[i] * (Real)(sizeof(Real) == 4 ? (double)t.finv_inc[i] : t.inv_inc[i]));
+            kb[i] = (int)least(most(u, Real(0)), Real(n[i] - 1));
         }
     }
-    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM> &q, double *x) const
+    static __device__ __forceinline__ double exact_x(const BoxPos<DIM, float> &q, int i)
+    {
+        return (double)q.hi[i] + (double)q.lo[i];
+    }
+    static __device__ __forceinline__ double exact_x(const BoxPos<DIM, double> &q, int i) { return q.hi[i]; }
+    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM, Real> &q, double *x) const
     {
         int kb[DIM];
         cell_box<DIM, TESS>(t, c, kb);
 #pragma unroll
         for (int i = 0; i < DIM; ++i)
-            x[i] = (((double)kb[i] + 0.5) + ((double)q.hi[i] + (double)q.lo[i])) * t.inc[i];
+            x[i] = (((double)kb[i] + 0.5) + exact_x(q, i)) * t.inc[i];
     }
     // the same rounded to float: the centre (k + 1/2) inc as a float and its
     // rest, and one rounding of the sum
-    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM> &q, float *x) const
+    __device__ __forceinline__ void to_absolute(const Tess &t, const BoxPos<DIM, Real> &q, float *x) const
     {
         int kb[DIM];
         cell_box<DIM, TESS>(t, c, kb);
@@ -315,33 +356,50 @@ struct WalkLocal {
     {
         to_absolute(t, p, x);
     }
-    __device__ __forceinline__ void where(const Tess &t, const BoxCand<DIM> &q, double *x) const
+    __device__ __forceinline__ void where(const Tess &t, const BoxCand<DIM, Real> &q, double *x) const
     {
         to_absolute(t, q.p, x);
     }
-    __device__ __forceinline__ void move(const BoxCand<DIM> &q, bool yes)
+    __device__ __forceinline__ void move(const BoxCand<DIM, Real> &q, bool yes)
     {
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {
             p.hi[i] = yes ? q.p.hi[i] : p.hi[i];
-            p.lo[i] = yes ? q.p.lo[i] : p.lo[i];
+            if constexpr (sizeof(Real) == 4) p.lo[i] = yes ? q.p.lo[i] : p.lo[i];
         }
         m = yes ? q.m : m;
     }
     // the box of a candidate, with its position relative to that box
-    __device__ __forceinline__ void shift_box(const Tess &t, BoxCand<DIM> &q, int *kb) const
+    __device__ __forceinline__ void shift_box(const Tess &t, BoxCand<DIM, Real> &q, int *kb) const
     {
         const int n[3] = {t.nC0, t.nC1, t.nC2};
         cell_box<DIM, TESS>(t, c, kb);
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {
-            const float s = fminf(fmaxf(floorf(q.x[i] + 0.5f), (float)-kb[i]), (float)(n[i] - 1 - kb[i]));
+            const Real s = least(most(floor(q.x[i] + Real(0.5)), Real(-kb[i])), Real(n[i] - 1 - kb[i]));
             kb[i] += (int)s;
             q.p.hi[i] -= s;
-            q.x[i] = q.p.hi[i] + q.p.lo[i];
+            q.x[i] = q.p.x(i);
         }
     }
-    __device__ __forceinline__ float advance(const float *map, BoxCand<DIM> &q) const
+    __device__ __forceinline__ Real advance(const Real *map, BoxCand<DIM, Real> &q) const
+    {
+        if constexpr (sizeof(Real) == 8) {
+            double len = 0.0;
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) {
+                double d = map[DIM * DIM + r];
+#pragma unroll
+                for (int k = 0; k < DIM; ++k) d = fma(map[k * DIM + r], p.hi[k], d);
+                q.x[r] = q.p.hi[r] = p.hi[r] + d;
+                len += fabs(d);
+            }
+            return len;
+        } else {
+            return advance_f(map, q);
+        }
+    }
+    __device__ __forceinline__ float advance_f(const float *map, BoxCand<DIM, float> &q) const
     {
         float mm[DIM * (DIM + 1)];
         load_cell<DIM>(map, mm);
@@ -387,17 +445,17 @@ struct WalkLocal {
 constexpr float kFar = 1e30f;  // distance to a facet on the domain boundary
 
 // Box cells (1D and type II): the box's faces.
-template <int DIM>
-struct WalkBox : WalkLocal<DIM, 2> {
-    using B = WalkLocal<DIM, 2>;
-    using Cand = BoxCand<DIM>;
+template <int DIM, typename Real>
+struct WalkBox : WalkLocal<DIM, 2, Real> {
+    using B = WalkLocal<DIM, 2, Real>;
+    using Cand = BoxCand<DIM, Real>;
     float flo[DIM], fhi[DIM];  // 1/2, or kFar where the domain ends
 
-    __device__ __forceinline__ float margin(const float *x) const
+    __device__ __forceinline__ Real margin(const Real *x) const
     {
-        float v = fminf(flo[0] + x[0], fhi[0] - x[0]);
+        Real v = least(flo[0] + x[0], fhi[0] - x[0]);
 #pragma unroll
-        for (int i = 1; i < DIM; ++i) v = fminf(v, fminf(flo[i] + x[i], fhi[i] - x[i]));
+        for (int i = 1; i < DIM; ++i) v = least(v, least(flo[i] + x[i], fhi[i] - x[i]));
         return v;
     }
     __device__ __forceinline__ void enter(const Tess &t, const int *kb)
@@ -417,12 +475,12 @@ struct WalkBox : WalkLocal<DIM, 2> {
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
     {
         int kb[DIM];
-        float r[DIM];
+        Real r[DIM];
         B::box_of(t, x, kb);
         B::set_local(t, x, kb);
         enter(t, kb);
 #pragma unroll
-        for (int i = 0; i < DIM; ++i) r[i] = B::p.hi[i] + B::p.lo[i];
+        for (int i = 0; i < DIM; ++i) r[i] = B::p.x(i);
         B::m = margin(r);
     }
     template <typename Elem>
@@ -432,11 +490,11 @@ struct WalkBox : WalkLocal<DIM, 2> {
         cell_box<DIM, 2>(t, cell, kb);
         B::set_local(t, x, kb);
         enter(t, kb);
-        B::m = 0.0f;
+        B::m = 0;
     }
-    __device__ __forceinline__ float step(const Tess &, const float *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
-        const float len = B::advance(map, q);
+        const Real len = B::advance(map, q);
         q.m = margin(q.x);
         return len;
     }
@@ -457,27 +515,31 @@ struct WalkBox : WalkLocal<DIM, 2> {
 // reference's rules (calc_2Dto2D.cu:53-148) continue it: beyond its side over
 // the side's width (|u| <= 1/2), and beyond a corner of the domain up to the
 // box's diagonal continued (|u| <= v).
-struct WalkTri : WalkLocal<2, 1> {
-    using B = WalkLocal<2, 1>;
-    using Cand = BoxCand<2>;
+template <typename Real>
+struct WalkTri : WalkLocal<2, 1, Real> {
+    using B = WalkLocal<2, 1, Real>;
+    using Cand = BoxCand<2, Real>;
+    using B::c;
+    using B::m;
+    using B::p;
     bool along_x;      // v is the y coordinate
-    unsigned sv;       // sign bit of v
+    bool neg;          // v points down it
     float side;        // 1/2, or kFar where the side ends the domain
     float ulo, uhi;    // 1/2 where the box's low / high face in u ends the domain, else kFar
 
-    __device__ __forceinline__ float margin(const float *x) const
+    __device__ __forceinline__ Real margin(const Real *x) const
     {
-        const float v = __uint_as_float(__float_as_uint(along_x ? x[1] : x[0]) ^ sv), u = along_x ? x[0] : x[1];
+        const Real v = flip(along_x ? x[1] : x[0], neg), u = along_x ? x[0] : x[1];
         // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
-        const float top = (u > uhi || u < -ulo) ? v : fminf(v, 0.5f);
-        return fminf(top - fabsf(u), side - v);
+        const Real top = (u > uhi || u < -ulo) ? v : least(v, Real(0.5));
+        return least(top - fabs(u), side - v);
     }
     __device__ __forceinline__ void enter(const Tess &t, const int *kb, bool up, bool right)
     {
         const int tri = up ? (right ? 2 : 3) : (right ? 1 : 0);
         c = (kb[0] + kb[1] * t.nC0) * 4 + tri;
         along_x = up == right;
-        sv = right ? 0u : 0x80000000u;
+        neg = !right;
         const int k = along_x ? kb[1] : kb[0], n = along_x ? t.nC1 : t.nC0;
         const int ku = along_x ? kb[0] : kb[1], nu = along_x ? t.nC0 : t.nC1;
         side = k == (right ? n - 1 : 0) ? kFar : 0.5f;
@@ -489,10 +551,10 @@ struct WalkTri : WalkLocal<2, 1> {
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
     {
         int kb[2];
-        box_of(t, x, kb);
-        set_local(t, x, kb);
-        const float r[2] = {p.hi[0] + p.lo[0], p.hi[1] + p.lo[1]};
-        enter(t, kb, r[0] < r[1], r[0] + r[1] > 0.0f);
+        B::box_of(t, x, kb);
+        B::set_local(t, x, kb);
+        const Real r[2] = {p.x(0), p.x(1)};
+        enter(t, kb, r[0] < r[1], r[0] + r[1] > Real(0));
         m = margin(r);
     }
     template <typename Elem>
@@ -500,23 +562,23 @@ struct WalkTri : WalkLocal<2, 1> {
     {
         int kb[2];
         cell_box<2, 1>(t, cell, kb);
-        set_local(t, x, kb);
+        B::set_local(t, x, kb);
         const int tri = cell & 3;
         enter(t, kb, tri >= 2, tri == 1 || tri == 2);
-        m = 0.0f;
+        m = 0;
     }
-    __device__ __forceinline__ float step(const Tess &, const float *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
-        const float len = advance(map, q);
+        const Real len = B::advance(map, q);
         q.m = margin(q.x);
         return len;
     }
-    __device__ __forceinline__ void take(const Cand &q, bool yes) { move(q, yes); }
+    __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
         int kb[2];
-        shift_box(t, q, kb);
-        enter(t, kb, q.x[0] < q.x[1], q.x[0] + q.x[1] > 0.0f);
+        B::shift_box(t, q, kb);
+        enter(t, kb, q.x[0] < q.x[1], q.x[0] + q.x[1] > Real(0));
         p = q.p;
         m = margin(q.x);
     }
@@ -530,30 +592,31 @@ struct WalkTri : WalkLocal<2, 1> {
 // as on its boundary (the reference clamps them, calc_3Dto3D.cu:55-60), hence
 // the clamped y in the sum.  The reference clamps z with the x box size: where
 // the two sizes differ, every candidate is looked up at its absolute position.
-struct WalkTet : WalkLocal<3, 1> {
-    using B = WalkLocal<3, 1>;
-    using Cand = BoxCand<3>;
-    unsigned sg[3];  // sign bits of sigma
+template <typename Real>
+struct WalkTet : WalkLocal<3, 1, Real> {
+    using B = WalkLocal<3, 1, Real>;
+    using Cand = BoxCand<3, Real>;
+    using B::c;
+    using B::m;
+    using B::p;
+    bool neg[3];     // signs of sigma
     float face[3];   // 1/2, or kFar where the face ends the domain (and for the centre)
     float low[3];    // -1/2 where the opposite face ends the domain, else -kFar
     bool centre;
 
-    __device__ __forceinline__ float margin(const float *x) const
+    __device__ __forceinline__ Real margin(const Real *x) const
     {
-        float y[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) y[i] = __uint_as_float(__float_as_uint(x[i]) ^ sg[i]);
-        float sum = -0.5f, far = kFar;
+        Real y[3], sum = Real(-0.5), far = kFar;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            sum += fmaxf(fminf(y[i], 0.5f), low[i]);
-            far = fminf(far, face[i] - y[i]);
+            y[i] = flip(x[i], neg[i]);
+            sum += most(least(y[i], Real(0.5)), Real(low[i]));
+            far = least(far, face[i] - y[i]);
         }
-        const float corner = fminf(sum, far);
         // the four corners' sums: sigma with an even number of signs flipped
-        const float a = y[0] + y[1], d = y[0] - y[1];
-        const float most = fmaxf(fabsf(a) + y[2], fabsf(d) - y[2]);
-        return centre ? 0.5f - most : corner;
+        const Real a = y[0] + y[1], d = y[0] - y[1];
+        const Real all = most(fabs(a) + y[2], fabs(d) - y[2]);
+        return centre ? Real(0.5) - all : least(sum, far);
     }
     __device__ __forceinline__ void enter(const Tess &t, int cell)
     {
@@ -565,31 +628,46 @@ struct WalkTet : WalkLocal<3, 1> {
         const bool odd = ((kb[0] ^ kb[1] ^ kb[2]) & 1) != 0;
         centre = tet == 0;
         // signs in fast_cell_3d_tet's turned coordinates (odd boxes: (x, y) -> (y, -x))
-        const bool n0 = tet == 1 || tet == 3, n1 = tet == 1 || tet == 4, n2 = tet == 3 || tet == 4;
-        const bool neg[3] = {odd ? !n1 : n0, odd ? n0 : n1, n2};
+        const bool n0 = tet == 1 || tet == 3, n1 = tet == 1 || tet == 4;
+        neg[0] = odd ? !n1 : n0;
+        neg[1] = odd ? n0 : n1;
+        neg[2] = tet == 3 || tet == 4;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            sg[i] = neg[i] ? 0x80000000u : 0u;
             face[i] = centre || kb[i] == (neg[i] ? 0 : n[i] - 1) ? kFar : 0.5f;
             low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
         }
     }
-    __device__ __forceinline__ int lookup(const Tess &t, const float *x, float &mq) const
+    static __device__ __forceinline__ int cell_at(const Tess &t, const float *a, float &mq)
     {
-        float a[3];
+        return fast_cell_3d_tet_m(t, a, mq);
+    }
+    static __device__ __forceinline__ int cell_at(const Tess &t, const double *a, double &mq)
+    {
+        float f[3], m32;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) f[i] = (float)a[i];
+        fast_cell_3d_tet_m(t, f, m32);
+        mq = fmax((double)m32 - 1e-6, 0.0);  // a lower bound still, whatever float rounded
+        return exact_cell<3, 1>(t, a);
+    }
+    // the cell of a position relative to the box of c
+    __device__ __forceinline__ int lookup(const Tess &t, const Real *x, Real &mq) const
+    {
+        Real a[3];
         int kb[3];
         cell_box<3, 1>(t, c, kb);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) a[i] = ((float)kb[i] + 0.5f + x[i]) * t.finc[i];
-        return fast_cell_3d_tet_m(t, a, mq);
+        for (int i = 0; i < 3; ++i) a[i] = ((Real)kb[i] + Real(0.5) + x[i]) * (Real)t.inc[i];
+        return cell_at(t, a, mq);
     }
     template <typename Elem>
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
     {
-        float a[3], mq;
+        Real a[3], mq;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) a[i] = (float)x[i];
-        place_in(t, x, fast_cell_3d_tet_m(t, a, mq));
+        for (int i = 0; i < 3; ++i) a[i] = (Real)x[i];
+        place_in(t, x, cell_at(t, a, mq));
         m = mq;
     }
     template <typename Elem>
@@ -598,42 +676,42 @@ struct WalkTet : WalkLocal<3, 1> {
         int kb[3];
         enter(t, cell);
         cell_box<3, 1>(t, cell, kb);
-        set_local(t, x, kb);
-        m = 0.0f;
+        B::set_local(t, x, kb);
+        m = 0;
     }
-    __device__ __forceinline__ float step(const Tess &t, const float *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &t, const Real *map, Cand &q) const
     {
-        const float len = advance(map, q);
+        const Real len = B::advance(map, q);
         if (t.inc[0] == t.inc[2]) {
             q.m = margin(q.x);
         } else if (lookup(t, q.x, q.m) != c) {
-            q.m = -1e-30f;  // outside, nothing known of how far
+            q.m = Real(-1e-30);  // outside, nothing known of how far
         }
         return len;
     }
-    __device__ __forceinline__ void take(const Cand &q, bool yes) { move(q, yes); }
+    __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
         double x[3];
-        float mq;
+        Real mq;
         const int cell = lookup(t, q.x, mq);
-        where(t, q, x);
+        B::where(t, q, x);
         place_in(t, x, cell);
         m = mq;
     }
 };
 
-template <int DIM, int TESS>
+template <int DIM, int TESS, typename Real>
 struct WalkerOf {
-    using type = WalkBox<DIM>;
+    using type = WalkBox<DIM, Real>;
 };
-template <>
-struct WalkerOf<2, 1> {
-    using type = WalkTri;
+template <typename Real>
+struct WalkerOf<2, 1, Real> {
+    using type = WalkTri<Real>;
 };
-template <>
-struct WalkerOf<3, 1> {
-    using type = WalkTet;
+template <typename Real>
+struct WalkerOf<3, 1, Real> {
+    using type = WalkTet<Real>;
 };
 
 // Per-warp queue of points that the first pass left over (entries, shared memory).
@@ -651,12 +729,12 @@ constexpr int kQueue = 64;
 // follow from the number of replaced ones (c_fb).
 template <int DIM, int TESS, int SCHEME, class Src, class Snk>
 __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, const JumpCfg &jc,
-                                               const JumpTables &tab, int64_t ws, int n_range, const Src &src,
+                                               const JumpTables<float> &tab, int64_t ws, int n_range, const Src &src,
                                                Snk &snk, unsigned long long &c_fast, unsigned long long &c_fb,
                                                unsigned long long &c_sub, unsigned long long &c_pts, int *claim,
                                                unsigned short *queues, ExactCross *ex)
 {
-    using Walker = typename WalkerOf<DIM, TESS>::type;
+    using Walker = typename WalkerOf<DIM, TESS, float>::type;
     using Cand = typename Walker::Cand;
     constexpr int NE = DIM * (DIM + 1);
     constexpr float kHuge = 1e30f;

@@ -114,7 +114,7 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
     int loaded = -1;
     const ArraySrc<DIM, Real> src{a.pts_in};
     ArraySnk<DIM, Real> snk{a.pts_out, a.clamp, a.clamp_lo, a.clamp_hi, 0ull};
-    JumpTables jt{nullptr, nullptr};
+    JumpTables<float> jt{nullptr, nullptr};
     ExactCross ex{nullptr, a.facets, a.nbr, a.nF, a.h_sub, a.max_crossings, 0ull, 0ull};
 
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
     Real *sT = sA + a.t.nC * NE;
     // per-landmark terms of the current tile, after the tables (a multiple of 8 bytes)
     constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
-    JumpTables jt{nullptr, nullptr};
+    JumpTables<float> jt{nullptr, nullptr};
     double *s_term = reinterpret_cast<double *>(
         smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     __shared__ unsigned long long s_claim;

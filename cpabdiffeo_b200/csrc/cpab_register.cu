@@ -484,7 +484,7 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 3 : 1) k_register_ll(
     constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
-    JumpTables jt{nullptr, nullptr};
+    JumpTables<float> jt{nullptr, nullptr};
     // the tile's point slots, after the tables (a multiple of 16 bytes), then the 32-point group sums of the
     // likelihood
     double2 *s_pos = reinterpret_cast<double2 *>(

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
     constexpr bool kJump = sizeof(Real) == 4;  // composed-step tables (cpab_jump.cuh)
-    JumpTables jt{nullptr, nullptr};
+    JumpTables<float> jt{nullptr, nullptr};
     double *s_pos = reinterpret_cast<double *>(
         smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     double *s_grp = s_pos + 3 * (size_t)a.tile_px;  // 32-voxel group sums of the likelihood
