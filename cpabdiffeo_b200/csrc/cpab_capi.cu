@@ -314,6 +314,9 @@ static int run_integrate(cpab_ctx *ctx, IntegrateArgs &a, int precision, int sch
                          cudaStream_t s)
 {
     LaunchCfg cfg = ctx->cfg;
+    // from 128 points per SM on (both sides measured at integrate_phases); a ragged launch, whose points are not
+    // known here, counts as large
+    a.phases = a.batch.tile_prefix || (int64_t)a.batch.N * a.batch.n_uniform >= (int64_t)num_sms() * 128;
     // small uniform launches: one CTA per tile (the persistent grid would leave CTAs idle)
     if (uniform_tiles_total > 0 && uniform_tiles_total < (int64_t)num_sms() * 2) cfg.grid = (int)uniform_tiles_total;
     if (cfg.grid > 0 && cfg.max_ctas > 0 && cfg.grid > cfg.max_ctas) cfg.grid = cfg.max_ctas;

@@ -256,7 +256,7 @@ CPAB_HD void exact_midpoint(double *p, const double *A, double h)
     double v[DIM], pm[DIM];
     exact_affine<DIM>(v, A, p);
 #pragma unroll
-    for (int i = 0; i < DIM; ++i) pm[i] = XADD(p[i], XDIV(XMUL(h, v[i]), 2.0));
+    for (int i = 0; i < DIM; ++i) pm[i] = XADD(p[i], XMUL(XMUL(h, v[i]), 0.5));  // / 2: the same double
     exact_affine<DIM>(v, A, pm);
 #pragma unroll
     for (int i = 0; i < DIM; ++i) p[i] = XADD(p[i], XMUL(v[i], h));
@@ -418,5 +418,145 @@ CPAB_HD void cell_box(const Tess &t, int c, int *kb)
     }
     kb[DIM - 1] = b;
 }
+
+// ---------------------------------------------------------------- facets of a cell
+//
+// Positions relative to a box: box units from its centre.  margin(x) is the
+// smallest of the functionals that bound the cell (coefficients 0, +-1 in the
+// coordinates): >= 0 in the cell, < 0 outside, up to rounding.  Facets on the
+// domain boundary do not count, the cells continue outside as in the
+// reference's lookup.  Either precision.
+
+constexpr float kFar = 1e30f;  // distance to a facet on the domain boundary
+
+CPAB_HD float flip(float v, bool neg) { return neg ? -v : v; }
+CPAB_HD double flip(double v, bool neg) { return neg ? -v : v; }
+CPAB_HD float least(float a, float b) { return fminf(a, b); }
+CPAB_HD double least(double a, double b) { return fmin(a, b); }
+CPAB_HD float most(float a, float b) { return fmaxf(a, b); }
+CPAB_HD double most(double a, double b) { return fmax(a, b); }
+CPAB_HD float size_of(float a) { return fabsf(a); }
+CPAB_HD double size_of(double a) { return fabs(a); }
+
+// Box cells (1D and type II): the box's faces.
+template <int DIM, int TESS>
+struct Facets {
+    float flo[DIM], fhi[DIM];  // 1/2, or kFar where the domain ends
+
+    CPAB_HD void enter(const Tess &t, int, const int *kb)
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < DIM; ++i) {
+            flo[i] = kb[i] > 0 ? 0.5f : kFar;
+            fhi[i] = kb[i] < n[i] - 1 ? 0.5f : kFar;
+        }
+    }
+    template <typename Real>
+    CPAB_HD Real margin(const Real *x) const
+    {
+        Real v = least(flo[0] + x[0], fhi[0] - x[0]);
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 1; i < DIM; ++i) v = least(v, least(flo[i] + x[i], fhi[i] - x[i]));
+        return v;
+    }
+};
+
+// 2D type I: four triangles per box between its diagonals, 0 at low y, then
+// counterclockwise.  With v the box coordinate towards a triangle's side and u
+// the one along it, the triangle is |u| <= v <= 1/2.  Outside the domain the
+// reference's rules (calc_2Dto2D.cu:53-148) continue it: beyond its side over
+// the side's width (|u| <= 1/2), and beyond a corner of the domain up to the
+// box's diagonal continued (|u| <= v).
+template <>
+struct Facets<2, 1> {
+    bool along_x;    // v is the y coordinate
+    bool neg;        // v points down it
+    float side;      // 1/2, or kFar where the side ends the domain
+    float ulo, uhi;  // 1/2 where the box's low / high face in u ends the domain, else kFar
+
+    CPAB_HD void enter(const Tess &t, int c, const int *kb)
+    {
+        const int tri = c & 3;
+        const bool up = tri >= 2, right = tri == 1 || tri == 2;
+        along_x = up == right;
+        neg = !right;
+        const int k = along_x ? kb[1] : kb[0], n = along_x ? t.nC1 : t.nC0;
+        const int ku = along_x ? kb[0] : kb[1], nu = along_x ? t.nC0 : t.nC1;
+        side = k == (right ? n - 1 : 0) ? kFar : 0.5f;
+        // where u's faces do not end the domain, u beyond 1/2 is outside the triangle whatever v
+        ulo = ku == 0 ? 0.5f : kFar;
+        uhi = ku == nu - 1 ? 0.5f : kFar;
+    }
+    template <typename Real>
+    CPAB_HD Real margin(const Real *x) const
+    {
+        const Real v = flip(along_x ? x[1] : x[0], neg), u = along_x ? x[0] : x[1];
+        // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
+        const Real top = (u > uhi || u < -ulo) ? v : least(v, Real(0.5));
+        return least(top - size_of(u), side - v);
+    }
+};
+
+// 3D type I: five tetrahedra per box, four at corners and the centre one.  In
+// box coordinates R a corner tetrahedron belongs to a corner sigma (signs of
+// product + in even boxes, - in odd ones): with y_a = sigma_a R_a it is
+// y0 + y1 + y2 >= 1/2 inside the box's three faces y_a <= 1/2 there; the centre
+// is where no corner's sum reaches 1/2.  Coordinates beyond the domain count
+// as on its boundary (the reference clamps them, calc_3Dto3D.cu:55-60), hence
+// the clamped y in the sums.  (The reference clamps z with the x box size:
+// where the two sizes differ, these facets do not describe its cells.)
+template <>
+struct Facets<3, 1> {
+    bool neg[3];    // signs of sigma
+    float face[3];  // 1/2, or kFar where the face ends the domain (and for the centre)
+    float low[3];   // -1/2 where the opposite face ends the domain, else -kFar
+    float cap[3];   // 1/2 (centre: where the face ends the domain, else kFar)
+    bool centre;
+
+    CPAB_HD void enter(const Tess &t, int c, const int *kb)
+    {
+        const int n[3] = {t.nC0, t.nC1, t.nC2};
+        const int tet = c - c / 5 * 5;
+        const bool odd = ((kb[0] ^ kb[1] ^ kb[2]) & 1) != 0;
+        centre = tet == 0;
+        // signs in exact_cell_3d_tet's turned coordinates (odd boxes: (x, y) -> (y, -x))
+        const bool n0 = tet == 1 || tet == 3, n1 = tet == 1 || tet == 4;
+        neg[0] = odd ? !n1 : n0;
+        neg[1] = odd ? n0 : n1;
+        neg[2] = tet == 3 || tet == 4;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < 3; ++i) {
+            const bool end = kb[i] == (neg[i] ? 0 : n[i] - 1);
+            face[i] = centre || end ? kFar : 0.5f;
+            low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
+            cap[i] = centre && !end ? kFar : 0.5f;
+        }
+    }
+    template <typename Real>
+    CPAB_HD Real margin(const Real *x) const
+    {
+        Real y[3], sum = Real(-0.5), far = kFar;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < 3; ++i) {
+            y[i] = flip(x[i], neg[i]);
+            far = least(far, face[i] - y[i]);
+            y[i] = most(least(y[i], Real(cap[i])), Real(low[i]));
+            sum += y[i];
+        }
+        // the four corners' sums: sigma with an even number of signs flipped
+        const Real a = y[0] + y[1], d = y[0] - y[1];
+        const Real all = most(size_of(a) + y[2], size_of(d) - y[2]);
+        return centre ? Real(0.5) - all : least(sum, far);
+    }
+};
 
 }  // namespace cpab

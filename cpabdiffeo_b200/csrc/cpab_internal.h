@@ -59,6 +59,7 @@ struct IntegrateArgs {
     double clamp_lo, clamp_hi;
     unsigned long long *counters;  // [CNT_N] or nullptr (slots below)
     int max_crossings;    // EXACT: give up after this many boundary crossings
+    int phases;           // FP64 REF: phase by phase (integrate_phases), for launches that fill the SMs
     int sort;             // REF/SIMPLE: process each tile's points in order of their start cell
     const volatile int *cancel;  // the context's cancel flag (device memory), polled between tiles, or nullptr
     const double *facets; // EXACT 2D/3D: [nC, nF, DIM+1] (outward unit normal, -offset) per cell facet

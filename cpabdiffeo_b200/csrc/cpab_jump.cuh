@@ -35,9 +35,9 @@
 // box units, |r| <= 1/2 inside) as a compensated pair, and the maps act on r:
 // rounding is then relative to a box, not to the domain, and the margin of a
 // candidate end point needs no cell lookup -- it is the smallest of the facet
-// functionals of the lane's current cell (WalkBox, WalkTri), negative when
-// the candidate left it.  The cell is looked up again only where a sub-step
-// leaves it.  3D tetrahedra (WalkTet) look every candidate up.
+// functionals of the lane's current cell (Facets), negative when the
+// candidate left it.  The cell is looked up again only where a sub-step leaves
+// it.
 //
 // Measured on 2D prior fields (64 cells, dt 0.02, 50 steps, 100 sub-steps
 // per leaving step): 11.4 units per point instead of 95; with r = 2 (every
@@ -282,19 +282,12 @@ struct BoxCand {
     Real m;
 };
 
-// -v where neg (a sign bit flipped, no branch)
-__device__ __forceinline__ float flip(float v, bool neg) { return neg ? -v : v; }
-__device__ __forceinline__ double flip(double v, bool neg) { return neg ? -v : v; }
-__device__ __forceinline__ float least(float a, float b) { return fminf(a, b); }
-__device__ __forceinline__ double least(double a, double b) { return fmin(a, b); }
-__device__ __forceinline__ float most(float a, float b) { return fmaxf(a, b); }
-__device__ __forceinline__ double most(double a, double b) { return fmax(a, b); }
-
 template <int DIM, int TESS, typename Real>
 struct WalkLocal {
     BoxPos<DIM, Real> p;
     int c;
     Real m;
+    Facets<DIM, TESS> f;
 
     __device__ __forceinline__ void set_local(const Tess &t, const double *x, const int *kb)
     {
@@ -442,34 +435,27 @@ struct WalkLocal {
     }
 };
 
-constexpr float kFar = 1e30f;  // distance to a facet on the domain boundary
-
-// Box cells (1D and type II): the box's faces.
+// Box cells (1D and type II).
 template <int DIM, typename Real>
 struct WalkBox : WalkLocal<DIM, 2, Real> {
     using B = WalkLocal<DIM, 2, Real>;
     using Cand = BoxCand<DIM, Real>;
-    float flo[DIM], fhi[DIM];  // 1/2, or kFar where the domain ends
+    using B::c;
+    using B::f;
+    using B::m;
+    using B::p;
 
-    __device__ __forceinline__ Real margin(const Real *x) const
-    {
-        Real v = least(flo[0] + x[0], fhi[0] - x[0]);
-#pragma unroll
-        for (int i = 1; i < DIM; ++i) v = least(v, least(flo[i] + x[i], fhi[i] - x[i]));
-        return v;
-    }
     __device__ __forceinline__ void enter(const Tess &t, const int *kb)
     {
         const int n[3] = {t.nC0, t.nC1, t.nC2};
         int stride = 1;
-        B::c = 0;
+        c = 0;
 #pragma unroll
         for (int i = 0; i < DIM; ++i) {
-            B::c += kb[i] * stride;
+            c += kb[i] * stride;
             stride *= n[i];
-            flo[i] = kb[i] > 0 ? 0.5f : kFar;
-            fhi[i] = kb[i] < n[i] - 1 ? 0.5f : kFar;
         }
+        f.enter(t, c, kb);
     }
     template <typename Elem>
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
@@ -480,8 +466,8 @@ struct WalkBox : WalkLocal<DIM, 2, Real> {
         B::set_local(t, x, kb);
         enter(t, kb);
 #pragma unroll
-        for (int i = 0; i < DIM; ++i) r[i] = B::p.x(i);
-        B::m = margin(r);
+        for (int i = 0; i < DIM; ++i) r[i] = p.x(i);
+        m = f.margin(r);
     }
     template <typename Elem>
     __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
@@ -490,12 +476,12 @@ struct WalkBox : WalkLocal<DIM, 2, Real> {
         cell_box<DIM, 2>(t, cell, kb);
         B::set_local(t, x, kb);
         enter(t, kb);
-        B::m = 0;
+        m = 0;
     }
     __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
         const Real len = B::advance(map, q);
-        q.m = margin(q.x);
+        q.m = f.margin(q.x);
         return len;
     }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
@@ -504,48 +490,26 @@ struct WalkBox : WalkLocal<DIM, 2, Real> {
         int kb[DIM];
         B::shift_box(t, q, kb);
         enter(t, kb);
-        B::p = q.p;
-        B::m = margin(q.x);
+        p = q.p;
+        m = f.margin(q.x);
     }
 };
 
-// 2D type I: four triangles per box between its diagonals, 0 at low y, then
-// counterclockwise.  With v the box coordinate towards a triangle's side and u
-// the one along it, the triangle is |u| <= v <= 1/2.  Outside the domain the
-// reference's rules (calc_2Dto2D.cu:53-148) continue it: beyond its side over
-// the side's width (|u| <= 1/2), and beyond a corner of the domain up to the
-// box's diagonal continued (|u| <= v).
+// 2D type I: the triangle by the signs of x - y and x + y, in the domain and
+// outside (Facets<2, 1>).
 template <typename Real>
 struct WalkTri : WalkLocal<2, 1, Real> {
     using B = WalkLocal<2, 1, Real>;
     using Cand = BoxCand<2, Real>;
     using B::c;
+    using B::f;
     using B::m;
     using B::p;
-    bool along_x;      // v is the y coordinate
-    bool neg;          // v points down it
-    float side;        // 1/2, or kFar where the side ends the domain
-    float ulo, uhi;    // 1/2 where the box's low / high face in u ends the domain, else kFar
 
-    __device__ __forceinline__ Real margin(const Real *x) const
-    {
-        const Real v = flip(along_x ? x[1] : x[0], neg), u = along_x ? x[0] : x[1];
-        // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
-        const Real top = (u > uhi || u < -ulo) ? v : least(v, Real(0.5));
-        return least(top - fabs(u), side - v);
-    }
     __device__ __forceinline__ void enter(const Tess &t, const int *kb, bool up, bool right)
     {
-        const int tri = up ? (right ? 2 : 3) : (right ? 1 : 0);
-        c = (kb[0] + kb[1] * t.nC0) * 4 + tri;
-        along_x = up == right;
-        neg = !right;
-        const int k = along_x ? kb[1] : kb[0], n = along_x ? t.nC1 : t.nC0;
-        const int ku = along_x ? kb[0] : kb[1], nu = along_x ? t.nC0 : t.nC1;
-        side = k == (right ? n - 1 : 0) ? kFar : 0.5f;
-        // where u's faces do not end the domain, u beyond 1/2 is outside the triangle whatever v
-        ulo = ku == 0 ? 0.5f : kFar;
-        uhi = ku == nu - 1 ? 0.5f : kFar;
+        c = (kb[0] + kb[1] * t.nC0) * 4 + (up ? (right ? 2 : 3) : (right ? 1 : 0));
+        f.enter(t, c, kb);
     }
     template <typename Elem>
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
@@ -555,22 +519,22 @@ struct WalkTri : WalkLocal<2, 1, Real> {
         B::set_local(t, x, kb);
         const Real r[2] = {p.x(0), p.x(1)};
         enter(t, kb, r[0] < r[1], r[0] + r[1] > Real(0));
-        m = margin(r);
+        m = f.margin(r);
     }
     template <typename Elem>
     __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
     {
         int kb[2];
+        c = cell;
         cell_box<2, 1>(t, cell, kb);
         B::set_local(t, x, kb);
-        const int tri = cell & 3;
-        enter(t, kb, tri >= 2, tri == 1 || tri == 2);
+        f.enter(t, cell, kb);
         m = 0;
     }
     __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
         const Real len = B::advance(map, q);
-        q.m = margin(q.x);
+        q.m = f.margin(q.x);
         return len;
     }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
@@ -580,74 +544,31 @@ struct WalkTri : WalkLocal<2, 1, Real> {
         B::shift_box(t, q, kb);
         enter(t, kb, q.x[0] < q.x[1], q.x[0] + q.x[1] > Real(0));
         p = q.p;
-        m = margin(q.x);
+        m = f.margin(q.x);
     }
 };
 
-// 3D type I: five tetrahedra per box, four at corners and the centre one.  In
-// box coordinates R a corner tetrahedron belongs to a corner sigma (signs of
-// product + in even boxes, - in odd ones): with y_a = sigma_a R_a it is
-// y0 + y1 + y2 >= 1/2 inside the box's three faces y_a <= 1/2 there; the centre
-// is where no corner's sum reaches 1/2.  Coordinates beyond the domain count
-// as on its boundary (the reference clamps them, calc_3Dto3D.cu:55-60), hence
-// the clamped y in the sum.  The reference clamps z with the x box size: where
-// the two sizes differ, every candidate is looked up at its absolute position.
+// 3D type I: a new cell is looked up at the absolute position, and so is every
+// candidate where the facets do not describe the reference's cells.
 template <typename Real>
 struct WalkTet : WalkLocal<3, 1, Real> {
     using B = WalkLocal<3, 1, Real>;
     using Cand = BoxCand<3, Real>;
     using B::c;
+    using B::f;
     using B::m;
     using B::p;
-    bool neg[3];     // signs of sigma
-    float face[3];   // 1/2, or kFar where the face ends the domain (and for the centre)
-    float low[3];    // -1/2 where the opposite face ends the domain, else -kFar
-    bool centre;
 
-    __device__ __forceinline__ Real margin(const Real *x) const
-    {
-        Real y[3], sum = Real(-0.5), far = kFar;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            y[i] = flip(x[i], neg[i]);
-            sum += most(least(y[i], Real(0.5)), Real(low[i]));
-            far = least(far, face[i] - y[i]);
-        }
-        // the four corners' sums: sigma with an even number of signs flipped
-        const Real a = y[0] + y[1], d = y[0] - y[1];
-        const Real all = most(fabs(a) + y[2], fabs(d) - y[2]);
-        return centre ? Real(0.5) - all : least(sum, far);
-    }
-    __device__ __forceinline__ void enter(const Tess &t, int cell)
-    {
-        const int n[3] = {t.nC0, t.nC1, t.nC2};
-        int kb[3];
-        c = cell;
-        cell_box<3, 1>(t, cell, kb);
-        const int tet = cell - cell / 5 * 5;
-        const bool odd = ((kb[0] ^ kb[1] ^ kb[2]) & 1) != 0;
-        centre = tet == 0;
-        // signs in fast_cell_3d_tet's turned coordinates (odd boxes: (x, y) -> (y, -x))
-        const bool n0 = tet == 1 || tet == 3, n1 = tet == 1 || tet == 4;
-        neg[0] = odd ? !n1 : n0;
-        neg[1] = odd ? n0 : n1;
-        neg[2] = tet == 3 || tet == 4;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            face[i] = centre || kb[i] == (neg[i] ? 0 : n[i] - 1) ? kFar : 0.5f;
-            low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
-        }
-    }
     static __device__ __forceinline__ int cell_at(const Tess &t, const float *a, float &mq)
     {
         return fast_cell_3d_tet_m(t, a, mq);
     }
     static __device__ __forceinline__ int cell_at(const Tess &t, const double *a, double &mq)
     {
-        float f[3], m32;
+        float x[3], m32;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) f[i] = (float)a[i];
-        fast_cell_3d_tet_m(t, f, m32);
+        for (int i = 0; i < 3; ++i) x[i] = (float)a[i];
+        fast_cell_3d_tet_m(t, x, m32);
         mq = fmax((double)m32 - 1e-6, 0.0);  // a lower bound still, whatever float rounded
         return exact_cell<3, 1>(t, a);
     }
@@ -674,8 +595,9 @@ struct WalkTet : WalkLocal<3, 1, Real> {
     __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
     {
         int kb[3];
-        enter(t, cell);
+        c = cell;
         cell_box<3, 1>(t, cell, kb);
+        f.enter(t, cell, kb);
         B::set_local(t, x, kb);
         m = 0;
     }
@@ -683,7 +605,7 @@ struct WalkTet : WalkLocal<3, 1, Real> {
     {
         const Real len = B::advance(map, q);
         if (t.inc[0] == t.inc[2]) {
-            q.m = margin(q.x);
+            q.m = f.margin(q.x);
         } else if (lookup(t, q.x, q.m) != c) {
             q.m = Real(-1e-30);  // outside, nothing known of how far
         }

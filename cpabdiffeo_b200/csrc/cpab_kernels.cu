@@ -90,7 +90,8 @@ __host__ __device__ inline size_t table_bytes(const IntegrateArgs &a)
     return (size_t)2 * a.t.nC * a.t.dim * (a.t.dim + 1) * sizeof(double);
 }
 
-template <int DIM, int TESS, typename Real, int SCHEME>
+// PHASES: FP64 reference scheme by integrate_phases.
+template <int DIM, int TESS, typename Real, int SCHEME, bool PHASES = false>
 __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
 {
     constexpr int NE = DIM * (DIM + 1);
@@ -99,8 +100,10 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
     constexpr bool kJump = sizeof(Real) == 4;
     Real *sA = reinterpret_cast<Real *>(smem_raw);
     Real *sT = sA + a.t.nC * NE;
-    // cell-sort scratch after the tables: histogram [nC], start cells and permutation [tile_pts]
-    int *s_hist = reinterpret_cast<int *>(smem_raw + table_bytes<Real>(a));
+    // PHASES: positions between the phases, after the tables
+    unsigned char *s_phase = smem_raw + table_bytes<Real>(a);
+    // cell-sort scratch: histogram [nC], start cells and permutation [tile_pts]
+    int *s_hist = reinterpret_cast<int *>(s_phase + (PHASES ? phase_scratch_bytes(DIM, a.batch.tile_pts) : 0));
     int *s_cell = s_hist + a.t.nC;
     int *s_perm = s_cell + a.batch.tile_pts;
     __shared__ TileInfo s_tile;
@@ -164,6 +167,9 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
         if constexpr (kJump)
             integrate_jump<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, ti.start, (int)n, src, snk,
                                               c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim), s_queue, &ex);
+        else if constexpr (PHASES)
+            integrate_phases<DIM, TESS>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, (int)n, h, src, snk, c_fast,
+                                        c_fb, c_sub, c_pts, perm, a.batch.tile_pts, s_phase);
         else
             integrate_range<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, ti.end, h, src,
                                                      snk, c_fast, c_fb, c_sub, c_pts, perm, ti.start, &s_claim,
@@ -197,6 +203,15 @@ template <int DIM, int TESS, typename Real, int SCHEME>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? kJumpCtas<DIM> : 1) k_integrate(IntegrateArgs a)
 {
     integrate_body<DIM, TESS, Real, SCHEME>(a);
+}
+
+// The FP64 reference scheme phase by phase.  4 CTAs of 256 threads per SM (2D,
+// 512 x 512 points there and back and a remap: 2 CTAs 708 us, 3: 642, 4: 632,
+// 5: 650); in 3D their registers would spill, 2.
+template <int DIM, int TESS>
+__global__ void __launch_bounds__(256, DIM < 3 ? 4 : 2) k_integrate_phases(IntegrateArgs a)
+{
+    integrate_body<DIM, TESS, double, SCHEME_REF, true>(a);
 }
 
 // The exact scheme's exit resolution (FP64, rare) would otherwise set the
@@ -545,6 +560,14 @@ static cudaError_t launch_integrate_t(const IntegrateArgs &a, const LaunchCfg &c
     void (*kern)(IntegrateArgs);
     if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
     else kern = k_integrate<DIM, TESS, Real, SCHEME>;
+    if constexpr (sizeof(Real) == 8 && SCHEME == SCHEME_REF) {
+        // phases where the launch has points enough to fill the SMs and their scratch fits beside the tables
+        const size_t with = smem + phase_scratch_bytes(DIM, a.batch.tile_pts);
+        if (a.phases && with + 1024 <= (size_t)max_smem_optin()) {
+            kern = k_integrate_phases<DIM, TESS>;
+            smem = with;
+        }
+    }
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
