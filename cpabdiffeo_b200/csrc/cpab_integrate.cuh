@@ -184,12 +184,15 @@ __device__ void stage_exact_substeps(const double *gA, const double *gT, int nC,
 // row-major [nC, DIM*(DIM+1)]), the facet tables, the sub-step length and
 // the lane's counters.
 // Parked exits a warp resolves together, and the votes the oldest may wait
-// (integrate_range).
+// (integrate_range, integrate_jump).  Resolving costs a few hundred FP64
+// instructions however many lanes take part; in a batch of 512 instances of
+// 8192 points (2D, 64 cells, FP32) 16 exits at a time took 1100 us, 24 995, 28
+// or 31 960, 32 978 (FP64, 64 such instances: 28 815, 31 848, 32 889).
 #ifndef CPAB_EXACT_CROSS_BATCH
-#define CPAB_EXACT_CROSS_BATCH 16
+#define CPAB_EXACT_CROSS_BATCH 28
 #endif
 #ifndef CPAB_EXACT_CROSS_WAIT
-#define CPAB_EXACT_CROSS_WAIT 96
+#define CPAB_EXACT_CROSS_WAIT 400
 #endif
 
 struct ExactCross {
@@ -274,7 +277,7 @@ __device__ __forceinline__ void velocity(const double *__restrict__ A, const dou
 // out = expm(t A)[p; 1] (out may alias p); false when kExactDeg terms do
 // not bring the omitted rest below FP64 rounding of the first term
 template <int DIM>
-__device__ __forceinline__ bool flow_taylor(const double *__restrict__ A, const double *p, double t, double *out)
+__device__ __noinline__ bool flow_taylor_any(const double *__restrict__ A, const double *p, double t, double *out)
 {
     const double *Ar = A;  // global, read through __ldg
     const double lnorm = affine_norm<DIM>(A);
@@ -318,7 +321,7 @@ __device__ __forceinline__ bool flow_taylor(const double *__restrict__ A, const 
 // safeguarded Newton iteration on that polynomial.  Returns NaN when
 // kExactDeg terms do not resolve g to that rounding.
 template <int DIM>
-__device__ __forceinline__ double facet_hit_time(const double *__restrict__ A, const double *__restrict__ F,
+__device__ __noinline__ double facet_hit_time_any(const double *__restrict__ A, const double *__restrict__ F,
                                                  const double *p, double s, double g0)
 {
     const double *Ar = A;  // global, read through __ldg
@@ -394,6 +397,144 @@ __device__ __forceinline__ double facet_hit_time(const double *__restrict__ A, c
     return 0.5 * (lo + hi);
 }
 
+// Both again, for the slow flows of ordinary sub-steps: with x = t |L| so small
+// that the rest after kShortDeg terms, at most x^8 / 9! (1 + x) of the first
+// one, is below kTaylorTol, the degree is fixed, the loops unroll and A stays
+// in registers.  (x <= 0.03 makes that rest 2e-18.)  With the exits' facets
+// picked before their times are computed (lanes used to enter the search at
+// whichever of the facets was theirs, one facet after the other) the batch of
+// 512 x 8192 points in 2D took 1100 us instead of 2015.
+constexpr int kShortDeg = 8;
+constexpr double kShortMax = 0.03;
+
+template <int DIM>
+struct AffineMap {
+    double a[DIM * (DIM + 1)], norm;
+    __device__ __forceinline__ void load(const double *__restrict__ A)
+    {
+        norm = 0.0;
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            double rs = 0.0;
+#pragma unroll
+            for (int m = 0; m <= DIM; ++m) {
+                a[r * (DIM + 1) + m] = __ldg(A + r * (DIM + 1) + m);
+                if (m < DIM) rs += fabs(a[r * (DIM + 1) + m]);
+            }
+            norm = fmax(norm, rs);
+        }
+    }
+    __device__ __forceinline__ void vel(const double *p, double *v) const
+    {
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            double s = a[r * (DIM + 1) + DIM];
+#pragma unroll
+            for (int m = 0; m < DIM; ++m) s = fma(a[r * (DIM + 1) + m], p[m], s);
+            v[r] = s;
+        }
+    }
+    __device__ __forceinline__ void lin(const double *u, double *v) const
+    {
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            double s = a[r * (DIM + 1)] * u[0];
+#pragma unroll
+            for (int m = 1; m < DIM; ++m) s = fma(a[r * (DIM + 1) + m], u[m], s);
+            v[r] = s;
+        }
+    }
+};
+
+template <int DIM>
+__device__ __forceinline__ bool flow_taylor(const AffineMap<DIM> &M, const double *__restrict__ A, const double *p,
+                                            double t, double *out)
+{
+    if (!(fabs(t) * M.norm <= kShortMax)) return flow_taylor_any<DIM>(A, p, t, out);
+    // p + t (v + t/2 L (v + t/3 L (v + ...)))
+    double v[DIM], w[DIM];
+    M.vel(p, v);
+#pragma unroll
+    for (int r = 0; r < DIM; ++r) w[r] = v[r];
+#pragma unroll
+    for (int k = kShortDeg; k > 1; --k) {
+        double lw[DIM];
+        M.lin(w, lw);
+        const double tk = t * (1.0 / k);
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) w[r] = fma(tk, lw[r], v[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < DIM; ++r) out[r] = fma(t, w[r], p[r]);
+    return true;
+}
+
+template <int DIM>
+__device__ __forceinline__ double facet_hit_time(const AffineMap<DIM> &M, const double *__restrict__ A,
+                                                 const double *__restrict__ F, const double *p, double s, double g0)
+{
+    double c[kShortDeg + 1], u[DIM], Fn[DIM], f1 = 0.0, un = 0.0;
+    M.vel(p, u);
+#pragma unroll
+    for (int r = 0; r < DIM; ++r) {
+        Fn[r] = __ldg(F + r);
+        f1 += fabs(Fn[r]);
+        un = fmax(un, fabs(u[r]));
+    }
+    c[0] = g0;
+    c[1] = 0.0;
+#pragma unroll
+    for (int r = 0; r < DIM; ++r) c[1] = fma(Fn[r], u[r], c[1]);
+    // the rest: f1 |u| s x^8 / 9! (1 + x) of g, to be below rounding of g over [0, s]; x^8 <= 0.03^4 x^4
+    const double x = s * M.norm, x2 = x * x;
+    if (!(x <= kShortMax && f1 * un * s * (x2 * x2) * (kShortMax * kShortMax * kShortMax * kShortMax * 1.03 / 362880) <=
+                                kTaylorTol * (fabs(g0) + fabs(c[1]) * s)))
+        return facet_hit_time_any<DIM>(A, F, p, s, g0);
+    double inv_fact = 1.0;
+#pragma unroll
+    for (int k = 2; k <= kShortDeg; ++k) {
+        double nu[DIM], d = 0.0;
+        M.lin(u, nu);
+#pragma unroll
+        for (int r = 0; r < DIM; ++r) {
+            u[r] = nu[r];
+            d = fma(Fn[r], u[r], d);
+        }
+        inv_fact *= 1.0 / k;
+        c[k] = d * inv_fact;
+    }
+    auto P = [&](double t, double &dP) {
+        double v = c[kShortDeg], dv = 0.0;
+#pragma unroll
+        for (int k = kShortDeg - 1; k >= 0; --k) {
+            dv = fma(dv, t, v);
+            v = fma(v, t, c[k]);
+        }
+        dP = dv;
+        return v;
+    };
+    // Newton with the slope's reciprocal in float (the polynomial is close to
+    // linear: the secant is off by x at most, the second iterate by 1e-7 of
+    // that), to the same end as facet_hit_time_any
+    auto over = [](double g, double d) { return g * (double)__frcp_rn((float)d); };
+    double lo = 0.0, hi = s, dP;
+    const double ps = P(s, dP);
+    if (!(ps > 0)) return s;
+    double t = s * over(-g0, ps - g0);
+    if (!(t > lo && t < hi)) t = 0.5 * (lo + hi);
+#pragma unroll 1
+    for (int it = 0; it < 60; ++it) {
+        const double g = P(t, dP);
+        if (g > 0) hi = t; else lo = t;
+        if (g == 0) return t;
+        double tn = t - over(g, dP);
+        if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
+        if (fabs(tn - t) <= 4.5e-16 * fabs(t) || hi - lo <= 4.5e-16 * hi) return tn;
+        t = tn;
+    }
+    return 0.5 * (lo + hi);
+}
+
 // A sub-step of length h from p in cell c ended at q outside c: the exact
 // flow from p, exit times through interior facets, the neighbour across the
 // exited facet, the rest of the sub-step there (and so on).  q becomes the
@@ -427,21 +568,28 @@ __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex
         }
         const double *A = ex.A + (size_t)c * NE;
         const double *Fc = ex.F + (size_t)c * ex.nF * NH;
+        AffineMap<DIM> M;
+        M.load(A);
         double tau = s;
         int kbest = -1;
+        // the facets with y beyond them first: lanes then resolve their hits together, whichever facet it is
+        unsigned beyond = 0;
 #pragma unroll 1
         for (int k = 0; k < ex.nF; ++k) {
-            if (__ldg(ex.nbr + c * ex.nF + k) < 0) continue;
             const double *F = Fc + k * NH;
-            double ge = __ldg(F + DIM), g0 = ge;
+            double ge = __ldg(F + DIM);
 #pragma unroll
-            for (int r = 0; r < DIM; ++r) {
-                const double n = __ldg(F + r);
-                ge = fma(n, y[r], ge);
-                g0 = fma(n, p[r], g0);
-            }
-            if (!(ge > 0)) continue;
-            const double r = (g0 >= 0) ? 0.0 : facet_hit_time<DIM>(A, F, p, s, g0);
+            for (int r = 0; r < DIM; ++r) ge = fma(__ldg(F + r), y[r], ge);
+            if (ge > 0 && __ldg(ex.nbr + c * ex.nF + k) >= 0) beyond |= 1u << k;
+        }
+#pragma unroll 1
+        for (; beyond; beyond &= beyond - 1) {
+            const int k = __ffs(beyond) - 1;
+            const double *F = Fc + k * NH;
+            double g0 = __ldg(F + DIM);
+#pragma unroll
+            for (int r = 0; r < DIM; ++r) g0 = fma(__ldg(F + r), p[r], g0);
+            const double r = (g0 >= 0) ? 0.0 : facet_hit_time<DIM>(M, A, F, p, s, g0);
             if (kbest < 0 || r < tau) {
                 tau = r;
                 kbest = k;
@@ -452,7 +600,7 @@ __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex
             end_at(y);
             return lookup_d<DIM, TESS>(t, y, Real(0));
         }
-        flow_taylor<DIM>(A, p, tau, p);
+        flow_taylor<DIM>(M, A, p, tau, p);
         s -= tau;
         c = __ldg(ex.nbr + c * ex.nF + kbest);
         ++ex.crossings;
@@ -460,7 +608,8 @@ __device__ __forceinline__ int exact_substep_cross(const Tess &t, ExactCross &ex
             end_at(p);
             return c;
         }
-        if (!flow_taylor<DIM>(ex.A + (size_t)c * NE, p, s, y)) {
+        M.load(ex.A + (size_t)c * NE);
+        if (!flow_taylor<DIM>(M, ex.A + (size_t)c * NE, p, s, y)) {
             // the neighbour's flow is too fast for the polynomial over the
             // rest of the sub-step: the reference scheme's sub-step end
             ++ex.unresolved;
