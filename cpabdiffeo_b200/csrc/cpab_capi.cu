@@ -310,19 +310,31 @@ static IntegrateArgs make_args(cpab_ctx *ctx, const double *signedA, const doubl
     return a;
 }
 
-static int run_integrate(cpab_ctx *ctx, IntegrateArgs &a, int precision, int scheme, int64_t uniform_tiles_total,
-                         cudaStream_t s)
+static int run_integrate(cpab_ctx *ctx, IntegrateArgs &a, int precision, int scheme, cudaStream_t s)
 {
+    Batch &b = a.batch;
+    b.tile_pts = ctx->cfg.tile_pts;
     LaunchCfg cfg = ctx->cfg;
     // from 128 points per SM on (both sides measured at integrate_phases); a ragged launch, whose points are not
     // known here, counts as large
     a.phases = a.batch.tile_prefix || (int64_t)a.batch.N * a.batch.n_uniform >= (int64_t)num_sms() * 128;
-    // small uniform launches: one CTA per tile (the persistent grid would leave CTAs idle)
-    if (uniform_tiles_total > 0 && uniform_tiles_total < (int64_t)num_sms() * 2) cfg.grid = (int)uniform_tiles_total;
-    if (cfg.grid > 0 && cfg.max_ctas > 0 && cfg.grid > cfg.max_ctas) cfg.grid = cfg.max_ctas;
-    cudaError_t e = (scheme == CPAB_SCHEME_EXACT && a.t.dim == 1) ? launch_integrate_exact1d(a, precision, cfg, s)
-                                                                   : launch_integrate(a, precision, scheme, cfg, s);
-    return cuda_status(ctx, e, "integrate launch");
+    if (scheme != CPAB_SCHEME_EXACT || a.t.dim != 1)
+        return cuda_status(ctx, launch_integrate(a, precision, scheme, cfg, s), "integrate launch");
+    if (b.offsets) {
+        // (the intervals take ranges of points, not tiles)
+        if (!exact1d_uses_intervals(a.t.nC, precision)) {
+            const cudaError_t e = launch_tile_prefix(b.offsets, b.tile_prefix, b.N, b.tile_pts, 0, s);
+            if (e != cudaSuccess) return cuda_status(ctx, e, "tile_prefix launch");
+        }
+    } else {
+        b.tile_pts = small_launch_tile((int64_t)b.N * b.n_uniform, b.tile_pts);
+        b.tiles_per_inst = (b.n_uniform + b.tile_pts - 1) / b.tile_pts;
+        // small launches: one CTA per tile (the persistent grid would leave CTAs idle)
+        const int64_t tiles = b.tiles_per_inst * b.N;
+        if (tiles < (int64_t)num_sms() * 2) cfg.grid = (int)tiles;
+        if (cfg.grid > 0 && cfg.max_ctas > 0 && cfg.grid > cfg.max_ctas) cfg.grid = cfg.max_ctas;
+    }
+    return cuda_status(ctx, launch_integrate_exact1d(a, precision, cfg, s), "integrate launch");
 }
 
 int cpab_calc_T(cpab_ctx *ctx, const double *signedA, const double *Trels, const void *pts, void *out,
@@ -339,9 +351,7 @@ int cpab_calc_T(cpab_ctx *ctx, const double *signedA, const double *Trels, const
     a.batch.n_uniform = nPts;
     a.batch.offsets = nullptr;
     a.batch.tile_prefix = nullptr;
-    a.batch.tile_pts = small_launch_tile(nPts, ctx->cfg.tile_pts);
-    a.batch.tiles_per_inst = (nPts + a.batch.tile_pts - 1) / a.batch.tile_pts;
-    return run_integrate(ctx, a, precision, scheme, a.batch.tiles_per_inst, (cudaStream_t)stream);
+    return run_integrate(ctx, a, precision, scheme, (cudaStream_t)stream);
 }
 
 size_t cpab_batched_workspace_bytes(int N)
@@ -370,27 +380,16 @@ int cpab_calc_T_batched(cpab_ctx *ctx, const double *signedA, const double *Trel
     cudaStream_t s = (cudaStream_t)stream;
     IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, scheme, dt, nTimeSteps, nStepsODE, counters);
     a.batch.N = N;
-    a.batch.tile_pts = ctx->cfg.tile_pts;
-    int64_t uniform_tiles = 0;
     if (offsets) {
         if (!workspace || workspace_bytes < cpab_batched_workspace_bytes(N))
             return fail(ctx, CPAB_NO_MEMORY, "workspace of %zu bytes needed", cpab_batched_workspace_bytes(N));
-        int64_t *prefix = static_cast<int64_t *>(workspace);
-        // (the 1D exact kernel's intervals take ranges of points, not tiles)
-        if (!(scheme == CPAB_SCHEME_EXACT && ctx->t.dim == 1 && exact1d_uses_intervals(ctx->t.nC, precision))) {
-            cudaError_t e = launch_tile_prefix(offsets, prefix, N, a.batch.tile_pts, s);
-            if (e != cudaSuccess) return cuda_status(ctx, e, "tile_prefix launch");
-        }
         a.batch.offsets = offsets;
-        a.batch.tile_prefix = prefix;
+        a.batch.tile_prefix = static_cast<int64_t *>(workspace);
     } else {
         if (n_uniform == 0) return CPAB_OK;
-        a.batch.tile_pts = small_launch_tile((int64_t)N * n_uniform, ctx->cfg.tile_pts);
         a.batch.n_uniform = n_uniform;
-        a.batch.tiles_per_inst = (n_uniform + a.batch.tile_pts - 1) / a.batch.tile_pts;
-        uniform_tiles = a.batch.tiles_per_inst * N;
     }
-    return run_integrate(ctx, a, precision, scheme, uniform_tiles, s);
+    return run_integrate(ctx, a, precision, scheme, s);
 }
 
 int cpab_calc_trajectory(cpab_ctx *ctx, const double *signedA, const double *Trels, const double *pts, double *traj,

@@ -68,14 +68,15 @@ __device__ __forceinline__ TileInfo decode_tile(const Batch &b, int64_t tile)
         return ti;
     }
     // first index with prefix > tile, minus one (skips empty instances)
-    int lo = 0, hi = b.N;  // prefix[0] = 0 <= tile < prefix[N]
+    int lo = 0, hi = b.N;  // 0 <= tile < prefix[N]; prefix[0], always 0, holds the points per tile
+    const int64_t tp = b.tile_prefix[0];
     while (hi - lo > 1) {
         int mid = (lo + hi) >> 1;
         if (b.tile_prefix[mid] <= tile) lo = mid; else hi = mid;
     }
     ti.inst = lo;
-    ti.start = b.offsets[lo] + (tile - b.tile_prefix[lo]) * b.tile_pts;
-    int64_t e = ti.start + b.tile_pts, lim = b.offsets[lo + 1];
+    ti.start = b.offsets[lo] + (tile - (lo ? b.tile_prefix[lo] : 0)) * tp;
+    int64_t e = ti.start + tp, lim = b.offsets[lo + 1];
     ti.end = e < lim ? e : lim;
     return ti;
 }

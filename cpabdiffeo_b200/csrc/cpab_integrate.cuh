@@ -915,14 +915,15 @@ __device__ __forceinline__ void integrate_phases(const Tess &t, int nT, int nODE
     constexpr int NE = DIM * (DIM + 1), kT = 2, kS = 4;  // burst lengths
     __shared__ int s_claim, s_nT, s_nS;
     const int cap = min(tile_pts, kChunk), lane = threadIdx.x & 31;
+    const int chunks = (n_range + cap - 1) / cap, each = chunks ? (n_range + chunks - 1) / chunks : 1;
     const unsigned lt = (1u << lane) - 1u;
     double *s_p = reinterpret_cast<double *>(scratch);       // [cap][DIM]
     int *s_c = reinterpret_cast<int *>(s_p + cap * DIM);     // cell
     int *s_left = s_c + cap;                                 // time steps to go
     unsigned short *l_T = reinterpret_cast<unsigned short *>(s_left + cap), *l_S = l_T + cap;
     unsigned n_fb = 0, n_pts = 0;
-    for (int b0 = 0; b0 < n_range; b0 += cap) {
-        const int m = min(cap, n_range - b0);
+    for (int b0 = 0; b0 < n_range; b0 += each) {
+        const int m = min(each, n_range - b0);
         auto point = [&](int i) { return perm ? perm[b0 + i] : b0 + i; };
         auto finish = [&](int i, const double *p) {
             snk.put(ws + point(i), p);

@@ -30,9 +30,9 @@ struct Batch {
     int N;
     int64_t n_uniform;
     const int64_t *offsets;      // [N+1] or nullptr
-    const int64_t *tile_prefix;  // [N+1] tiles per instance (prefix) or nullptr
+    int64_t *tile_prefix;        // [N+1] tiles per instance (prefix; [0]: points per tile) or nullptr
     int64_t tiles_per_inst;      // uniform batches
-    int tile_pts;                // points per CTA tile
+    int tile_pts;                // points per CTA tile (ragged: at most)
 };
 
 // Composed-step tables of the FP32 integration (cpab_jump.cuh): nT levels of

@@ -17,16 +17,20 @@
 // tables are staged in shared memory (converted to float in FP32 mode).
 #include <mutex>
 
+#include <algorithm>
+
 #include "cpab_integrate.cuh"
 #include "cpab_jump.cuh"
 #include "cpab_launch.h"
 
 namespace cpab {
 
-// tile_prefix[i] = sum_{j<i} ceil(n_j / tile_pts); one block, sequential
-// chunks per thread, then a block scan of the chunk sums.
-__global__ void k_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts)
+// tile_prefix[i] = sum_{j<i} ceil(n_j / tile), tile_prefix[0] = tile; one
+// block, sequential chunks per thread, then a block scan of the chunk sums.
+// ctas > 0: the tile that shares the points out evenly (balanced_tile).
+__global__ void k_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, int ctas)
 {
+    if (ctas > 0) tile_pts = balanced_tile(max((long long)(offsets[N] - offsets[0]), 0ll), N, true, tile_pts, ctas);
     __shared__ int64_t part[1024];
     const int tid = threadIdx.x, nt = blockDim.x;
     const int per = (N + nt - 1) / nt;
@@ -46,7 +50,7 @@ __global__ void k_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, in
     __syncthreads();
     int64_t acc = part[tid];
     for (int i = b; i < e; ++i) {
-        prefix[i] = acc;
+        prefix[i] = i == 0 ? tile_pts : acc;
         int64_t n = offsets[i + 1] - offsets[i];
         acc += n > 0 ? (n + tile_pts - 1) / tile_pts : 0;
     }
@@ -553,26 +557,48 @@ static int grid_for(int64_t n, int block, int per_sm = 8)
 }
 
 template <int DIM, int TESS, typename Real, int SCHEME>
-static cudaError_t launch_integrate_t(const IntegrateArgs &a, const LaunchCfg &cfg, cudaStream_t s)
+static cudaError_t launch_integrate_t(IntegrateArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    size_t smem = table_bytes<Real>(a);
-    if (sizeof(Real) == 8 && a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)a.batch.tile_pts) * sizeof(int);
+    Batch &b = a.batch;
     void (*kern)(IntegrateArgs);
-    if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
-    else kern = k_integrate<DIM, TESS, Real, SCHEME>;
-    if constexpr (sizeof(Real) == 8 && SCHEME == SCHEME_REF) {
-        // phases where the launch has points enough to fill the SMs and their scratch fits beside the tables
-        const size_t with = smem + phase_scratch_bytes(DIM, a.batch.tile_pts);
-        if (a.phases && with + 1024 <= (size_t)max_smem_optin()) {
-            kern = k_integrate_phases<DIM, TESS>;
-            smem = with;
+    size_t smem;
+    auto pick = [&](int tile) {  // the kernel and its shared memory at this many points per tile
+        smem = table_bytes<Real>(a);
+        if (sizeof(Real) == 8 && a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)tile) * sizeof(int);
+        if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
+        else kern = k_integrate<DIM, TESS, Real, SCHEME>;
+        if constexpr (sizeof(Real) == 8 && SCHEME == SCHEME_REF) {
+            // phases where the launch has points enough to fill the SMs and their scratch fits beside the tables
+            const size_t with = smem + phase_scratch_bytes(DIM, tile);
+            if (a.phases && with + 1024 <= (size_t)max_smem_optin()) {
+                kern = k_integrate_phases<DIM, TESS>;
+                smem = with;
+            }
         }
-    }
-    if (smem > kSmemOptInAbove) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem <= kSmemOptInAbove) return cudaSuccess;
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+    int grid = 0;
+    if (b.offsets) {
+        cudaError_t e = pick(b.tile_pts);
         if (e != cudaSuccess) return e;
+        grid = persistent_grid(kern, cfg, smem);
+        e = launch_tile_prefix(b.offsets, b.tile_prefix, b.N, b.tile_pts, grid, s);
+        if (e != cudaSuccess) return e;
+    } else {
+        // smaller tiles need less scratch, which may let more CTAs run, whose tiles are smaller again
+        const int most = b.tile_pts;
+        for (int pass = 0; pass < (sizeof(Real) == 8 ? 3 : 1); ++pass) {
+            const cudaError_t e = pick(b.tile_pts);
+            if (e != cudaSuccess) return e;
+            grid = persistent_grid(kern, cfg, smem);
+            b.tile_pts = balanced_tile((int64_t)b.N * b.n_uniform, b.N, false, most, grid);
+            b.tiles_per_inst = (b.n_uniform + b.tile_pts - 1) / b.tile_pts;
+        }
+        const cudaError_t e = pick(b.tile_pts);
+        if (e != cudaSuccess) return e;
+        grid = (int)std::min((int64_t)grid, b.tiles_per_inst * b.N);
     }
-    int grid = cfg.grid > 0 ? cfg.grid : persistent_grid(kern, cfg, smem);
     kern<<<grid, cfg.block, smem, s>>>(a);
     return cudaGetLastError();
 }
@@ -605,9 +631,9 @@ cudaError_t launch_integrate(const IntegrateArgs &a, int prec, int scheme, const
                      : launch_integrate_dt<3, 2>(a, prec, scheme, cfg, s);
 }
 
-cudaError_t launch_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, cudaStream_t s)
+cudaError_t launch_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, int ctas, cudaStream_t s)
 {
-    k_tile_prefix<<<1, 1024, 0, s>>>(offsets, prefix, N, tile_pts);
+    k_tile_prefix<<<1, 1024, 0, s>>>(offsets, prefix, N, tile_pts, ctas);
     return cudaGetLastError();
 }
 

@@ -41,6 +41,35 @@ inline int small_launch_tile(int64_t total, int tile_pts)
     if (t < 64) t = 64;
     return (int)(t < tile_pts ? t : tile_pts);
 }
+// Points per tile of an integration of `total` points by `ctas` persistent
+// CTAs: the configured tile where every CTA gets two of them or more; for
+// fewer points one or two tiles for every CTA, all of one size (a multiple of
+// 32, at least 64), of N ragged instances with room for as many half empty
+// last tiles.  A few CTAs with a tile more than the others would set
+// the launch's time.  Measured, us, with tiles of 2048 points (uniform: a
+// quarter of an SM's share) before and these: FP32 ragged, 16 x 10 k points
+// 116 and 87, 200 x 2.7 k 321 and 212, 48 x 28 k 300 and 278; exact scheme, 64 x
+// 5 k 308 and 171; 3D, 262144 points 205 and 163; FP64, 64 x 8192 551 and 458.
+// From two tiles per CTA on, larger tiles or shares of consecutive points lose
+// more to points that cost alike side by side than they save at their ends
+// (1024 x 8192: 793 with tiles of 2048, 841 in one share per CTA).
+__host__ __device__ inline int balanced_tile(int64_t total, int N, bool ragged, int tile_pts, int ctas)
+{
+    const int64_t most = (int64_t)ctas * tile_pts;
+    if (total >= 2 * most || N < 1) return tile_pts;
+    const int64_t slots = total > most ? 2 * (int64_t)ctas : ctas;
+    int64_t t;
+    if (ragged) {
+        const int64_t n = N / 2 < slots / 2 ? slots - N / 2 : slots - slots / 2;
+        t = (total + n - 1) / n;
+    } else {  // a whole number of tiles per instance
+        const int64_t n = slots > N ? slots / N : 1, len = total / N;
+        t = (len + n - 1) / n;
+    }
+    t = (t + 31) / 32 * 32;
+    if (t < 64) t = 64;
+    return (int)(t < tile_pts ? t : tile_pts);
+}
 int persistent_grid_impl(const void *kern, const LaunchCfg &cfg, size_t smem);
 template <typename K>
 inline int persistent_grid(K kern, const LaunchCfg &cfg, size_t smem)
@@ -52,7 +81,7 @@ cudaError_t launch_integrate(const IntegrateArgs &a, int prec, int scheme, const
 cudaError_t launch_integrate_exact1d(const IntegrateArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s);
 size_t exact1d_smem_bytes(int nC, int tile_pts, int sort, int prec);
 bool exact1d_uses_intervals(int nC, int prec);
-cudaError_t launch_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, cudaStream_t s);
+cudaError_t launch_tile_prefix(const int64_t *offsets, int64_t *prefix, int N, int tile_pts, int ctas, cudaStream_t s);
 cudaError_t launch_trajectory(const IntegrateArgs &a, int64_t nPts, cudaStream_t s);
 cudaError_t launch_cell_idx(const Tess &t, const double *pts, int32_t *out, int64_t n, cudaStream_t s);
 cudaError_t launch_calc_v(const Tess &t, const double *A, const double *pts, double *out, int64_t n, cudaStream_t s);
