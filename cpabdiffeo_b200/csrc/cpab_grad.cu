@@ -45,6 +45,7 @@
 // backward: one step at a time 30.8 ms -- 4.8 of 32 lanes active, a fallback
 // step holding up its warp -- this 4.0 ms.
 #include <algorithm>
+#include <climits>
 
 #include "cpab_integrate.cuh"
 #include "cpab_jump.cuh"
@@ -200,6 +201,12 @@ constexpr int kMoves = 48, kSaves = 24;
 // first (the 3D case above: 8 lanes 3.98 ms, 4 4.11, 16 4.54).
 constexpr int kGroup = 8;
 
+// Points a warp may have left for later, and the units of its first go at a
+// point (3D, 320 cells, 8 x 262144 points, value and gradient: 4.20 ms without
+// the queue, 4.26 with 4 units first, 4.28 with 6, 3.99 with 10, 4.06 with 16; a
+// longer queue no better).
+constexpr int kGradQueue = 64, kGradUnits = 10;
+
 // One point on its way through calc_T (the phases of integrate_jump, for one
 // lane on its own).
 template <int DIM, int TESS, typename Real>
@@ -339,11 +346,26 @@ __global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
     const int64_t n = a.n_per_inst;
     const Real *pts = static_cast<const Real *>(a.pts), *gout = static_cast<const Real *>(a.grad_out);
     Real *gin = static_cast<Real *>(a.grad_in);
-    // 32 points per warp at a time
-    for (int64_t j0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane; j0 < n;
-         j0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t gi = (int64_t)inst * n + j0 + lane;
-        const bool have = j0 + lane < n;
+    // 32 points per warp at a time: the next 32 of the instance, as far as a
+    // few units take them, or 32 of those that this left over (most points
+    // make a few moves, some make dozens: together, the few set the pace of
+    // the warp).  A warp with one go at the points takes them to their end.
+    int64_t *queue = reinterpret_cast<int64_t *>(smem_raw + jump_bytes(jc, DIM, nC, sizeof(Real))) +
+                     (threadIdx.x >> 5) * kGradQueue;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t j0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) - lane;
+    const bool once = !a.queue || n <= stride;
+    int queued = 0;
+    for (;;) {
+        const bool next = j0 < n && queued <= kGradQueue - 32;
+        if (!next && queued == 0) break;
+        const int64_t j = next ? j0 + lane : lane < queued ? queue[max(queued - 32, 0) + lane] : 0;
+        bool have = next ? j < n : lane < queued;
+        const int most_units = next && !once ? kGradUnits : INT_MAX;
+        if (next) j0 += stride;
+        else queued = max(queued - 32, 0);
+        __syncwarp();
+        const int64_t gi = (int64_t)inst * n + j;
         Real x[DIM], g[DIM], r[kMoves][DIM];
         int mi[kMoves];
         Path<DIM, TESS, Real> save[kSaves], s;
@@ -351,7 +373,7 @@ __global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
         if (have) {
             load_pt<DIM, Real>(pts, gi, x);
             s.begin(a.t, jc, x, a.nTimeSteps);
-            while (!s.done()) {
+            for (int u = 0; u < most_units && !s.done(); ++u) {
                 if (k == kMoves) {
                     ++block;
                     k = 0;
@@ -359,6 +381,17 @@ __global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
                 }
                 k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
             }
+        }
+        const bool later = have && !s.done();
+        const unsigned put = __ballot_sync(FULL, later);
+        if (later) {
+            queue[queued + __popc(put & ((1u << lane) - 1u))] = j;
+            have = false;
+            k = block = 0;
+        }
+        queued += __popc(put);
+        __syncwarp();
+        if (have) {
             // dLoss/d(position in the box)
             load_pt<DIM, Real>(gout, gi, g);
 #pragma unroll
@@ -678,16 +711,21 @@ static cudaError_t launch_grad_t(const GradArgs &a, cudaStream_t s)
 }
 
 template <int DIM, int TESS, typename Real>
-static cudaError_t launch_grad_ref_t(const GradArgs &a, cudaStream_t s)
+static cudaError_t launch_grad_ref_t(GradArgs a, cudaStream_t s)
 {
-    const size_t smem = jump_bytes(a.jump, DIM, a.t.nC, sizeof(Real));
+    LaunchCfg cfg;
+    cfg.block = a.n_per_inst * a.N >= (int64_t)num_sms() * 512 ? 256 : 64;
+    // the warps' queues, where they fit beside the tables and two CTAs do not become one
+    size_t smem = jump_bytes(a.jump, DIM, a.t.nC, sizeof(Real));
+    const size_t with = smem + cfg.block / 32 * kGradQueue * sizeof(int64_t);
+    const size_t most = (size_t)max_smem_optin() - 1024;
+    a.queue = with <= most && (with <= most / 2 || smem > most / 2);
+    if (a.queue) smem = with;
     auto kern = k_grad_ref<DIM, TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    LaunchCfg cfg;
-    cfg.block = a.n_per_inst * a.N >= (int64_t)num_sms() * 512 ? 256 : 64;
     // one wave: a CTA over it would run alone after all others
     int64_t bx = (a.n_per_inst + cfg.block - 1) / cfg.block;
     const int64_t cap = std::max<int64_t>(1, persistent_grid(kern, cfg, smem) / a.N);

@@ -27,6 +27,7 @@ struct GradArgs {
     int64_t n_per_inst;
     double dt;
     int nTimeSteps, nStepsODE, ck;
+    int queue;               // the launch gives the warps room for a queue of points (reference scheme)
 };
 
 cudaError_t launch_grad_simple(const GradArgs &a, cudaStream_t s);
