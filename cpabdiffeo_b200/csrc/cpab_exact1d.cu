@@ -618,10 +618,13 @@ __device__ bool build_intervals(const Exact1D &e, const Transit &tr, const Inter
         if (!(it.bp[k] <= it.bp[k + 1])) s_bad = 1;  // bisection would mean nothing
         Interval o;
         o.iv = o.za = o.ad = 0.0f;
-        // stays: the middle; moving: the end where the cell's velocity is smaller
-        const bool at_low = (a > 0) == (side == 2);
+        // stays: the middle; moving: the end where the cell's velocity is smaller.  Ending in the first cell, the
+        // low end: results next to zero are then sums of positive terms, right to float rounding of themselves
+        // (from the middle or the high end, of the cell's width: 1.7e-4 of results around 1e-6 before)
+        const bool first = (side == 1 ? c : tr.cn[q.rec].x) == 0;
+        const bool at_low = (a > 0) == (side == 2) || first;
         const float high = fminf(it.bp[k + 1], 1.0f);
-        o.x0 = side == 1 ? 0.5f * (it.bp[k] + high) : (at_low ? it.bp[k] : high);
+        o.x0 = side == 1 && !first ? 0.5f * (it.bp[k] + high) : (at_low ? it.bp[k] : high);
         const double x0 = o.x0, vc = a * x0 + b;
         double y0;
         bool ok;
@@ -646,6 +649,8 @@ __device__ bool build_intervals(const Exact1D &e, const Transit &tr, const Inter
             o.visits = abs((q.rec >> 1) - c) + 1;
             // resolved: the anchor moves as the interval does, away from the zero of the velocity
             ok = fabs(vc) > 1e-6 && (vc > 0) == (ve > 0);
+            // log1p far below the anchor's velocity is not
+            if (first) ok = ok && fabs(a * (double)high + b) >= 0.1 * fabs(vc);
         }
         o.y0h = (float)y0;
         o.y0l = (float)(y0 - (double)o.y0h);
