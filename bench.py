@@ -615,7 +615,8 @@ def bench_2d(args, torch, dev, exact: bool = False) -> dict:
                          "frac": achieved / peaks["fp32_simt_tflops"],
                          "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off",
                          "flop_model": f"per step 2*{C_CELL_2D}+{M_2D}, per midpoint sub-step "
-                                       f"{C_CELL_2D}+2*{M_2D}+8 (algorithmic, before compensation)",
+                                       f"{C_CELL_2D}+2*{M_2D}+8 (of the scheme's steps; composed steps take "
+                                       "several of them at once, so more is achieved than executed)",
                          "kernel_ms": kern_ms, "algorithmic_flop_per_launch": flops,
                          "traffic": TRAFFIC_2D_BYTES_PER_LAUNCH},
             "error_vs_fp64_oracle": {"max_abs": err, "points_checked": 4 * npt, "tolerance": 1e-5,
@@ -845,7 +846,7 @@ def main():
 
     from cpabdiffeo_b200 import autotune
     tuned = autotune.tune(sp, sp.tables_from_theta(theta, DT, 1), pts, offsets, _lib.SCHEME_EXACT, **p)
-    # the step (prologue + tile prefix + integration) captured once in a CUDA graph, replayed per step
+    # the step (prologue + integration) captured once in a CUDA graph, replayed per step
     graph_step = sp.capture_batched(args.theta, pts, out, offsets=offsets, scheme=_lib.SCHEME_EXACT, **p)
     graph_step.theta.copy_(theta)
     k_ev = []
@@ -1014,7 +1015,7 @@ def main():
                        "nC": NC, "integration_time": 1.0,
                        "scheme": "closed form across cells (ClosedFormInt restated: hitting times in FP64)",
                        "precision": "f32 points, f64 hitting times and expm",
-                       "step": "CUDA graph replay: theta -> A -> expm prologue, tile prefix, persistent integration",
+                       "step": "CUDA graph replay: theta -> A -> expm prologue, persistent integration",
                        "l2": "inputs larger than L2 (352 MB of points per GPU)",
                        "parallelism": f"independent shards x{world}"},
             "e2e": {"value": n_total * world * args.steps / (ms_e2e * 1e-3), "unit": UNIT,
@@ -1024,7 +1025,7 @@ def main():
                     "link_bound_points_per_s": n_total * world / (link_ms * 1e-3),
                     "pipeline": f"{args.e2e_chunks} instance groups (1/4, 1/2, 1, ..., 1, 1/2, 1/4 of the points), "
                                 "3 streams (copy in / integrate / copy out), pinned host buffers"},
-            "gpu_launches": 3 * args.steps,
+            "gpu_launches": 2 * args.steps,
             "clocks": clk.summary(),
             "work": {"cell_visits": int(cnt_h[0]), "points": int(cnt_h[3]), "failed": int(cnt_h[4])},
             "load_balance": load_balance,
@@ -1037,12 +1038,13 @@ def main():
     if rank == 0:
         peaks = measured_peaks(torch)
         achieved = flops / (kern_ms * 1e-3) / 1e12
-        line["roofline"] = {"bound": "fp64", "kernel": "k_exact1d<float>", "achieved": achieved,
+        line["roofline"] = {"bound": "fp64", "kernel": "k_exact1d_intervals", "achieved": achieved,
                             "peak": peaks["fp64_tflops"], "unit": "TFLOP/s",
                             "frac": achieved / peaks["fp64_tflops"],
                             "peak_source": "measured here: cuBLAS DGEMM 4096^3",
                             "flop_model": f"{EXACT_FLOP_PER_VISIT} per cell visit + {EXACT_FLOP_PER_POINT} per point "
-                                          "(log/exp counted as 20)",
+                                          "(log/exp counted as 20): the point-by-point walk's work, most of which "
+                                          "the kernel's intervals of the flow map spare",
                             "kernel_ms": kern_ms, "step_ms_events": step_ms,
                             "traffic": TRAFFIC_EXACT1D_BYTES_PER_POINT * n_total,
                             "traffic_note": "ncu DRAM bytes of one launch on the 2048-theta case, scaled by points",
@@ -1056,7 +1058,7 @@ def main():
             "bound": "fp32", "kernel": "k_integrate<1, float, ref>", "achieved": ach_ref,
             "peak": peaks["fp32_simt_tflops"], "unit": "TFLOP/s", "frac": ach_ref / peaks["fp32_simt_tflops"],
             "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off",
-            "flop_model": "per step 2*5+2, per midpoint sub-step 5+2*2+4 (algorithmic)"}
+            "flop_model": "per step 2*5+2, per midpoint sub-step 5+2*2+4 (of the scheme's steps)"}
         # errors: the timed FP32 result and the FP64 run against the FP64 closed form (oracle) on 64
         # instances; both GPU schemes against the reference's calc_T scheme in FP64 on 8
         from oracle import oracle as O

@@ -25,13 +25,11 @@ constexpr size_t kSmemOptInAbove = 40 * 1024;
 int num_sms();
 int max_smem_optin();
 
-// Points per tile of a uniform integration launch over `total` points: the
-// configured tile, or a smaller one (a multiple of 32, at least 64) when the
-// launch has too few points to give every SM four tiles -- one transform of a
-// few hundred thousand points would otherwise occupy fewer SMs than the GPU
-// has.  Per-point results do not depend on the tiling.  (The likelihood
-// kernels keep the configured tile: their sums follow the tiles, and a tile
-// that depended on the batch would break "the same alone and in a batch".)
+// Points per tile of a uniform 1D exact or a likelihood launch over `total`
+// points: the configured tile, or a smaller one (a multiple of 32, at least 64)
+// when the launch has too few points to give every SM four tiles -- one
+// transform of a few hundred thousand points would otherwise occupy fewer SMs
+// than the GPU has.  Per-point results do not depend on the tiling.
 inline int small_launch_tile(int64_t total, int tile_pts)
 {
     const int64_t want = 4 * (int64_t)num_sms();

@@ -129,11 +129,12 @@ int cpab_set_clamp(cpab_ctx *ctx, int enable, double lo, double hi);
 
 /* Launch shape of the integration kernel: threads per CTA (32..256, a
  * multiple of 32), resident CTAs per SM of the persistent grid, points per
- * CTA tile.  0 keeps the current value.  Used by the autotuner. */
+ * CTA tile (at most: a launch with fewer than two such tiles per CTA shares its
+ * points out evenly).  0 keeps the current value.  Used by the autotuner. */
 int cpab_set_launch(cpab_ctx *ctx, int block, int ctas_per_sm, int tile_pts);
 
 /* Cell-sort the points of each CTA tile by start cell before integrating
- * (REF / SIMPLE schemes): lanes of a warp then share cells (shared-memory
+ * (FP64; FP32 launches ignore it): lanes of a warp then share cells (shared-memory
  * broadcasts, coherent branches).  Results are unchanged (every point is
  * integrated on its own).  Off by default; the autotuner decides.  No
  * reference counterpart (the reference launches one thread per point in input
