@@ -508,14 +508,18 @@ struct Facets<2, 1> {
 // y0 + y1 + y2 >= 1/2 inside the box's three faces y_a <= 1/2 there; the centre
 // is where no corner's sum reaches 1/2.  Coordinates beyond the domain count
 // as on its boundary (the reference clamps them, calc_3Dto3D.cu:55-60), hence
-// the clamped y in the sums.  (The reference clamps z with the x box size:
-// where the two sizes differ, these facets do not describe its cells.)
+// the clamped y in the sums: there the margin does not tell a cell from its
+// neighbours for certain (past a corner of the domain every coordinate is
+// clamped, and the sums of a corner and of the centre are both 0 over all of
+// it), so margin also says how far past the domain the point is (`over`).
+// (The reference clamps z with the x box size: where the two sizes differ,
+// these facets do not describe its cells.)
 template <>
 struct Facets<3, 1> {
     bool neg[3];    // signs of sigma
     float face[3];  // 1/2, or kFar where the face ends the domain (and for the centre)
     float low[3];   // -1/2 where the opposite face ends the domain, else -kFar
-    float cap[3];   // 1/2 (centre: where the face ends the domain, else kFar)
+    float cap[3];   // 1/2 where the face ends the domain, else kFar
     bool centre;
 
     CPAB_HD void enter(const Tess &t, int c, const int *kb)
@@ -536,20 +540,28 @@ struct Facets<3, 1> {
             const bool end = kb[i] == (neg[i] ? 0 : n[i] - 1);
             face[i] = centre || end ? kFar : 0.5f;
             low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
-            cap[i] = centre && !end ? kFar : 0.5f;
+            cap[i] = end ? 0.5f : kFar;
         }
     }
     template <typename Real>
     CPAB_HD Real margin(const Real *x) const
     {
+        Real over;
+        return margin(x, over);
+    }
+    template <typename Real>
+    CPAB_HD Real margin(const Real *x, Real &over) const
+    {
         Real y[3], sum = Real(-0.5), far = kFar;
+        over = 0;
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
         for (int i = 0; i < 3; ++i) {
-            y[i] = flip(x[i], neg[i]);
-            far = least(far, face[i] - y[i]);
-            y[i] = most(least(y[i], Real(cap[i])), Real(low[i]));
+            const Real f = flip(x[i], neg[i]);
+            far = least(far, face[i] - f);
+            y[i] = most(least(f, Real(cap[i])), Real(low[i]));
+            over = most(over, size_of(f - y[i]));
             sum += y[i];
         }
         // the four corners' sums: sigma with an even number of signs flipped

@@ -207,79 +207,6 @@ constexpr int kGroup = 8;
 // longer queue no better).
 constexpr int kGradQueue = 64, kGradUnits = 10;
 
-// One point on its way through calc_T (the phases of integrate_jump, for one
-// lane on its own).
-template <int DIM, int TESS, typename Real>
-struct Path {
-    using Walker = typename WalkerOf<DIM, TESS, Real>::type;
-    Walker w;
-    Real per_m;
-    int left, steps, row, kshift, top;
-    bool sub;
-
-    __device__ __forceinline__ void to_steps(const JumpCfg &jc, int nC, int n)
-    {
-        left = n;
-        sub = false;
-        row = w.c;
-        kshift = nC;
-        top = jc.nT - 1;
-        per_m = Real(1e30);
-    }
-    __device__ __forceinline__ void to_substeps(const JumpCfg &jc, int nC, int n)
-    {
-        left = n;
-        sub = true;
-        row = jc.nT * nC + w.c;
-        kshift = 2 * nC;
-        top = jc.nS - 1;
-    }
-    __device__ __forceinline__ void begin(const Tess &t, const JumpCfg &jc, const Real *x, int nT)
-    {
-        w.place(t, x);
-        steps = 0;
-        to_steps(jc, t.nC, nT);
-    }
-    __device__ __forceinline__ bool done() const { return left == 0; }
-    // One unit; true when it moved, by the table row mi from r.
-    __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE,
-                                         int &mi, Real *r)
-    {
-        constexpr int NE = DIM * (DIM + 1);
-        const int nC = t.nC, lg = 31 - __clz(max(min(left, (int)(w.m * per_m)), 1));
-        const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
-        typename Walker::Cand q;
-        mi = l * nC + row;
-        const Real need = w.step(t, tab.map + (size_t)mi * NE, q) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
-        const bool stays = !(q.m < Real(0));
-        const bool take = stays && (l == 0 || most(w.m, q.m) >= need);
-        if (take || (l == 0 && sub)) {
-#pragma unroll
-            for (int i = 0; i < DIM; ++i) r[i] = w.p.x(i);
-            left -= n;
-            if (take) {
-                w.take(q, true);
-            } else {
-                w.leave(t, q);
-                per_m = Real(1e30);
-                row = jc.nT * nC + w.c;
-            }
-            if (left == 0 && sub) to_steps(jc, nC, --steps);
-            return true;
-        }
-        // dropped: see integrate_jump
-        per_m = (stays ? Real(0.5) : Real(0.999)) * Real(l == 0 ? nODE : n) /
-                (stays ? most(w.m, Real(1e-12)) : w.m - q.m);
-        if (l == 0) {
-            steps = left;
-            const Real keep = per_m;
-            to_substeps(jc, nC, nODE);
-            per_m = keep;
-        }
-        return false;
-    }
-};
-
 // Add each lane's NE values to the sums at G (null: nothing to add; `key`
 // tells the sums apart).  Lanes with the same key -- neighbouring points make
 // the same moves -- are added up in the warp first: the sums are spread over

@@ -253,9 +253,10 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
 //   place(t, x)          at the absolute position x (looks the cell up)
 //   place_in(t, x, c)    the same, in the given cell (margin unknown: 0)
 //   position(t, x)       the absolute position
-//   step(t, map, q)      q: the candidate end of one composed step with the
+//   step(t, map, q, one) q: the candidate end of one composed step with the
 //                        column-major map; returns |d|_1 in box units; q.m is
-//                        its margin, negative when it left the cell
+//                        its margin, negative when it left the cell (of more
+//                        than one step, also where that is not certain)
 //   take(q, yes)         moves to q, in the same cell, when yes
 //   leave(t, q)          moves to q, looking its cell up
 //   where(t, q, x)       absolute position of a candidate
@@ -478,7 +479,7 @@ struct WalkBox : WalkLocal<DIM, 2, Real> {
         enter(t, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q, bool) const
     {
         const Real len = B::advance(map, q);
         q.m = f.margin(q.x);
@@ -531,7 +532,7 @@ struct WalkTri : WalkLocal<2, 1, Real> {
         f.enter(t, cell, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q, bool) const
     {
         const Real len = B::advance(map, q);
         q.m = f.margin(q.x);
@@ -549,7 +550,15 @@ struct WalkTri : WalkLocal<2, 1, Real> {
 };
 
 // 3D type I: a new cell is looked up at the absolute position, and so is every
-// candidate where the facets do not describe the reference's cells.
+// candidate where the facets do not describe the reference's cells.  A
+// candidate past the domain, where the lookup takes the nearest point inside
+// and the margin is no distance (Facets<3, 1>), is in the cell when the lookup
+// says so, one step from the last; more than one step never end there.  Points
+// within kOver of the domain's boundary (box units) count as inside: those on
+// it stay on it up to rounding.
+template <typename Real>
+constexpr Real kOver = sizeof(Real) == 4 ? Real(1e-6) : Real(1e-12);
+
 template <typename Real>
 struct WalkTet : WalkLocal<3, 1, Real> {
     using B = WalkLocal<3, 1, Real>;
@@ -601,11 +610,15 @@ struct WalkTet : WalkLocal<3, 1, Real> {
         B::set_local(t, x, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &t, const Real *map, Cand &q) const
+    __device__ __forceinline__ Real step(const Tess &t, const Real *map, Cand &q, bool one) const
     {
         const Real len = B::advance(map, q);
         if (t.inc[0] == t.inc[2]) {
-            q.m = f.margin(q.x);
+            Real over, mq;
+            q.m = f.margin(q.x, over);
+            // (negative beyond rounding: outside for certain)
+            if (over > kOver<Real> && !(q.m < Real(-1e-5)))
+                q.m = one && lookup(t, q.x, mq) == c ? Real(0) : Real(-1e-30);
         } else if (lookup(t, q.x, q.m) != c) {
             q.m = Real(-1e-30);  // outside, nothing known of how far
         }
@@ -634,6 +647,79 @@ struct WalkerOf<2, 1, Real> {
 template <typename Real>
 struct WalkerOf<3, 1, Real> {
     using type = WalkTet<Real>;
+};
+
+// One point on its way through calc_T (the phases of integrate_jump, for one
+// lane on its own).
+template <int DIM, int TESS, typename Real>
+struct Path {
+    using Walker = typename WalkerOf<DIM, TESS, Real>::type;
+    Walker w;
+    Real per_m;
+    int left, steps, row, kshift, top;
+    bool sub;
+
+    __device__ __forceinline__ void to_steps(const JumpCfg &jc, int nC, int n)
+    {
+        left = n;
+        sub = false;
+        row = w.c;
+        kshift = nC;
+        top = jc.nT - 1;
+        per_m = Real(1e30);
+    }
+    __device__ __forceinline__ void to_substeps(const JumpCfg &jc, int nC, int n)
+    {
+        left = n;
+        sub = true;
+        row = jc.nT * nC + w.c;
+        kshift = 2 * nC;
+        top = jc.nS - 1;
+    }
+    __device__ __forceinline__ void begin(const Tess &t, const JumpCfg &jc, const Real *x, int nT)
+    {
+        w.place(t, x);
+        steps = 0;
+        to_steps(jc, t.nC, nT);
+    }
+    __device__ __forceinline__ bool done() const { return left == 0; }
+    // One unit; true when it moved, by the table row mi from r.
+    __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE,
+                                         int &mi, Real *r)
+    {
+        constexpr int NE = DIM * (DIM + 1);
+        const int nC = t.nC, lg = 31 - __clz(max(min(left, (int)(w.m * per_m)), 1));
+        const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
+        typename Walker::Cand q;
+        mi = l * nC + row;
+        const Real need = w.step(t, tab.map + (size_t)mi * NE, q, l == 0) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
+        const bool stays = !(q.m < Real(0));
+        const bool take = stays && (l == 0 || most(w.m, q.m) >= need);
+        if (take || (l == 0 && sub)) {
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) r[i] = w.p.x(i);
+            left -= n;
+            if (take) {
+                w.take(q, true);
+            } else {
+                w.leave(t, q);
+                per_m = Real(1e30);
+                row = jc.nT * nC + w.c;
+            }
+            if (left == 0 && sub) to_steps(jc, nC, --steps);
+            return true;
+        }
+        // dropped: see integrate_jump
+        per_m = (stays ? Real(0.5) : Real(0.999)) * Real(l == 0 ? nODE : n) /
+                (stays ? most(w.m, Real(1e-12)) : w.m - q.m);
+        if (l == 0) {
+            steps = left;
+            const Real keep = per_m;
+            to_substeps(jc, nC, nODE);
+            per_m = keep;
+        }
+        return false;
+    }
 };
 
 // Per-warp queue of points that the first pass left over (entries, shared memory).
@@ -743,7 +829,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                     int n;
                     const int l = level(max(togo, 1), jc.nT - 1, n);
                     Cand q;
-                    const float need = v.step(t, tab.map + (l + v.c) * NE, q) * tab.kap[l + v.c - nC];
+                    const float need = v.step(t, tab.map + (l + v.c) * NE, q, l == 0) * tab.kap[l + v.c - nC];
                     go = go && !(q.m < 0.0f) && (l == 0 || fmaxf(v.m, q.m) >= need);
                     v.take(q, go);
                     togo -= go ? n : 0;
@@ -788,7 +874,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                 int n;
                 const int l = level(max(min(left, (int)(w.m * per_m)), 1), top, n);
                 Cand q;
-                const float need = w.step(t, tab.map + (l + row) * NE, q) * tab.kap[l + row - kshift];
+                const float need = w.step(t, tab.map + (l + row) * NE, q, l == 0) * tab.kap[l + row - kshift];
                 const bool stays = !(q.m < 0.0f);  // NaN stays
                 const bool take = go && stays && (l == 0 || fmaxf(w.m, q.m) >= need);
                 // Dropped: the exit is estimated where the margin is used up at
@@ -827,7 +913,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
         if (resolve && park) {
             // the parked sub-step's end, recomputed with the same arithmetic
             Cand q;
-            w.step(t, tab.map + row * NE, q);
+            w.step(t, tab.map + row * NE, q, true);
             if (SCHEME == SCHEME_EXACT) {
                 double from[DIM], to[DIM];
                 w.position(t, from);

@@ -1,0 +1,90 @@
+"""Composed steps (cpabdiffeo_b200/csrc/cpab_jump.cuh), compiled as host code,
+against single steps in the reference's arithmetic: the whole trajectory of
+points in the domain, on its faces and corners and beyond them, fields that
+keep the domain and fields that do not.  CPU only.
+
+FP64: the two take the same steps unless rounding decides which side of a
+facet a point is on, so they differ by rounding (1e-16 a step, up to 5100
+steps, grown by a flow that expands by less than 1e3): 1e-9.
+"""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from cpabdiffeo_b200.space import Prior, build_space
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    out = tmp_path_factory.mktemp("jump") / "libjumphost.so"
+    cxx = "/usr/bin/g++" if Path("/usr/bin/g++").exists() else "g++"
+    subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-fno-fast-math", "-w",
+                    "-I", "/usr/local/cuda/include", "-I", str(ROOT / "cpabdiffeo_b200" / "csrc"),
+                    "-I", str(ROOT / "tests"), str(ROOT / "tests" / "jump_host.cpp"), "-o", str(out)], check=True)
+    return C.CDLL(str(out))
+
+
+def _expm_affine(M):
+    """expm of [M; 0] (M [.., D, D+1]) by its Taylor sum of M / 2^8, squared back."""
+    D = M.shape[-2]
+    Z = np.zeros(M.shape[:-2] + (D + 1, D + 1))
+    Z[..., :D, :] = M / 256
+    E = term = np.broadcast_to(np.eye(D + 1), Z.shape)
+    for k in range(1, 13):
+        term = term @ Z / k
+        E = E + term
+    for _ in range(8):
+        E = E @ E
+    return E[..., :D, :]
+
+
+def _walk(lib, nCs, tess, top, x, dt, nT, nODE, f32=False, r_least=1, seed=0, closed=True):
+    dim = len(nCs)
+    geo = build_space(dim, nCs, tess, xmaxs=top, zero_v_across_bdry=(closed,) * dim)
+    rng = np.random.default_rng(seed)
+    A = (geo.B @ Prior.create(geo, 0.15, 0.5).sample(1, rng)[0]).reshape(geo.nC, dim, dim + 1)
+    A, T = (np.ascontiguousarray(a) for a in (A, _expm_affine(dt * A)))
+    x = np.ascontiguousarray(x, np.float64)
+    got, want = np.empty_like(x), np.empty_like(x)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    inc = np.asarray(top) / np.asarray(nCs)
+    assert lib.jump_walk(dim, 1 if tess == "I" else 2, (C.c_int * 3)(*nCs), (C.c_double * 3)(*inc), int(f32), p(A), p(T),
+                         p(x), p(got), p(want), C.c_long(len(x)), nT, nODE, C.c_double(dt), r_least) == 1
+    return np.abs(got - want).max(1)
+
+
+def _points(rng, nCs, top, n, beyond):
+    """Uniform up to `beyond` (of a box) outside the domain on every side, a third of them past a corner of it."""
+    top = np.asarray(top, float)
+    inc = top / np.asarray(nCs)
+    x = rng.uniform(-beyond, 1 + beyond, (n, len(nCs))) * inc + rng.integers(0, np.asarray(nCs), (n, len(nCs))) * inc
+    d = rng.uniform(0, beyond, (n // 3, len(nCs))) * inc
+    x[: n // 3] = np.where(rng.uniform(size=d.shape) < 0.5, -d, top + d)
+    return x
+
+
+TETS = [((2, 2, 2), (1.0,) * 3), ((4, 4, 4), (1.0,) * 3), ((2, 3, 2), (1.0, 2.0, 1.0)), ((4, 2, 3), (1.0,) * 3),
+        ((2, 2, 4), (1.0,) * 3)]
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+@pytest.mark.parametrize("nCs,top,beyond,closed", [(*c, *b) for c in TETS for b in ((0.8, True), (0.0, False))] +
+                         [((1, 1, 1), (1.0,) * 3, b, False) for b in (0.8, 0.0)])  # (closed: no such field)
+def test_tet_keep_test_past_corners(lib, nCs, top, beyond, closed, seed):
+    """3D type I, one step at a time: a step is kept exactly when its end is in the cell, also where the point is
+    past the domain and the reference's lookup takes the coordinates of the nearest point inside.  FP32: a point
+    within float rounding of a facet (1e-7 of a box; some 1e-5 to 1e-4 of the points meet one) may part."""
+    rng = np.random.default_rng(40 + seed)
+    x = _points(rng, nCs, top, 6000, beyond)
+    err = _walk(lib, nCs, "I", top, x, 0.02, 50, 10, r_least=31, seed=seed, closed=closed)
+    print(nCs, beyond, closed, f"max {err.max():.2e} share beyond 1e-9: {(err > 1e-9).mean():.2e}")
+    assert err.max() < 1e-9
+    x = x.astype(np.float32)
+    err = _walk(lib, nCs, "I", top, x, 0.02, 50, 10, f32=True, r_least=31, seed=seed, closed=closed)
+    print(f"FP32: max {err.max():.2e} share beyond 1e-5: {(err > 1e-5).mean():.2e}")
+    assert (err > 1e-5).mean() <= 5e-4
