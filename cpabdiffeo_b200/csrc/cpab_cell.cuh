@@ -497,8 +497,11 @@ struct Facets<2, 1> {
     {
         const Real v = flip(along_x ? x[1] : x[0], neg), u = along_x ? x[0] : x[1];
         // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
-        const Real top = (u > uhi || u < -ulo) ? v : least(v, Real(0.5));
-        return least(top - size_of(u), side - v);
+        const bool hi = u > uhi, lo = u < -ulo;
+        const Real top = hi || lo ? v : least(v, Real(0.5));
+        // (and its other side stays half a box from the middle, unless that ends the domain too)
+        const Real other = hi ? Real(ulo < kFar ? kFar : 0.5f) + u : lo ? Real(uhi < kFar ? kFar : 0.5f) - u : Real(kFar);
+        return least(least(top - size_of(u), side - v), other);
     }
 };
 
@@ -512,14 +515,15 @@ struct Facets<2, 1> {
 // neighbours for certain (past a corner of the domain every coordinate is
 // clamped, and the sums of a corner and of the centre are both 0 over all of
 // it), so margin also says how far past the domain the point is (`over`).
-// (The reference clamps z with the x box size: where the two sizes differ,
-// these facets do not describe its cells.)
+// The reference clamps z with the x box size.  Where that is the smaller one,
+// the clamp lies inside the domain and takes the place of its top here; where
+// it is the larger one, these facets do not describe the cells past the top.
 template <>
 struct Facets<3, 1> {
     bool neg[3];    // signs of sigma
     float face[3];  // 1/2, or kFar where the face ends the domain (and for the centre)
     float low[3];   // -1/2 where the opposite face ends the domain, else -kFar
-    float cap[3];   // 1/2 where the face ends the domain, else kFar
+    float cap[3];   // 1/2 where the face ends the domain (z: where it is clamped), else kFar
     bool centre;
 
     CPAB_HD void enter(const Tess &t, int c, const int *kb)
@@ -537,10 +541,15 @@ struct Facets<3, 1> {
 #pragma unroll
 #endif
         for (int i = 0; i < 3; ++i) {
-            const bool end = kb[i] == (neg[i] ? 0 : n[i] - 1);
-            face[i] = centre || end ? kFar : 0.5f;
-            low[i] = kb[i] == (neg[i] ? n[i] - 1 : 0) ? -0.5f : -kFar;
-            cap[i] = end ? 0.5f : kFar;
+            const float lo = kb[i] == 0 ? 0.5f : kFar;
+            float hi = kb[i] == n[i] - 1 ? 0.5f : kFar;
+            if (i == 2 && t.inc[0] < t.inc[2]) {
+                const float z = (float)(t.hi[2] * t.inv_inc[2] - ((double)kb[2] + 0.5));
+                if (z < 0.5f) hi = z;
+            }
+            cap[i] = neg[i] ? lo : hi;
+            low[i] = neg[i] ? -hi : -lo;
+            face[i] = centre || cap[i] < kFar ? kFar : 0.5f;
         }
     }
     template <typename Real>

@@ -25,6 +25,16 @@
 // tabulated per cell and level with 2 % to spare for the float arithmetic
 // and for S being the flow only up to O(h^2).
 //
+// The argument takes facets that are planes.  The tetrahedra's are bent where
+// the domain ends (or z is clamped): beyond, the lookup takes the nearest
+// coordinate inside.  A jump therefore starts and ends inside, and in a box
+// that touches an end its margin is twice the above: between its ends the path
+// may pass the end by e_i(s) <= B_i s (tau - s) / 2 in coordinate i, B_i
+// bounding that coordinate's second derivative, sum B_i <= B; the facet's
+// functional of the clamped coordinates differs from g by sum e_i at most, and
+// g(s) + sum e_i(s) <= (tau - s) / tau (-m + 2 B tau s / 2) <= 0 for
+// m >= tau^2 B.
+//
 // A jump that is not certain is dropped, and the exit estimated from the rate
 // at which the dropped candidate lost its margin (`per_m`); the next jumps aim
 // short of it (8.7 units per point; 11.4 by bisection down the levels).  Level
@@ -215,6 +225,16 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
             for (int r = 0; r < DIM; ++r) s += fabs(a[r * NH + k]) * t.inv_inc[r];
             rho = fmax(rho, s * t.inc[k]);
         }
+        // twice the margin where a facet is bent in the box
+        float bent = 1.0f;
+        if (DIM == 3 && TESS == 1) {
+            int kb[DIM];
+            cell_box<DIM, TESS>(t, c, kb);
+            const int n[3] = {t.nC0, t.nC1, t.nC2};
+#pragma unroll
+            for (int r = 0; r < DIM; ++r)
+                if (kb[r] == 0 || kb[r] == n[r] - 1 || (r == 2 && (double)(kb[r] + 1) * t.inc[r] >= t.hi[2])) bent = 2.0f;
+        }
         const int levels = sub ? jc.nS : jc.nT, row0 = sub ? jc.nT : 0;
         const int kap0 = sub ? (jc.nT > 0 ? jc.nT - 1 : 0) : 0;
 #pragma unroll 1
@@ -233,7 +253,7 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
             if (l > 0) {
                 const float x = (float)(rho * tau), em = expm1f(x), room = 2.0f - em / x;
                 kap[(size_t)(kap0 + l - 1) * nC + c] =
-                    x < 1e-6f ? 1e-6f : (x < 1.2f ? 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
+                    x < 1e-6f ? 1e-6f : (x < 1.2f ? bent * 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
             }
             if (l + 1 < levels) {
 #pragma unroll 1
@@ -549,11 +569,10 @@ struct WalkTri : WalkLocal<2, 1, Real> {
     }
 };
 
-// 3D type I: a new cell is looked up at the absolute position, and so is every
-// candidate where the facets do not describe the reference's cells.  A
-// candidate past the domain, where the lookup takes the nearest point inside
-// and the margin is no distance (Facets<3, 1>), is in the cell when the lookup
-// says so, one step from the last; more than one step never end there.  Points
+// 3D type I: a new cell is looked up at the absolute position.  A candidate past
+// the domain, where the lookup takes the nearest point inside and the margin is
+// no distance (Facets<3, 1>), is in the cell when the lookup says so, one step
+// from the last; more than one step never end there, nor (m = 0) start.  Points
 // within kOver of the domain's boundary (box units) count as inside: those on
 // it stay on it up to rounding.
 template <typename Real>
@@ -598,7 +617,14 @@ struct WalkTet : WalkLocal<3, 1, Real> {
 #pragma unroll
         for (int i = 0; i < 3; ++i) a[i] = (Real)x[i];
         place_in(t, x, cell_at(t, a, mq));
-        m = mq;
+        set_margin(mq);
+    }
+    __device__ __forceinline__ void set_margin(Real mq)
+    {
+        const Real r[3] = {p.x(0), p.x(1), p.x(2)};
+        Real over;
+        f.margin(r, over);
+        m = over > kOver<Real> ? Real(0) : mq;
     }
     template <typename Elem>
     __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
@@ -613,15 +639,11 @@ struct WalkTet : WalkLocal<3, 1, Real> {
     __device__ __forceinline__ Real step(const Tess &t, const Real *map, Cand &q, bool one) const
     {
         const Real len = B::advance(map, q);
-        if (t.inc[0] == t.inc[2]) {
-            Real over, mq;
-            q.m = f.margin(q.x, over);
-            // (negative beyond rounding: outside for certain)
-            if (over > kOver<Real> && !(q.m < Real(-1e-5)))
-                q.m = one && lookup(t, q.x, mq) == c ? Real(0) : Real(-1e-30);
-        } else if (lookup(t, q.x, q.m) != c) {
-            q.m = Real(-1e-30);  // outside, nothing known of how far
-        }
+        Real over, mq;
+        q.m = f.margin(q.x, over);
+        // (negative beyond rounding: outside for certain, where the facets describe the cells)
+        if (over > kOver<Real> && !(q.m < Real(-1e-5) && t.inc[0] <= t.inc[2]))
+            q.m = one && lookup(t, q.x, mq) == c ? Real(0) : Real(-1e-30);
         return len;
     }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
@@ -632,7 +654,7 @@ struct WalkTet : WalkLocal<3, 1, Real> {
         const int cell = lookup(t, q.x, mq);
         B::where(t, q, x);
         place_in(t, x, cell);
-        m = mq;
+        set_margin(mq);
     }
 };
 
@@ -830,7 +852,9 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                     const int l = level(max(togo, 1), jc.nT - 1, n);
                     Cand q;
                     const float need = v.step(t, tab.map + (l + v.c) * NE, q, l == 0) * tab.kap[l + v.c - nC];
-                    go = go && !(q.m < 0.0f) && (l == 0 || fmaxf(v.m, q.m) >= need);
+                    // (a tetrahedron's margin of 0 may mean past the domain, where no jump starts)
+                    const bool sure = fmaxf(v.m, q.m) >= need && (DIM < 3 || TESS == 2 || v.m > 0.0f);
+                    go = go && !(q.m < 0.0f) && (l == 0 || sure);
                     v.take(q, go);
                     togo -= go ? n : 0;
                     go = go && togo > 0;

@@ -3,6 +3,7 @@
 
 #include <vector>
 
+#include "cell_facets_host.cpp"
 #include "cpab_jump.cuh"
 
 using namespace cpab;

@@ -43,11 +43,13 @@ def _expm_affine(M):
     return E[..., :D, :]
 
 
-def _walk(lib, nCs, tess, top, x, dt, nT, nODE, f32=False, r_least=1, seed=0, closed=True):
+def _walk(lib, nCs, tess, top, x, dt, nT, nODE, f32=False, r_least=1, seed=0, closed=True, wild=0.0):
     dim = len(nCs)
     geo = build_space(dim, nCs, tess, xmaxs=top, zero_v_across_bdry=(closed,) * dim)
     rng = np.random.default_rng(seed)
     A = (geo.B @ Prior.create(geo, 0.15, 0.5).sample(1, rng)[0]).reshape(geo.nC, dim, dim + 1)
+    if wild:  # any piecewise-affine field: it turns and jumps from cell to cell
+        A = rng.normal(0, wild, A.shape)
     A, T = (np.ascontiguousarray(a) for a in (A, _expm_affine(dt * A)))
     x = np.ascontiguousarray(x, np.float64)
     got, want = np.empty_like(x), np.empty_like(x)
@@ -88,3 +90,37 @@ def test_tet_keep_test_past_corners(lib, nCs, top, beyond, closed, seed):
     err = _walk(lib, nCs, "I", top, x, 0.02, 50, 10, f32=True, r_least=31, seed=seed, closed=closed)
     print(f"FP32: max {err.max():.2e} share beyond 1e-5: {(err > 1e-5).mean():.2e}")
     assert (err > 1e-5).mean() <= 5e-4
+
+
+@pytest.mark.parametrize("wild", [0.0, 0.6])  # a prior field, and one that turns and jumps from cell to cell
+@pytest.mark.parametrize("nCs,tess,top,closed", [
+    ((2, 2, 4), "I", (1.0,) * 3, True), ((2, 2, 4), "I", (1.0,) * 3, False), ((4, 2, 3), "I", (1.0,) * 3, True),
+    ((4, 2, 3), "I", (1.0,) * 3, False), ((1, 1, 1), "I", (1.0,) * 3, False), ((2, 3, 2), "I", (1.0, 2.0, 1.0), True),
+    ((2, 3, 2), "II", (1.0,) * 3, False), ((1, 1), "I", (1.0,) * 2, False), ((5, 3), "I", (1.0, 2.0), False),
+    ((3, 2), "II", (1.0,) * 2, False), ((5,), "II", (1.0,), False)])
+def test_jumps_equal_single_steps(lib, nCs, tess, top, closed, wild):
+    """Jumps take the steps that the scheme would: points in the domain and past it, boxes of any shape (3D type I:
+    also where the reference clamps z inside the domain or beyond its top)."""
+    rng = np.random.default_rng(50)
+    x = _points(rng, nCs, top, 20000, 0.5)
+    err = _walk(lib, nCs, tess, top, x, 0.02, 50, 10, seed=2, closed=closed, wild=wild)
+    print(nCs, tess, closed, wild, f"max {err.max():.2e} share beyond 1e-9: {(err > 1e-9).mean():.2e}")
+    assert err.max() < 1e-9
+
+
+@pytest.mark.parametrize("nCs", [(1, 1), (1, 3), (2, 1), (4, 4)])
+def test_triangle_margin_is_a_distance(lib, nCs):
+    """2D type I: no displacement shorter than the margin (|.|_1, box units) leaves the cell, past a corner of the
+    domain either, where a triangle keeps only the side towards the domain."""
+    rng = np.random.default_rng(51)
+    n, inc = 200000, 1.0 / np.asarray(nCs)
+    x = _points(rng, nCs, (1.0, 1.0), n, 3.0)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    c, c2, m = np.empty(n, np.int32), np.empty(n, np.int32), np.empty(n, np.float32)
+    args = 2, 1, (C.c_int * 3)(*nCs), (C.c_double * 3)(*inc)
+    assert lib.facet_margins(*args, p(x), p(x), p(c), p(c2), p(m), C.c_long(n)) == 1
+    step = rng.standard_normal((n, 2)) * np.where(rng.uniform(size=(n, 2)) < 0.4, 0.0, 1.0) + 1e-9
+    step *= (np.maximum(np.minimum(m, 20.0) - 1e-4, 0) / np.abs(step).sum(1))[:, None]
+    y = np.ascontiguousarray(x + step * inc)
+    assert lib.facet_margins(*args, p(y), p(y), p(c2), p(c2.copy()), p(m.copy()), C.c_long(n)) == 1
+    np.testing.assert_array_equal(c2[m > 1e-3], c[m > 1e-3])
