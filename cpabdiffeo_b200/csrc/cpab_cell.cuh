@@ -437,6 +437,8 @@ CPAB_HD float most(float a, float b) { return fmaxf(a, b); }
 CPAB_HD double most(double a, double b) { return fmax(a, b); }
 CPAB_HD float size_of(float a) { return fabsf(a); }
 CPAB_HD double size_of(double a) { return fabs(a); }
+CPAB_HD float fused(float a, float b, float c) { return fmaf(a, b, c); }
+CPAB_HD double fused(double a, double b, double c) { return fma(a, b, c); }
 
 // Box cells (1D and type II): the box's faces.
 template <int DIM, int TESS>
@@ -477,7 +479,7 @@ struct Facets<2, 1> {
     bool along_x;    // v is the y coordinate
     bool neg;        // v points down it
     float side;      // 1/2, or kFar where the side ends the domain
-    float ulo, uhi;  // 1/2 where the box's low / high face in u ends the domain, else kFar
+    float ulo, uhi;  // beyond such a side: 1/2 at the box's faces in u inside the domain, else kFar
 
     CPAB_HD void enter(const Tess &t, int c, const int *kb)
     {
@@ -487,21 +489,16 @@ struct Facets<2, 1> {
         neg = !right;
         const int k = along_x ? kb[1] : kb[0], n = along_x ? t.nC1 : t.nC0;
         const int ku = along_x ? kb[0] : kb[1], nu = along_x ? t.nC0 : t.nC1;
-        side = k == (right ? n - 1 : 0) ? kFar : 0.5f;
-        // where u's faces do not end the domain, u beyond 1/2 is outside the triangle whatever v
-        ulo = ku == 0 ? 0.5f : kFar;
-        uhi = ku == nu - 1 ? 0.5f : kFar;
+        const bool end = k == (right ? n - 1 : 0);
+        side = end ? kFar : 0.5f;
+        ulo = end && ku > 0 ? 0.5f : kFar;
+        uhi = end && ku < nu - 1 ? 0.5f : kFar;
     }
     template <typename Real>
     CPAB_HD Real margin(const Real *x) const
     {
         const Real v = flip(along_x ? x[1] : x[0], neg), u = along_x ? x[0] : x[1];
-        // beyond a corner of the domain, v itself counts (only where the side ends the domain can v exceed 1/2)
-        const bool hi = u > uhi, lo = u < -ulo;
-        const Real top = hi || lo ? v : least(v, Real(0.5));
-        // (and its other side stays half a box from the middle, unless that ends the domain too)
-        const Real other = hi ? Real(ulo < kFar ? kFar : 0.5f) + u : lo ? Real(uhi < kFar ? kFar : 0.5f) - u : Real(kFar);
-        return least(least(top - size_of(u), side - v), other);
+        return least(least(v - size_of(u), side - v), least(ulo + u, uhi - u));
     }
 };
 
@@ -514,8 +511,7 @@ struct Facets<2, 1> {
 // the clamped y in the sums: there the margin does not tell a cell from its
 // neighbours for certain (past a corner of the domain every coordinate is
 // clamped, and the sums of a corner and of the centre are both 0 over all of
-// it), so margin also says how far past the domain the point is (`over`).
-// The reference clamps z with the x box size.  Where that is the smaller one,
+// it).  The reference clamps z with the x box size.  Where that is the smaller one,
 // the clamp lies inside the domain and takes the place of its top here; where
 // it is the larger one, these facets do not describe the cells past the top.
 template <>
@@ -555,14 +551,7 @@ struct Facets<3, 1> {
     template <typename Real>
     CPAB_HD Real margin(const Real *x) const
     {
-        Real over;
-        return margin(x, over);
-    }
-    template <typename Real>
-    CPAB_HD Real margin(const Real *x, Real &over) const
-    {
         Real y[3], sum = Real(-0.5), far = kFar;
-        over = 0;
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
@@ -570,13 +559,58 @@ struct Facets<3, 1> {
             const Real f = flip(x[i], neg[i]);
             far = least(far, face[i] - f);
             y[i] = most(least(f, Real(cap[i])), Real(low[i]));
-            over = most(over, size_of(f - y[i]));
             sum += y[i];
         }
         // the four corners' sums: sigma with an even number of signs flipped
         const Real a = y[0] + y[1], d = y[0] - y[1];
         const Real all = most(size_of(a) + y[2], size_of(d) - y[2]);
         return centre ? Real(0.5) - all : least(sum, far);
+    }
+};
+
+// The same cells up to the domain's ends only: margin is that of Facets inside
+// the domain, or within kOver (box units) of it, and below kPast beyond, where
+// the clamped coordinates would say nothing certain.  One multiply-add per end
+// takes the place of Facets' clamps: kSteep (end + kOver - y), the steepness
+// keeping it out of the minimum inside.
+template <typename Real>
+struct InnerTet {
+    static constexpr Real kOver = sizeof(Real) == 4 ? Real(1e-6) : Real(1e-12);
+    static constexpr Real kSteep = sizeof(Real) == 4 ? Real(1e36f) : Real(1e200);
+    static constexpr Real kPast = Real(-1e20);
+    bool neg[3], centre;
+    Real steep[3], hi[3], lo[3];  // towards sigma: face (steep 1) or end (kSteep); away from it: end
+
+    CPAB_HD void enter(const Tess &t, int c, const int *kb)
+    {
+        Facets<3, 1> f;
+        f.enter(t, c, kb);
+        centre = f.centre;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < 3; ++i) {
+            neg[i] = f.neg[i];
+            const bool face = f.face[i] < kFar;
+            steep[i] = face ? Real(1) : kSteep;
+            hi[i] = face ? Real(0.5) : f.cap[i] < kFar ? kSteep * (Real(f.cap[i]) + kOver) : Real(INFINITY);
+            lo[i] = f.low[i] > -kFar ? kSteep * (kOver - Real(f.low[i])) : Real(INFINITY);
+        }
+    }
+    CPAB_HD Real margin(const Real *x) const
+    {
+        Real y[3], sum = Real(-0.5), far = kFar;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int i = 0; i < 3; ++i) {
+            y[i] = flip(x[i], neg[i]);
+            far = least(far, least(fused(-steep[i], y[i], hi[i]), fused(kSteep, y[i], lo[i])));
+            sum += y[i];
+        }
+        const Real a = y[0] + y[1], d = y[0] - y[1];
+        const Real all = most(size_of(a) + y[2], size_of(d) - y[2]);
+        return least(centre ? Real(0.5) - all : sum, far);
     }
 };
 

@@ -273,10 +273,11 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
 //   place(t, x)          at the absolute position x (looks the cell up)
 //   place_in(t, x, c)    the same, in the given cell (margin unknown: 0)
 //   position(t, x)       the absolute position
-//   step(t, map, q, one) q: the candidate end of one composed step with the
+//   step(t, map, q)      q: the candidate end of one composed step with the
 //                        column-major map; returns |d|_1 in box units; q.m is
-//                        its margin, negative when it left the cell (of more
-//                        than one step, also where that is not certain)
+//                        its margin, negative when it left the cell
+//   keeps(t, q)          after a single step with q.m < 0: whether it is in the
+//                        cell all the same (kept out of the units' way)
 //   take(q, yes)         moves to q, in the same cell, when yes
 //   leave(t, q)          moves to q, looking its cell up
 //   where(t, q, x)       absolute position of a candidate
@@ -304,11 +305,20 @@ struct BoxCand {
 };
 
 template <int DIM, int TESS, typename Real>
+struct FacetsOf {
+    using type = Facets<DIM, TESS>;
+};
+template <typename Real>
+struct FacetsOf<3, 1, Real> {
+    using type = InnerTet<Real>;
+};
+
+template <int DIM, int TESS, typename Real>
 struct WalkLocal {
     BoxPos<DIM, Real> p;
     int c;
     Real m;
-    Facets<DIM, TESS> f;
+    typename FacetsOf<DIM, TESS, Real>::type f;
 
     __device__ __forceinline__ void set_local(const Tess &t, const double *x, const int *kb)
     {
@@ -499,12 +509,13 @@ struct WalkBox : WalkLocal<DIM, 2, Real> {
         enter(t, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q, bool) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
         const Real len = B::advance(map, q);
         q.m = f.margin(q.x);
         return len;
     }
+    __device__ __forceinline__ bool keeps(const Tess &, const Cand &) const { return false; }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
@@ -552,12 +563,13 @@ struct WalkTri : WalkLocal<2, 1, Real> {
         f.enter(t, cell, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q, bool) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
         const Real len = B::advance(map, q);
         q.m = f.margin(q.x);
         return len;
     }
+    __device__ __forceinline__ bool keeps(const Tess &, const Cand &) const { return false; }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
@@ -570,14 +582,11 @@ struct WalkTri : WalkLocal<2, 1, Real> {
 };
 
 // 3D type I: a new cell is looked up at the absolute position.  A candidate past
-// the domain, where the lookup takes the nearest point inside and the margin is
-// no distance (Facets<3, 1>), is in the cell when the lookup says so, one step
-// from the last; more than one step never end there, nor (m = 0) start.  Points
-// within kOver of the domain's boundary (box units) count as inside: those on
-// it stay on it up to rounding.
-template <typename Real>
-constexpr Real kOver = sizeof(Real) == 4 ? Real(1e-6) : Real(1e-12);
-
+// the domain, where the lookup takes the nearest point inside and no margin is
+// a distance, is outside to a step (InnerTet: q.m < kPast); of a single step
+// `keeps` then asks the lookup.  Jumps never end there, nor (m = 0) start.
+// Points on the domain's boundary, which stay there up to rounding, count as
+// inside.
 template <typename Real>
 struct WalkTet : WalkLocal<3, 1, Real> {
     using B = WalkLocal<3, 1, Real>;
@@ -587,44 +596,31 @@ struct WalkTet : WalkLocal<3, 1, Real> {
     using B::m;
     using B::p;
 
-    static __device__ __forceinline__ int cell_at(const Tess &t, const float *a, float &mq)
-    {
-        return fast_cell_3d_tet_m(t, a, mq);
-    }
-    static __device__ __forceinline__ int cell_at(const Tess &t, const double *a, double &mq)
-    {
-        float x[3], m32;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) x[i] = (float)a[i];
-        fast_cell_3d_tet_m(t, x, m32);
-        mq = fmax((double)m32 - 1e-6, 0.0);  // a lower bound still, whatever float rounded
-        return exact_cell<3, 1>(t, a);
-    }
+    static __device__ __forceinline__ int cell_at(const Tess &t, const float *a) { return fast_cell<3, 1>(t, a); }
+    static __device__ __forceinline__ int cell_at(const Tess &t, const double *a) { return exact_cell<3, 1>(t, a); }
     // the cell of a position relative to the box of c
-    __device__ __forceinline__ int lookup(const Tess &t, const Real *x, Real &mq) const
+    __device__ __forceinline__ int lookup(const Tess &t, const Real *x) const
     {
         Real a[3];
         int kb[3];
         cell_box<3, 1>(t, c, kb);
 #pragma unroll
         for (int i = 0; i < 3; ++i) a[i] = ((Real)kb[i] + Real(0.5) + x[i]) * (Real)t.inc[i];
-        return cell_at(t, a, mq);
+        return cell_at(t, a);
     }
     template <typename Elem>
     __device__ __forceinline__ void place(const Tess &t, const Elem *x)
     {
-        Real a[3], mq;
+        Real a[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) a[i] = (Real)x[i];
-        place_in(t, x, cell_at(t, a, mq));
-        set_margin(mq);
+        place_in(t, x, cell_at(t, a));
+        set_margin();
     }
-    __device__ __forceinline__ void set_margin(Real mq)
+    __device__ __forceinline__ void set_margin()
     {
         const Real r[3] = {p.x(0), p.x(1), p.x(2)};
-        Real over;
-        f.margin(r, over);
-        m = over > kOver<Real> ? Real(0) : mq;
+        m = most(f.margin(r), Real(0));
     }
     template <typename Elem>
     __device__ __forceinline__ void place_in(const Tess &t, const Elem *x, int cell)
@@ -636,25 +632,24 @@ struct WalkTet : WalkLocal<3, 1, Real> {
         B::set_local(t, x, kb);
         m = 0;
     }
-    __device__ __forceinline__ Real step(const Tess &t, const Real *map, Cand &q, bool one) const
+    __device__ __forceinline__ Real step(const Tess &, const Real *map, Cand &q) const
     {
         const Real len = B::advance(map, q);
-        Real over, mq;
-        q.m = f.margin(q.x, over);
-        // (negative beyond rounding: outside for certain, where the facets describe the cells)
-        if (over > kOver<Real> && !(q.m < Real(-1e-5) && t.inc[0] <= t.inc[2]))
-            q.m = one && lookup(t, q.x, mq) == c ? Real(0) : Real(-1e-30);
+        q.m = f.margin(q.x);
         return len;
+    }
+    __device__ __forceinline__ bool keeps(const Tess &t, const Cand &q) const
+    {
+        return q.m < InnerTet<Real>::kPast && lookup(t, q.x) == c;
     }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
         double x[3];
-        Real mq;
-        const int cell = lookup(t, q.x, mq);
+        const int cell = lookup(t, q.x);
         B::where(t, q, x);
         place_in(t, x, cell);
-        set_margin(mq);
+        set_margin();
     }
 };
 
@@ -705,6 +700,8 @@ struct Path {
         to_steps(jc, t.nC, nT);
     }
     __device__ __forceinline__ bool done() const { return left == 0; }
+    // (of a candidate past the domain only that it is outside is known)
+    static __device__ __forceinline__ Real lost(Real m) { return DIM == 3 && TESS == 1 ? most(m, Real(-1)) : m; }
     // One unit; true when it moved, by the table row mi from r.
     __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE,
                                          int &mi, Real *r)
@@ -714,8 +711,12 @@ struct Path {
         const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
         typename Walker::Cand q;
         mi = l * nC + row;
-        const Real need = w.step(t, tab.map + (size_t)mi * NE, q, l == 0) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
-        const bool stays = !(q.m < Real(0));
+        const Real need = w.step(t, tab.map + (size_t)mi * NE, q) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
+        bool stays = !(q.m < Real(0));
+        if (!stays && l == 0 && w.keeps(t, q)) {
+            stays = true;
+            q.m = 0;
+        }
         const bool take = stays && (l == 0 || most(w.m, q.m) >= need);
         if (take || (l == 0 && sub)) {
 #pragma unroll
@@ -733,7 +734,7 @@ struct Path {
         }
         // dropped: see integrate_jump
         per_m = (stays ? Real(0.5) : Real(0.999)) * Real(l == 0 ? nODE : n) /
-                (stays ? most(w.m, Real(1e-12)) : w.m - q.m);
+                (stays ? most(w.m, Real(1e-12)) : w.m - lost(q.m));
         if (l == 0) {
             steps = left;
             const Real keep = per_m;
@@ -767,6 +768,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
     using Walker = typename WalkerOf<DIM, TESS, float>::type;
     using Cand = typename Walker::Cand;
     constexpr int NE = DIM * (DIM + 1);
+    constexpr bool kTet = DIM == 3 && TESS == 1;
     constexpr float kHuge = 1e30f;
     const int lane = threadIdx.x & 31, nC = t.nC;
     const unsigned lt = (1u << lane) - 1u;
@@ -851,9 +853,9 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                     int n;
                     const int l = level(max(togo, 1), jc.nT - 1, n);
                     Cand q;
-                    const float need = v.step(t, tab.map + (l + v.c) * NE, q, l == 0) * tab.kap[l + v.c - nC];
+                    const float need = v.step(t, tab.map + (l + v.c) * NE, q) * tab.kap[l + v.c - nC];
                     // (a tetrahedron's margin of 0 may mean past the domain, where no jump starts)
-                    const bool sure = fmaxf(v.m, q.m) >= need && (DIM < 3 || TESS == 2 || v.m > 0.0f);
+                    const bool sure = fmaxf(v.m, q.m) >= need && (!kTet || v.m > 0.0f);
                     go = go && !(q.m < 0.0f) && (l == 0 || sure);
                     v.take(q, go);
                     togo -= go ? n : 0;
@@ -892,26 +894,39 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
         // units without branches: lanes that wait run along without effect
 #pragma unroll 1
         for (int h = 0; h < kRounds; ++h) {
-            bool go = active && !park && left > 0, out = false;
+            bool go = active && !park && left > 0, out = false, past = false;
 #pragma unroll
             for (int u = 0; u < kUnits; ++u) {
                 int n;
                 const int l = level(max(min(left, (int)(w.m * per_m)), 1), top, n);
                 Cand q;
-                const float need = w.step(t, tab.map + (l + row) * NE, q, l == 0) * tab.kap[l + row - kshift];
+                const float need = w.step(t, tab.map + (l + row) * NE, q) * tab.kap[l + row - kshift];
                 const bool stays = !(q.m < 0.0f);  // NaN stays
                 const bool take = go && stays && (l == 0 || fmaxf(w.m, q.m) >= need);
                 // Dropped: the exit is estimated where the margin is used up at
                 // the rate it was lost (a candidate inside, but not certain:
                 // at half its steps).  The estimate stays below n steps, so the
                 // next jump from here is a shorter one.
-                if (go && !take)
+                if (go && !take) {
                     per_m = __fdividef((stays ? 0.5f : 0.999f) * (float)(l == 0 && !sub ? nODE : n),
-                                       stays ? fmaxf(w.m, 1e-12f) : w.m - q.m);
+                                       stays ? fmaxf(w.m, 1e-12f) : w.m - (kTet ? fmaxf(q.m, -1.0f) : q.m));
+                    if (kTet) past = q.m < InnerTet<float>::kPast;
+                }
                 out = out || (go && !take && l == 0);
                 w.take(q, take);
                 left -= take ? n : 0;
                 go = go && !out && left > 0;
+            }
+            if (kTet && out && past) {
+                // past the domain: the lookup says whether the step left the cell
+                Cand q;
+                w.step(t, tab.map + row * NE, q);
+                if (w.keeps(t, q)) {
+                    q.m = 0.0f;
+                    w.take(q, true);
+                    --left;
+                    out = false;
+                }
             }
             if (SCHEME == SCHEME_SIMPLE) {
                 park = park || out;
@@ -937,7 +952,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
         if (resolve && park) {
             // the parked sub-step's end, recomputed with the same arithmetic
             Cand q;
-            w.step(t, tab.map + row * NE, q, true);
+            w.step(t, tab.map + row * NE, q);
             if (SCHEME == SCHEME_EXACT) {
                 double from[DIM], to[DIM];
                 w.position(t, from);
