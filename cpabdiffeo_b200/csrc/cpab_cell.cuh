@@ -437,6 +437,16 @@ CPAB_HD float most(float a, float b) { return fmaxf(a, b); }
 CPAB_HD double most(double a, double b) { return fmax(a, b); }
 CPAB_HD float size_of(float a) { return fabsf(a); }
 CPAB_HD double size_of(double a) { return fabs(a); }
+// towards zero, saturating; NaN -> 0 (a conversion on the device)
+template <typename Real>
+CPAB_HD int whole(Real v)
+{
+#ifdef __CUDA_ARCH__
+    return (int)v;
+#else
+    return v >= Real(2147483647) ? 2147483647 : v > Real(-2147483648.0) ? (int)v : v == v ? -2147483647 - 1 : 0;
+#endif
+}
 CPAB_HD float fused(float a, float b, float c) { return fmaf(a, b, c); }
 CPAB_HD double fused(double a, double b, double c) { return fma(a, b, c); }
 

@@ -33,7 +33,9 @@
 // bounding that coordinate's second derivative, sum B_i <= B; the facet's
 // functional of the clamped coordinates differs from g by sum e_i at most, and
 // g(s) + sum e_i(s) <= (tau - s) / tau (-m + 2 B tau s / 2) <= 0 for
-// m >= tau^2 B.
+// m >= tau^2 B.  With x boxes larger than z boxes the cells past the top are
+// others altogether (the lookup folds z back into the box): no jumps in a box
+// below it whose field crosses it.
 //
 // A jump that is not certain is dropped, and the exit estimated from the rate
 // at which the dropped candidate lost its margin (`per_m`); the next jumps aim
@@ -227,13 +229,21 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
         }
         // twice the margin where a facet is bent in the box
         float bent = 1.0f;
-        if (DIM == 3 && TESS == 1) {
+        if constexpr (DIM == 3 && TESS == 1) {
             int kb[DIM];
             cell_box<DIM, TESS>(t, c, kb);
             const int n[3] = {t.nC0, t.nC1, t.nC2};
 #pragma unroll
             for (int r = 0; r < DIM; ++r)
                 if (kb[r] == 0 || kb[r] == n[r] - 1 || (r == 2 && (double)(kb[r] + 1) * t.inc[r] >= t.hi[2])) bent = 2.0f;
+            if (t.inc[0] > t.inc[2] && kb[DIM - 1] == n[2] - 1) {
+                // the velocity across the top, at its middle and the most it differs from that
+                const double *az = a + 2 * NH;
+                const double ax = az[0] * t.inc[0], ay = az[1] * t.inc[1], top = az[2] * t.span[2] + az[3];
+                const double mid = ax * (kb[0] + 0.5) + ay * (kb[1] + 0.5) + top;
+                const double size = fabs(ax) * (kb[0] + 1) + fabs(ay) * (kb[1] + 1) + fabs(az[2] * t.span[2]) + fabs(az[3]);
+                if (!(fabs(mid) + 0.5 * (fabs(ax) + fabs(ay)) <= 1e-12 * size)) bent = CUDART_INF_F;
+            }
         }
         const int levels = sub ? jc.nS : jc.nT, row0 = sub ? jc.nT : 0;
         const int kap0 = sub ? (jc.nT > 0 ? jc.nT - 1 : 0) : 0;
@@ -253,7 +263,7 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
             if (l > 0) {
                 const float x = (float)(rho * tau), em = expm1f(x), room = 2.0f - em / x;
                 kap[(size_t)(kap0 + l - 1) * nC + c] =
-                    x < 1e-6f ? 1e-6f : (x < 1.2f ? bent * 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
+                    x < 1e-6f && bent < 3.0f ? 1e-6f : (x < 1.2f ? bent * 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
             }
             if (l + 1 < levels) {
 #pragma unroll 1
@@ -707,7 +717,7 @@ struct Path {
                                          int &mi, Real *r)
     {
         constexpr int NE = DIM * (DIM + 1);
-        const int nC = t.nC, lg = 31 - __clz(max(min(left, (int)(w.m * per_m)), 1));
+        const int nC = t.nC, lg = 31 - __clz(max(min(left, whole(w.m * per_m)), 1));
         const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
         typename Walker::Cand q;
         mi = l * nC + row;
@@ -898,7 +908,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
 #pragma unroll
             for (int u = 0; u < kUnits; ++u) {
                 int n;
-                const int l = level(max(min(left, (int)(w.m * per_m)), 1), top, n);
+                const int l = level(max(min(left, whole(w.m * per_m)), 1), top, n);
                 Cand q;
                 const float need = w.step(t, tab.map + (l + row) * NE, q) * tab.kap[l + row - kshift];
                 const bool stays = !(q.m < 0.0f);  // NaN stays

@@ -43,11 +43,12 @@ def _expm_affine(M):
     return E[..., :D, :]
 
 
-def _walk(lib, nCs, tess, top, x, dt, nT, nODE, f32=False, r_least=1, seed=0, closed=True, wild=0.0):
+def _walk(lib, nCs, tess, top, x, dt, nT, nODE, f32=False, r_least=1, seed=0, closed=True, wild=0.0, A=None):
     dim = len(nCs)
     geo = build_space(dim, nCs, tess, xmaxs=top, zero_v_across_bdry=(closed,) * dim)
     rng = np.random.default_rng(seed)
-    A = (geo.B @ Prior.create(geo, 0.15, 0.5).sample(1, rng)[0]).reshape(geo.nC, dim, dim + 1)
+    if A is None:
+        A = (geo.B @ Prior.create(geo, 0.15, 0.5).sample(1, rng)[0]).reshape(geo.nC, dim, dim + 1)
     if wild:  # any piecewise-affine field: it turns and jumps from cell to cell
         A = rng.normal(0, wild, A.shape)
     A, T = (np.ascontiguousarray(a) for a in (A, _expm_affine(dt * A)))
