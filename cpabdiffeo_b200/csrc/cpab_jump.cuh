@@ -16,7 +16,7 @@
 //     bounds the second derivative of every facet functional along the path
 //     over the jump's time tau: a functional g with g(0), g(tau) <= 0, one of
 //     them <= -tau^2 B / 2 and |g''| <= B stays <= 0 in between.
-// With L the cell's linear part in box units, rho = |L|_1, x = rho tau: the
+// With L the cell's linear part in box units, rho = |L|_1, x = rho |tau|: the
 // path's velocity is e^{L t} v0, so B <= rho e^x |v0|_1 (facet functionals
 // have coefficients 0, +-1), and its displacement d = tau phi(L tau) v0,
 // phi(z) = (e^z - 1)/z, gives |v0|_1 <= |d|_1 / (tau (2 - phi(x))).  So the
@@ -261,7 +261,7 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
                 m[DIM * DIM + r] = (Real)(off * t.inv_inc[r]);
             }
             if (l > 0) {
-                const float x = (float)(rho * tau), em = expm1f(x), room = 2.0f - em / x;
+                const float x = (float)(rho * fabs(tau)), em = expm1f(x), room = 2.0f - em / x;
                 kap[(size_t)(kap0 + l - 1) * nC + c] =
                     x < 1e-6f && bent < 3.0f ? 1e-6f : (x < 1.2f ? bent * 0.51f * x * (1.0f + em) / room : CUDART_INF_F);
             }

@@ -125,3 +125,17 @@ def test_triangle_margin_is_a_distance(lib, nCs):
     y = np.ascontiguousarray(x + step * inc)
     assert lib.facet_margins(*args, p(y), p(y), p(c2), p(c2.copy()), p(m.copy()), C.c_long(n)) == 1
     np.testing.assert_array_equal(c2[m > 1e-3], c[m > 1e-3])
+
+
+@pytest.mark.parametrize("dt", [0.02, -0.02])
+def test_arcs_over_a_face_in_either_direction_of_time(lib, dt):
+    """Circles around a point near a face that reach over it by up to a fifth of their radius: a jump from before the
+    arc to behind it would miss the cell beyond, where nothing moves.  A negative dt is a flow like any other."""
+    rng = np.random.default_rng(52)
+    ang, r = rng.uniform(0, 2 * np.pi, 4000), rng.uniform(0.04, 0.06, 4000)
+    x = np.stack([0.45 + r * np.cos(ang), 0.5 + r * np.sin(ang)], 1)
+    A = np.zeros((2, 2, 3))
+    A[0] = [[0, -1, 0.5], [1, 0, -0.45]]
+    err = _walk(lib, (2, 1), "II", (1.0, 1.0), x, dt, 64, 10, A=A)
+    print(dt, f"max {err.max():.2e} share beyond 1e-9: {(err > 1e-9).mean():.2e}")
+    assert err.max() < 1e-9
