@@ -275,7 +275,7 @@ static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *T
         need = exact1d_smem_bytes(ctx->t.nC, ctx->cfg.tile_pts, ctx->cfg.sort,
                                   precision == CPAB_F64 ? PREC_F64 : PREC_F32);
     } else {
-        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx);
+        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx) + kIntegrateStatic;
     }
     if (need > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch (%zu bytes) exceed shared memory", need);

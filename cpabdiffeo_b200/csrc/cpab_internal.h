@@ -41,6 +41,7 @@ struct Batch {
 // for k = log2 of a step count.
 struct JumpCfg {
     int nT, nS, r, mul;
+    int queue;  // the launch gives the warps room for their queues
 };
 
 struct IntegrateArgs {

@@ -76,10 +76,11 @@ template <int DIM>
 constexpr int kJumpCtas = DIM == 3 ? 2 : 4;
 
 // Shared memory of the tables: the maps (increments M - I, column-major),
-// then kappa of every level above 0.
+// then kappa of every level above 0.  (Level 0 reads kappa too and ignores it:
+// an entry before its own table's, in the maps where there is none.)
 __host__ __device__ inline size_t jump_bytes(const JumpCfg &j, int dim, int nC, size_t el = sizeof(float))
 {
-    const size_t kap = (size_t)(j.nT > 0 ? j.nT - 1 : 0) + j.nS;  // one row to spare: level 0 reads a row too
+    const size_t kap = (size_t)(j.nT > 0 ? j.nT - 1 : 0) + j.nS - 1;
     const size_t b = ((size_t)(j.nT + j.nS) * dim * (dim + 1) + kap) * nC * el;
     return (b + 15) & ~(size_t)15;
 }
@@ -104,7 +105,7 @@ inline JumpCfg jump_cfg(int dim, int nC, int nTimeSteps, int nStepsODE, int sche
     const int lt = log2i(nTimeSteps);
     int ls = log2i(scheme == SCHEME_SIMPLE ? (long long)nTimeSteps * nStepsODE : nStepsODE);
     if (ls > 8) ls = 8;
-    JumpCfg j{0, 0, 0, 0};
+    JumpCfg j{0, 0, 0, 0, 0};
     for (int r : {1, 2, 3, 4, 5, 6, 31}) {
         if (r < r_least) continue;
         j.r = r;
@@ -757,6 +758,7 @@ struct Path {
 
 // Per-warp queue of points that the first pass left over (entries, shared memory).
 constexpr int kQueue = 64;
+__host__ __device__ inline size_t queue_bytes(int block) { return (size_t)(block / 32) * kQueue * sizeof(unsigned short); }
 
 // The FP32 twin of integrate_range.  Warps claim 32 points of the range at a
 // time and try to carry them through all their closed-form steps at once
@@ -840,6 +842,16 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
     auto refill = [&]() {
         const unsigned idle = __ballot_sync(FULL, !active);
         const int want = __popc(idle);
+        if (!queues) {
+            int b = 0;
+            if (lane == 0) b = atomicAdd(claim, want);
+            b = __shfl_sync(FULL, b, 0);
+            more = b + want < n_range;
+            const int k = b + __popc(idle & lt);
+            if (!active && k < n_range) start(k);
+            __syncwarp();
+            return;
+        }
         while (more && queued < want) {
             int b = 0;
             if (lane == 0) b = atomicAdd(claim, 32);

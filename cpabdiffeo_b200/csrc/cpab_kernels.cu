@@ -112,7 +112,8 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
     int *s_perm = s_cell + a.batch.tile_pts;
     __shared__ TileInfo s_tile;
     __shared__ unsigned long long s_claim;
-    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
+    // float: the warps' queues, after the tables
+    unsigned short *s_queue = a.jump.queue ? reinterpret_cast<unsigned short *>(smem_raw + table_bytes<Real>(a)) : nullptr;
 
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
@@ -564,6 +565,7 @@ static cudaError_t launch_integrate_t(IntegrateArgs a, const LaunchCfg &cfg, cud
     size_t smem;
     auto pick = [&](int tile) {  // the kernel and its shared memory at this many points per tile
         smem = table_bytes<Real>(a);
+        if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
         if (sizeof(Real) == 8 && a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)tile) * sizeof(int);
         if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
         else kern = k_integrate<DIM, TESS, Real, SCHEME>;

@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
     double *s_term = reinterpret_cast<double *>(
         smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     __shared__ unsigned long long s_claim;
-    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
+    // float: the warps' queues, after all else
+    unsigned short *s_queue = a.jump.queue ? reinterpret_cast<unsigned short *>(s_term + a.tile_pts) : nullptr;
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t tpi = ((int64_t)a.n_lm + a.tile_pts - 1) / a.tile_pts;
@@ -135,9 +136,10 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
 }
 
 template <int DIM, int TESS, typename Real>
-cudaError_t launch_t(const LandmarkArgs &a, const LaunchCfg &cfg, cudaStream_t s)
+cudaError_t launch_t(LandmarkArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = landmark_smem_bytes(a.t, a.tile_pts, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    size_t smem = landmark_smem_bytes(a.t, a.tile_pts, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
     auto kern = k_landmark_ll<DIM, TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

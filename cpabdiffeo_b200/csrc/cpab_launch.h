@@ -22,6 +22,9 @@ struct LaunchCfg {
 // dynamic size exceeds this (their static shared memory comes on top).
 constexpr size_t kSmemOptInAbove = 40 * 1024;
 
+// Static shared memory of k_integrate* (48 bytes), and at most of any kernel that integrates.
+constexpr size_t kIntegrateStatic = 48, kStaticSmem = 320;
+
 int num_sms();
 int max_smem_optin();
 
@@ -67,6 +70,14 @@ __host__ __device__ inline int balanced_tile(int64_t total, int N, bool ragged, 
     t = (t + 31) / 32 * 32;
     if (t < 64) t = 64;
     return (int)(t < tile_pts ? t : tile_pts);
+}
+// Room for the warps' queues of an FP32 integration (integrate_jump), `bytes`,
+// behind its other shared memory; false, and none, where that fills an SM.
+inline bool add_queue(size_t &smem, size_t bytes)
+{
+    if (smem + bytes + kStaticSmem > (size_t)max_smem_optin()) return false;
+    smem += bytes;
+    return true;
 }
 int persistent_grid_impl(const void *kern, const LaunchCfg &cfg, size_t smem);
 template <typename K>

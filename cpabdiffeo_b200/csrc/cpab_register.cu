@@ -491,7 +491,8 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 3 : 1) k_register_ll(
         smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     double *s_grp = reinterpret_cast<double *>(s_pos + a.tile_px);
     __shared__ unsigned long long s_claim;
-    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
+    // float: the warps' queues, after all else
+    unsigned short *s_queue = a.jump.queue ? reinterpret_cast<unsigned short *>(s_grp + (a.tile_px + 31) / 32) : nullptr;
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t npx = (int64_t)a.H * a.W;
@@ -572,9 +573,10 @@ size_t register_smem_bytes(int nC, int tile_px, int prec, const JumpCfg &jump)
 }
 
 template <int TESS, typename Real>
-static cudaError_t launch_register_t(const RegisterArgs &a, const LaunchCfg &cfg, cudaStream_t s)
+static cudaError_t launch_register_t(RegisterArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = register_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    size_t smem = register_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
     auto kern = k_register_ll<TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

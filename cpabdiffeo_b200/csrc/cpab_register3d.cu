@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
         smem_raw + (kJump ? jump_bytes(a.jump, DIM, a.t.nC) : (size_t)2 * a.t.nC * NE * sizeof(double)));
     double *s_grp = s_pos + 3 * (size_t)a.tile_px;  // 32-voxel group sums of the likelihood
     __shared__ unsigned long long s_claim;
-    __shared__ unsigned short s_queue[sizeof(Real) == 4 ? 8 * kQueue : 1];  // at most 8 warps
+    // float: the warps' queues, after all else
+    unsigned short *s_queue = a.jump.queue ? reinterpret_cast<unsigned short *>(s_grp + (a.tile_px + 31) / 32) : nullptr;
     const int tab = a.t.nC * NE;
     const Real h = (Real)(a.dt / (double)a.nStepsODE);
     const int64_t nvx = (int64_t)a.H * a.W * a.D;
@@ -257,9 +258,10 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
 }
 
 template <int TESS, typename Real>
-cudaError_t launch_register3d_t(const Register3dArgs &a, const LaunchCfg &cfg, cudaStream_t s)
+cudaError_t launch_register3d_t(Register3dArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
-    const size_t smem = register3d_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    size_t smem = register3d_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
+    if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
     auto kern = k_register3d_ll<TESS, Real>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
