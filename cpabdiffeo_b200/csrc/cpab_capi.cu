@@ -10,10 +10,10 @@ using namespace cpab;
 
 thread_local char cpab::g_thread_err[512];
 
-// Tile scratch of a cell-sorted launch next to the tables.
-static size_t sort_smem(const cpab_ctx *c)
+// Tile scratch of a cell-sorted launch next to the tables (FP32 launches don't sort).
+static size_t sort_smem(const cpab_ctx *c, int prec)
 {
-    return c->cfg.sort ? ((size_t)c->t.nC + 2 * (size_t)c->cfg.tile_pts) * sizeof(int) : 0;
+    return c->cfg.sort && prec == CPAB_F64 ? ((size_t)c->t.nC + 2 * (size_t)c->cfg.tile_pts) * sizeof(int) : 0;
 }
 
 JumpCfg cpab::ctx_jump(const cpab_ctx *c, int nTimeSteps, int nStepsODE, int scheme, size_t scratch)
@@ -26,7 +26,7 @@ static size_t tables_smem(const cpab_ctx *c, int prec, int scheme, int nTimeStep
 {
     // float64: A and T; float32: the composed-step tables
     if (prec == CPAB_F64) return (size_t)c->t.nC * cell_len(c) * 2 * 8;
-    return jump_bytes(ctx_jump(c, nTimeSteps, nStepsODE, scheme, sort_smem(c)), c->t.dim, c->t.nC);
+    return jump_bytes(ctx_jump(c, nTimeSteps, nStepsODE, scheme, 0), c->t.dim, c->t.nC);
 }
 
 int cpab::max_smem_optin()
@@ -275,7 +275,7 @@ static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *T
         need = exact1d_smem_bytes(ctx->t.nC, ctx->cfg.tile_pts, ctx->cfg.sort,
                                   precision == CPAB_F64 ? PREC_F64 : PREC_F32);
     } else {
-        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx) + kIntegrateStatic;
+        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx, precision) + kIntegrateStatic;
     }
     if (need > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch (%zu bytes) exceed shared memory", need);
@@ -306,7 +306,7 @@ static IntegrateArgs make_args(cpab_ctx *ctx, const double *signedA, const doubl
     a.facets = ctx->facets_dev;
     a.nbr = ctx->nbr_dev;
     a.nF = ctx->nF;
-    a.jump = ctx_jump(ctx, nTimeSteps, nStepsODE, scheme, sort_smem(ctx));
+    a.jump = ctx_jump(ctx, nTimeSteps, nStepsODE, scheme, 0);
     return a;
 }
 

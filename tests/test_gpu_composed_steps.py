@@ -84,3 +84,18 @@ def test_wide_spaces_and_nan(nCs):
     err = (got.double() - want)[keep].abs().amax(1)
     # the field jumps across faces, so a point at a face may part: allow 1 %
     assert (err > 1e-5).double().mean().item() <= 1e-2
+
+
+@pytest.mark.parametrize("nCs", [(16, 16), (24, 24), (6, 6, 6), (1500, 1)])
+def test_cell_sorting_changes_nothing(nCs):
+    """FP32 ignores it: the same table levels, so the same bits."""
+    dim = len(nCs)
+    rng = np.random.default_rng(5)
+    sp = CpaSpace([0.0] * dim, [1.0] * dim, nCs, tess="II", device=DEV)
+    tables = sp.tables_from_A(torch.as_tensor(rng.normal(0, 0.2, (1, sp.D)), device=DEV), 0.02)
+    x = torch.as_tensor(rng.uniform(0, 1, (20000, dim)), dtype=torch.float32, device=DEV)
+    got = []
+    for sort, tile in ((False, 2048), (True, 2048), (True, 16384)):
+        sp.set_launch(tile_pts=tile, cell_sort=sort)
+        got.append(sp.calc_T_batched(tables, x, torch.empty_like(x), dt=0.02, nTimeSteps=50, nStepsODEsolver=100))
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])

@@ -67,3 +67,16 @@ def test_likelihoods(ctx, prec):
             args = [h, BASE, BASE, 1, BASE, BASE] + [64] * dim + [0.05, prec, 0.02, 50, 100, BASE, None, None, 0, None, None]
             st = (lib.cpab_register_ll if dim == 2 else lib.cpab_register3d_ll)(*args)
             assert st == want, (dim, cells, lib.cpab_last_error_string(h))
+
+
+@pytest.mark.parametrize("scheme", [0, 1])
+@pytest.mark.parametrize("dim,nCs", [(1, (100,)), (2, (4, 4)), (2, (69, 70)), (3, (4, 4, 4))])
+def test_fp32_needs_no_room_to_sort(ctx, dim, nCs, scheme):
+    """FP32 launches ignore cell sorting: it takes nothing from the space or the tile."""
+    lib, make = ctx
+    h = make(dim, 2, nCs)
+    lib.cpab_set_cell_sort(h, 1)
+    for tile in (2048, 65536):
+        lib.cpab_set_launch(h, 0, 0, tile)
+        st = lib.cpab_calc_T(h, BASE, BASE, BASE, BASE, 0, F32, scheme, 0.02, 50, 100, None, None)
+        assert st == OK, (tile, lib.cpab_last_error_string(h))
