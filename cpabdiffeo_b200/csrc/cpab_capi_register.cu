@@ -632,8 +632,13 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
     CPAB_CHECK_ALIGN(ctx, {B, 8, "B"}, {signedA, 8, "signedA"}, {Trels, 8, "Trels"}, {pts, pa, "pts"},
                      {grad_out, pa, "grad_out"}, {out, pa, "out"}, {grad_pts, pa, "grad_pts"}, {gA, 8, "gA"},
                      {dtheta, 8, "dtheta"}, {workspace, 8, "workspace"});
-    // tables (reference scheme: the closed-form steps too) in shared memory
-    if ((size_t)2 * ctx->t.nC * cell_len(ctx) * 8 > (size_t)max_smem_optin())
+    // tables in shared memory: A and the sums (midpoint scheme), the composed steps (reference scheme), of which
+    // level 0 alone takes as many bytes in FP64
+    const size_t el = precision == CPAB_F64 ? 8 : 4;
+    const size_t rows = (size_t)n_per_inst / ((size_t)ctx->t.nC * (ctx->t.dim + 1));
+    const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el, rows);
+    if ((size_t)2 * ctx->t.nC * cell_len(ctx) * 8 > (size_t)max_smem_optin() ||
+        (ref && jump_bytes(jump, ctx->t.dim, ctx->t.nC, el) > (size_t)max_smem_optin()))
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables exceed shared memory");
     const size_t ck_bytes = cpab_grad_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck);
     const size_t need = ref ? cpab_grad_ref_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck) : ck_bytes;
@@ -669,9 +674,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
             e = cudaMemsetAsync(a.gT, 0, 2 * sum_bytes, s);
             // The sums of the levels above 0 take the place of the checkpoints.  As many levels as one
             // checkpoint has room for, so that the result does not depend on ck.
-            const size_t rows = (size_t)n_per_inst / ((size_t)ctx->t.nC * (ctx->t.dim + 1));
-            const size_t el = precision == CPAB_F64 ? 8 : 4, most = (size_t)max_smem_optin() - 1024;
-            a.jump = grad_jump(ctx, nTimeSteps, nStepsODE, most, el, rows);
+            a.jump = jump;
             a.gL = static_cast<double *>(workspace);
             const size_t extra = (size_t)(a.jump.nT - 1 + a.jump.nS - 1);
             if (e == cudaSuccess && extra) e = cudaMemsetAsync(a.gL, 0, extra * N * DA * sizeof(double), s);
