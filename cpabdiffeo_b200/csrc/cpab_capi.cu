@@ -411,6 +411,17 @@ int cpab_calc_trajectory(cpab_ctx *ctx, const double *signedA, const double *Tre
 
 }  // extern "C"
 
+int cpab::transform_points(cpab_ctx *ctx, const double *signedA, const double *Trels, const void *pts, void *out, int N,
+                           int64_t n_per_inst, int precision, double dt, int nTimeSteps, int nStepsODE, cudaStream_t s)
+{
+    IntegrateArgs a = make_args(ctx, signedA, Trels, pts, out, CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE, nullptr);
+    a.clamp = a.sort = 0;
+    a.cancel = nullptr;
+    a.batch.N = N;
+    a.batch.n_uniform = n_per_inst;
+    return run_integrate(ctx, a, precision, CPAB_SCHEME_REF, s);
+}
+
 // ---------------------------------------------------------------------------
 // Allocation-free ragged batch (cpab_calc_T_batched_noalloc).
 //

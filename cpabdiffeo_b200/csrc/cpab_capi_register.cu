@@ -686,8 +686,8 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         if (e != cudaSuccess) return cuda_status(ctx, e, "grad launch");
     }
     if (ref && out && n_per_inst > 0) {
-        const int st = cpab_calc_T_batched(ctx, signedA, Trels, pts, out, N, nullptr, n_per_inst, nullptr, 0, precision,
-                                           CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE, nullptr, stream);
+        const int st = transform_points(ctx, signedA, Trels, pts, out, N, n_per_inst, precision, dt, nTimeSteps,
+                                        nStepsODE, s);
         if (st != CPAB_OK) return st;
     }
     if (dtheta) {

@@ -94,6 +94,9 @@ inline const volatile int *cancel_ptr(const cpab_ctx *c)
 int max_smem_optin();
 // The FP32 integration's table levels, `scratch` bytes of shared memory being needed beside them.
 JumpCfg ctx_jump(const cpab_ctx *c, int nTimeSteps, int nStepsODE, int scheme, size_t scratch);
+// calc_T of N x n points as the kernels know it: no checks, no clamp, no cancel flag; out may be pts.
+int transform_points(cpab_ctx *c, const double *signedA, const double *Trels, const void *pts, void *out, int N,
+                     int64_t n_per_inst, int precision, double dt, int nTimeSteps, int nStepsODE, cudaStream_t s);
 int build_facets(const Tess &t, const int *nCs, std::vector<double> &F, std::vector<int> &nbr);
 
 }  // namespace cpab
