@@ -9,7 +9,8 @@ scheme="ref" (default): the forward is calc_T, the reference scheme
 leaves its cell); the backward (cpab_grad_theta_ref) re-runs it through
 composed steps and propagates dLoss/dT(x) back along the branch the forward
 took, mapping the per-cell dLoss/dT to dLoss/dA through the adjoint Frechet
-derivative of expm (`ck` only sizes its scratch).
+derivative of expm (it keeps no checkpoints: `ck` and the memory budget are
+scheme="simple"'s).
 scheme="simple": the forward is calc_T_simple (nTimeSteps * nStepsODE
 midpoint sub-steps) and the backward (cpab_grad_theta) goes through every
 sub-step.  Either is the exact gradient of the discrete map.  theta is
@@ -39,6 +40,10 @@ def checkpoint_stride(space: CpaSpace, N: int, n: int, nT: int, budget_bytes: in
         if -(-nT // ck) * per_ck <= budget_bytes:
             return ck
     return nT
+
+
+# Per-cell sums of composed steps that the reference scheme's adjoint can use, and their bytes at a time.
+_LEVEL_SUMS, _LEVEL_BYTES = 16, 128 << 20
 
 
 class _Transform(torch.autograd.Function):
@@ -71,10 +76,14 @@ class _Transform(torch.autograd.Function):
         gpts = torch.empty_like(pts) if ctx.need_pts_grad else None
         c = sp._ctx
         if ctx.ref:
-            wsb = int(c.lib.cpab_grad_ref_workspace_bytes(c.h, N, n, ctx.nT, ctx.ck))
+            # the least that is asked for, and room for the sums
+            one = _LEVEL_SUMS * sp.D * 8
+            ck = ctx.nT if ctx.ck >= 1 else ctx.ck  # (refused below)
+            wsb = int(c.lib.cpab_grad_ref_workspace_bytes(c.h, N, n, ctx.nT, ck)) + \
+                one * min(N, max(_LEVEL_BYTES // one, 1))
             ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=pts.device)
             c.check(c.lib.cpab_grad_theta_ref(c.h, _lib.ptr(sp.B), sp.d, _lib.ptr(sA), _lib.ptr(Tr), N, _lib.ptr(pts),
-                                              n, _lib.ptr(g), prec, ctx.dt, ctx.nT, ctx.nODE, ctx.sign, ctx.ck, None,
+                                              n, _lib.ptr(g), prec, ctx.dt, ctx.nT, ctx.nODE, ctx.sign, ck, None,
                                               _lib.ptr(gpts), _lib.ptr(gA), _lib.ptr(dtheta), _lib.ptr(ws),
                                               ws.numel(), _lib.stream_ptr()))
         else:

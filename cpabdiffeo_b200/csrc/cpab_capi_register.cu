@@ -2,6 +2,8 @@
 // kernels (declared in include/cpab_b200.h).
 #include <cmath>
 
+#include <algorithm>
+
 #include "cpab_ctx.h"
 #include "cpab_landmarks.h"
 #include "cpab_reduce.cuh"
@@ -595,12 +597,18 @@ size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_i
 
 }  // extern "C"
 
-// Levels of the adjoint's tables: as calc_T's, sparser where there is room for
-// fewer than `rows` sums beside level 0.
-static JumpCfg grad_jump(const cpab_ctx *ctx, int nTimeSteps, int nStepsODE, size_t most, size_t el, size_t rows)
+// The sums of one instance's levels above 0.
+static size_t grad_level_bytes(const cpab_ctx *ctx, const JumpCfg &j)
+{
+    return (size_t)(j.nT - 1 + j.nS - 1) * ctx->t.nC * cell_len(ctx) * sizeof(double);
+}
+
+// Levels of the adjoint's tables: calc_T's, sparser where the sums of one
+// instance beside level 0 take more than `room` bytes.
+static JumpCfg grad_jump(const cpab_ctx *ctx, int nTimeSteps, int nStepsODE, size_t most, size_t el, size_t room)
 {
     JumpCfg j = jump_cfg(ctx->t.dim, ctx->t.nC, nTimeSteps, nStepsODE, SCHEME_REF, most, el);
-    while (j.r < 31 && (size_t)(j.nT - 1 + j.nS - 1) > rows)
+    while (j.r < 31 && grad_level_bytes(ctx, j) > room)
         j = jump_cfg(ctx->t.dim, ctx->t.nC, nTimeSteps, nStepsODE, SCHEME_REF, most, el, j.r + 1);
     return j;
 }
@@ -635,13 +643,16 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
     // tables in shared memory: A and the sums (midpoint scheme), the composed steps (reference scheme), of which
     // level 0 alone takes as many bytes in FP64
     const size_t el = precision == CPAB_F64 ? 8 : 4;
-    const size_t rows = (size_t)n_per_inst / ((size_t)ctx->t.nC * (ctx->t.dim + 1));
-    const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el, rows);
+    const size_t ck_bytes = cpab_grad_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck);
+    const size_t need = ref ? cpab_grad_ref_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck) : ck_bytes;
+    // Reference scheme: the sums of the levels above 0 take the checkpoints' place.  Which levels there are depends on
+    // what one checkpoint has room for, and on what the caller gives beyond the size asked for, not on ck.
+    const size_t spare = workspace && workspace_bytes > need ? workspace_bytes - need : 0;
+    const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el,
+                                   (size_t)N * n_per_inst * ctx->t.dim * sizeof(double) + spare);
     if ((size_t)2 * ctx->t.nC * cell_len(ctx) * 8 > (size_t)max_smem_optin() ||
         (ref && jump_bytes(jump, ctx->t.dim, ctx->t.nC, el) > (size_t)max_smem_optin()))
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables exceed shared memory");
-    const size_t ck_bytes = cpab_grad_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck);
-    const size_t need = ref ? cpab_grad_ref_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck) : ck_bytes;
     if (n_per_inst > 0 && (!workspace || workspace_bytes < need))
         return fail(ctx, CPAB_NO_MEMORY, "workspace of %zu bytes needed", need);
     cudaStream_t s = (cudaStream_t)stream;
@@ -669,17 +680,30 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         a.h_sub = dt / (double)nStepsODE;
         if (ref) {
             const size_t sum_bytes = align256((size_t)N * DA * sizeof(double));
-            a.gT = reinterpret_cast<double *>(static_cast<char *>(workspace) + ck_bytes);
-            a.gS = reinterpret_cast<double *>(static_cast<char *>(workspace) + ck_bytes + sum_bytes);
+            a.gT = static_cast<double *>(workspace);
+            a.gS = reinterpret_cast<double *>(static_cast<char *>(workspace) + sum_bytes);
+            a.gL = reinterpret_cast<double *>(static_cast<char *>(workspace) + 2 * sum_bytes);
             e = cudaMemsetAsync(a.gT, 0, 2 * sum_bytes, s);
-            // The sums of the levels above 0 take the place of the checkpoints.  As many levels as one
-            // checkpoint has room for, so that the result does not depend on ck.
             a.jump = jump;
-            a.gL = static_cast<double *>(workspace);
-            const size_t extra = (size_t)(a.jump.nT - 1 + a.jump.nS - 1);
-            if (e == cudaSuccess && extra) e = cudaMemsetAsync(a.gL, 0, extra * N * DA * sizeof(double), s);
-            if (e != cudaSuccess) return cuda_status(ctx, e, "gradient sums reset");
-            e = launch_grad_ref(a, precision == CPAB_F64 ? PREC_F64 : PREC_F32, s);
+            // as many instances at a time as there is room for the sums of
+            const size_t one = grad_level_bytes(ctx, jump), pt = (size_t)n_per_inst * ctx->t.dim * el;
+            const size_t fit = one ? (ck_bytes + spare) / one : (size_t)N;
+            const int step = (int)std::min<size_t>(std::max<size_t>(fit, 1), (size_t)N);
+            const int prec = precision == CPAB_F64 ? PREC_F64 : PREC_F32;
+            for (int i = 0; i < N && e == cudaSuccess; i += step) {
+                GradArgs b = a;
+                b.N = std::min(step, N - i);
+                b.A += (size_t)i * DA;
+                b.T += (size_t)i * DA;
+                b.pts = static_cast<const char *>(a.pts) + i * pt;
+                b.grad_out = static_cast<const char *>(a.grad_out) + i * pt;
+                if (a.grad_in) b.grad_in = static_cast<char *>(a.grad_in) + i * pt;
+                b.gA += (size_t)i * DA;
+                b.gT += (size_t)i * DA;
+                b.gS += (size_t)i * DA;
+                if (one) e = cudaMemsetAsync(b.gL, 0, one * b.N, s);
+                if (e == cudaSuccess) e = launch_grad_ref(b, prec, s);
+            }
         } else {
             e = launch_grad_simple(a, s);
         }

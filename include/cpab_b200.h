@@ -399,10 +399,13 @@ int cpab_grad_theta(cpab_ctx *ctx, const double *B, int d, const double *signedA
                     int ck, double *out, double *grad_pts, double *gA, double *dtheta, void *workspace,
                     size_t workspace_bytes, void *stream);
 
-/* Scratch bytes of cpab_grad_theta_ref: room for checkpoints every ck time
- * steps (which hold per-cell sums of composed steps instead; ck does not
- * change the result or the time) plus two per-cell sums [N, nC, ne]
- * (dLoss/dTrels, dLoss/d(sub-step map)). */
+/* Scratch bytes that cpab_grad_theta_ref asks for: room for checkpoints every
+ * ck time steps plus two per-cell sums [N, nC, ne] (dLoss/dTrels,
+ * dLoss/d(sub-step map)).  The checkpoints' place holds per-cell sums of
+ * composed steps; ck does not change the result.  A larger workspace gives them
+ * more room: up to 16 [nC, ne] sums (8 bytes each) per instance are put to use,
+ * which matters where points are few -- with less room it takes shorter
+ * composed steps, or the instances in several launches. */
 size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_inst, int nTimeSteps, int ck);
 
 /* Gradient of a scalar loss of T(x) through the reference scheme (calc_T:
