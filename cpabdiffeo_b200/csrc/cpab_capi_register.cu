@@ -680,9 +680,13 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         a.h_sub = dt / (double)nStepsODE;
         if (ref) {
             const size_t sum_bytes = align256((size_t)N * DA * sizeof(double));
-            a.gT = static_cast<double *>(workspace);
-            a.gS = reinterpret_cast<double *>(static_cast<char *>(workspace) + sum_bytes);
-            a.gL = reinterpret_cast<double *>(static_cast<char *>(workspace) + 2 * sum_bytes);
+            // the sums of level 0 at the far end: the atomic additions of both are limited by the memory they hit, which
+            // is usually faster apart (3D, 320 cells, 8 x 262144 points, twelve placements each: 2.97 to 3.25 ms,
+            // side by side 3.23 to 3.48)
+            char *end = static_cast<char *>(workspace) + workspace_bytes / 256 * 256 - 2 * sum_bytes;
+            a.gL = static_cast<double *>(workspace);
+            a.gT = reinterpret_cast<double *>(end);
+            a.gS = reinterpret_cast<double *>(end + sum_bytes);
             e = cudaMemsetAsync(a.gT, 0, 2 * sum_bytes, s);
             a.jump = jump;
             // as many instances at a time as there is room for the sums of
