@@ -647,7 +647,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
     const size_t need = ref ? cpab_grad_ref_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck) : ck_bytes;
     // Reference scheme: the sums of the levels above 0 take the checkpoints' place.  Which levels there are depends on
     // what one checkpoint has room for, and on what the caller gives beyond the size asked for, not on ck.
-    const size_t spare = workspace && workspace_bytes > need ? workspace_bytes - need : 0;
+    const size_t spare = workspace && workspace_bytes > need ? (workspace_bytes - need) / 256 * 256 : 0;
     const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el,
                                    (size_t)N * n_per_inst * ctx->t.dim * sizeof(double) + spare);
     if ((size_t)2 * ctx->t.nC * cell_len(ctx) * 8 > (size_t)max_smem_optin() ||

@@ -25,7 +25,7 @@ def test_any_workspace(nCs, tess, n):
     w = torch.as_tensor(rng.normal(0, 1, (N * n, dim)), device=DEV)
     c, p, one = sp._ctx, _lib.ptr, 16 * sp.D * 8
     got = []
-    for ck, more in ((nT, 0), (1, 0), (nT, one), (nT, 2 * one + 8), (nT, 3 * one), (nT, N * one), (nT, 100 * one)):
+    for ck, more in ((nT, 0), (1, 0), (nT, one), (nT, 2 * one + 8), (nT, one // 16 + 255), (nT, 3 * one), (nT, N * one), (nT, 100 * one)):
         least = c.lib.cpab_grad_ref_workspace_bytes(c.h, N, n, nT, ck)
         ws = torch.full((least + more + 256,), 255, dtype=torch.uint8, device=DEV)  # NaN everywhere
         gA, gx = torch.empty_like(A), torch.empty_like(x)
