@@ -650,6 +650,11 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
     const size_t spare = workspace && workspace_bytes > need ? (workspace_bytes - need) / 256 * 256 : 0;
     const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el,
                                    (size_t)N * n_per_inst * ctx->t.dim * sizeof(double) + spare);
+    // FP32: with calc_T's own levels the kernel's forward is calc_T, bit for bit (into out, but not over pts, which
+    // long lists are replayed from)
+    const size_t pt_bytes = (size_t)N * n_per_inst * ctx->t.dim * el;
+    const bool same = precision == CPAB_F32 && !overlaps(pts, pt_bytes, out, pt_bytes) &&
+                      jump.r == ctx_jump(ctx, nTimeSteps, nStepsODE, SCHEME_REF, 0).r;
     if ((size_t)2 * ctx->t.nC * cell_len(ctx) * 8 > (size_t)max_smem_optin() ||
         (ref && jump_bytes(jump, ctx->t.dim, ctx->t.nC, el) > (size_t)max_smem_optin()))
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables exceed shared memory");
@@ -667,7 +672,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         a.T = Trels;
         a.pts = pts;
         a.grad_out = grad_out;
-        a.out = static_cast<double *>(out);
+        a.out = out;
         a.grad_in = grad_pts;
         a.gA = gA;
         a.ckpt = static_cast<double *>(workspace);
@@ -689,6 +694,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
             a.gS = reinterpret_cast<double *>(end + sum_bytes);
             e = cudaMemsetAsync(a.gT, 0, 2 * sum_bytes, s);
             a.jump = jump;
+            if (!same) a.out = nullptr;
             // as many instances at a time as there is room for the sums of
             const size_t one = grad_level_bytes(ctx, jump), pt = (size_t)n_per_inst * ctx->t.dim * el;
             const size_t fit = one ? (ck_bytes + spare) / one : (size_t)N;
@@ -701,6 +707,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
                 b.T += (size_t)i * DA;
                 b.pts = static_cast<const char *>(a.pts) + i * pt;
                 b.grad_out = static_cast<const char *>(a.grad_out) + i * pt;
+                if (a.out) b.out = static_cast<char *>(a.out) + i * pt;
                 if (a.grad_in) b.grad_in = static_cast<char *>(a.grad_in) + i * pt;
                 b.gA += (size_t)i * DA;
                 b.gT += (size_t)i * DA;
@@ -713,7 +720,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
         }
         if (e != cudaSuccess) return cuda_status(ctx, e, "grad launch");
     }
-    if (ref && out && n_per_inst > 0) {
+    if (ref && out && !same && n_per_inst > 0) {
         const int st = transform_points(ctx, signedA, Trels, pts, out, N, n_per_inst, precision, dt, nTimeSteps,
                                         nStepsODE, s);
         if (st != CPAB_OK) return st;

@@ -35,8 +35,8 @@
 //     dA_c += dt L(X^T, dT_c),  X = dt [A_c; 0],
 // L the Frechet derivative of expm, read off the top-right block of
 // expm([[X^T, G], [0, X^T]]), and k_substep_map_adjoint.  This is the exact
-// gradient of the discrete map along the branch the forward took (kept /
-// fallback, cells); where a perturbation flips a branch the map itself jumps
+// gradient of the discrete map along the branch calc_T takes (kept / fallback,
+// cells; Path); where a perturbation flips a branch the map itself jumps
 // by the sub-steps' discretisation error.  Nothing is checkpointed: the list
 // holds kMoves moves of a trajectory (most take 5 to 30) in local memory, and
 // a longer one is replayed in blocks from saved states.
@@ -256,13 +256,78 @@ __device__ __forceinline__ void add_grouped(double *G, int key, const Real *v)
     }
 }
 
+// Value and adjoint of one point that a Path left in doubt, by single steps in calc_T's arithmetic; mi, r and save
+// are the caller's lists.  Out of line, for points so rare that its lanes may go alone.
+template <int DIM, int TESS>
+__device__ __noinline__ void exact_point(const GradArgs &a, const double *map, int inst, int64_t gi, int *mi,
+                                         double (*r)[DIM], ExactPath<DIM, TESS> *save)
+{
+    constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
+    const int nC = a.t.nC, tab = nC * NE, s_row = a.jump.nT * nC;
+    const double *A = a.A + (size_t)inst * tab, *T = a.T + (size_t)inst * tab;
+    double *gT = a.gT + (size_t)inst * tab, *gS = a.gS + (size_t)inst * tab;
+    double x[DIM], g[DIM];
+    load_pt<DIM, double>(a.pts, gi, x);
+    load_pt<DIM, double>(a.grad_out, gi, g);
+#pragma unroll
+    for (int i = 0; i < DIM; ++i) g[i] *= a.t.inc[i];
+    ExactPath<DIM, TESS> s;
+    InCell<DIM, TESS> here;
+    int k = 0, block = 0;
+    s.begin(a.t, x, a.nTimeSteps);
+    here.enter(a.t, s.c);
+    while (!s.done()) {
+        if (k == kMoves) {
+            ++block;
+            k = 0;
+            if (block < kSaves) save[block] = s;
+        }
+        k += s.step(a.t, A, T, a.h_sub, a.nStepsODE, s_row, here, mi[k], r[k]) ? 1 : 0;
+    }
+    for (;;) {
+        while (k > 0) {
+            --k;
+            const bool sub = mi[k] >= s_row;
+            double *G = sub ? gS + (size_t)(mi[k] - s_row) * NE : gT + (size_t)mi[k] * NE;
+            const double *M = map + (size_t)mi[k] * NE;
+            double gn[DIM];
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) {
+                gn[c] = g[c];
+#pragma unroll
+                for (int i = 0; i < DIM; ++i) {
+                    atomicAdd(G + i * NH + c, g[i] * r[k][c]);
+                    gn[c] += M[c * DIM + i] * g[i];
+                }
+                atomicAdd(G + c * NH + DIM, g[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < DIM; ++c) g[c] = gn[c];
+        }
+        if (block == 0) break;
+        --block;
+        const int from = min(block, kSaves - 1);
+        if (from == 0) s.begin(a.t, x, a.nTimeSteps);
+        else s = save[from];
+        here.enter(a.t, s.c);
+        for (int skip = block - from; skip >= 0; --skip)
+            for (k = 0; k < kMoves;) k += s.step(a.t, A, T, a.h_sub, a.nStepsODE, s_row, here, mi[k], r[k]) ? 1 : 0;
+    }
+    if (a.grad_in) {
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) g[i] *= a.t.inv_inc[i];
+        store_pt<DIM, double>(a.grad_in, gi, g);
+    }
+}
+
 template <int DIM, int TESS, typename Real>
-__global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
+__global__ void __launch_bounds__(256) k_grad_ref(const __grid_constant__ GradArgs a)
 {
     constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nC = a.t.nC, tab = nC * NE, inst = blockIdx.y, lane = threadIdx.x & 31;
     const JumpCfg jc = a.jump;
+    constexpr bool kF64 = sizeof(Real) == 8;
     const JumpTables<Real> jt = stage_jump<DIM, TESS, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t, jc,
                                                             a.dt, a.h_sub, false, smem_raw);
     __syncthreads();
@@ -307,6 +372,21 @@ __global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
                     if (block < kSaves) save[block] = s;
                 }
                 k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
+                if constexpr (kF64) {
+                    if (s.again) break;
+                }
+            }
+            if (s.done() && a.out) {
+                // (FP32: the end calc_T comes to)
+                s.w.position(a.t, x);
+                store_pt<DIM, Real>(a.out, gi, x);
+            }
+        }
+        if constexpr (kF64) {
+            if (have && s.again) {
+                exact_point<DIM, TESS>(a, jt.map, inst, gi, mi, r, reinterpret_cast<ExactPath<DIM, TESS> *>(save));
+                have = false;
+                k = block = 0;
             }
         }
         const bool later = have && !s.done();
@@ -361,11 +441,15 @@ __global__ void __launch_bounds__(256) k_grad_ref(GradArgs a)
                 // the block before, replayed from the latest saved state at or before its start
                 --block;
                 const int from = min(block, kSaves - 1);
-                if (from == 0) s.begin(a.t, jc, x, a.nTimeSteps);
-                else s = save[from];
-                for (int skip = (block - from) * kMoves; skip > 0;)
-                    skip -= s.unit(a.t, jc, jt, a.nStepsODE, mi[0], r[0]) ? 1 : 0;
-                for (k = 0; k < kMoves;) k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
+                if (from == 0) {
+                    load_pt<DIM, Real>(pts, gi, x);
+                    s.begin(a.t, jc, x, a.nTimeSteps);
+                } else {
+                    s = save[from];
+                }
+                // whole blocks of moves up to this one, the last in the list
+                for (int skip = block - from; skip >= 0; --skip)
+                    for (k = 0; k < kMoves;) k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
             }
         }
         if (gin && have) {

@@ -15,7 +15,7 @@ struct GradArgs {
     const double *T;         // [N, nC, ne] their closed-form steps expm(dt A) (reference scheme)
     const void *pts;         // [N * n, DIM] start points
     const void *grad_out;    // [N * n, DIM] dLoss/dT(x)
-    double *out;             // [N * n, DIM] T(x) or nullptr (midpoint scheme)
+    void *out;               // [N * n, DIM] T(x) or nullptr (FP64 reference scheme: nullptr)
     void *grad_in;           // [N * n, DIM] dLoss/dx or nullptr
     double *gA;              // [N, nC, ne] dLoss/d(signed A), accumulated (zero on entry)
     double *gT;              // [N, nC, ne] dLoss/dT scratch, zero on entry (reference scheme)

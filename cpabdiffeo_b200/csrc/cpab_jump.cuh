@@ -653,6 +653,16 @@ struct WalkTet : WalkLocal<3, 1, Real> {
     {
         return q.m < InnerTet<Real>::kPast && lookup(t, q.x) == c;
     }
+    // the margin of x past the domain, by the clamped coordinates (0: not known)
+    __device__ __forceinline__ Real margin_past(const Tess &t, const Real *x) const
+    {
+        if (t.inc[0] > t.inc[2]) return 0;
+        int kb[3];
+        Facets<3, 1> clamped;
+        cell_box<3, 1>(t, c, kb);
+        clamped.enter(t, c, kb);
+        return clamped.margin(x);
+    }
     __device__ __forceinline__ void take(const Cand &q, bool yes) { B::move(q, yes); }
     __device__ __forceinline__ void leave(const Tess &t, Cand &q)
     {
@@ -677,11 +687,94 @@ struct WalkerOf<3, 1, Real> {
     using type = WalkTet<Real>;
 };
 
-// One point on its way through calc_T (the phases of integrate_jump, for one
-// lane on its own).
+// One point on its way through calc_T, for the adjoint: the moves that calc_T
+// makes, so that the gradient is that of its branch at every step.
+//
+// FP32: the decisions of integrate_jump for one lane on its own (whose first
+// pass makes the same moves where it gets through).
+//
+// FP64: calc_T goes step by step in the reference's arithmetic, this in jumps,
+// so positions differ by rounding: `err` (|.|_1, box units) gains kRound reach a
+// step, `reach` bounding the position in boxes, and grows or shrinks with a
+// move's linear part.  A decision that a margin within 2 err makes (a jump's
+// ends beyond that leave 3/4 of it in between) is in doubt (`again`), and the
+// point is left to ExactPath: some 1e-9 to 1e-6 of the points, by how far and how
+// often they go, and those of grids that move along a facet.
+
+// calc_T in its FP64 arithmetic: at x in cell c (`here`, entered by the caller), `left` closed-form steps to go, or
+// sub-steps of the first of `steps`.
+template <int DIM, int TESS>
+struct ExactPath {
+    double x[DIM];
+    int c, left, steps;
+    bool sub;
+
+    __device__ __forceinline__ void begin(const Tess &t, const double *from, int nT)
+    {
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) x[i] = from[i];
+        c = exact_cell<DIM, TESS>(t, x);
+        left = nT;
+        steps = 0;
+        sub = false;
+    }
+    __device__ __forceinline__ bool done() const { return left == 0; }
+    // One step, as a move from r in the box of its cell by row mi of level 0 (s_row: the first of the sub-steps'); false:
+    // none, but the finding that sub-steps follow.
+    __device__ __forceinline__ bool step(const Tess &t, const double *A, const double *T, double h, int nODE, int s_row,
+                                         InCell<DIM, TESS> &here, int &mi, double *r)
+    {
+        constexpr int NE = DIM * (DIM + 1);
+        double y[DIM];
+        if (sub) {
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) y[i] = x[i];
+            exact_midpoint<DIM>(y, A + (size_t)c * NE, h);
+        } else {
+            exact_affine<DIM>(y, T + (size_t)c * NE, x);
+        }
+        const int in = here.holds(t, y), cy = in > 0 ? c : in < 0 && !sub ? -1 : exact_cell<DIM, TESS>(t, y);
+        if (!sub && cy != c) {
+            steps = left;
+            left = nODE;
+            sub = true;
+            return false;
+        }
+        mi = (sub ? s_row : 0) + c;
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) {
+            r[i] = fma(x[i], t.inv_inc[i], -here.ctr[i]);
+            x[i] = y[i];
+        }
+        if (cy != c) here.enter(t, cy);
+        c = cy;
+        --left;
+        if (sub && left == 0) {
+            sub = false;
+            left = --steps;
+        }
+        return true;
+    }
+};
+
+// What an FP64 Path keeps beside its walker to follow calc_T.
+template <typename Real>
+struct PathExtra {
+};
+template <>
+struct PathExtra<double> {
+    bool again;
+    double err, reach;
+};
+
 template <int DIM, int TESS, typename Real>
-struct Path {
+struct Path : PathExtra<Real> {
     using Walker = typename WalkerOf<DIM, TESS, Real>::type;
+    static constexpr int NE = DIM * (DIM + 1);
+    static constexpr bool kTet = DIM == 3 && TESS == 1, kF64 = sizeof(Real) == 8;
+    // A step's roundings in calc_T's arithmetic, relative to the position: 2 D + 1 of u = 1.1e-16 in a closed-form
+    // step, 1 in a sub-step and h|A| (3 D + 1) in its velocities.  (Those here are relative to the box, and fewer.)
+    static constexpr double kRound = (3 * DIM + 2) * 1.1102230246251565e-16;
     Walker w;
     Real per_m;
     int left, steps, row, kshift, top;
@@ -706,29 +799,70 @@ struct Path {
     }
     __device__ __forceinline__ void begin(const Tess &t, const JumpCfg &jc, const Real *x, int nT)
     {
-        w.place(t, x);
         steps = 0;
+        if constexpr (kF64) {
+            w.place_in(t, x, exact_cell<DIM, TESS>(t, x));
+            Real r[DIM];
+            this->again = false;
+            this->reach = t.nC0 + t.nC1 + t.nC2;
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) {
+                r[i] = w.p.x(i);
+                this->reach += fabs(r[i]);
+            }
+            this->err = kRound * this->reach;
+            w.m = most(w.f.margin(r), Real(0));
+        } else {
+            w.place(t, x);
+        }
         to_steps(jc, t.nC, nT);
     }
     __device__ __forceinline__ bool done() const { return left == 0; }
     // (of a candidate past the domain only that it is outside is known)
-    static __device__ __forceinline__ Real lost(Real m) { return DIM == 3 && TESS == 1 ? most(m, Real(-1)) : m; }
+    static __device__ __forceinline__ Real lost(Real m) { return kTet ? most(m, Real(-1)) : m; }
+    static __device__ __forceinline__ float rate(float a, float b) { return __fdividef(a, b); }
+    static __device__ __forceinline__ double rate(double a, double b) { return a / b; }
     // One unit; true when it moved, by the table row mi from r.
-    __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE,
-                                         int &mi, Real *r)
+    __device__ __forceinline__ bool unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab, int nODE, int &mi,
+                                         Real *r)
     {
-        constexpr int NE = DIM * (DIM + 1);
         const int nC = t.nC, lg = 31 - __clz(max(min(left, whole(w.m * per_m)), 1));
         const int l = min((lg * jc.mul) >> 5, top), n = 1 << (l * jc.r);
         typename Walker::Cand q;
         mi = l * nC + row;
-        const Real need = w.step(t, tab.map + (size_t)mi * NE, q) * (l > 0 ? tab.kap[mi - kshift] : Real(0));
-        bool stays = !(q.m < Real(0));
-        if (!stays && l == 0 && w.keeps(t, q)) {
-            stays = true;
-            q.m = 0;
+        const Real *m = tab.map + (size_t)mi * NE;
+        const Real len = w.step(t, m, q), need = len * (l > 0 ? tab.kap[mi - kshift] : Real(0));
+        bool stays = !(q.m < Real(0)), take = stays && (l == 0 || most(w.m, q.m) >= need);
+        if constexpr (kF64) {
+            if (take || l == 0) {
+                double norm = 0.0, known = l == 0 ? size_of(q.m) : q.m;
+#pragma unroll
+                for (int k = 0; k < DIM; ++k) {
+                    double col = 0.0;
+#pragma unroll
+                    for (int i = 0; i < DIM; ++i) col += fabs(m[k * DIM + i] + (i == k ? 1.0 : 0.0));
+                    norm = fmax(norm, col);
+                }
+                const double reach = this->reach + len;
+                // (within a jump a rounding grows by e^x <= 1 + 2 kappa at most)
+                const double steps_err = n * (kRound * reach) * (l > 0 ? 1.0 + 2.0 * tab.kap[mi - kshift] : 1.0);
+                const double err = fma(this->err, norm, steps_err);
+                if constexpr (kTet) {
+                    if (q.m < InnerTet<Real>::kPast) known = size_of(w.margin_past(t, q.x));
+                }
+                // (3D type I: within the domain's tolerance a margin holds to three times that)
+                if (!(known > 2 * err + (kTet ? 4 * InnerTet<Real>::kOver : 0.0))) this->again = true;
+                if (take || sub) {
+                    this->err = err;
+                    this->reach = reach;
+                }
+            }
         }
-        const bool take = stays && (l == 0 || most(w.m, q.m) >= need);
+        if (!stays && l == 0 && w.keeps(t, q)) {
+            take = true;
+            q.m = 0;
+            per_m = Real(1e30);
+        }
         if (take || (l == 0 && sub)) {
 #pragma unroll
             for (int i = 0; i < DIM; ++i) r[i] = w.p.x(i);
@@ -737,6 +871,13 @@ struct Path {
                 w.take(q, true);
             } else {
                 w.leave(t, q);
+                if constexpr (kF64) {
+                    double known = w.m;
+                    if constexpr (kTet) {
+                        if (w.m == 0) known = w.margin_past(t, w.p.hi);
+                    }
+                    if (!(known > 2 * this->err)) this->again = true;
+                }
                 per_m = Real(1e30);
                 row = jc.nT * nC + w.c;
             }
@@ -744,13 +885,11 @@ struct Path {
             return true;
         }
         // dropped: see integrate_jump
-        per_m = (stays ? Real(0.5) : Real(0.999)) * Real(l == 0 ? nODE : n) /
-                (stays ? most(w.m, Real(1e-12)) : w.m - lost(q.m));
+        per_m = rate((stays ? Real(0.5) : Real(0.999)) * Real(l == 0 && !sub ? nODE : n),
+                     stays ? most(w.m, Real(1e-12)) : w.m - lost(q.m));
         if (l == 0) {
             steps = left;
-            const Real keep = per_m;
             to_substeps(jc, nC, nODE);
-            per_m = keep;
         }
         return false;
     }
@@ -876,8 +1015,8 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                     const int l = level(max(togo, 1), jc.nT - 1, n);
                     Cand q;
                     const float need = v.step(t, tab.map + (l + v.c) * NE, q) * tab.kap[l + v.c - nC];
-                    // (a tetrahedron's margin of 0 may mean past the domain, where no jump starts)
-                    const bool sure = fmaxf(v.m, q.m) >= need && (!kTet || v.m > 0.0f);
+                    // (from a margin of 0 single steps: as below, and a tetrahedron's may mean past the domain)
+                    const bool sure = fmaxf(v.m, q.m) >= need && v.m > 0.0f;
                     go = go && !(q.m < 0.0f) && (l == 0 || sure);
                     v.take(q, go);
                     togo -= go ? n : 0;
@@ -948,6 +1087,7 @@ __device__ __forceinline__ void integrate_jump(const Tess &t, int nT, int nODE, 
                     w.take(q, true);
                     --left;
                     out = false;
+                    per_m = kHuge;
                 }
             }
             if (SCHEME == SCHEME_SIMPLE) {

@@ -421,7 +421,10 @@ size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_i
  * step (closed-form step or fallback, and every sub-step's cell), runs of
  * steps inside a cell composed, and maps the per-cell dLoss/dTrels and
  * dLoss/d(sub-step map) to dLoss/dA, the former through the adjoint Frechet
- * derivative of expm.  Workspace: cpab_grad_ref_workspace_bytes.
+ * derivative of expm.  FP64: that is calc_T's own branch for every point; FP32:
+ * likewise where the workspace holds the sums of all levels of one instance, else
+ * a point within float rounding of a facet may take the other side.
+ * Workspace: cpab_grad_ref_workspace_bytes.
  * nStepsODE <= 256. */
 int cpab_grad_theta_ref(cpab_ctx *ctx, const double *B, int d, const double *signedA, const double *Trels, int N,
                         const void *pts, int64_t n_per_inst, const void *grad_out, int precision, double dt,

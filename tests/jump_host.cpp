@@ -25,9 +25,19 @@ static void walk(const Tess &t, const double *A, const double *T, const double *
         for (int k = 0; k < DIM; ++k) p[k] = (Real)x[i * DIM + k];
         Path<DIM, TESS, Real> s;
         s.begin(t, jc, p, nT);
-        for (int mi; !s.done();) s.unit(t, jc, tab, nODE, mi, r);
+        int mi;
+        while (!s.done()) s.unit(t, jc, tab, nODE, mi, r);
         Real y[DIM];
         s.w.position(t, y);
+        if constexpr (sizeof(Real) == 8) {
+            if (s.again) {
+                ExactPath<DIM, TESS> e;
+                InCell<DIM, TESS> here;
+                e.begin(t, p, nT);
+                for (here.enter(t, e.c); !e.done();) e.step(t, A, T, h, nODE, jc.nT * t.nC, here, mi, r);
+                for (int k = 0; k < DIM; ++k) y[k] = e.x[k];
+            }
+        }
         double q[DIM];
         for (int k = 0; k < DIM; ++k) {
             got[i * DIM + k] = y[k];
@@ -63,4 +73,90 @@ extern "C" int jump_walk(int dim, int tess, const int *nCs, const double *incs, 
     if (f32) go(float());
     else go(double());
     return 1;
+}
+
+// dLoss/dx of n points for dLoss/dT(x) = g: `got` down the list of the adjoint's moves, `want` down the steps of the
+// reference's arithmetic; returns how many points the former took step by step.
+template <int DIM, int TESS>
+static long adjoint(const Tess &t, const double *A, const double *T, const double *x, const double *g, double *got,
+                    double *want, long n, int nT, int nODE, double dt)
+{
+    constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
+    const JumpCfg jc = jump_cfg(DIM, t.nC, nT, nODE, SCHEME_REF, (size_t)227 * 1024, 8);
+    const double h = dt / nODE;
+    std::vector<double> smem(jump_bytes(jc, DIM, t.nC, 8) / 8 + 2);
+    const JumpTables<double> tab =
+        stage_jump<DIM, TESS, double>(A, T, t, jc, dt, h, false, reinterpret_cast<unsigned char *>(smem.data()));
+    long exact = 0;
+    std::vector<int> rows;
+    for (long i = 0; i < n; ++i) {
+        double r[DIM], v[DIM], q[DIM];
+        int mi;
+        Path<DIM, TESS, double> s;
+        rows.clear();
+        for (s.begin(t, jc, x + i * DIM, nT); !s.done() && !s.again;)
+            if (s.unit(t, jc, tab, nODE, mi, r)) rows.push_back(mi);
+        if (s.again) {
+            ExactPath<DIM, TESS> e;
+            rows.clear();
+            InCell<DIM, TESS> here;
+            e.begin(t, x + i * DIM, nT);
+            for (here.enter(t, e.c); !e.done();)
+                if (e.step(t, A, T, h, nODE, jc.nT * t.nC, here, mi, r)) rows.push_back(mi);
+            ++exact;
+        }
+        auto back = [&](const double *M, bool columns, bool plus_one) {
+            double o[DIM];
+            for (int c = 0; c < DIM; ++c) {
+                o[c] = plus_one ? v[c] : 0.0;
+                for (int k = 0; k < DIM; ++k) o[c] += (columns ? M[c * DIM + k] : M[k * NH + c]) * v[k];
+            }
+            for (int c = 0; c < DIM; ++c) v[c] = o[c];
+        };
+        for (int k = 0; k < DIM; ++k) v[k] = g[i * DIM + k] * t.inc[k];
+        for (size_t k = rows.size(); k-- > 0;) back(tab.map + (size_t)rows[k] * NE, true, true);
+        for (int k = 0; k < DIM; ++k) got[i * DIM + k] = v[k] * t.inv_inc[k];
+
+        rows.clear();  // cells; sub-steps as -1 - cell
+        for (int k = 0; k < DIM; ++k) q[k] = x[i * DIM + k];
+        for (int step = 0; step < nT; ++step) {
+            const int c = exact_cell<DIM, TESS>(t, q);
+            double e[DIM];
+            exact_affine<DIM>(e, T + c * NE, q);
+            if (exact_cell<DIM, TESS>(t, e) == c) {
+                for (int k = 0; k < DIM; ++k) q[k] = e[k];
+                rows.push_back(c);
+                continue;
+            }
+            for (int k = 0; k < nODE; ++k) {
+                const int cc = exact_cell<DIM, TESS>(t, q);
+                exact_midpoint<DIM>(q, A + cc * NE, h);
+                rows.push_back(-1 - cc);
+            }
+        }
+        for (int k = 0; k < DIM; ++k) v[k] = g[i * DIM + k];
+        for (size_t k = rows.size(); k-- > 0;) {
+            if (rows[k] >= 0) {
+                back(T + rows[k] * NE, false, false);
+            } else {
+                double D[NE];
+                midpoint_increment<DIM>(A + (-1 - rows[k]) * NE, h, D);
+                back(D, false, true);
+            }
+        }
+        for (int k = 0; k < DIM; ++k) want[i * DIM + k] = v[k];
+    }
+    return exact;
+}
+
+extern "C" long jump_adjoint(int dim, int tess, const int *nCs, const double *incs, const double *A, const double *T,
+                             const double *x, const double *g, double *got, double *want, long n, int nT, int nODE, double dt)
+{
+    Tess t;
+    if (!make_tess(dim, tess, nCs, incs, t)) return -1;
+    if (dim == 1) return adjoint<1, 2>(t, A, T, x, g, got, want, n, nT, nODE, dt);
+    if (dim == 2 && tess == 1) return adjoint<2, 1>(t, A, T, x, g, got, want, n, nT, nODE, dt);
+    if (dim == 2) return adjoint<2, 2>(t, A, T, x, g, got, want, n, nT, nODE, dt);
+    if (tess == 1) return adjoint<3, 1>(t, A, T, x, g, got, want, n, nT, nODE, dt);
+    return adjoint<3, 2>(t, A, T, x, g, got, want, n, nT, nODE, dt);
 }

@@ -139,3 +139,39 @@ def test_arcs_over_a_face_in_either_direction_of_time(lib, dt):
     err = _walk(lib, (2, 1), "II", (1.0, 1.0), x, dt, 64, 10, A=A)
     print(dt, f"max {err.max():.2e} share beyond 1e-9: {(err > 1e-9).mean():.2e}")
     assert err.max() < 1e-9
+
+
+@pytest.mark.parametrize("wild", [0.0, 0.6])
+@pytest.mark.parametrize("nCs,tess,top,closed", [
+    ((7,), "II", (1.0,), True), ((4, 4), "I", (1.0, 1.0), True), ((5, 3), "I", (1.0, 1.0), False),
+    ((3, 7), "II", (1.0, 1.0), True), ((3, 3, 3), "I", (1.0,) * 3, True), ((2, 2, 2), "I", (1.0,) * 3, False),
+    ((2, 3, 5), "II", (1.0,) * 3, True)])
+def test_adjoint_follows_calc_T(lib, nCs, tess, top, closed, wild):
+    """The adjoint's FP64 moves are calc_T's steps: of every point, also on faces, edges, corners and diagonals of boxes
+    (where only the reference's own arithmetic says which cell it is in) and past the domain, dT/dx along its branch.
+    Rounding of up to 5000 steps, grown by the flow: 1e-8 of the largest entry.  Step by step go only those that come
+    within rounding of a facet after the start, or past the domain in 3D type I."""
+    dim, nT, nODE, dt = len(nCs), 50, 100, 0.02
+    rng = np.random.default_rng(60)
+    geo = build_space(dim, nCs, tess, xmaxs=top, zero_v_across_bdry=(closed,) * dim)
+    A = (geo.B @ Prior.create(geo, 0.15, 0.5).sample(1, rng)[0]).reshape(geo.nC, dim, dim + 1)
+    if wild:
+        A = rng.normal(0, wild, A.shape)
+    A, T = (np.ascontiguousarray(a) for a in (A, _expm_affine(dt * A)))
+    inc, n = np.asarray(top) / np.asarray(nCs), 1500
+    on = (rng.integers(0, np.asarray(nCs) + 1, (n, dim)) + rng.choice([0.0, 0.25, 0.5, 0.75], (n, dim))) * inc  # facets
+    free = rng.uniform(-0.3, 1.3, (n, dim)) * top
+    for name, x in (("inside", rng.uniform(0, 1, (n, dim)) * top), ("facets", np.where(on <= top, on, free * 0.7 + 0.15)),
+                    ("around", free)):
+        x = np.ascontiguousarray(x)
+        g = rng.standard_normal((n, dim))
+        got, want = np.empty_like(x), np.empty_like(x)
+        p = lambda a: a.ctypes.data_as(C.c_void_p)
+        lib.jump_adjoint.restype = C.c_long
+        k = lib.jump_adjoint(dim, 1 if tess == "I" else 2, (C.c_int * 3)(*nCs), (C.c_double * 3)(*inc), p(A), p(T), p(x), p(g),
+                             p(got), p(want), C.c_long(n), nT, nODE, C.c_double(dt))
+        err = np.abs(got - want).max(1) / np.abs(want).max()
+        print(nCs, tess, name, f"max {err.max():.1e} beyond 1e-8: {(err > 1e-8).mean():.1e} step by step: {k / n:.1e}")
+        assert err.max() < 1e-8
+        if name == "inside" and not wild and closed:
+            assert k <= 2
