@@ -94,8 +94,8 @@ __host__ __device__ inline size_t table_bytes(const IntegrateArgs &a)
     return (size_t)2 * a.t.nC * a.t.dim * (a.t.dim + 1) * sizeof(double);
 }
 
-// PHASES: FP64 reference scheme by integrate_phases.
-template <int DIM, int TESS, typename Real, int SCHEME, bool PHASES = false>
+// PHASES: FP64 reference scheme by integrate_phases; ONE: FP64 bursts of one (one_at_a_time).
+template <int DIM, int TESS, typename Real, int SCHEME, bool PHASES, bool ONE>
 __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
 {
     constexpr int NE = DIM * (DIM + 1);
@@ -173,10 +173,10 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
             integrate_jump<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, a.jump, jt, ti.start, (int)n, src, snk,
                                               c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim), s_queue, &ex);
         else if constexpr (PHASES)
-            integrate_phases<DIM, TESS>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, (int)n, h, src, snk, c_fast,
+            integrate_phases<DIM, TESS, ONE>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, (int)n, h, src, snk, c_fast,
                                         c_fb, c_sub, c_pts, perm, a.batch.tile_pts, s_phase);
         else
-            integrate_range<DIM, TESS, SCHEME>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, ti.end, h, src,
+            integrate_range<DIM, TESS, SCHEME, ONE>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, ti.start, ti.end, h, src,
                                                      snk, c_fast, c_fb, c_sub, c_pts, perm, ti.start, &s_claim,
                                                      perm ? s_cell : nullptr, &ex);
         __syncthreads();
@@ -204,19 +204,19 @@ __device__ __forceinline__ void integrate_body(const IntegrateArgs &a)
     }
 }
 
-template <int DIM, int TESS, typename Real, int SCHEME>
+template <int DIM, int TESS, typename Real, int SCHEME, bool ONE>
 __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? kJumpCtas<DIM> : 1) k_integrate(IntegrateArgs a)
 {
-    integrate_body<DIM, TESS, Real, SCHEME>(a);
+    integrate_body<DIM, TESS, Real, SCHEME, false, ONE>(a);
 }
 
 // The FP64 reference scheme phase by phase.  4 CTAs of 256 threads per SM (2D,
 // 512 x 512 points there and back and a remap: 2 CTAs 708 us, 3: 642, 4: 632,
 // 5: 650); in 3D their registers would spill, 2.
-template <int DIM, int TESS>
+template <int DIM, int TESS, bool ONE>
 __global__ void __launch_bounds__(256, DIM < 3 ? 4 : 2) k_integrate_phases(IntegrateArgs a)
 {
-    integrate_body<DIM, TESS, double, SCHEME_REF, true>(a);
+    integrate_body<DIM, TESS, double, SCHEME_REF, true, ONE>(a);
 }
 
 // The exact scheme's exit resolution (FP64, rare) would otherwise set the
@@ -225,10 +225,10 @@ __global__ void __launch_bounds__(256, DIM < 3 ? 4 : 2) k_integrate_phases(Integ
 #ifndef CPAB_EXACT_MIN_BLOCKS
 #define CPAB_EXACT_MIN_BLOCKS 3
 #endif
-template <int DIM, int TESS, typename Real>
+template <int DIM, int TESS, typename Real, bool ONE>
 __global__ void __launch_bounds__(256, CPAB_EXACT_MIN_BLOCKS) k_integrate_exact(IntegrateArgs a)
 {
-    integrate_body<DIM, TESS, Real, SCHEME_EXACT>(a);
+    integrate_body<DIM, TESS, Real, SCHEME_EXACT, false, ONE>(a);
 }
 
 // ------------------------------------------------------------ trajectory
@@ -557,7 +557,7 @@ static int grid_for(int64_t n, int block, int per_sm = 8)
     return (int)g;
 }
 
-template <int DIM, int TESS, typename Real, int SCHEME>
+template <int DIM, int TESS, typename Real, int SCHEME, bool ONE = false>
 static cudaError_t launch_integrate_t(IntegrateArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
     Batch &b = a.batch;
@@ -567,13 +567,13 @@ static cudaError_t launch_integrate_t(IntegrateArgs a, const LaunchCfg &cfg, cud
         smem = table_bytes<Real>(a);
         if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
         if (sizeof(Real) == 8 && a.sort) smem += ((size_t)a.t.nC + 2 * (size_t)tile) * sizeof(int);
-        if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real>;
-        else kern = k_integrate<DIM, TESS, Real, SCHEME>;
+        if constexpr (SCHEME == SCHEME_EXACT) kern = k_integrate_exact<DIM, TESS, Real, ONE>;
+        else kern = k_integrate<DIM, TESS, Real, SCHEME, ONE>;
         if constexpr (sizeof(Real) == 8 && SCHEME == SCHEME_REF) {
             // phases where the launch has points enough to fill the SMs and their scratch fits beside the tables
             const size_t with = smem + phase_scratch_bytes(DIM, tile);
             if (a.phases && with + 1024 <= (size_t)max_smem_optin()) {
-                kern = k_integrate_phases<DIM, TESS>;
+                kern = k_integrate_phases<DIM, TESS, ONE>;
                 smem = with;
             }
         }
@@ -609,6 +609,13 @@ template <int DIM, int TESS>
 static cudaError_t launch_integrate_dt(const IntegrateArgs &a, int prec, int scheme, const LaunchCfg &cfg,
                                        cudaStream_t s)
 {
+    if constexpr (DIM == 3 && TESS == 1) {
+        if (prec == PREC_F64 && one_at_a_time(a.t)) {
+            if (scheme == SCHEME_EXACT) return launch_integrate_t<DIM, TESS, double, SCHEME_EXACT, true>(a, cfg, s);
+            if (scheme == SCHEME_REF) return launch_integrate_t<DIM, TESS, double, SCHEME_REF, true>(a, cfg, s);
+            return launch_integrate_t<DIM, TESS, double, SCHEME_SIMPLE, true>(a, cfg, s);
+        }
+    }
     if constexpr (DIM > 1) {
         // the 2D/3D exact scheme (1D has its own kernel, k_exact1d)
         if (scheme == SCHEME_EXACT)

@@ -67,7 +67,7 @@ struct LandmarkSnk {
     }
 };
 
-template <int DIM, int TESS, typename Real>
+template <int DIM, int TESS, typename Real, bool ONE>
 __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
 {
     constexpr int NE = DIM * (DIM + 1);
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
                                                   snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
                                                   s_queue, nullptr);
         else
-            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, end, h,
+            integrate_range<DIM, TESS, SCHEME_REF, ONE>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, end, h,
                                                          src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         double acc = 0.0;
@@ -135,12 +135,12 @@ __global__ void __launch_bounds__(256) k_landmark_ll(LandmarkArgs a)
     }
 }
 
-template <int DIM, int TESS, typename Real>
+template <int DIM, int TESS, typename Real, bool ONE = false>
 cudaError_t launch_t(LandmarkArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
     size_t smem = landmark_smem_bytes(a.t, a.tile_pts, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
     if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
-    auto kern = k_landmark_ll<DIM, TESS, Real>;
+    auto kern = k_landmark_ll<DIM, TESS, Real, ONE>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -155,6 +155,9 @@ cudaError_t launch_t(LandmarkArgs a, const LaunchCfg &cfg, cudaStream_t s)
 template <int DIM, int TESS>
 cudaError_t launch_dt(const LandmarkArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s)
 {
+    if constexpr (DIM == 3 && TESS == 1) {
+        if (prec == PREC_F64 && one_at_a_time(a.t)) return launch_t<DIM, TESS, double, true>(a, cfg, s);
+    }
     return prec == PREC_F64 ? launch_t<DIM, TESS, double>(a, cfg, s) : launch_t<DIM, TESS, float>(a, cfg, s);
 }
 

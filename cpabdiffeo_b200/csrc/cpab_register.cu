@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 4 ? 3 : 1) k_register_ll(
                                                   snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
                                                   s_queue, nullptr);
         else
-            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
+            integrate_range<DIM, TESS, SCHEME_REF, false>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
                                                          src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         const float *img = a.src + base, *ref = a.dst + base;

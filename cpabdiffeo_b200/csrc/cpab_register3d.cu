@@ -170,7 +170,7 @@ struct SlotSnk3 {
     }
 };
 
-template <int TESS, typename Real>
+template <int TESS, typename Real, bool ONE>
 __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
 {
     constexpr int DIM = 3, NE = 12;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
                                                   snk, c_fast, c_fb, c_sub, c_pts, reinterpret_cast<int *>(&s_claim),
                                                   s_queue, nullptr);
         else
-            integrate_range<DIM, TESS, SCHEME_REF>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
+            integrate_range<DIM, TESS, SCHEME_REF, ONE>(a.t, a.nTimeSteps, a.nStepsODE, sA, sT, start, start + n, h,
                                                          src, snk, c_fast, c_fb, c_sub, c_pts, nullptr, 0, &s_claim);
         __syncthreads();
         const float *img = a.src + base, *ref = a.dst + base;
@@ -257,12 +257,12 @@ __global__ void __launch_bounds__(256) k_register3d_ll(Register3dArgs a)
     }
 }
 
-template <int TESS, typename Real>
+template <int TESS, typename Real, bool ONE = false>
 cudaError_t launch_register3d_t(Register3dArgs a, const LaunchCfg &cfg, cudaStream_t s)
 {
     size_t smem = register3d_smem_bytes(a.t.nC, a.tile_px, sizeof(Real) == 8 ? PREC_F64 : PREC_F32, a.jump);
     if (sizeof(Real) == 4) a.jump.queue = add_queue(smem, queue_bytes(cfg.block));
-    auto kern = k_register3d_ll<TESS, Real>;
+    auto kern = k_register3d_ll<TESS, Real, ONE>;
     if (smem > kSmemOptInAbove) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -299,6 +299,7 @@ cudaError_t launch_remap3d_ssd(const Remap3dArgs &a, int map_prec, cudaStream_t 
 
 cudaError_t launch_register3d_ll(const Register3dArgs &a, int prec, const LaunchCfg &cfg, cudaStream_t s)
 {
+    if (prec == PREC_F64 && one_at_a_time(a.t)) return launch_register3d_t<1, double, true>(a, cfg, s);
     if (a.t.tess == 1)
         return prec == PREC_F64 ? launch_register3d_t<1, double>(a, cfg, s) : launch_register3d_t<1, float>(a, cfg, s);
     return prec == PREC_F64 ? launch_register3d_t<2, double>(a, cfg, s) : launch_register3d_t<2, float>(a, cfg, s);

@@ -109,6 +109,24 @@ def test_jumps_equal_single_steps(lib, nCs, tess, top, closed, wild):
     assert err.max() < 1e-9
 
 
+@pytest.mark.parametrize("nCs", [(4, 2, 3), (2, 2, 4), (3, 3, 2), (1, 1, 5), (5, 1, 1)])
+def test_tet_sign_with_any_boxes(lib, nCs):
+    """3D type I with x and z boxes of different sizes, where the reference clamps z inside the domain or beyond its top:
+    a point whose margin is beyond 1e-5 is in the cell or is not, as its sign says (with x boxes the larger ones, below
+    the top).  The FP64 integration decides by it."""
+    rng = np.random.default_rng(53)
+    n, inc = 300000, 1.0 / np.asarray(nCs)
+    x = _points(rng, nCs, (1.0,) * 3, n, 0.8)
+    y = np.ascontiguousarray(x + rng.normal(0, 1, (n, 3)) * inc * 10.0 ** rng.uniform(-6, -0.3, (n, 1)))
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    c, d, m = np.empty(n, np.int32), np.empty(n, np.int32), np.empty(n, np.float32)
+    assert lib.facet_margins(3, 1, (C.c_int * 3)(*nCs), (C.c_double * 3)(*inc), p(x), p(y), p(c), p(d), p(m), C.c_long(n)) == 1
+    known = np.ones(n, bool) if inc[0] <= inc[2] else (x[:, 2] < 1) & (y[:, 2] < 1)
+    np.testing.assert_array_equal(c[known & (m > 1e-5)], d[known & (m > 1e-5)])
+    assert not (c == d)[known & (m < -1e-5)].any()
+    assert (known & (m > 1e-5)).mean() > 0.2 and (known & (m < -1e-5)).mean() > 0.02
+
+
 @pytest.mark.parametrize("nCs", [(1, 1), (1, 3), (2, 1), (4, 4)])
 def test_triangle_margin_is_a_distance(lib, nCs):
     """2D type I: no displacement shorter than the margin (|.|_1, box units) leaves the cell, past a corner of the
