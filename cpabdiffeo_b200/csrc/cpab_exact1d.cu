@@ -734,7 +734,16 @@ __device__ __forceinline__ int find_instance(const int64_t *off, int N, int64_t 
     return lo;
 }
 
-constexpr int kIvUnroll = 4, kIvMinRange = 1024;
+// Instances of fewer points than kIvFew take the walk, whose table is built
+// five times as fast: an instance of 1000 points takes as long either way (4096
+// instances of 100 cells: 256 points 50 and 108 us, 512 84 and 127, 1000 134 and
+// 142).  The number of an instance's own points decides, nothing of the batch,
+// so results do not depend on that.
+// A CTA's range is at least kIvMinRange points (kWalkMinRange where instances
+// are that small on average), which the build of a table is worth; uniform
+// instances of up to kIvPart points per CTA are cut into equal parts, so that
+// no CTA builds two tables.
+constexpr int kIvUnroll = 4, kIvFew = 1024, kIvMinRange = 1024, kWalkMinRange = 128, kIvPart = 4096;
 
 // 4 resident CTAs of 256 threads (64 registers): 0.77 ms on the batch above; 3, 5, 6: 0.86, 0.84, 0.86.
 __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
@@ -765,9 +774,21 @@ __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
     // this CTA's contiguous range of points, whole warps of 32
     const int64_t p0 = a.batch.offsets ? a.batch.offsets[0] : 0;
     const int64_t p1 = a.batch.offsets ? a.batch.offsets[a.batch.N] : (int64_t)a.batch.N * a.batch.n_uniform;
-    int64_t len = (p1 - p0 + gridDim.x - 1) / gridDim.x;
-    len = (max(len, (int64_t)kIvMinRange) + 31) / 32 * 32;
-    const int64_t first = p0 + len * blockIdx.x, last = min(first + len, p1);
+    const int64_t total = p1 - p0, mean = total / max(a.batch.N, 1);
+    int64_t len = (total + gridDim.x - 1) / gridDim.x;
+    len = (max(len, (int64_t)(mean < kIvFew ? kWalkMinRange : kIvMinRange)) + 31) / 32 * 32;
+    int64_t first = p0 + len * blockIdx.x, last = min(first + len, p1);
+    if (!a.batch.offsets && (int64_t)a.batch.N <= gridDim.x) {
+        const int64_t n = a.batch.n_uniform, cuts = gridDim.x / a.batch.N;
+        const int64_t part = max((n + cuts - 1) / cuts, (int64_t)(n < kIvFew ? 64 : kIvMinRange));
+        const int64_t parts = (n + part - 1) / part;
+        if (part <= kIvPart) {
+            const int64_t i = blockIdx.x / parts;
+            if (i >= a.batch.N) return;
+            first = i * n + (blockIdx.x - i * parts) * part;
+            last = min(first + part, (i + 1) * n);
+        }
+    }
     if (first >= last) return;
     if (a.batch.offsets) {
         if (threadIdx.x < 32) {
@@ -798,7 +819,8 @@ __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
         __syncthreads();
         build_transit(e, tr);
         __syncthreads();
-        const bool use = build_intervals(e, tr, it, T_total);
+        const int64_t size = a.batch.offsets ? a.batch.offsets[inst + 1] - a.batch.offsets[inst] : a.batch.n_uniform;
+        const bool use = size >= kIvFew && build_intervals(e, tr, it, T_total);
         // the cancel flag is polled every 16 K points
         constexpr int kChunk = 16384;
         for (; pos < end; pos += kChunk, ++chunk) {
