@@ -167,7 +167,9 @@ __device__ void build_transit(const Exact1D &e, Transit tr)
 // cell is the record of entering that cell (when that record leads on in the
 // same direction; else points near a zero of the velocity take any time and
 // nothing is skipped).  The margin keeps every skipped comparison true for
-// all points of the cell whatever their rounding.
+// all points of the cell: that record enters 1e-12 inside the vertex, and a
+// point on it takes up to 1e-12 / v longer (v at least 1e-8, or it never
+// leaves); times are logarithms over a, each rounded to some 1e-15 / a.
 __device__ void build_skip(const Exact1D &e, const Transit &tr, double t_total)
 {
     for (int i = threadIdx.x; i < 2 * e.nC; i += blockDim.x) {
@@ -176,7 +178,10 @@ __device__ void build_skip(const Exact1D &e, const Transit &tr, double t_total)
         if (0 <= cn && cn < e.nC) {
             s.rec = record_of(cn, c);
             if (tr.cn[i].x == c && tr.cn[i].y == s.rec) {
-                const double t_min = t_total - tr.te[i].x - 1e-9 * (1.0 + fabs(t_total));
+                const double ac = e.A[2 * c], bc = e.A[2 * c + 1], far = vert(e, c + (i & 1));
+                const double v = fmax(1e-8, fmin(fabs(ac * far + bc), fabs(ac * tr.te[i].y + bc)));
+                const double t_min = t_total - tr.te[i].x - 1e-9 * (1.0 + fabs(t_total)) - 2e-12 / v -
+                                     (near0(ac) ? 0.0 : 2e-15 * fabs(e.ia[c]));
                 // one direction has at most nC - 1 crossings
                 while (s.hops < e.nC && s.cum + tr.te[s.rec].x < t_min) {
                     const int next = tr.cn[s.rec].y;
