@@ -179,8 +179,8 @@ __device__ void build_skip(const Exact1D &e, const Transit &tr, double t_total)
             s.rec = record_of(cn, c);
             if (tr.cn[i].x == c && tr.cn[i].y == s.rec) {
                 const double ac = e.A[2 * c], bc = e.A[2 * c + 1], far = vert(e, c + (i & 1));
-                const double v = fmax(1e-8, fmin(fabs(ac * far + bc), fabs(ac * tr.te[i].y + bc)));
-                const double t_min = t_total - tr.te[i].x - 1e-9 * (1.0 + fabs(t_total)) - 2e-12 / v -
+                const float v = fmaxf(1e-8f, (float)fmin(fabs(ac * far + bc), fabs(ac * tr.te[i].y + bc)));
+                const double t_min = t_total - tr.te[i].x - 1e-9 * (1.0 + fabs(t_total)) - (double)__fdividef(2e-12f, v) -
                                      (near0(ac) ? 0.0 : 2e-15 * fabs(e.ia[c]));
                 // one direction has at most nC - 1 crossings
                 while (s.hops < e.nC && s.cum + tr.te[s.rec].x < t_min) {
@@ -267,6 +267,9 @@ __device__ __forceinline__ int sort_key(const Exact1D &e, float x)
 // 96 bytes, so what follows is 16-byte aligned -- and, when cell-sorting,
 // sorted start points and results in input order [tile_pts] (Real), the
 // permutation [tile_pts] (16-bit) and the histogram [nC] (int).
+// Instances of fewer points than this walk without the table, whose making takes longer than it saves (FP64, 4096
+// instances of 128 points 47.9 us with it, 43.9 without, of 256 points 55.8 and 59.4, of 512 75.8 and 97.5).
+constexpr int kSkipFew = 256;
 size_t exact1d_skip_bytes(int nC) { return (size_t)nC * 2 * sizeof(Skip); }
 
 size_t exact1d_smem_bytes(int nC, int tile_pts, int sort, int prec)
@@ -303,10 +306,11 @@ __global__ void __launch_bounds__(256, CPAB_EXACT1D_MIN_BLOCKS) k_exact1d(Integr
     Transit tr;
     tr.te = reinterpret_cast<double2 *>(s_lx + 2 * nC);
     tr.cn = reinterpret_cast<int2 *>(tr.te + 2 * nC);
-    tr.skip = skip ? reinterpret_cast<Skip *>(tr.cn + 2 * nC) : nullptr;
+    Skip *const skips = skip ? reinterpret_cast<Skip *>(tr.cn + 2 * nC) : nullptr;
+    tr.skip = nullptr;
     // cell-sort scratch (see exact1d_smem_bytes)
     const int tp = a.batch.tile_pts;
-    Real *s_xs = reinterpret_cast<Real *>(skip ? (void *)(tr.skip + 2 * nC) : (void *)(tr.cn + 2 * nC));
+    Real *s_xs = reinterpret_cast<Real *>(skip ? (void *)(skips + 2 * nC) : (void *)(tr.cn + 2 * nC));
     Real *s_y = s_xs + tp;
     unsigned short *s_perm = reinterpret_cast<unsigned short *>(s_y + tp);
     // the histogram after the 16-bit permutation, rounded up to a 4-byte boundary
@@ -362,7 +366,9 @@ __global__ void __launch_bounds__(256, CPAB_EXACT1D_MIN_BLOCKS) k_exact1d(Integr
             build_transit(e, tr);
             loaded = ti.inst;
             __syncthreads();
-            if (skip) {
+            const int64_t size = a.batch.offsets ? a.batch.offsets[ti.inst + 1] - a.batch.offsets[ti.inst] : a.batch.n_uniform;
+            tr.skip = size >= kSkipFew ? skips : nullptr;
+            if (tr.skip) {
                 build_skip(e, tr, T_total);
                 __syncthreads();
             }
@@ -748,7 +754,7 @@ __device__ __forceinline__ int find_instance(const int64_t *off, int N, int64_t 
 // are that small on average), which the build of a table is worth; uniform
 // instances of up to kIvPart points per CTA are cut into equal parts, so that
 // no CTA builds two tables.
-constexpr int kIvUnroll = 4, kIvFew = 1024, kIvMinRange = 1024, kWalkMinRange = 128, kIvPart = 4096;
+constexpr int kIvUnroll = 4, kIvFew = 1024, kIvMinRange = 1024, kWalkMinRange = 32, kIvPart = 4096;
 
 // 4 resident CTAs of 256 threads (64 registers): 0.77 ms on the batch above; 3, 5, 6: 0.86, 0.84, 0.86.
 __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
