@@ -15,13 +15,12 @@
 // Layout in HBM: points row-major [nPts, DIM] (the reference's layout);
 // per-instance tables [N, nC, DIM*(DIM+1)] float64; the current instance's
 // tables are staged in shared memory (converted to float in FP32 mode).
-#include <mutex>
-
 #include <algorithm>
 
 #include "cpab_integrate.cuh"
 #include "cpab_jump.cuh"
 #include "cpab_launch.h"
+#include "cpab_occupancy.h"
 
 namespace cpab {
 
@@ -518,31 +517,14 @@ int num_sms()
 
 // Persistent grid: SMs x resident CTAs of this kernel at this block size and
 // shared memory (capped by cfg.ctas_per_sm when that is smaller).
-// Occupancy queries are cached per (kernel, block, shared memory) so that a
-// launch inside stream capture makes no query.
+// A launch that was made before, at that size, makes no query.
 int persistent_grid_impl(const void *kern, const LaunchCfg &cfg, size_t smem)
 {
-    struct Key {
-        const void *k;
-        int block;
-        size_t smem;
-        int per_sm;
-    };
-    static Key cache[64];
-    static int n_cached = 0;
-    static std::mutex mu;
-    int per_sm = 0;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        for (int i = 0; i < n_cached; ++i)
-            if (cache[i].k == kern && cache[i].block == cfg.block && cache[i].smem == smem) per_sm = cache[i].per_sm;
-        if (per_sm == 0) {
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, cfg.block, smem) != cudaSuccess ||
-                per_sm < 1)
-                per_sm = 1;
-            if (n_cached < 64) cache[n_cached++] = Key{kern, cfg.block, smem, per_sm};
-        }
-    }
+    static OccupancyCache cache;
+    int per_sm = cache.get(kern, cfg.block, smem, [&] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, cfg.block, smem) == cudaSuccess && n > 0 ? n : 1;
+    });
     if (cfg.ctas_per_sm > 0 && cfg.ctas_per_sm < per_sm) per_sm = cfg.ctas_per_sm;
     const int g = num_sms() * per_sm;
     return (cfg.max_ctas > 0 && cfg.max_ctas < g) ? cfg.max_ctas : g;
