@@ -246,7 +246,8 @@ int cpab_calc_v(cpab_ctx *ctx, const double *A, const double *pts, double *vel, 
 }
 
 static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *Trels, const void *pts, void *out,
-                           int64_t nPts, int precision, int scheme, double dt, int nTimeSteps, int nStepsODE)
+                           int64_t nPts, int precision, int scheme, double dt, int nTimeSteps, int nStepsODE,
+                           size_t static_smem = kIntegrateStatic)
 {
     if (precision != CPAB_F64 && precision != CPAB_F32)
         return fail(ctx, CPAB_BAD_DTYPE, "precision must be CPAB_F64 or CPAB_F32");
@@ -275,7 +276,7 @@ static int check_integrate(cpab_ctx *ctx, const double *signedA, const double *T
         need = exact1d_smem_bytes(ctx->t.nC, ctx->cfg.tile_pts, ctx->cfg.sort,
                                   precision == CPAB_F64 ? PREC_F64 : PREC_F32);
     } else {
-        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx, precision) + kIntegrateStatic;
+        need = tables_smem(ctx, precision, scheme, nTimeSteps, nStepsODE) + sort_smem(ctx, precision) + static_smem;
     }
     if (need > (size_t)max_smem_optin())
         return fail(ctx, CPAB_UNSUPPORTED, "cell tables and tile scratch (%zu bytes) exceed shared memory", need);
@@ -397,7 +398,7 @@ int cpab_calc_trajectory(cpab_ctx *ctx, const double *signedA, const double *Tre
 {
     if (!ctx) return fail(nullptr, CPAB_BAD_ARG, "ctx is NULL");
     if (!Trels) return fail(ctx, CPAB_BAD_ARG, "Trels is NULL");
-    int st = check_integrate(ctx, signedA, Trels, pts, traj, 0, CPAB_F64, CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE);
+    int st = check_integrate(ctx, signedA, Trels, pts, traj, 0, CPAB_F64, CPAB_SCHEME_REF, dt, nTimeSteps, nStepsODE, 0);
     if (st != CPAB_OK) return st;
     if (nPts < 0) return fail(ctx, CPAB_BAD_SHAPE, "nPts < 0");
     if (nPts == 0) return CPAB_OK;

@@ -80,3 +80,13 @@ def test_fp32_needs_no_room_to_sort(ctx, dim, nCs, scheme):
         lib.cpab_set_launch(h, 0, 0, tile)
         st = lib.cpab_calc_T(h, BASE, BASE, BASE, BASE, 0, F32, scheme, 0.02, 50, 100, None, None)
         assert st == OK, (tile, lib.cpab_last_error_string(h))
+
+
+def test_trajectory(ctx):
+    """Its kernel keeps nothing beside the tables."""
+    lib, make = ctx
+    for dim in (1, 2, 3):
+        n = LIMIT // (2 * dim * (dim + 1) * 8)
+        for cells, want in ((n, OK), (n + 1, UNSUPPORTED)):
+            h = make(dim, 2, [cells] + [1] * (dim - 1))
+            assert lib.cpab_calc_trajectory(h, BASE, BASE, BASE, BASE, 0, 0.02, 50, 100, None) == want, (dim, cells)
