@@ -12,10 +12,14 @@
 // endpoint (sign change / zero velocity), with the reference's 1e-16 and
 // 1e-12 nudges at endpoints and its np.allclose(., 0) tests (|.| <= 1e-8).
 //
-// Hitting times are double in both precisions.  The FP32 mode stores the
-// points in float, takes the first cell's exit time as a difference of
-// logarithms (per-cell exit logarithms staged with the tables) and the
-// final position's exponential in float (cf_crossing_f32, cf_phi_f32).
+// FP64 walks, with double hitting times throughout.  FP32 (float points) takes
+// intervals of the flow map where an instance has the points for it: their ends
+// and anchors come from double hitting times, and a point is one formula in
+// float from its anchor on (k_exact1d_intervals); the error stays that of the
+// walk, 2.2e-8 of the norm.  Other points and instances walk in double; in
+// spaces of too many cells for the intervals' tables FP32 walks with the first
+// exit time as a difference of logarithms and the last exponential in float
+// (cf_crossing_f32, cf_phi_f32).
 #include <math_constants.h>
 
 #include "cpab_device.cuh"
@@ -813,7 +817,7 @@ __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
     int inst = s_inst;
     const float *in = static_cast<const float *>(a.pts_in);
     float *out = static_cast<float *>(a.pts_out);
-    unsigned c_pts = 0, c_fail = 0, c_nan = 0, chunk = 0;
+    unsigned c_pts = 0, c_fail = 0, c_nan = 0;
     unsigned long long c_visits = 0;
     bool stop = false;
     for (int64_t pos = first; pos < last && inst < a.batch.N && !stop; ++inst) {
@@ -834,7 +838,7 @@ __global__ void __launch_bounds__(256, 4) k_exact1d_intervals(IntegrateArgs a)
         const bool use = size >= kIvFew && build_intervals(e, tr, it, T_total);
         // the cancel flag is polled every 16 K points
         constexpr int kChunk = 16384;
-        for (; pos < end; pos += kChunk, ++chunk) {
+        for (; pos < end; pos += kChunk) {
             if (cta_cancelled(a.cancel, a.counters)) {
                 stop = true;
                 break;

@@ -38,17 +38,6 @@ struct PState;
 template <int DIM>
 struct PState<DIM, double> {
     double p[DIM];
-    __device__ __forceinline__ void set(const double *x)
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) p[i] = x[i];
-    }
-    __device__ __forceinline__ void get(double *x) const
-    {
-#pragma unroll
-        for (int i = 0; i < DIM; ++i) x[i] = p[i];
-    }
-    __device__ __forceinline__ const double *lookup() const { return p; }
 };
 
 template <int DIM>

@@ -52,9 +52,8 @@
 // it.
 //
 // Measured on 2D prior fields (64 cells, dt 0.02, 50 steps, 100 sub-steps
-// per leaving step): 11.4 units per point instead of 95; with r = 2 (every
-// fourth power) 13.5.  8.4 M points in 1024 instances: 3.17 ms with one step
-// per unit, 0.73 ms.
+// per leaving step): 8.7 units per point instead of 95.  8.4 M points in 1024
+// instances: 3.17 ms with one step per unit, 0.73 ms.
 // FP32 error against 64 bits of the registration likelihood (256 fields x
 // 256^2 pixels): 5.1e-8 before, 2.8e-8.
 #pragma once
