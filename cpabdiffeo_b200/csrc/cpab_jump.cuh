@@ -22,8 +22,8 @@
 // phi(z) = (e^z - 1)/z, gives |v0|_1 <= |d|_1 / (tau (2 - phi(x))).  So the
 // margin needed is |d|_1 kappa with
 //     kappa = 1/2 x e^x / (2 - phi(x))        (x < 1.2, else no jump),
-// tabulated per cell and level with 2 % to spare for the float arithmetic
-// and for S being the flow only up to O(h^2).
+// tabulated per cell and level with 2 % to spare for the float arithmetic.  (The
+// midpoint sub-steps' flow is that of log(S) / h, for which rho is raised.)
 //
 // The argument takes facets that are planes.  The tetrahedra's are bent where
 // the domain ends (or z is clamped): beyond, the lookup takes the nearest
@@ -227,6 +227,8 @@ __device__ __forceinline__ JumpTables<Real> stage_jump(const double *gA, const d
             for (int r = 0; r < DIM; ++r) s += fabs(a[r * NH + k]) * t.inv_inc[r];
             rho = fmax(rho, s * t.inc[k]);
         }
+        // the midpoint map's flow is that of log(S) / h = L - h^2 L^3 / 6 + ...: at most this much steeper
+        if (sub && !exact_sub) rho *= 1.0 + h * h * rho * rho / 3.0;
         // twice the margin where a facet is bent in the box
         float bent = 1.0f;
         if constexpr (DIM == 3 && TESS == 1) {

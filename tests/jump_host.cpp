@@ -160,3 +160,17 @@ extern "C" long jump_adjoint(int dim, int tess, const int *nCs, const double *in
     if (tess == 1) return adjoint<3, 1>(t, A, T, x, g, got, want, n, nT, nODE, dt);
     return adjoint<3, 2>(t, A, T, x, g, got, want, n, nT, nODE, dt);
 }
+
+// kappa of every level above 0 of the sub-step's map, per cell: the tables' value; returns how many levels (2D type II).
+extern "C" int jump_kappa(const int *nCs, const double *incs, const double *A, const double *T, int nT, int nODE, double dt,
+                          double *kappa)
+{
+    Tess t;
+    if (!make_tess(2, 2, nCs, incs, t)) return -1;
+    const JumpCfg jc = jump_cfg(2, t.nC, nT, nODE, SCHEME_REF, (size_t)227 * 1024, 8);
+    std::vector<double> smem(jump_bytes(jc, 2, t.nC, 8) / 8 + 2);
+    const JumpTables<double> tab =
+        stage_jump<2, 2, double>(A, T, t, jc, dt, dt / nODE, false, reinterpret_cast<unsigned char *>(smem.data()));
+    for (int l = 0; l < (jc.nS - 1) * t.nC; ++l) kappa[l] = tab.kap[(jc.nT - 1) * t.nC + l];
+    return jc.nS - 1;
+}

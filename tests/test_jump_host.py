@@ -193,3 +193,26 @@ def test_adjoint_follows_calc_T(lib, nCs, tess, top, closed, wild):
         assert err.max() < 1e-8
         if name == "inside" and not wild and closed:
             assert k <= 2
+
+
+@pytest.mark.parametrize("size", [0.01, 0.1, 0.3, 0.5])  # of h L, h the sub-step
+def test_kappa_covers_the_flow_of_the_substeps(lib, size):
+    """The margin a jump of sub-steps needs is that of the flow through their ends, whose field is log(S) / h, S the
+    midpoint map: up to 9 % steeper than the cell's own where the sub-steps are coarse."""
+    from scipy.linalg import logm
+    rng = np.random.default_rng(54)
+    nCs, nODE, h = (6, 5), 4, 0.125
+    n, inc = 30, 1.0 / np.asarray(nCs)
+    A = rng.normal(0, 1, (n, 2, 3))
+    A[:, :, :2] *= (size / h / np.abs(A[:, :, :2] * inc[None, None] / inc[None, :, None]).sum(1).max(1))[:, None, None]
+    T, kappa = np.ascontiguousarray(_expm_affine(nODE * h * A)), np.empty((2, n))
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    assert lib.jump_kappa((C.c_int * 2)(*nCs), (C.c_double * 2)(*inc), p(A), p(T), 8, nODE, C.c_double(nODE * h), p(kappa)) == 2
+    for c in range(n):
+        L = A[c, :, :2]
+        S = np.eye(2) + h * L + h * h / 2 * L @ L
+        Lf = logm(S).real / h * inc[None] / inc[:, None]
+        for l in range(2):
+            x = np.abs(Lf).sum(0).max() * h * 2 ** (l + 1)
+            if kappa[l, c] < 1e29 and x < 1.4:
+                assert kappa[l, c] >= 0.5 * x * np.exp(x) / (2 - np.expm1(x) / x)
