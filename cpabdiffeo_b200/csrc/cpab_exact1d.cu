@@ -173,7 +173,8 @@ __device__ void build_transit(const Exact1D &e, Transit tr)
 // nothing is skipped).  The margin keeps every skipped comparison true for
 // all points of the cell: that record enters 1e-12 inside the vertex, and a
 // point on it takes up to 1e-12 / v longer (v at least 1e-8, or it never
-// leaves); times are logarithms over a, each rounded to some 1e-15 / a.
+// leaves: 1e-4); times are logarithms over a, each rounded to some 1e-15 / a (a
+// at least 1e-8: 1e-7).
 __device__ void build_skip(const Exact1D &e, const Transit &tr, double t_total)
 {
     for (int i = threadIdx.x; i < 2 * e.nC; i += blockDim.x) {
@@ -182,10 +183,7 @@ __device__ void build_skip(const Exact1D &e, const Transit &tr, double t_total)
         if (0 <= cn && cn < e.nC) {
             s.rec = record_of(cn, c);
             if (tr.cn[i].x == c && tr.cn[i].y == s.rec) {
-                const double ac = e.A[2 * c], bc = e.A[2 * c + 1], far = vert(e, c + (i & 1));
-                const float v = fmaxf(1e-8f, (float)fmin(fabs(ac * far + bc), fabs(ac * tr.te[i].y + bc)));
-                const double t_min = t_total - tr.te[i].x - 1e-9 * (1.0 + fabs(t_total)) - (double)__fdividef(2e-12f, v) -
-                                     (near0(ac) ? 0.0 : 2e-15 * fabs(e.ia[c]));
+                const double t_min = t_total - tr.te[i].x - (3e-4 + 1e-9 * fabs(t_total));
                 // one direction has at most nC - 1 crossings
                 while (s.hops < e.nC && s.cum + tr.te[s.rec].x < t_min) {
                     const int next = tr.cn[s.rec].y;
