@@ -4,9 +4,9 @@ Workload (the batched 1D configuration): [0,1] split into nC=100 equal
 cells, zero-velocity boundary; 4096 theta from the Gaussian prior (length
 scale 0.1, variance 1); instance i transforms its own n_i = floor(10^U(3,5))
 uniform points (~8.8e7 in total), FP32 points; integration time 1.0.  The
-timed step integrates in closed form across cell boundaries (hitting times
-in FP64, cpab/cpa1d/calcs/ClosedFormInt.py restated on the GPU): one fused
-prologue launch (theta -> A -> expm for all 4096) and one persistent
+timed step integrates in closed form across cell boundaries
+(cpab/cpa1d/calcs/ClosedFormInt.py restated on the GPU: intervals of the flow
+map with ends from FP64 hitting times, evaluated in FP32): one fused prologue launch (theta -> A -> expm for all 4096) and one persistent
 integration launch.  Each run checks the result against the reference's own
 calc_T scheme in FP64 (dt=0.02 x 50 steps, nStepsODE=100) on a sample of
 instances and reports the error (must stay <= 1e-5); the same workload
@@ -66,10 +66,10 @@ def parse():
                     choices=["batched_1d", "batched_2d_nc64", "exact_2d_nc64", "remap_ssd", "mcmc_c3", "serving"],
                     help="batched_1d: the headline (1D nC=100, 4096 theta, ragged); batched_2d_nc64: the reference "
                          "scheme in FP32 on 2D tess I 4x4 (nC=64), 4096 theta x 8192 points, for the "
-                         "integration kernel's FP32 roofline; exact_2d_nc64: the same through the exact scheme "
+                         "integration kernel's use of issue slots; exact_2d_nc64: the same through the exact scheme "
                          "(facet hitting times); remap_ssd: remap + SSD of 256 pairs of 256x256 "
                          "images through FP32 maps, for its HBM roofline; mcmc_c3: 256-chain MCMC registration of "
-                         "256x256 FP32 image pairs, for the fused likelihood kernel's roofline; serving: only the "
+                         "256x256 FP32 image pairs, for the fused likelihood kernel; serving: only the "
                          "serving legs (capacity, 200 req/s, sustained, 2000 req/s), one JSON line")
     return ap.parse_args()
 
@@ -188,53 +188,40 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm), "source": self.source}
 
 
-_PEAKS: dict = {}
 
 
-def measured_peaks(torch) -> dict:
-    """FP32 / FP64 SIMT throughput measured here (cuBLAS SGEMM with TF32 off,
-    DGEMM): the denominators for the integration kernel, which runs on the
-    FP32 / FP64 pipes.  HBM from MEASURED_PEAKS.json."""
-    if _PEAKS:
-        return _PEAKS
-    out = _PEAKS
+def measured_peaks() -> dict:
+    """This card's HBM rate (GB/s), from MEASURED_PEAKS.json."""
     try:
-        out.update(json.loads((ROOT / "MEASURED_PEAKS.json").read_text()))
+        return json.loads((ROOT / "MEASURED_PEAKS.json").read_text())
     except (OSError, ValueError):
-        out["hbm_gbs"] = 6650.0
-    prev = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = False
-    for name, dt, n in (("fp32_simt_tflops", torch.float32, 8192), ("fp64_tflops", torch.float64, 4096)):
-        a = torch.randn(n, n, device="cuda", dtype=dt)
-        b = torch.randn(n, n, device="cuda", dtype=dt)
-        for _ in range(2):
-            a @ b
-        torch.cuda.synchronize()
-        s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        best = 1e30
-        for _ in range(5):
-            s.record()
-            a @ b
-            e.record()
-            e.synchronize()
-            best = min(best, s.elapsed_time(e))
-        out[name] = 2 * n ** 3 / (best * 1e-3) / 1e12
-        del a, b
-    torch.backends.cuda.matmul.allow_tf32 = prev
-    return out
+        return {"hbm_gbs": 6650.0}
 
 
 # DRAM bytes per launch measured with ncu (dram__bytes_read.sum +
 # dram__bytes_write.sum, one captured launch of the timed region):
-#  * k_exact1d_intervals on the 2048-theta case (42.7 M points): 308.7 MB, 7.22 B/point,
+#  * k_exact1d_intervals on the 2048-theta case (42.7 M points): 302.9 MB, 7.09 B/point,
 #    scaled to a launch by the points it processes;
 #  * k_integrate on the 2D 4096 x 8192-point workload: 543.7 MB per launch;
 #  * k_remap_ssd_bulk on 256 pairs of 256^2 images: 273.0 MB per launch.
-TRAFFIC_EXACT1D_BYTES_PER_POINT = 308.66e6 / 42737756
+TRAFFIC_EXACT1D_BYTES_PER_POINT = 302.89e6 / 42737756
 # Pipe utilisation of k_exact1d_intervals from the same capture (ncu, % of each
 # pipe's peak over the elapsed cycles; issue over the active ones).
-PIPES_EXACT1D = {"fp64_pct": 3.6, "fp32_fma_pct": 20.5, "fp32_fma_heavy_pct_elapsed": 20.8, "alu_pct": 26.4,
-                 "issue_active_pct": 63.5, "source": "ncu, one launch of the 2048-theta case"}
+PIPES_EXACT1D = {"fp64_pct": 3.8, "fp32_fma_pct": 20.5, "fp32_fma_heavy_pct_elapsed": 20.8, "alu_pct": 26.4,
+                 "issue_active_pct": 66.0, "source": "ncu, one launch of the 2048-theta case"}
+# Issue slots used (ncu, smsp__issue_active.avg.pct_of_peak_sustained_active, one launch of the timed region each):
+# what bounds the integration kernels, which run far below every pipe's and DRAM's rates.
+ISSUE_PCT = {"ref_2d": 72.1, "exact_2d": 64.4, "register": 60.1}
+
+
+def issue_roofline(kernel: str, pct: float, kern_ms: float, scheme_tflops: float, model: str, **more) -> dict:
+    """The share of issue slots used; beside it, without a fraction, the rate of the scheme's own operations, most of
+    which composed steps and intervals spare."""
+    return {"bound": "issue", "kernel": kernel, "achieved": pct, "peak": 100.0, "unit": "% of issue slots (ncu)",
+            "frac": pct / 100.0, "kernel_ms": kern_ms, "scheme_equivalent_tflops": scheme_tflops,
+            "scheme_equivalent_model": model, **more}
+
+
 TRAFFIC_2D_BYTES_PER_LAUNCH = 543.74e6
 TRAFFIC_REMAP_BYTES_PER_LAUNCH = 272.95e6
 
@@ -578,7 +565,6 @@ def bench_2d(args, torch, dev, exact: bool = False) -> dict:
     sp.calc_T_batched(sp.tables_from_theta(theta, DT, 1), x, out, counters=cnt, scheme=scheme, **p)
     cnt_h = cnt.cpu().numpy()
     flops = flops_ref_2d(cnt_h)
-    peaks = measured_peaks(torch)
     achieved = flops / (kern_ms * 1e-3) / 1e12
     # error against the FP64 oracle of the reference scheme on the first 4 instances
     from oracle import oracle as O
@@ -609,16 +595,10 @@ def bench_2d(args, torch, dev, exact: bool = False) -> dict:
             "gpu_launches": 2 * args.steps, "clocks": clk.summary(), "launch": tuned,
             "work": {"kept_steps": int(cnt_h[0]), "fallback_steps": int(cnt_h[1]), "substeps": int(cnt_h[2]),
                      "points": int(cnt_h[3]), "crossings": int(cnt_h[_lib.CNT_CROSSINGS])},
-            "roofline": {"bound": "fp32", "kernel": f"k_integrate<2, tess I, float, {'exact' if exact else 'ref'}>",
-                         "achieved": achieved,
-                         "peak": peaks["fp32_simt_tflops"], "unit": "TFLOP/s",
-                         "frac": achieved / peaks["fp32_simt_tflops"],
-                         "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off",
-                         "flop_model": f"per step 2*{C_CELL_2D}+{M_2D}, per midpoint sub-step "
-                                       f"{C_CELL_2D}+2*{M_2D}+8 (of the scheme's steps; composed steps take "
-                                       "several of them at once, so more is achieved than executed)",
-                         "kernel_ms": kern_ms, "algorithmic_flop_per_launch": flops,
-                         "traffic": TRAFFIC_2D_BYTES_PER_LAUNCH},
+            "roofline": issue_roofline(f"k_integrate<2, tess I, float, {'exact' if exact else 'ref'}>",
+                                       ISSUE_PCT["exact_2d" if exact else "ref_2d"], kern_ms, achieved,
+                                       f"per step of the scheme 2*{C_CELL_2D}+{M_2D}, per sub-step {C_CELL_2D}+2*{M_2D}+8",
+                                       traffic=TRAFFIC_2D_BYTES_PER_LAUNCH),
             "error_vs_fp64_oracle": {"max_abs": err, "points_checked": 4 * npt, "tolerance": 1e-5,
                                      "oracle": "exact scheme (oracle/cpab_oracle_exact.c)" if exact
                                      else "reference scheme (calc_T restated)",
@@ -659,7 +639,7 @@ def remap_ssd_c3(torch, dev, theta, src, dst, reps: int = 10) -> dict:
     torch.cuda.nvtx.range_pop()
     ms_r = float(np.median(times))
     nbytes = 16 * C * H * W
-    pk = measured_peaks(torch).get("hbm_gbs")
+    pk = measured_peaks().get("hbm_gbs")
     ach = nbytes / (ms_r * 1e-3) / 1e9
     return {"ms": ms_r, "images": C, "side": H, "algorithmic_bytes": nbytes, "achieved_gbs": ach,
             "hbm_peak_gbs": pk, "frac": ach / pk if pk else None,
@@ -716,7 +696,6 @@ def bench_mcmc_c3(args, torch, dev) -> dict:
     kern_ms = ks.elapsed_time(ke) / 5
     cnt_h = cnt.cpu().numpy()
     flops = flops_ref_2d(cnt_h)
-    peaks = measured_peaks(torch)
     achieved = flops / (kern_ms * 1e-3) / 1e12
     return {"metric": METRIC, "value": C * H * H / (ms * 1e-3), "unit": "pixels/s", "n_gpus": 1,
             "steps": steps, "warmup": 10 * max(1, -(-args.warmup // 10)), "ms_per_step": ms,
@@ -728,13 +707,9 @@ def bench_mcmc_c3(args, torch, dev) -> dict:
             "gpu_launches": 4 * steps, "clocks": clk.summary(),
             "work": {"kept_steps": int(cnt_h[0]), "fallback_steps": int(cnt_h[1]), "substeps": int(cnt_h[2]),
                      "pixels": int(cnt_h[3])},
-            "roofline": {"bound": "fp32", "kernel": "k_register_ll<tess I, float>", "achieved": achieved,
-                         "peak": peaks["fp32_simt_tflops"], "unit": "TFLOP/s",
-                         "frac": achieved / peaks["fp32_simt_tflops"],
-                         "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off",
-                         "flop_model": "the integration's algorithmic FLOPs as for the 2D workload (sampling and SSD "
-                                       "not counted)",
-                         "kernel_ms": kern_ms, "algorithmic_flop_per_launch": flops, "traffic": None}}
+            "roofline": issue_roofline("k_register_ll<tess I, float>", ISSUE_PCT["register"], kern_ms, achieved,
+                                       "the integration's operations as for the 2D workload (sampling and SSD not "
+                                       "counted)", traffic=None)}
 
 
 def bench_remap(args, torch, dev) -> dict:
@@ -1013,8 +988,9 @@ def main():
             "data": "synthetic (seeded prior draws, log-uniform ragged sizes, uniform points)",
             "config": {"workload": WORKLOAD, "n_theta_per_gpu": args.theta, "points_per_gpu": n_total,
                        "nC": NC, "integration_time": 1.0,
-                       "scheme": "closed form across cells (ClosedFormInt restated: hitting times in FP64)",
-                       "precision": "f32 points, f64 hitting times and expm",
+                       "scheme": "closed form across cells (ClosedFormInt restated: intervals of the flow map, their ends "
+                                 "from FP64 hitting times)",
+                       "precision": "f32 points and evaluation, f64 interval tables and expm",
                        "step": "CUDA graph replay: theta -> A -> expm prologue, persistent integration",
                        "l2": "inputs larger than L2 (352 MB of points per GPU)",
                        "parallelism": f"independent shards x{world}"},
@@ -1036,29 +1012,14 @@ def main():
                                "launch": tuned_ref},
             "launch": tuned}
     if rank == 0:
-        peaks = measured_peaks(torch)
-        achieved = flops / (kern_ms * 1e-3) / 1e12
-        line["roofline"] = {"bound": "fp64", "kernel": "k_exact1d_intervals", "achieved": achieved,
-                            "peak": peaks["fp64_tflops"], "unit": "TFLOP/s",
-                            "frac": achieved / peaks["fp64_tflops"],
-                            "peak_source": "measured here: cuBLAS DGEMM 4096^3",
-                            "flop_model": f"{EXACT_FLOP_PER_VISIT} per cell visit + {EXACT_FLOP_PER_POINT} per point "
-                                          "(log/exp counted as 20): the point-by-point walk's work, most of which "
-                                          "the kernel's intervals of the flow map spare",
-                            "kernel_ms": kern_ms, "step_ms_events": step_ms,
-                            "traffic": TRAFFIC_EXACT1D_BYTES_PER_POINT * n_total,
-                            "traffic_note": "ncu DRAM bytes of one launch on the 2048-theta case, scaled by points",
-                            "pipes_ncu": PIPES_EXACT1D,
-                            "algorithmic_flop_per_launch": flops,
-                            "hbm_achieved_gbs": 2 * pts_h.nbytes / (kern_ms * 1e-3) / 1e9,
-                            "hbm_peak_gbs": peaks.get("hbm_gbs")}
+        line["roofline"] = issue_roofline(
+            "k_exact1d_intervals", PIPES_EXACT1D["issue_active_pct"], kern_ms, flops / (kern_ms * 1e-3) / 1e12,
+            f"the point-by-point walk: {EXACT_FLOP_PER_VISIT} per cell visit + {EXACT_FLOP_PER_POINT} per point (log/exp "
+            "counted as 20)", step_ms_events=step_ms, traffic=TRAFFIC_EXACT1D_BYTES_PER_POINT * n_total,
+            traffic_note="ncu DRAM bytes of one launch on the 2048-theta case, scaled by points", pipes_ncu=PIPES_EXACT1D,
+            hbm_achieved_gbs=2 * pts_h.nbytes / (kern_ms * 1e-3) / 1e9, hbm_peak_gbs=measured_peaks().get("hbm_gbs"))
         flops_ref = flops_from_counters(cnt_ref.cpu().numpy(), 1)
-        ach_ref = flops_ref / (ms_ref * 1e-3) / 1e12
-        line["ref_scheme_gpu"]["roofline"] = {
-            "bound": "fp32", "kernel": "k_integrate<1, float, ref>", "achieved": ach_ref,
-            "peak": peaks["fp32_simt_tflops"], "unit": "TFLOP/s", "frac": ach_ref / peaks["fp32_simt_tflops"],
-            "peak_source": "measured here: cuBLAS SGEMM 8192^3, TF32 off",
-            "flop_model": "per step 2*5+2, per midpoint sub-step 5+2*2+4 (of the scheme's steps)"}
+        line["ref_scheme_gpu"]["scheme_equivalent_tflops"] = flops_ref / (ms_ref * 1e-3) / 1e12
         # errors: the timed FP32 result and the FP64 run against the FP64 closed form (oracle) on 64
         # instances; both GPU schemes against the reference's calc_T scheme in FP64 on 8
         from oracle import oracle as O
