@@ -645,11 +645,17 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
     const size_t el = precision == CPAB_F64 ? 8 : 4;
     const size_t ck_bytes = cpab_grad_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck);
     const size_t need = ref ? cpab_grad_ref_workspace_bytes(ctx, N, n_per_inst, nTimeSteps, ck) : ck_bytes;
-    // Reference scheme: the sums of the levels above 0 take the checkpoints' place.  Which levels there are depends on
-    // what one checkpoint has room for, and on what the caller gives beyond the size asked for, not on ck.
+    // Reference scheme: the sums of the levels above 0 take the checkpoints' place, and what the caller gives beyond the
+    // size asked for.  Level 0 alone where instances have few points for their cells, whose tables and sums would cost
+    // more than they save (3D, 320 cells, 4000 x 4 points: 5.9 ms with all levels, 3.4 without; 2000 x 30: 4.0 and 4.4;
+    // 2D, 64 cells, 20000 x 4: 1.8 and 5.1; 1D, 20 cells, 60000 x 1: 1.7 and 8.5).  The instances go in at most 12
+    // launches, each some 0.15 ms, else with sparser levels.
     const size_t spare = workspace && workspace_bytes > need ? (workspace_bytes - need) / 256 * 256 : 0;
+    const size_t room = ck_bytes + spare;
     const JumpCfg jump = grad_jump(ctx, nTimeSteps, nStepsODE, (size_t)max_smem_optin() - 1024, el,
-                                   (size_t)N * n_per_inst * ctx->t.dim * sizeof(double) + spare);
+                                   256 * n_per_inst < (int64_t)ctx->t.nC * cell_len(ctx)
+                                       ? 0
+                                       : std::min(room, 12 * (room / (size_t)N)));
     // FP32: with calc_T's own levels the kernel's forward is calc_T, bit for bit (into out, but not over pts, which
     // long lists are replayed from)
     const size_t pt_bytes = (size_t)N * n_per_inst * ctx->t.dim * el;
@@ -697,7 +703,7 @@ static int grad_impl(cpab_ctx *ctx, const double *B, int d, const double *signed
             if (!same) a.out = nullptr;
             // as many instances at a time as there is room for the sums of
             const size_t one = grad_level_bytes(ctx, jump), pt = (size_t)n_per_inst * ctx->t.dim * el;
-            const size_t fit = one ? (ck_bytes + spare) / one : (size_t)N;
+            const size_t fit = one ? room / one : (size_t)N;
             const int step = (int)std::min<size_t>(std::max<size_t>(fit, 1), (size_t)N);
             const int prec = precision == CPAB_F64 ? PREC_F64 : PREC_F32;
             for (int i = 0; i < N && e == cudaSuccess; i += step) {

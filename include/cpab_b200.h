@@ -402,10 +402,10 @@ int cpab_grad_theta(cpab_ctx *ctx, const double *B, int d, const double *signedA
 /* Scratch bytes that cpab_grad_theta_ref asks for: room for checkpoints every
  * ck time steps plus two per-cell sums [N, nC, ne] (dLoss/dTrels,
  * dLoss/d(sub-step map)).  The checkpoints' place holds per-cell sums of
- * composed steps; ck does not change the result.  A larger workspace gives them
- * more room: up to 16 [nC, ne] sums (8 bytes each) per instance are put to use,
- * which matters where points are few -- with less room it takes shorter
- * composed steps, or the instances in several launches. */
+ * composed steps; ck changes the result by rounding only.  A larger workspace
+ * gives them more room: up to 16 [nC, ne] sums (8 bytes each) per instance are
+ * put to use, which matters where points are few -- with less room it takes
+ * shorter composed steps, or the instances in several launches. */
 size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_inst, int nTimeSteps, int ck);
 
 /* Gradient of a scalar loss of T(x) through the reference scheme (calc_T:
@@ -422,8 +422,9 @@ size_t cpab_grad_ref_workspace_bytes(const cpab_ctx *ctx, int N, int64_t n_per_i
  * steps inside a cell composed, and maps the per-cell dLoss/dTrels and
  * dLoss/d(sub-step map) to dLoss/dA, the former through the adjoint Frechet
  * derivative of expm.  FP64: that is calc_T's own branch for every point; FP32:
- * likewise where the workspace holds the sums of all levels of one instance, else
- * a point within float rounding of a facet may take the other side.
+ * likewise with room for the sums of all levels of a twelfth of the instances and
+ * nC ne / 256 points in each, else a point within float rounding of a facet may take
+ * the other side.
  * Workspace: cpab_grad_ref_workspace_bytes.
  * nStepsODE <= 256. */
 int cpab_grad_theta_ref(cpab_ctx *ctx, const double *B, int d, const double *signedA, const double *Trels, int N,
