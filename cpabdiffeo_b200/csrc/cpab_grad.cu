@@ -256,40 +256,59 @@ __device__ __forceinline__ void add_grouped(double *G, int key, const Real *v)
     }
 }
 
-// Value and adjoint of one point that a Path left in doubt, by single steps in calc_T's arithmetic; mi, r and save
-// are the caller's lists.  Out of line, for points so rare that its lanes may go alone.
+// Where the sums of table row `key` of this instance are.
+template <int NE>
+__device__ __forceinline__ double *sums_of(const GradArgs &a, int inst, int key)
+{
+    const int nC = a.t.nC, s_row = a.jump.nT * nC;
+    const bool sub = key >= s_row;
+    const int rel = key - (sub ? s_row : 0);
+    const size_t tab = (size_t)nC * NE;
+    if (rel < nC) return (sub ? a.gS : a.gT) + inst * tab + (size_t)rel * NE;
+    return a.gL + inst * (a.jump.nT - 1 + a.jump.nS - 1) * tab + (size_t)(rel - nC + (sub ? (a.jump.nT - 1) * nC : 0)) * NE;
+}
+
+// Value and adjoint of one point, its doubtful decisions settled in calc_T's arithmetic; mi, r and save are the
+// caller's lists.  Out of line, for points so rare that their lanes may go alone.
 template <int DIM, int TESS>
-__device__ __noinline__ void exact_point(const GradArgs &a, const double *map, int inst, int64_t gi, int *mi,
-                                         double (*r)[DIM], ExactPath<DIM, TESS> *save)
+__device__ __noinline__ void careful_point(const GradArgs &a, JumpTables<double> jt, int inst, int64_t gi, int *mi,
+                                           double (*r)[DIM], Path<DIM, TESS, double> *save)
 {
     constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
-    const int nC = a.t.nC, tab = nC * NE, s_row = a.jump.nT * nC;
-    const double *A = a.A + (size_t)inst * tab, *T = a.T + (size_t)inst * tab;
-    double *gT = a.gT + (size_t)inst * tab, *gS = a.gS + (size_t)inst * tab;
+    const size_t tab = (size_t)a.t.nC * NE;
+    const double *x0 = static_cast<const double *>(a.pts) + gi * DIM;
     double x[DIM], g[DIM];
     load_pt<DIM, double>(a.pts, gi, x);
     load_pt<DIM, double>(a.grad_out, gi, g);
 #pragma unroll
     for (int i = 0; i < DIM; ++i) g[i] *= a.t.inc[i];
-    ExactPath<DIM, TESS> s;
-    InCell<DIM, TESS> here;
+    Path<DIM, TESS, double> s;
+    ExactPath<DIM, TESS> e;
+    e.c = -1;
     int k = 0, block = 0;
-    s.begin(a.t, x, a.nTimeSteps);
-    here.enter(a.t, s.c);
-    while (!s.done()) {
-        if (k == kMoves) {
-            ++block;
-            k = 0;
-            if (block < kSaves) save[block] = s;
-        }
-        k += s.step(a.t, A, T, a.h_sub, a.nStepsODE, s_row, here, mi[k], r[k]) ? 1 : 0;
-    }
+    auto unit = [&] {
+        k += s.settled_unit(a.t, a.jump, jt, a.A + inst * tab, a.T + inst * tab, a.h_sub, a.nTimeSteps, a.nStepsODE, x0, e,
+                            mi[k], r[k]) ? 1 : 0;
+    };
+    int todo = -1;  // blocks to replay, the first time as many as there are
     for (;;) {
+        const int from = todo < 0 ? 0 : min(todo, kSaves - 1);
+        if (from == 0) s.begin(a.t, a.jump, x, a.nTimeSteps);
+        else s = save[from];
+        k = 0;
+        block = from;
+        while (todo < 0 ? !s.done() : block < todo || k < kMoves) {
+            if (k == kMoves) {
+                ++block;
+                k = 0;
+                if (todo < 0 && block < kSaves) save[block] = s;
+            }
+            unit();
+        }
         while (k > 0) {
             --k;
-            const bool sub = mi[k] >= s_row;
-            double *G = sub ? gS + (size_t)(mi[k] - s_row) * NE : gT + (size_t)mi[k] * NE;
-            const double *M = map + (size_t)mi[k] * NE;
+            double *G = sums_of<NE>(a, inst, mi[k]);
+            const double *M = jt.map + (size_t)mi[k] * NE;
             double gn[DIM];
 #pragma unroll
             for (int c = 0; c < DIM; ++c) {
@@ -304,14 +323,8 @@ __device__ __noinline__ void exact_point(const GradArgs &a, const double *map, i
 #pragma unroll
             for (int c = 0; c < DIM; ++c) g[c] = gn[c];
         }
-        if (block == 0) break;
-        --block;
-        const int from = min(block, kSaves - 1);
-        if (from == 0) s.begin(a.t, x, a.nTimeSteps);
-        else s = save[from];
-        here.enter(a.t, s.c);
-        for (int skip = block - from; skip >= 0; --skip)
-            for (k = 0; k < kMoves;) k += s.step(a.t, A, T, a.h_sub, a.nStepsODE, s_row, here, mi[k], r[k]) ? 1 : 0;
+        todo = block - 1;
+        if (todo < 0) break;
     }
     if (a.grad_in) {
 #pragma unroll
@@ -320,14 +333,18 @@ __device__ __noinline__ void exact_point(const GradArgs &a, const double *map, i
     }
 }
 
+// Resident CTAs per SM the registers must allow (0: the compiler's choice, 48 registers in 1D, 101 in 3D): 2D FP32, 16 x
+// 65536 points, 3 CTAs 593 us, 4 633; FP64 as many as without careful_point's registers (1D 64, else 128).
+template <int DIM, typename Real>
+constexpr int kGradCtas = sizeof(Real) == 4 ? (DIM == 2 ? 3 : 0) : DIM == 1 ? 4 : 2;
+
 template <int DIM, int TESS, typename Real>
-__global__ void __launch_bounds__(256) k_grad_ref(const __grid_constant__ GradArgs a)
+__global__ void __launch_bounds__(256, kGradCtas<DIM, Real>) k_grad_ref(const __grid_constant__ GradArgs a)
 {
     constexpr int NE = DIM * (DIM + 1), NH = DIM + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nC = a.t.nC, tab = nC * NE, inst = blockIdx.y, lane = threadIdx.x & 31;
     const JumpCfg jc = a.jump;
-    constexpr bool kF64 = sizeof(Real) == 8;
     const JumpTables<Real> jt = stage_jump<DIM, TESS, Real>(a.A + (size_t)inst * tab, a.T + (size_t)inst * tab, a.t, jc,
                                                             a.dt, a.h_sub, false, smem_raw);
     __syncthreads();
@@ -372,9 +389,7 @@ __global__ void __launch_bounds__(256) k_grad_ref(const __grid_constant__ GradAr
                     if (block < kSaves) save[block] = s;
                 }
                 k += s.unit(a.t, jc, jt, a.nStepsODE, mi[k], r[k]) ? 1 : 0;
-                if constexpr (kF64) {
-                    if (s.again) break;
-                }
+                if (s.doubtful()) break;
             }
             if (s.done() && a.out) {
                 // (FP32: the end calc_T comes to)
@@ -382,9 +397,9 @@ __global__ void __launch_bounds__(256) k_grad_ref(const __grid_constant__ GradAr
                 store_pt<DIM, Real>(a.out, gi, x);
             }
         }
-        if constexpr (kF64) {
-            if (have && s.again) {
-                exact_point<DIM, TESS>(a, jt.map, inst, gi, mi, r, reinterpret_cast<ExactPath<DIM, TESS> *>(save));
+        if constexpr (sizeof(Real) == 8) {
+            if (have && s.doubtful()) {
+                careful_point<DIM, TESS>(a, jt, inst, gi, mi, r, save);
                 have = false;
                 k = block = 0;
             }

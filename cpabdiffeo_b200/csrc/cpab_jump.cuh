@@ -698,9 +698,11 @@ struct WalkerOf<3, 1, Real> {
 // so positions differ by rounding: `err` (|.|_1, box units) gains kRound reach a
 // step, `reach` bounding the position in boxes, and grows or shrinks with a
 // move's linear part.  A decision that a margin within 2 err makes (a jump's
-// ends beyond that leave 3/4 of it in between) is in doubt (`again`), and the
-// point is left to ExactPath: some 1e-9 to 1e-6 of the points, by how far and how
-// often they go, and those of grids that move along a facet.
+// ends beyond that leave 3/4 of it in between) is in doubt, and ExactPath, which
+// goes step by step from the start of the point or from where it was last
+// asked, catches up, makes it, and hands over its position (settled_unit): some 1e-7
+// of the points, and those of grids that move along a facet, on each of their
+// steps.
 
 // calc_T in its FP64 arithmetic: at x in cell c (`here`, entered by the caller), `left` closed-form steps to go, or
 // sub-steps of the first of `steps`.
@@ -756,7 +758,38 @@ struct ExactPath {
         }
         return true;
     }
+    // how far a path has come that has `n` closed-form steps to go, or as many sub-steps of the first of k: < 0: not as
+    // far as this one, 0: as far
+    __device__ __forceinline__ int behind(bool s, int n, int k) const
+    {
+        const int mine = sub ? steps : left, its = s ? k : n;
+        if (mine != its) return mine - its;
+        if (sub != s) return sub ? -1 : 1;
+        return sub ? left - n : 0;
+    }
 };
+
+// Take e to where a path (see `behind`) of the point at x0 stands, from its last place or, where that is ahead, from the
+// start, and, `one` more step on; what step() returned.  Out of line: rare, and its lookups would take the registers of
+// the jumps around it.
+template <int DIM, int TESS>
+__device__ __noinline__ bool catch_up(const Tess &t, const double *A, const double *T, double h, int nT, int nODE, int s_row,
+                                      const double *x0, bool sub, int left, int steps, bool one, ExactPath<DIM, TESS> &e,
+                                      int &mi, double *r)
+{
+    if (e.c < 0 || e.behind(sub, left, steps) < 0) {
+        double x[DIM];
+#pragma unroll
+        for (int i = 0; i < DIM; ++i) x[i] = x0[i];
+        e.begin(t, x, nT);
+    }
+    InCell<DIM, TESS> here;
+    here.enter(t, e.c);
+    int row;
+    double from[DIM];
+    while (!e.done() && e.behind(sub, left, steps) > 0) e.step(t, A, T, h, nODE, s_row, here, row, from);
+    return one && !e.done() && e.step(t, A, T, h, nODE, s_row, here, mi, r);
+}
 
 // What an FP64 Path keeps beside its walker to follow calc_T.
 template <typename Real>
@@ -764,7 +797,7 @@ struct PathExtra {
 };
 template <>
 struct PathExtra<double> {
-    bool again;
+    bool doubt_step, doubt_cell;  // of the last unit: its decision; the cell its sub-step ended in
     double err, reach;
 };
 
@@ -804,7 +837,7 @@ struct Path : PathExtra<Real> {
         if constexpr (kF64) {
             w.place_in(t, x, exact_cell<DIM, TESS>(t, x));
             Real r[DIM];
-            this->again = false;
+            this->doubt_step = this->doubt_cell = false;
             this->reach = t.nC0 + t.nC1 + t.nC2;
 #pragma unroll
             for (int i = 0; i < DIM; ++i) {
@@ -852,7 +885,7 @@ struct Path : PathExtra<Real> {
                     if (q.m < InnerTet<Real>::kPast) known = size_of(w.margin_past(t, q.x));
                 }
                 // (3D type I: within the domain's tolerance a margin holds to three times that)
-                if (!(known > 2 * err + (kTet ? 4 * InnerTet<Real>::kOver : 0.0))) this->again = true;
+                this->doubt_step = !(known > 2 * err + (kTet ? 4 * InnerTet<Real>::kOver : 0.0));
                 if (take || sub) {
                     this->err = err;
                     this->reach = reach;
@@ -877,7 +910,7 @@ struct Path : PathExtra<Real> {
                     if constexpr (kTet) {
                         if (w.m == 0) known = w.margin_past(t, w.p.hi);
                     }
-                    if (!(known > 2 * this->err)) this->again = true;
+                    this->doubt_cell = !(known > 2 * this->err);
                 }
                 per_m = Real(1e30);
                 row = jc.nT * nC + w.c;
@@ -893,6 +926,39 @@ struct Path : PathExtra<Real> {
             to_substeps(jc, nC, nODE);
         }
         return false;
+    }
+    __device__ __forceinline__ bool doubtful() const
+    {
+        if constexpr (kF64) return this->doubt_step || this->doubt_cell;
+        return false;
+    }
+    // A unit (true when it moved), its doubts settled.  A, T: the tables' signed A and Trel, x0 the point's start.
+    __device__ __forceinline__ bool settled_unit(const Tess &t, const JumpCfg &jc, const JumpTables<Real> &tab,
+                                                 const double *A, const double *T, double h, int nT, int nODE,
+                                                 const Real *x0, ExactPath<DIM, TESS> &e, int &mi, Real *r)
+    {
+        const bool sub_before = sub;
+        const int left_before = left, steps_before = steps;
+        bool moved = unit(t, jc, tab, nODE, mi, r);
+        if constexpr (kF64) {
+            if (!doubtful()) return moved;
+            const bool one = this->doubt_step;
+            const bool did = catch_up<DIM, TESS>(t, A, T, h, nT, nODE, jc.nT * t.nC, x0, one ? sub_before : sub,
+                                                 one ? left_before : left, one ? steps_before : steps, one, e, mi, r);
+            if (one) moved = did;
+            this->doubt_step = this->doubt_cell = false;
+            w.place_in(t, e.x, e.c);
+            Real p[DIM];
+#pragma unroll
+            for (int i = 0; i < DIM; ++i) p[i] = w.p.x(i);
+            w.m = most(w.f.margin(p), Real(0));
+            this->err = kRound * this->reach;
+            if (e.sub) to_substeps(jc, t.nC, e.left);
+            else to_steps(jc, t.nC, e.left);
+            steps = e.steps;
+            per_m = Real(1e30);
+        }
+        return moved;
     }
 };
 

@@ -25,19 +25,12 @@ static void walk(const Tess &t, const double *A, const double *T, const double *
         for (int k = 0; k < DIM; ++k) p[k] = (Real)x[i * DIM + k];
         Path<DIM, TESS, Real> s;
         s.begin(t, jc, p, nT);
+        ExactPath<DIM, TESS> e;
+        e.c = -1;
         int mi;
-        while (!s.done()) s.unit(t, jc, tab, nODE, mi, r);
+        while (!s.done()) s.settled_unit(t, jc, tab, A, T, h, nT, nODE, p, e, mi, r);
         Real y[DIM];
         s.w.position(t, y);
-        if constexpr (sizeof(Real) == 8) {
-            if (s.again) {
-                ExactPath<DIM, TESS> e;
-                InCell<DIM, TESS> here;
-                e.begin(t, p, nT);
-                for (here.enter(t, e.c); !e.done();) e.step(t, A, T, h, nODE, jc.nT * t.nC, here, mi, r);
-                for (int k = 0; k < DIM; ++k) y[k] = e.x[k];
-            }
-        }
         double q[DIM];
         for (int k = 0; k < DIM; ++k) {
             got[i * DIM + k] = y[k];
@@ -93,18 +86,12 @@ static long adjoint(const Tess &t, const double *A, const double *T, const doubl
         double r[DIM], v[DIM], q[DIM];
         int mi;
         Path<DIM, TESS, double> s;
+        ExactPath<DIM, TESS> e;
+        e.c = -1;
         rows.clear();
-        for (s.begin(t, jc, x + i * DIM, nT); !s.done() && !s.again;)
-            if (s.unit(t, jc, tab, nODE, mi, r)) rows.push_back(mi);
-        if (s.again) {
-            ExactPath<DIM, TESS> e;
-            rows.clear();
-            InCell<DIM, TESS> here;
-            e.begin(t, x + i * DIM, nT);
-            for (here.enter(t, e.c); !e.done();)
-                if (e.step(t, A, T, h, nODE, jc.nT * t.nC, here, mi, r)) rows.push_back(mi);
-            ++exact;
-        }
+        for (s.begin(t, jc, x + i * DIM, nT); !s.done();)
+            if (s.settled_unit(t, jc, tab, A, T, h, nT, nODE, x + i * DIM, e, mi, r)) rows.push_back(mi);
+        exact += e.c >= 0;
         auto back = [&](const double *M, bool columns, bool plus_one) {
             double o[DIM];
             for (int c = 0; c < DIM; ++c) {

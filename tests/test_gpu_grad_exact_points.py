@@ -1,5 +1,5 @@
 """FP64 gradients through calc_T of points that move along a facet, which the
-adjoint takes step by step in the reference's arithmetic (exact_point), among
+adjoint takes step by step in the reference's arithmetic (careful_point), among
 others that it takes in jumps: dLoss/dA and dLoss/dx against torch's through the
 same steps.  1e-10 of the largest entry: some 30 steps, rounded differently."""
 import ctypes as C
